@@ -40,19 +40,19 @@ __device__ __forceinline__ float exp2f_approx(float x) {
 }
 
 // step_function, layer.cu:81-84.  Three flavours, selected at compile time:
-//   0  the reference's own expression, compiled without fast-math (libdevice expf, IEEE divide):
-//      equal pre-activations give bit-equal activations; about 21 instructions;
+//   0  the reference's own expression, 1 / (1 + expf(-v)) with CUDA's expf and an IEEE division: equal
+//      pre-activations give bit-equal activations;
 //   1  the short form: one multiply, ex2.approx.ftz, one add, rcp.approx.ftz -- four dependent
-//      instructions, written with the flush-to-zero forms explicitly (the non-ftz forms that
-//      __expf / __fdividef compile to without fast-math carry range checks and rescaling around
-//      each special-function instruction); a flushed subnormal only ever turns an activation of
-//      ~1e-38 into 0.  About 1e-6 relative from flavour 0 per evaluation for |v| <= 16 (the
+//      instructions.  The flush-to-zero forms are written out because they measured faster here than
+//      __expf and __fdividef; a flushed subnormal only ever turns an activation of ~1e-38 into 0.
+//      About 1e-6 relative from flavour 0 per evaluation for |v| <= 16 (the
 //      multiplication by log2e is rounded before the exponential).  What the fused kernels of the 28x28 net use when
 //      fast_sigmoid is set: on the network's outputs it is as close to the fp64 oracle as flavour 0
 //      (2.1e-6 over 65,536 images);
-//   2  the same two special-function instructions with the argument reduced in two FMA steps
-//      (n = round(-v*log2e), r = -v - n*ln2 exactly) and one Newton step on the reciprocal: about 12
-//      instructions, a few 1e-7 from flavour 0 per evaluation (selectable for the widened net).
+//   2  the same two approximate instructions with the argument reduced as in Cody and Waite, "Software
+//      Manual for the Elementary Functions" (1980): n = round(x / ln 2), r = x - n * ln 2 with ln 2 cut into
+//      a 16-bit head (n * head is exact for |n| < 256) and its tail; then one Newton step on the reciprocal.
+//      About 12 instructions, a few 1e-7 from flavour 0 per evaluation (selectable for the widened net).
 template <int FLAVOR>
 __device__ __forceinline__ float sigmoidf(float v) {
   if constexpr (FLAVOR == 1) {
@@ -65,8 +65,9 @@ __device__ __forceinline__ float sigmoidf(float v) {
     const float magic = 12582912.0f;                       // 1.5 * 2^23: adding it rounds to integer
     const float t = fmaf(x, 1.4426950408889634f, magic);
     const float n = t - magic;                              // round(x * log2e)
-    float r = fmaf(n, -0.693145751953125f, x);              // x - n*ln2_hi (exact)
-    r = fmaf(n, -1.4286068203094173e-6f, r);                // ... - n*ln2_lo
+    constexpr double ln2 = 0.69314718055994530942, head = 45426.0 / 65536.0;   // head = ln2 in 16 bits
+    float r = fmaf(n, (float)-head, x);                     // x - n * head (exact)
+    r = fmaf(n, (float)(head - ln2), r);                    // ... - n * tail
     const float m = exp2f_approx(r * 1.4426950408889634f);  // 2^(r*log2e), |r| <= 0.35
     const float e = __int_as_float(__float_as_int(m) + (__float_as_int(t) << 23));  // * 2^n
     const float d = 1.0f + e;

@@ -132,8 +132,8 @@ int cnn_net_params_device(cnn_net* net, float** d_params);
 /* Sigmoid of the fused kernels (the per-operator kernels always use the reference's expression):
  *   0 = the reference's own expression 1/(1+expf(-v)) with IEEE division (layer.cu:81-84): equal
  *       pre-activations give bit-equal activations, about 21 instructions per evaluation;
- *   non-zero (default) = the short form, ex2.approx and rcp.approx (the special-function instructions
- *       expf and the division are themselves built on), four instructions, about 1e-6 relative per
+ *   non-zero (default) = the short form, the approximate instructions ex2.approx and rcp.approx,
+ *       four instructions, about 1e-6 relative per
  *       evaluation.  On the network's outputs the two are equally close to an fp64 evaluation: 2.1e-6
  *       over the 65,536 images of benchmark configuration 2, where the fp32 oracle itself is 4.0e-6 away
  *       (tests/test_gpu_forward.py prints both).
