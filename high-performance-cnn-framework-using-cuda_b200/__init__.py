@@ -568,18 +568,18 @@ def persample_phase_clocks():
 
 
 def forward_tc_phase_clocks():
-    """The same for the tensor-core forward kernel: float64 [16 warps][16 stamps] of CTA 0 of the last
-    launch (warp 0 finisher, 1 MMA issue, 2-3 loaders, 4-15 epilogue), or None without the
+    """The same for the tensor-core forward kernel: float64 [20 warps][16 stamps] of CTA 0 of the last
+    launch (warp 0 finisher, 1 MMA issue, 2-7 loaders, 8-19 epilogue), or None without the
     instrumented build."""
     lib = load_library()
     try:
         fn = lib.cnn_debug_phase_clocks_tc
     except AttributeError:
         return None
-    out = (C.c_longlong * 256)()
+    out = (C.c_longlong * 320)()
     fn.restype = C.c_int
     _check(fn(out))
-    return np.array(out[:], dtype=np.float64).reshape(16, 16)
+    return np.array(out[:], dtype=np.float64).reshape(20, 16)
 
 
 def synth_images_device(seed: int, first_index: int, n: int, d_images, d_labels=None, stream=None) -> None:

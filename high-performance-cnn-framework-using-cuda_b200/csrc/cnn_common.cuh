@@ -39,6 +39,39 @@ __device__ __forceinline__ float exp2f_approx(float x) {
   return y;
 }
 
+__device__ __forceinline__ float rcp_approx(float x) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
+// Two floats in one 64-bit register pair and the packed fp32 instructions on them (sm_100): one issue slot for two
+// lanes' worth of arithmetic, each half rounded like the scalar instruction.
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
+  f32x2 v;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
+  return v;
+}
+__device__ __forceinline__ void unpack2(f32x2 v, float& lo, float& hi) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+  f32x2 d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+  f32x2 d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+
 // step_function, layer.cu:81-84.  Three flavours, selected at compile time:
 //   0  the reference's own expression, 1 / (1 + expf(-v)) with CUDA's expf and an IEEE division: equal
 //      pre-activations give bit-equal activations;
@@ -56,10 +89,7 @@ __device__ __forceinline__ float exp2f_approx(float x) {
 template <int FLAVOR>
 __device__ __forceinline__ float sigmoidf(float v) {
   if constexpr (FLAVOR == 1) {
-    const float d = 1.0f + exp2f_approx(v * -1.4426950408889634f);
-    float q;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(q) : "f"(d));
-    return q;
+    return rcp_approx(1.0f + exp2f_approx(v * -1.4426950408889634f));
   } else if constexpr (FLAVOR == 2) {
     const float x = fminf(fmaxf(-v, -87.0f), 87.0f);
     const float magic = 12582912.0f;                       // 1.5 * 2^23: adding it rounds to integer
@@ -71,8 +101,7 @@ __device__ __forceinline__ float sigmoidf(float v) {
     const float m = exp2f_approx(r * 1.4426950408889634f);  // 2^(r*log2e), |r| <= 0.35
     const float e = __int_as_float(__float_as_int(m) + (__float_as_int(t) << 23));  // * 2^n
     const float d = 1.0f + e;
-    float q;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(q) : "f"(d));
+    const float q = rcp_approx(d);
     const float err = fmaf(-d, q, 1.0f);
     return fmaf(q, err, q);
   } else {

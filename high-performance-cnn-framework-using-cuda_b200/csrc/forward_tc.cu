@@ -2,99 +2,113 @@
 // 94 % of the forward MACs) on the 5th-generation tensor cores (tcgen05, accumulators in tensor
 // memory), and everything after it -- bias, sigmoid, shared 4x4 subsample, sigmoid, FC 216->10,
 // sigmoid, argmax -- done by the epilogue warps straight out of tensor memory.  Selected with the
-// option "forward_path" = 1 (three tf32 passes, fp32-level accuracy) or 2 (one tf32 pass and a
-// tanh.approx sigmoid: an explicitly reduced-precision inference mode).
+// option "forward_path" = 1 (three passes, fp32-level accuracy; the default for large batches, fp32 images
+// or uint8 pixels) or 2 (one pass and a tanh.approx sigmoid: an explicitly reduced-precision inference mode).
 //
-// The convolution as a GEMM WITHOUT an im2col copy.  A CTA sees its images as one matrix of stacked
-// image rows, R[r][c] with r = 28 * image + y (28 floats per row, contiguous in HBM as they are).
-// For kernel row i the conv is a product with a banded (Toeplitz) weight matrix,
-//     out[r][x][f] = sum_i sum_c R[r + i][c] * T_i[c][x][f],   T_i[c][x][f] = Wc[f][i][c - x] (0 <= c-x < 5),
-// so the A operand of kernel row i is the SAME tile of image rows, started i rows further down: in
-// the un-swizzled K-major shared-memory layout a row is 16 bytes inside each 16-byte column chunk
-// ([chunk][row][4 floats]), and a matrix descriptor may start at any row.  The band is cut into two
-// blocks of 12 output columns (16 input columns, K = 16 per kernel row), and because the weights are
-// shift-invariant both blocks use the same B operand: 5 x [80 x 16] tf32 values, 25 KB.  One tile of
-// 128 stacked rows (4.57 images) costs 2 blocks x 5 kernel rows x 2 K-steps = 20 MMAs of
-// 128 x 80 x 8 per pass.  Rows y = 24..27 of every image produce junk (they run into the next image)
-// and are discarded: 24 of 28 tensor-memory lanes carry results.
+// The convolution as a GEMM WITHOUT an im2col copy.  For kernel row i the conv is a product of image rows
+// with a banded (Toeplitz) weight matrix,
+//     out[y][x][f] = sum_i sum_c R[y + i][c] * T_i[c][x][f],   T_i[c][x][f] = Wc[f][i][c - x] (0 <= c-x < 5),
+// so the A operand of kernel row i is the SAME tile of image rows, started i rows further down: in the
+// un-swizzled K-major shared-memory layout a row is 16 bytes inside each 16-byte column chunk
+// ([chunk][row][8 fp16]), and a matrix descriptor may start at any row.  M is made of groups of 8 output
+// rows (the layout's core matrices); a group keeps the 12 input rows it needs, so the group stride is
+// 12 rows and an image's 24 output rows are exactly three groups: no output row is computed for nothing.
+// (Stacking whole images, 28 rows each, wasted 4 rows in 28 of everything below: tensor work, sigmoids, epilogue.)
+// The band is cut into two blocks of 12 output columns (16 input columns, K = 16 per kernel row = one MMA),
+// and because the weights are shift-invariant both blocks use the same B operand: 5 x [80 x 16] values.
+// Column chunks are kept at columns 0-7, 8-15, 12-19, 20-27, so that both blocks start on a chunk.
+// One tile of 16 groups (5.33 images) costs 10 MMAs of 128 x 80 x 16 per pass.
 //
-// Accuracy.  Path 1 splits both operands into a tf32-exact high part and the remainder and issues
-// hi*hi + lo*hi + hi*lo (three passes, fp32 accumulation): pre-activations agree with the fp32 SIMT
-// kernel to a few 1e-7, the 1e-5 parity bar holds.  Path 2 feeds the fp32 bit patterns as they are
-// (the tensor core reads 19 of the 32 bits) and evaluates sigmoid(v) = 0.5 + 0.5 * tanh.approx(v / 2):
-// outputs within about 1e-4, argmax equal wherever the top-two margin is clear of that.
+// Accuracy.  Path 1 splits both operands into an fp16 high part and an fp16 remainder and issues hi*hi + lo*hi +
+// hi*lo (fp32 accumulation): 22-23 significant bits of either operand take part, what is left out is lo*lo,
+// about 2^-24 relative.  fp16 instead of tf32 halves the MMAs (K = 16 per instruction at the same operand bytes,
+// and operand bytes are what an MMA of this shape costs) at one more bit of mantissa.  Its range does not cover
+// fp32's, so weights and pixels are scaled by powers of two that follow the largest weight w (undone, exactly, in the
+// epilogue's bias FMA): weights so that w lies between 256 and 512, pixels by more than 25 w, which keeps what a pixel's
+// parts lose (2^-25 of the scaled value, absolute) below 2^-24 in any pre-activation, whatever the pixels.  An image
+// with a scaled pixel of 65,520 or more (a pixel of 1,000 to 2,000 where w = 1: its pre-activations are no longer
+// of order one) is noticed by the loader, and a finisher warp computes it in plain fp32 instead (slow, 0.1 ms
+// per image; no image data is expected there).
+// Path 2 uses the high parts only (11 significant bits, as tf32) and one special-function operation
+// per activation: outputs within about 1e-4, argmax equal wherever the top-two margin is clear of that.
 //
-// Pipeline (one CTA per SM, 16 warps, everything handed over through mbarriers with bounded waits):
-//   warps 2-3   load 136 stacked rows per tile straight into the operand layout with 16-byte
-//               cp.async copies (contiguous on the global side; eight slabs: path 2 keeps six tiles
-//               in flight, path 1 uses them as four (high, low) pairs and splits its own chunks in
-//               place after they land);
-//   warp 1      issues the tile's MMAs into one of three 160-column accumulators and commits to
+// Pipeline (one CTA per SM, 20 warps, everything handed over through mbarriers with bounded waits):
+//   warps 4-7   fetch the tile's rows -- consecutive in HBM -- by one bulk copy per tile, three tiles ahead, convert
+//               them to fp16 high and low parts and store them in the operand layout, 16 bytes per store (uint8
+//               pixels go through a 256-entry table of both parts of pixel / 255.0).  (Loads into registers one
+//               tile ahead left the copy's latency, 2,300 cycles per tile, in the path: cost 4 us of 136);
+//   warp 3      issues the tile's MMAs into one of three 160-column accumulators and commits to
 //               mbarriers (the whole warp runs the loop, an elected lane issues: see wide_tc.cuh);
-//   warps 4-15  three epilogue groups of four warps (one per 32-lane quarter of tensor memory), one
-//               tile each: tcgen05.ld of 8 columns (one window column, two maps) at a time, software
+//   warps 8-19  three epilogue groups of four warps (one per 32-lane quarter of tensor memory), one
+//               tile each: tcgen05.ld of 8 columns (one window row of two maps) at a time, software
 //               pipelined; bias, sigmoid, the window row's four subsample taps; the four rows of a
 //               window are four adjacent lanes (reduce-scatter by shuffles); subsample sigmoid; the
-//               window row's share of the FC into shared memory, counted on the image's mbarrier;
-//   warp 0      finishes images in order, three at a time: adds the six window rows' FC sums, output
+//               activation into the image's slot in shared memory, window rows counted on its mbarrier;
+//   warps 0-2   finish images in order, three at a time in turn: FC 216 -> 10 (lane = every 32nd subsample
+//               output, so the weights are read once for three images), reduce-scatter, output
 //               sigmoid, argmax (lowest index wins ties), 44 bytes per image to HBM.
-// Measured on a B200, 65,536 images: path 2 0.131 ms (5.0e8 images/s; the special-function unit -- one
-// tanh per conv output -- and shared-memory bandwidth bound it), path 1 0.46 ms (three passes' operand
-// traffic plus 3,682 exact sigmoids per image: no faster than the fp32 SIMT kernel's 0.39 ms).
+//
+// Measured on a B200 (tf32 operands over stacked images before, now): 65,536 fp32 images 213 -> 137 us, 30,011 uint8 images
+// 151 us (CUDA-core kernel) -> 65 us, path 2 on 65,536 images 122 -> 98 us.  What bounds it now, per tile of 5.33 images
+// (2,900 cycles): the shared-memory data pipe (30 MMAs fetch 195 KB of operands, the other warps move 75 KB), and next
+// the special-function unit (1,600 cycles) and instruction issue (1,700); path 2: the special-function unit, 73 % busy.
+#include <type_traits>
+
+#include "cluster_exchange.cuh"
 #include "net.cuh"
 #include "wide_tc.cuh"
 #include "phase_clocks.cuh"
 
 namespace cnn {
 
-constexpr int kTfThreads = 512;
-constexpr int kTfSlabsTotal = 8;             // operand slabs in shared memory: path 1 uses them as 4 (high, low)
-                                             // pairs with 2 tiles of look-ahead, path 2 as 8 with 6
+constexpr int kTfThreads = 640;
+constexpr int kTfSlabsTotal = 6;             // operand slabs in shared memory: path 1 uses them as 3 (high, low)
+                                             // pairs, path 2 as 6
+constexpr int kTfRaw = 4;                    // tiles of raw image rows in shared memory
 constexpr int kTfAcc = 3;                    // accumulators in tensor memory
-constexpr int kTfRows = 128;                 // stacked rows per tile = tensor-memory lanes
-constexpr int kTfSlabRows = 136;             // + the 4 rows the last kernel row reaches, padded to 8
-constexpr int kTfChunks = 7;                 // 16-byte chunks of a 28-float image row
-constexpr int kTfItems = kTfChunks * kTfSlabRows;              // 952 16-byte copies per tile
-constexpr unsigned kTfChunkStride = (kTfSlabRows + 1) * 16;    // 2,192 B between column chunks of a slab: one row of
-                                                               // padding, so that the seven chunks of an image row
-                                                               // (written by adjacent lanes) fall into different banks
-constexpr int kTfSlabBytes = 15360;                            // 7 x 2,192 = 15,344, rounded up
+constexpr int kTfGroups = 16;                // groups of 8 output rows per tile (M = 128)
+constexpr int kTfGroupsImg = 3;              // groups per image
+constexpr int kTfGroupRows = 12;             // input rows a group keeps: 8 + 4
+constexpr unsigned kTfGroupStride = kTfGroupRows * 16;                       // 192 B
+constexpr unsigned kTfChunkStride = kTfGroups * kTfGroupStride + 32;         // 3,104 B: the 32 B put the four chunks of a
+                                                                             // row into different banks for the loader
+constexpr int kTfSlabBytes = 4 * kTfChunkStride;                             // 12,416
 constexpr int kTfBN = 80;                    // MMA N of one 12-column block: 72 used, padded to 16n
-constexpr unsigned kTfBChunk = kTfBN * 16;   // 1,280 B between the K chunks of a B block
-constexpr unsigned kTfBRow = 4 * kTfBChunk;  // 5,120 B per kernel row (K = 16)
-constexpr int kTfBBytes = 5 * kTfBRow;       // 25,600
+constexpr unsigned kTfBChunk = kTfBN * 16;   // 1,280 B between the two K chunks of a kernel row
+constexpr unsigned kTfBRow = 2 * kTfBChunk;  // 2,560 B per kernel row (K = 16)
+constexpr int kTfBBytes = 5 * kTfBRow;       // 12,800
 constexpr int kTfDCols = 2 * kTfBN;          // 160 accumulator columns per tile
 constexpr int kTfSlots = 32;                 // images whose FC sums may be in flight (ring)
-constexpr int kTfLoaders = 64;               // threads of warps 2-3
-constexpr int kTfEpiWarp0 = 4;
-constexpr int kTfWfBlock = 124;              // floats per (window row, lane-in-window) block of the FC table:
-                                             // 2 blocks x 5 slots x 12, padded to 31 x 16 B (conflict-free LDS.128)
+constexpr int kTfRange = 128;                // ring of out-of-range marks: more images than can be between loader and finisher
+constexpr int kTfFinishers = 3;
+constexpr int kTfMmaWarp = 3;
+constexpr int kTfLoadWarp0 = 4, kTfLoaders = 128;
+constexpr int kTfUnits = kTfGroups * kTfGroupRows * 4 / kTfLoaders;   // 6 chunk rows (8 pixels) per loader thread and tile
+constexpr int kTfEpiWarp0 = 8;
+constexpr float kTfMaxExp = 31.f;            // (1 + 2^31)^4 is still finite
+constexpr int kTfFcIn = 7;                   // subsample outputs per lane of a finisher warp: 216 = 6.75 x 32
+constexpr int kTfAsStride = 32 * kTfFcIn;    // 224
+
+constexpr int kTfRawPixels = kTfGroups * 8 * kH + 6 * 4 * kH;   // a tile meets six images at most, four halo rows each
 
 struct TfSmem {
-  alignas(128) unsigned char slab[kTfSlabsTotal][kTfSlabBytes];   // path 1: slab s = high part, slab s + 4 = low part
+  alignas(128) float raw[kTfRaw][kTfRawPixels];               // image rows as they lie in HBM (fp32, or uint8 in the first quarter)
+  alignas(128) unsigned char slab[kTfSlabsTotal][kTfSlabBytes];   // path 1: slab s = high part, slab s + 3 = low part
   alignas(128) unsigned char b_hi[kTfBBytes];
   alignas(128) unsigned char b_lo[kTfBBytes];                 // path 1 only
-  alignas(16) float wf[7 * 4 * kTfWfBlock];   // FC weights as the epilogue lanes read them (see fill loop)
-  alignas(16) float part[kTfSlots][6][12];    // FC sums of (image slot, window row)
+  alignas(16) float wf[kTfFcIn][3][32][4];    // FC weights of subsample output 32 j + lane: ten, padded to twelve
+  alignas(16) float as[kTfSlots][kTfAsStride];   // subsample activations of an image: [window row][6 * window column + map]
+  unsigned lut[256];                          // uint8 pixels only: fp16 parts of pixel / 255.0, high part in the low half
   float bc[8], ws[16], bs[4], bf[12];
-  unsigned long long a_full[kTfSlabsTotal], a_free[kTfSlabsTotal], d_full[kTfAcc], d_free[kTfAcc], img_done[kTfSlots];
-  int finished;                               // images this CTA has written out (slot reuse guard)
+  unsigned long long raw_full[kTfRaw], raw_free[kTfRaw];
+  unsigned long long a_full[kTfSlabsTotal], a_free[kTfSlabsTotal], d_full[2 * kTfAcc], d_free[2 * kTfAcc], img_done[kTfSlots];
+  unsigned char out_of_range[kTfRange];
+  int finished[kTfFinishers];                            // image triples that each finisher warp has written out (slot reuse guard)
   unsigned tmem_base;
   long long clock_base;                       // phase clocks only
 };
 
-CNN_PHASE_TABLE(g_phase_clocks_tc, 16)
-#ifdef CNN_PHASE_CLOCKS
-__device__ long long g_tc_cta_times[160][4];   // per CTA: global timer (ns) at entry, after set-up, after the loops, at exit
-__device__ __forceinline__ long long global_ns() {
-  long long t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
-#define TC_CTA_TIME(i) do { if (threadIdx.x == 0 && blockIdx.x < 160) g_tc_cta_times[blockIdx.x][i] = global_ns(); } while (0)
-#else
-#define TC_CTA_TIME(i) do { } while (0)
-#endif
+CNN_PHASE_TABLE(g_phase_clocks_tc, 20)
 
 // Eight consecutive fp32 columns of this warp's 32 tensor-memory lanes; not waited for.
 __device__ __forceinline__ void tmem_ld8_nowait(unsigned taddr, unsigned (&r)[8]) {
@@ -116,14 +130,6 @@ __device__ __forceinline__ float tanh_approx(float x) {
   return y;
 }
 
-// 1 / (1 + 2^t): the sigmoid of a pre-activation that arrives already multiplied by -log2(e).
-__device__ __forceinline__ float sigmoid_of_scaled(float t) {
-  const float d = 1.0f + exp2f_approx(t);
-  float q;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(q) : "f"(d));
-  return q;
-}
-
 // Bounded spin on a counter in shared memory (same limit and status convention as mbar_wait_bounded).
 __device__ __forceinline__ void wait_counter_bounded(const int* counter, int at_least, int* status, bool& gave_up) {
   if (gave_up) return;
@@ -138,83 +144,172 @@ __device__ __forceinline__ void wait_counter_bounded(const int* counter, int at_
   }
 }
 
-// PATH 1: three tf32 passes, sigmoid flavour SIG (0 or 1).  PATH 2: one pass, tanh sigmoid.
-template <int PATH, int SIG>
+// FC sums (without bias) of one image in plain fp32 by one warp, lane k < 10 returns sum k: the way out for images whose
+// pixels do not fit fp16.  Lanes own windows; kept out of line and rolled so that it costs the hot code nothing.
+template <int SIG>
+__device__ __noinline__ float image_fc_plain(const float* __restrict__ image, const float* __restrict__ params, int lane) {
+  float mine = 0.f;
+#pragma unroll 1
+  for (int w0 = 0; w0 < 36; w0 += 32) {
+    const int w = w0 + lane;
+    const bool live = w < 36;
+    const float* base = image + (live ? (4 * (w / 6)) * kH + 4 * (w % 6) : 0);
+#pragma unroll 1
+    for (int f = 0; f < kF; ++f) {
+      float zs = params[kOffBs];
+#pragma unroll 1
+      for (int o = 0; o < 16; ++o) {
+        float acc = params[kOffBc + f];
+#pragma unroll 1
+        for (int t = 0; t < 25; ++t)
+          acc = fmaf(params[kOffWc + f * 25 + t], base[(o / 4 + t / 5) * kH + o % 4 + t % 5], acc);
+        zs = fmaf(params[kOffWs + o], sigmoidf<SIG>(acc), zs);
+      }
+      const float as = live ? sigmoidf<SIG>(zs) : 0.f;
+#pragma unroll 1
+      for (int k = 0; k < kOut; ++k) {
+        float v = live ? params[kOffWf + k * kS + f * 36 + w] * as : 0.f;
+#pragma unroll
+        for (int m = 16; m > 0; m >>= 1) v += __shfl_xor_sync(0xffffffffu, v, m);
+        if (lane == k) mine += v;
+      }
+    }
+  }
+  return mine;
+}
+
+// PATH 1: three passes, sigmoid flavour SIG (0 or 1).  PATH 2: one pass, tanh sigmoid.  U8: `images` points at
+// uint8 pixels and the kernel applies the reference's ingest, float(pixel / 255.0) (mnist.h:145, main.cu:57-65).
+template <int PATH, int SIG, bool U8>
 __global__ void __launch_bounds__(kTfThreads, 1)
-k_forward_tc(const float* __restrict__ images, long n, long imgs_per_cta, const float* __restrict__ params,
+k_forward_tc(const void* __restrict__ images, long n, long imgs_per_cta, const float* __restrict__ params,
              float* __restrict__ out, int* __restrict__ argmax, int* __restrict__ status) {
   extern __shared__ unsigned char smem_raw[];
   TfSmem& sm = *reinterpret_cast<TfSmem*>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~(uintptr_t)127);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   constexpr bool kPrecise = (PATH == 1);
   constexpr int kTfSlabs = kPrecise ? kTfSlabsTotal / 2 : kTfSlabsTotal;   // slabs in flight
-  constexpr int kTfAhead = kTfSlabs - 2;    // tiles a loader thread keeps in flight beyond the one it completes
   // Path 2 computes tanh(v / 2): conv weights and bias are halved.  Path 1 with the short sigmoid form folds
-  // the form's multiplication by -log2(e) into them, so an activation is add, ex2, add, rcp.
-  constexpr bool kScaled = kPrecise && (SIG == 1);
-  constexpr float kPre = kPrecise ? (kScaled ? -1.4426950408889634f : 1.0f) : 0.5f;
+  // the form's multiplication by -log2(e) into them.
+  constexpr bool kShort = kPrecise && (SIG == 1);
+  constexpr float kPre = kPrecise ? (kShort ? -1.4426950408889634f : 1.0f) : 0.5f;
 
-  TC_CTA_TIME(0);
   const long img0 = (long)blockIdx.x * imgs_per_cta;
   const long imgs_here_l = (n - img0) < imgs_per_cta ? (n - img0) : imgs_per_cta;
   const int imgs_here = imgs_here_l > 0 ? (int)imgs_here_l : 0;
-  const int rows_here = imgs_here * kH;
-  const int n_tiles = (rows_here + kTfRows - 1) / kTfRows;
-  const long rows_total = n * kH;
-  const long row0 = img0 * kH;
+  const int n_groups = imgs_here * kTfGroupsImg;
+  const int n_tiles = (n_groups + kTfGroups - 1) / kTfGroups;
 
-  // ---- set-up: B operand (banded weights), FC table, small parameters, barriers, tensor memory -----
-  for (int e = tid; e < 5 * kTfBN * 16; e += kTfThreads) {
-    const int i = e / (kTfBN * 16), rem = e % (kTfBN * 16);
-    const int nn = rem / 16, c = rem % 16;
-    float v = 0.f;
-    if (nn < 72) {   // accumulator column nn = 24 * (window column in the block) + 4 * map + (column in the window)
-      const int qq = nn / 24, f = (nn % 24) / 4, j = nn % 4;
-      const int d = c - (4 * qq + j);
-      if (d >= 0 && d < 5) v = kPre * params[kOffWc + f * 25 + i * 5 + d];
-    }
-    float hi, lo;
-    tc::split_tf32(v, hi, lo);
-    const unsigned off = (unsigned)i * kTfBRow + (unsigned)(c >> 2) * kTfBChunk + (unsigned)nn * 16u + (unsigned)(c & 3) * 4u;
-    *reinterpret_cast<float*>(sm.b_hi + off) = hi;
-    if (kPrecise) *reinterpret_cast<float*>(sm.b_lo + off) = lo;
-  }
-  // FC table: block (window row p, lane-in-window r) holds, for column block xb and slot i, the ten
-  // weights of the subsample output that lane r ends up with after the reduce-scatter: sum number
-  // e = 9 * (r & 1) + 5 * (r >> 1) + i of the block (e = 6 * window column + map); the fifth slot of the
-  // lanes with r >= 2 is empty (zeros), and so is the junk window row p = 6.
-  for (int e = tid; e < 7 * 4 * kTfWfBlock; e += kTfThreads) {
-    const int blk = e / kTfWfBlock, w = e % kTfWfBlock;
-    const int p = blk >> 2, r = blk & 3;
-    float v = 0.f;
-    if (w < 120 && p < 6) {
-      const int xb = w / 60, i = (w % 60) / 12, k = w % 12;
-      const bool empty = (r >= 2) && (i == 4);
-      if (!empty && k < kOut) {
-        const int idx = 18 * xb + 9 * (r & 1) + 5 * (r >> 1) + i;   // 6 * q + f over the whole row
-        const int q = idx / 6, f = idx % 6;
-        v = params[kOffWf + k * kS + f * 36 + p * 6 + q];
-      }
-    }
-    sm.wf[e] = v;
-  }
-  if (tid < kF) sm.bc[tid] = kPre * params[kOffBc + tid];
-  if (tid < 16) sm.ws[tid] = params[kOffWs + tid];
-  if (tid == 0) { sm.bs[0] = params[kOffBs]; sm.finished = 0; }
-  if (tid < 12) sm.bf[tid] = (tid < kOut) ? params[kOffBf + tid] : 0.f;
+  // ---- set-up that touches nothing of the kernel before this one ------------------------------------
+  pdl_launch_dependents();
   if (tid == 0) {
+    for (int s = 0; s < kTfRaw; ++s) {
+      mbar_init(&sm.raw_full[s], 1);
+      mbar_init(&sm.raw_free[s], kTfLoaders / 32);
+    }
     for (int s = 0; s < kTfSlabs; ++s) {
-      mbar_init(&sm.a_full[s], kTfLoaders);
+      mbar_init(&sm.a_full[s], kTfLoaders / 32);
       mbar_init(&sm.a_free[s], 1);
     }
-    for (int s = 0; s < kTfAcc; ++s) {
+    for (int s = 0; s < 2 * kTfAcc; ++s) {      // one pair per column block of an accumulator
       mbar_init(&sm.d_full[s], 1);
       mbar_init(&sm.d_free[s], 4);
     }
     for (int s = 0; s < kTfSlots; ++s) mbar_init(&sm.img_done[s], 6);
     mbar_fence_init();
+    for (int w = 0; w < kTfFinishers; ++w) sm.finished[w] = 0;
   }
-  if (warp == 1) tc::tmem_alloc(&sm.tmem_base, 512);
+  if (tid < kTfRange) sm.out_of_range[tid] = 0;
+  if (tid < 8 * kTfSlots) sm.as[tid >> 3][216 + (tid & 7)] = 0.f;     // the padding meets zero weights and has to be finite
+  if (warp == kTfMmaWarp) tc::tmem_alloc(&sm.tmem_base, 512);
+  pdl_wait();
+
+  // ---- loaders: the first copies leave now ------------------------------------------------------------------
+  const int lt = tid - 32 * kTfLoadWarp0;
+  const bool loader = lt >= 0 && lt < kTfLoaders;
+  // group g of this CTA starts 224 g + 112 (g / 3) pixels into its images: 8 rows further per group, 12 more per image
+  auto group_pixel = [](int g) { return 8 * kH * g + 4 * kH * (g / kTfGroupsImg); };
+  auto fetch = [&](int k) {       // one thread: the rows of tile k, from its first group's first to its last group's twelfth
+    constexpr unsigned kBytes = U8 ? 1u : 4u;
+    const int g0 = k * kTfGroups, g1 = min(g0 + kTfGroups, n_groups) - 1;
+    const int first = group_pixel(g0);
+    const unsigned bytes = (unsigned)(group_pixel(g1) + kTfGroupRows * kH - first) * kBytes;
+    unsigned long long* bar = &sm.raw_full[k % kTfRaw];
+    mbar_expect_tx(bar, bytes);
+    bulk_g2s(sm.raw[k % kTfRaw], static_cast<const unsigned char*>(images) + (size_t)(img0 * kImg + first) * kBytes, bytes, bar);
+  };
+
+  if (tid == 0)        // the thread that initialised the barriers
+    for (int k = 0; k < kTfRaw - 1 && k < n_tiles; ++k) fetch(k);
+
+  // ---- set-up: weight scale, B operand (banded weights), FC table, small parameters -------------------------
+  float wmax = 0.f;
+  bool finite = true;
+#pragma unroll
+  for (int j = 0; j < 5; ++j) {
+    const int e = lane + 32 * j;      // the 150 weights and 6 biases
+    if (e < kOffBc + kF) {
+      const float a = fabsf(params[e]);
+      finite = finite && (a <= 3.402823466e38f);
+      if (e < kOffBc) wmax = fmaxf(wmax, a);
+    }
+  }
+#pragma unroll
+  for (int m = 16; m > 0; m >>= 1) wmax = fmaxf(wmax, __shfl_xor_sync(0xffffffffu, wmax, m));
+  const bool plain = !__all_sync(0xffffffffu, finite);    // parameters that fp16 cannot stand in for: every image in plain fp32
+  // With 2^E <= max |kPre * w| < 2^(E+1) weights are scaled by 2^(8-E) and pixels by 2^(E+5): the accumulator carries 2^13.
+  int wexp = (int)((__float_as_uint(fabsf(kPre) * wmax) >> 23) & 255u) - 127;
+  wexp = wexp > 90 ? 90 : (wexp < -90 ? -90 : wexp);
+  const float w_scale = __int_as_float((127 + 8 - wexp) << 23), px_scale = __int_as_float((127 + 5 + wexp) << 23);
+  constexpr float w_unscale = 1.0f / 8192.0f;
+  if (U8 && tid < 256) {
+    const float v = (float)((double)tid / 255.0) * px_scale;
+    const __half hi = __float2half_rn(v);
+    const __half lo = __float2half_rn(v - __half2float(hi));
+    sm.lut[tid] = (unsigned)__half_as_ushort(hi) | ((unsigned)__half_as_ushort(lo) << 16);
+  }
+
+  for (int e = tid; e < 5 * 2 * kTfBN; e += kTfThreads) {     // one 16-byte row of a chunk: 8 columns of one accumulator column
+    const int i = e / (2 * kTfBN), rem = e % (2 * kTfBN);
+    const int ch = rem / kTfBN, nn = rem % kTfBN;
+    // accumulator column nn = 24 * (window column in the block) + 8 * (map / 2) + 2 * (column in the window) + map % 2
+    const int qq = nn / 24, r = nn % 24, f = 2 * (r / 8) + (r & 1), x = 4 * qq + ((r & 7) >> 1);
+    float w[5];
+#pragma unroll
+    for (int d = 0; d < 5; ++d) w[d] = (nn < 72) ? kPre * params[kOffWc + f * 25 + i * 5 + d] : 0.f;
+    __half2 hi[4], lo[4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      float t[2];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int d = 8 * ch + 2 * c + h - x;
+        t[h] = 0.f;
+#pragma unroll
+        for (int dd = 0; dd < 5; ++dd) t[h] = (d == dd) ? w[dd] : t[h];
+      }
+      tc::split_f16x2(t[0], t[1], w_scale, hi[c], lo[c]);
+    }
+    const unsigned off = (unsigned)i * kTfBRow + (unsigned)ch * kTfBChunk + (unsigned)nn * 16u;
+    *reinterpret_cast<uint4*>(sm.b_hi + off) = *reinterpret_cast<uint4*>(hi);
+    if (kPrecise) *reinterpret_cast<uint4*>(sm.b_lo + off) = *reinterpret_cast<uint4*>(lo);
+  }
+  if (tid < kTfAsStride) {       // FC table
+    const int p = tid / 36, q = (tid % 36) / 6, f = tid % 6;
+    const float* wf = params + kOffWf + (tid < kS ? f * 36 + p * 6 + q : 0);
+    float w[12];
+#pragma unroll
+    for (int k = 0; k < 12; ++k) w[k] = (tid < kS && k < kOut) ? wf[(k < kOut ? k : 0) * kS] : 0.f;
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+      *reinterpret_cast<float4*>(sm.wf[tid >> 5][k][tid & 31]) = make_float4(w[4 * k], w[4 * k + 1], w[4 * k + 2], w[4 * k + 3]);
+  } else if (tid >= 256 && tid < 256 + 64) {
+    const int t = tid - 256;
+    if (t < 16) sm.ws[t] = params[kOffWs + t];
+    else if (t < 28) sm.bf[t - 16] = (t - 16 < kOut) ? params[kOffBf + t - 16] : 0.f;
+    else if (t < 28 + kF) sm.bc[t - 28] = kPre * params[kOffBc + t - 28];
+    else if (t == 40) sm.bs[0] = params[kOffBs];
+  }
   tc::fence_async_smem();      // the B operand was written through the generic proxy
   tc::fence_before_sync();
   __syncthreads();
@@ -223,26 +318,64 @@ k_forward_tc(const float* __restrict__ images, long n, long imgs_per_cta, const 
 
   bool gave_up = false;
   CNN_PHASE_BEGIN(blockIdx.x == 0, sm.clock_base)
-  TC_CTA_TIME(1);
 
-  if (warp == 0) {
-    // ================= finisher: images in order, three at a time ===================================
+  if (warp < kTfFinishers) {
+    // ================= finishers: images in order, three at a time in turn ===========================
     const int li = lane / 10, k = lane % 10;
-    for (int base = 0; base < imgs_here; base += 3) {
+    for (int base = 3 * warp, turn = 0; base < imgs_here; base += 3 * kTfFinishers) {
       const int img = base + li;
       const bool active = (lane < 30) && (img < imgs_here);
-      const int slot = img & (kTfSlots - 1);
-      float o = 0.f;
       CNN_PHASE(0);
-      if (active) {
-        mbar_wait_bounded(&sm.img_done[slot], (unsigned)(img / kTfSlots) & 1u, status, gave_up);
-        float z = 0.f;
+      const float* as[3];
 #pragma unroll
-        for (int p = 0; p < 6; ++p) z += sm.part[slot][p][k];
-        z += sm.bf[k];
-        CNN_PHASE(1);
-        o = kPrecise ? sigmoidf<SIG>(z) : fmaf(0.5f, tanh_approx(0.5f * z), 0.5f);
+      for (int j = 0; j < 3; ++j) {
+        const int slot = (base + j) & (kTfSlots - 1);
+        as[j] = &sm.as[slot][lane];
+        if (base + j < imgs_here) mbar_wait_bounded(&sm.img_done[slot], (unsigned)((base + j) / kTfSlots) & 1u, status, gave_up);
       }
+      CNN_PHASE(1);
+      f32x2 fc2[3][kOut / 2];
+#pragma unroll
+      for (int j = 0; j < 3; ++j)
+#pragma unroll
+        for (int kk = 0; kk < kOut / 2; ++kk) fc2[j][kk] = pack2(0.f, 0.f);
+#pragma unroll
+      for (int i = 0; i < kTfFcIn; ++i) {
+        const ulonglong2 w0 = *reinterpret_cast<const ulonglong2*>(sm.wf[i][0][lane]);
+        const ulonglong2 w1 = *reinterpret_cast<const ulonglong2*>(sm.wf[i][1][lane]);
+        const f32x2 w4 = *reinterpret_cast<const f32x2*>(sm.wf[i][2][lane]);
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+          const float a = as[j][32 * i];
+          const f32x2 a2 = pack2(a, a);
+          fc2[j][0] = fma2(w0.x, a2, fc2[j][0]); fc2[j][1] = fma2(w0.y, a2, fc2[j][1]); fc2[j][2] = fma2(w1.x, a2, fc2[j][2]);
+          fc2[j][3] = fma2(w1.y, a2, fc2[j][3]); fc2[j][4] = fma2(w4, a2, fc2[j][4]);
+        }
+      }
+      float sums[32];
+      sums[30] = sums[31] = 0.f;
+#pragma unroll
+      for (int j = 0; j < 3; ++j)
+#pragma unroll
+        for (int kk = 0; kk < kOut / 2; ++kk) unpack2(fc2[j][kk], sums[10 * j + 2 * kk], sums[10 * j + 2 * kk + 1]);
+      float z = warp_reduce_scatter32(sums, lane);      // lane 10 li + k: sum k of image base + li
+      bool bad = !U8 && active && (plain || sm.out_of_range[img & (kTfRange - 1)] != 0);
+      if (U8 && plain) bad = active;
+      if (__any_sync(0xffffffffu, bad)) {
+        if constexpr (!U8) {
+          for (int j = 0; j < 3; ++j) {
+            if (!__shfl_sync(0xffffffffu, (int)bad, 10 * j)) continue;
+            const float s = image_fc_plain<kPrecise ? SIG : 1>(static_cast<const float*>(images) + (img0 + base + j) * kImg, params, lane);
+            const float sk = __shfl_sync(0xffffffffu, s, k);
+            if (li == j) z = sk;
+          }
+        } else {
+          z = active ? __int_as_float(0x7fffffff) : 0.f;    // parameters that are not finite
+        }
+        if (bad && k == 0) sm.out_of_range[img & (kTfRange - 1)] = 0;
+      }
+      z += sm.bf[k];
+      const float o = kPrecise ? sigmoidf<SIG>(z) : fmaf(0.5f, tanh_approx(0.5f * z), 0.5f);
       __syncwarp();
       // classify(): strict '<' scan from index 0, so the lowest index wins ties.
       float bv = __shfl_sync(0xffffffffu, o, li * 10);
@@ -257,12 +390,12 @@ k_forward_tc(const float* __restrict__ images, long n, long imgs_per_cta, const 
         if (argmax && k == 0) argmax[img0 + img] = best;
       }
       __syncwarp();
-      if (lane == 0) *reinterpret_cast<volatile int*>(&sm.finished) = base + 3;   // these slots may be reused
+      if (lane == 0) *reinterpret_cast<volatile int*>(&sm.finished[warp]) = ++turn;   // these slots may be reused
       CNN_PHASE(2);
     }
-  } else if (warp == 1) {
+  } else if (warp == kTfMmaWarp) {
     // ================= MMA issue: the whole warp runs the loop, one elected lane issues ============
-    const unsigned idesc = tc::idesc_tf32(kTfRows, kTfBN, 0, 0);
+    const unsigned idesc = tc::idesc_f16(128, kTfBN);
     // descriptors differ only in their 14-bit start-address field: base + (byte offset >> 4)
     const unsigned long long bd_hi = tc::smem_desc(smem_u32(sm.b_hi), kTfBChunk, 128);
     const unsigned long long bd_lo = tc::smem_desc(smem_u32(sm.b_lo), kTfBChunk, 128);
@@ -271,132 +404,131 @@ k_forward_tc(const float* __restrict__ images, long n, long imgs_per_cta, const 
       CNN_PHASE(0);
       mbar_wait_bounded(&sm.a_full[s], (unsigned)(k / kTfSlabs) & 1u, status, gave_up);
       CNN_PHASE(1);
-      mbar_wait_bounded(&sm.d_free[b], ((unsigned)(k / kTfAcc) & 1u) ^ 1u, status, gave_up);
       CNN_PHASE(2);
-      __syncwarp();
-      tc::fence_after_sync();
-      const unsigned long long ad_hi = tc::smem_desc(smem_u32(sm.slab[s]), kTfChunkStride, 128);
-      const unsigned long long ad_lo = tc::smem_desc(smem_u32(sm.slab[s + kTfSlabsTotal / 2]), kTfChunkStride, 128);
+      const unsigned long long ad_hi = tc::smem_desc(smem_u32(sm.slab[s]), kTfChunkStride, kTfGroupStride);
+      const unsigned long long ad_lo = tc::smem_desc(smem_u32(sm.slab[(s + kTfSlabsTotal / 2) % kTfSlabsTotal]), kTfChunkStride, kTfGroupStride);
       const unsigned d_tile = tmem_base + (unsigned)(b * kTfDCols);
-      constexpr int kPasses = kPrecise ? 3 : 1;
-      // The loops over column block and pass stay rolled, the ten MMAs of one (block, pass) are written out.
-      // Four roles share this SM's instruction cache: with all 60 MMAs of path 1 written out (and the
-      // epilogue's two column blocks as well) the kernel's hot code no longer fitted -- instruction-cache
-      // hit rate 56 %, CTAs between 211 and 340 us depending on how many SMs of their GPC were fetching
-      // from the next cache level at the same time.  Rolled completely, the loop overhead between two
-      // MMAs (dependent address arithmetic, branch) showed: 76-91 cycles per MMA instead of 53.
+      // Four roles share this SM's instruction cache, so the loop over the two column blocks stays rolled; the MMAs
+      // of one block are written out (with dependent address arithmetic between two MMAs they cost 76-91 cycles
+      // each instead of 53).
 #pragma unroll 1
       for (int xb = 0; xb < 2; ++xb) {
-        unsigned accumulate = 0;
+        // The two column blocks of an accumulator are handed over and freed one by one: while an epilogue group works on
+        // the second block of its tile, the first block of its next tile (three tiles on) is computed, so it never
+        // waits for its own MMAs.
+        mbar_wait_bounded(&sm.d_free[2 * b + xb], ((unsigned)(k / kTfAcc) & 1u) ^ 1u, status, gave_up);
+        __syncwarp();
+        tc::fence_after_sync();
         const unsigned d_blk = d_tile + (unsigned)(xb * kTfBN);
-        const unsigned a_blk = ((unsigned)(3 * xb) * kTfChunkStride) >> 4;
-#pragma unroll 1
-        for (int pass = 0; pass < kPasses; ++pass) {
+        const unsigned a_blk = ((unsigned)(2 * xb) * kTfChunkStride) >> 4;
+#pragma unroll
+        for (int pass = 0; pass < (kPrecise ? 3 : 1); ++pass) {
           const unsigned long long a_d = ((pass == 1) ? ad_lo : ad_hi) + a_blk;
           const unsigned long long b_d = (pass == 2) ? bd_lo : bd_hi;
 #pragma unroll
-          for (int i = 0; i < 5; ++i) {
-#pragma unroll
-            for (int ks = 0; ks < 2; ++ks) {
-              constexpr unsigned kSixteen = 16u;
-              const unsigned a_off = (unsigned)(2 * ks) * kTfChunkStride + (unsigned)i * kSixteen;
-              const unsigned b_off = (unsigned)i * kTfBRow + (unsigned)(2 * ks) * kTfBChunk;
-              tc::mma_tf32_elect(d_blk, a_d + (a_off >> 4), b_d + (b_off >> 4), idesc, accumulate);
-              accumulate = 1;
-            }
-          }
+          for (int i = 0; i < 5; ++i)
+            tc::mma_f16_elect(d_blk, a_d + (unsigned)i, b_d + (unsigned)i * (kTfBRow >> 4), idesc, (pass | i) ? 1u : 0u);
         }
+        tc::mma_commit_elect(&sm.d_full[2 * b + xb]);    // the block is complete ...
       }
-      tc::mma_commit_elect(&sm.d_full[b]);    // the accumulator is complete ...
-      tc::mma_commit_elect(&sm.a_free[s]);    // ... and the slab may be overwritten
+      tc::mma_commit_elect(&sm.a_free[s]);               // ... and after both the slab may be overwritten
       CNN_PHASE(3);
     }
-  } else if (warp < kTfEpiWarp0) {
+  } else if (loader) {
     // ================= loaders: image rows -> operand slabs ==========================================
-    // Thread lt copies the same 15 items of every tile: item t = lt + 64 j is the t-th 16-byte piece of the
-    // tile's 15,232 contiguous bytes in HBM (row t / 7, column chunk t % 7), so a warp's copies cover 512
-    // contiguous bytes: four 128-byte requests instead of 32.  The offsets are computed once.
-    const int lt = tid - 64;                         // 0..63
-    constexpr int kPerThread = (kTfItems + kTfLoaders - 1) / kTfLoaders;   // 15
-    unsigned soff[kPerThread];                       // byte offset in the slab
-    int goff[kPerThread], irow[kPerThread];          // float offset from the tile's first row; row (>= 136: no item)
+    // Unit u = (group, row, chunk), chunk fastest: eight consecutive lanes store two rows of the four chunks without a bank
+    // conflict.  A thread's units u + 128 j repeat after three, eight groups further on.
+    typedef typename std::conditional<U8, unsigned, float4>::type Piece;     // four pixels
+    int ugroup[3], ugoff[3];
+    unsigned usoff[3];
 #pragma unroll
-    for (int j = 0; j < kPerThread; ++j) {
-      const int t = lt + kTfLoaders * j;
-      const int row = t / kTfChunks, chunk = t - row * kTfChunks;
-      soff[j] = (unsigned)chunk * kTfChunkStride + (unsigned)row * 16u;
-      goff[j] = t * 4;
-      irow[j] = (t < kTfItems) ? row : (1 << 20);
+    for (int j = 0; j < 3; ++j) {
+      const int u = lt + kTfLoaders * j;
+      const int r = u % (4 * kTfGroupRows), row = r >> 2, chunk = r & 3;
+      ugroup[j] = u / (4 * kTfGroupRows);
+      ugoff[j] = row * 7 + 2 * chunk - (chunk >> 1);                          // columns 0, 8, 12, 20
+      usoff[j] = (unsigned)chunk * kTfChunkStride + (unsigned)(ugroup[j] * kTfGroupRows + row) * 16u;
     }
-    auto rows_avail = [&](int kk) {                  // rows of tile kk that exist in the batch (junk lanes beyond)
-      const long left = rows_total - (row0 + (long)kk * kTfRows);
-      return (int)(left < kTfSlabRows ? left : kTfSlabRows);
-    };
-    auto finish_tile = [&](int kk) {
-      const int s = kk % kTfSlabs;
-      if (kPrecise) {
-        // split this thread's own chunks in place: the high part stays, the remainder goes to the low slab
-        const int avail = rows_avail(kk);
-        unsigned char* hi_s = sm.slab[s];
-        unsigned char* lo_s = sm.slab[s + kTfSlabsTotal / 2];
-        // five items at a time: the loads of a batch are issued together (a store to the slab would
-        // otherwise order every following load behind it)
+    for (int k = 0; k < n_tiles; ++k) {
+      const int s = k % kTfSlabs, r = k % kTfRaw;
+      CNN_PHASE(0);
+      if (lt == 0 && k + kTfRaw - 1 < n_tiles) {       // the buffer of tile k - 1 is next
+        if (k > 0) mbar_wait_bounded(&sm.raw_free[(k - 1) % kTfRaw], (unsigned)((k - 1) / kTfRaw) & 1u, status, gave_up);
+        fetch(k + kTfRaw - 1);
+      }
+      __syncwarp();
+      mbar_wait_bounded(&sm.raw_full[r], (unsigned)(k / kTfRaw) & 1u, status, gave_up);
+      CNN_PHASE(1);
+      // Groups past the last image read what the buffer held before: their output rows are never looked at.
+      const Piece* raw = reinterpret_cast<const Piece*>(sm.raw[r]) - group_pixel(k * kTfGroups) / 4;
+      Piece v[kTfUnits][2];
 #pragma unroll
-        for (int j0 = 0; j0 < kPerThread; j0 += 5) {
-          float4 v[5];
+      for (int j = 0; j < kTfUnits; ++j) {
+        const Piece* p = raw + group_pixel(k * kTfGroups + ugroup[j % 3] + (kTfGroups / 2) * (j / 3)) / 4 + ugoff[j % 3];
+        v[j][0] = p[0];
+        v[j][1] = p[1];
+      }
+      mbar_wait_bounded(&sm.a_free[s], ((unsigned)(k / kTfSlabs) & 1u) ^ 1u, status, gave_up);
+      CNN_PHASE(2);
+      unsigned char* hi_s = sm.slab[s];
+      unsigned char* lo_s = sm.slab[(s + kTfSlabsTotal / 2) % kTfSlabsTotal];
+      __half2 top = __floats2half2_rn(0.f, 0.f);
 #pragma unroll
-          for (int jj = 0; jj < 5; ++jj)
-            if (irow[j0 + jj] < avail) v[jj] = *reinterpret_cast<const float4*>(hi_s + soff[j0 + jj]);
+      for (int j = 0; j < kTfUnits; ++j) {
+        unsigned hi[4], lo[4];
+        const bool live = k * kTfGroups + ugroup[j % 3] + (kTfGroups / 2) * (j / 3) < n_groups;
 #pragma unroll
-          for (int jj = 0; jj < 5; ++jj) {
-            if (irow[j0 + jj] < avail) {
-              float4 hi, lo;
-              tc::split_tf32(v[jj].x, hi.x, lo.x); tc::split_tf32(v[jj].y, hi.y, lo.y);
-              tc::split_tf32(v[jj].z, hi.z, lo.z); tc::split_tf32(v[jj].w, hi.w, lo.w);
-              *reinterpret_cast<float4*>(hi_s + soff[j0 + jj]) = hi;
-              *reinterpret_cast<float4*>(lo_s + soff[j0 + jj]) = lo;
-            }
+        for (int h = 0; h < 2; ++h) {
+          if constexpr (U8) {
+            const unsigned b = v[j][h];
+            const unsigned e0 = sm.lut[b & 255u], e1 = sm.lut[(b >> 8) & 255u], e2 = sm.lut[(b >> 16) & 255u], e3 = sm.lut[b >> 24];
+            hi[2 * h] = __byte_perm(e0, e1, 0x5410); hi[2 * h + 1] = __byte_perm(e2, e3, 0x5410);
+            lo[2 * h] = __byte_perm(e0, e1, 0x7632); lo[2 * h + 1] = __byte_perm(e2, e3, 0x7632);
+          } else {
+            __half2 h0, h1, l0, l1;
+            tc::split_f16x2(v[j][h].x, v[j][h].y, px_scale, h0, l0);
+            tc::split_f16x2(v[j][h].z, v[j][h].w, px_scale, h1, l1);
+            if (live) top = __hmax2_nan(top, __hmax2_nan(__habs2(h0), __habs2(h1)));
+            hi[2 * h] = *reinterpret_cast<unsigned*>(&h0); hi[2 * h + 1] = *reinterpret_cast<unsigned*>(&h1);
+            lo[2 * h] = *reinterpret_cast<unsigned*>(&l0); lo[2 * h + 1] = *reinterpret_cast<unsigned*>(&l1);
           }
+        }
+        const unsigned o = usoff[j % 3] + (unsigned)(j / 3) * ((kTfGroups / 2) * kTfGroupStride);
+        *reinterpret_cast<uint4*>(hi_s + o) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+        if (kPrecise) *reinterpret_cast<uint4*>(lo_s + o) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+      }
+      if constexpr (!U8) {
+        const float2 t = __half22float2(top);
+        const float big = (t.x != t.x || t.y != t.y) ? 1e30f : fmaxf(t.x, t.y);
+        // fp16 holds magnitudes below 65,520: a larger scaled pixel (or one that is not a number) marks the tile's images
+        if (!(big < 65536.f)) {
+          const int first = (k * kTfGroups) / kTfGroupsImg, last = (k * kTfGroups + kTfGroups - 1) / kTfGroupsImg;
+          for (int im = first; im <= last; ++im)
+            if (im < imgs_here) sm.out_of_range[im & (kTfRange - 1)] = 1;
         }
       }
       tc::fence_async_smem();    // generic-proxy writes -> visible to the tensor core's operand reads
-      mbar_arrive(&sm.a_full[s]);
-    };
-    for (int k = 0; k < n_tiles + kTfAhead; ++k) {
-      // first hand over the oldest tile in flight (its hand-over must not wait for a slab to come free) ...
-      CNN_PHASE(0);
-      if (k >= kTfAhead) {
-        cp_async_wait<kTfAhead - 1>();   // this thread's copies of tile k - kTfAhead have landed
-        CNN_PHASE(1);
-        finish_tile(k - kTfAhead);
-        CNN_PHASE(2);
+      __syncwarp();
+      if (lane == 0) {
+        mbar_arrive(&sm.raw_free[r]);
+        mbar_arrive(&sm.a_full[s]);
       }
-      // ... then start tile k
-      if (k < n_tiles) {
-        const int s = k % kTfSlabs;
-        mbar_wait_bounded(&sm.a_free[s], ((unsigned)(k / kTfSlabs) & 1u) ^ 1u, status, gave_up);
-        CNN_PHASE(3);
-        const int avail = rows_avail(k);
-        const float* src = images + (row0 + (long)k * kTfRows) * kH;
-        unsigned char* dst = sm.slab[s];
-#pragma unroll
-        for (int j = 0; j < kPerThread; ++j)
-          if (irow[j] < avail) cp_async16(dst + soff[j], src + goff[j]);   // rows past the batch stay as they are
-      }
-      cp_async_commit();                 // (an empty group past the last tile keeps the count uniform)
-      CNN_PHASE(4);
+      CNN_PHASE(3);
     }
-  } else {
+  } else if (warp >= kTfEpiWarp0) {
     // ================= epilogue ====================================================================
     const int group = (warp - kTfEpiWarp0) >> 2;   // accumulator / tile residue this group owns
     const int quarter = warp & 3;                  // tensor-memory lanes 32 * quarter ..
-    const int rsub = lane & 3;                     // row of the 4x4 window (28, 32 and 128 are multiples of 4)
-    float wsr[4];
+    const int rsub = lane & 3;                     // row of the 4x4 window
+    f32x2 ws2[4], bc2[kF / 2];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) wsr[j] = (kPrecise ? 1.0f : 0.5f) * sm.ws[rsub * 4 + j];
-    float bcr[kF];
+    for (int j = 0; j < 4; ++j) {
+      const float w = (kPrecise ? 1.0f : 0.5f) * sm.ws[rsub * 4 + j];
+      ws2[j] = pack2(w, w);
+    }
 #pragma unroll
-    for (int f = 0; f < kF; ++f) bcr[f] = sm.bc[f];
+    for (int f = 0; f < kF; f += 2) bc2[f / 2] = pack2(sm.bc[f], sm.bc[f + 1]);
+    const f32x2 unscale2 = pack2(w_unscale, w_unscale), one2 = pack2(1.f, 1.f);
     // path 2: sum_j ws * (0.5 + 0.5 t) = sum_j (0.5 ws) t + 0.5 * sum(ws); the constant goes into the bias
     float bs_eff = sm.bs[0];
     if (!kPrecise) {
@@ -409,56 +541,86 @@ k_forward_tc(const float* __restrict__ images, long n, long imgs_per_cta, const 
 
     for (int k = group; k < n_tiles; k += kTfAcc) {
       CNN_PHASE(0);
-      mbar_wait_bounded(&sm.d_full[group], (unsigned)(k / kTfAcc) & 1u, status, gave_up);
-      CNN_PHASE(1);
-      tc::fence_after_sync();
-      const int R = k * kTfRows + quarter * 32 + lane;     // stacked row of this lane inside the CTA
-      const int img_l = R / kH;
-      const int y = R - img_l * kH;
-      const int p = y >> 2;
-      const bool valid = (img_l < imgs_here) && (p < 6);
+      const int g = k * kTfGroups + quarter * 4 + (lane >> 3);     // group of 8 output rows this lane's row belongs to
+      const int img_l = g / kTfGroupsImg;
+      const int p = 2 * (g - img_l * kTfGroupsImg) + ((lane >> 2) & 1);   // window row
+      const bool valid = img_l < imgs_here;
       const unsigned t0 = tmem_base + (unsigned)(group * kTfDCols) + ((unsigned)(quarter * 32) << 16);
-      const float* wblock = &sm.wf[((p < 6 ? p : 6) * 4 + rsub) * kTfWfBlock];
-
-      float fc[kOut];
-#pragma unroll
-      for (int kk = 0; kk < kOut; ++kk) fc[kk] = 0.f;
-      unsigned cur[8], nxt[8];
-      tmem_ld8_nowait(t0, cur);
-      tmem_wait8(cur);
+      const int slot = img_l & (kTfSlots - 1);
+      {   // the slots of this quarter's two or three images are free again: the images that had them, kTfSlots ago, lie in
+          // the triple of the last one and the triple before it, of different finisher warps
+        const int t = ((k * kTfGroups + quarter * 4 + 3) / kTfGroupsImg - kTfSlots) / 3;
+        if (k * kTfGroups + quarter * 4 + 3 >= kTfGroupsImg * kTfSlots) {
+          wait_counter_bounded(&sm.finished[t % kTfFinishers], t / kTfFinishers + 1, status, gave_up);
+          if (t > 0) wait_counter_bounded(&sm.finished[(t - 1) % kTfFinishers], (t - 1) / kTfFinishers + 1, status, gave_up);
+        }
+      }
+      // after the reduce-scatter lane r = rsub holds sums 9 (r & 1) + 5 (r >> 1) + i of a block, i < 5 - (r >> 1)
+      float* as_dst = &sm.as[slot][p * 36 + (b0 ? 9 : 0) + (b1 ? 5 : 0)];
+      CNN_PHASE(1);
       // (the column-block loop stays rolled to keep the epilogue's code inside the instruction cache)
 #pragma unroll 1
       for (int xb = 0; xb < 2; ++xb) {              // one 12-column block = three window columns
+        mbar_wait_bounded(&sm.d_full[2 * group + xb], (unsigned)(k / kTfAcc) & 1u, status, gave_up);
+        if (xb == 0) CNN_PHASE(2); else CNN_PHASE(5);
+        __syncwarp();
+        tc::fence_after_sync();
+        unsigned nxt[8];
+        tmem_ld8_nowait(t0 + (unsigned)(xb * kTfBN), nxt);
+        tmem_wait8(nxt);
         float z[18];
+        f32x2 d2[4];               // the row's four activations before the reciprocal (of two maps), one step behind
+        // Step ch turns 8 accumulator columns (window column ch / 3, maps 2 * (ch % 3) + {0, 1}) into exponentials and
+        // finishes the columns of step ch - 1, so that two chains of dependent instructions are always under way.
 #pragma unroll
-        for (int ch = 0; ch < 9; ++ch) {            // 8 accumulator columns: window column ch / 3, maps 2 * (ch % 3) + {0, 1}
-          const bool last = (ch == 8) && (xb == 1);
-          if (ch < 8) {
-            tmem_ld8_nowait(t0 + (unsigned)(xb * kTfBN + (ch + 1) * 8), nxt);
-          } else if (xb == 0) {
-            tmem_ld8_nowait(t0 + (unsigned)kTfBN, nxt);
-          } else {
-            // the last columns of this accumulator are in registers: hand it back to the MMA warp
-            tc::fence_before_sync();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&sm.d_free[group]);
+        for (int ch = 0; ch < 10; ++ch) {
+          f32x2 e2[4];
+          if (ch < 9) {
+            if (ch > 0) tmem_wait8(nxt);
+            // the window row's four columns of two maps: t = unscale * acc + bias
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+              e2[j] = fma2(pack2(__uint_as_float(nxt[2 * j]), __uint_as_float(nxt[2 * j + 1])), unscale2, bc2[ch % 3]);
+            if (ch < 8) {
+              tmem_ld8_nowait(t0 + (unsigned)(xb * kTfBN + (ch + 1) * 8), nxt);
+            } else {
+              // the last columns of this block are in registers: hand it back to the MMA warp
+              tc::fence_before_sync();
+              __syncwarp();
+              if (lane == 0) mbar_arrive(&sm.d_free[2 * group + xb]);
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              float x, y;
+              unpack2(e2[j], x, y);
+              if (kShort) e2[j] = pack2(exp2f_approx(fminf(x, kTfMaxExp)), exp2f_approx(fminf(y, kTfMaxExp)));
+              else if (kPrecise) e2[j] = pack2(sigmoidf<SIG>(x), sigmoidf<SIG>(y));
+              else e2[j] = pack2(tanh_approx(x), tanh_approx(y));
+            }
           }
-          // eight independent activations, written in stages so that their chains interleave
-          float av[8];
+          if (ch > 0) {
+            f32x2 z2;
+            if constexpr (kShort) {
+              // sum_j ws_j / d_j with d_j = 1 + 2^t_j over one common denominator: one reciprocal for four activations
+              // (the special-function unit would bound the kernel: 1.25 operations per activation instead of 2).
+              // t is capped at 31 so that the product of four stays finite: an activation below 4.7e-10 counts as 4.7e-10,
+              // far below the rounding of the sum it enters.
+              const f32x2 d01 = mul2(d2[0], d2[1]), d23 = mul2(d2[2], d2[3]);
+              float x, y;
+              unpack2(mul2(d01, d23), x, y);
+              const f32x2 n01 = fma2(ws2[0], d2[1], mul2(ws2[1], d2[0])), n23 = fma2(ws2[2], d2[3], mul2(ws2[3], d2[2]));
+              z2 = mul2(pack2(rcp_approx(x), rcp_approx(y)), fma2(n01, d23, mul2(n23, d01)));
+            } else {
+              z2 = fma2(ws2[3], d2[3], fma2(ws2[2], d2[2], fma2(ws2[1], d2[1], mul2(ws2[0], d2[0]))));
+            }
+            unpack2(z2, z[2 * (ch - 1)], z[2 * (ch - 1) + 1]);    // sums 6 * (window column) + map
+          }
+          if (ch < 9) {
 #pragma unroll
-          for (int c = 0; c < 8; ++c) av[c] = __uint_as_float(cur[c]) + bcr[2 * (ch % 3) + (c >> 2)];
-#pragma unroll
-          for (int c = 0; c < 8; ++c)
-            av[c] = kScaled ? sigmoid_of_scaled(av[c]) : (kPrecise ? sigmoidf<SIG>(av[c]) : tanh_approx(av[c]));
-          z[(ch / 3) * 6 + 2 * (ch % 3)] = fmaf(wsr[3], av[3], fmaf(wsr[2], av[2], fmaf(wsr[1], av[1], wsr[0] * av[0])));
-          z[(ch / 3) * 6 + 2 * (ch % 3) + 1] = fmaf(wsr[3], av[7], fmaf(wsr[2], av[6], fmaf(wsr[1], av[5], wsr[0] * av[4])));
-          if (!last) {
-            tmem_wait8(nxt);
-#pragma unroll
-            for (int e = 0; e < 8; ++e) cur[e] = nxt[e];
+            for (int j = 0; j < 4; ++j) d2[j] = kShort ? add2(e2[j], one2) : e2[j];
           }
         }
-        if (xb == 0) CNN_PHASE(2); else CNN_PHASE(4);
+        if (xb == 0) CNN_PHASE(3); else CNN_PHASE(6);
         // ---- the window's four rows are lanes 4g..4g+3: reduce-scatter the block's 18 sums -----------
         // step 1 (lane bit 0): 9 each; step 2 (lane bit 1): 5 / 4 (+ one empty slot)
         float w9[9];
@@ -476,52 +638,29 @@ k_forward_tc(const float* __restrict__ images, long n, long imgs_per_cta, const 
           const float keep = b1 ? hi9 : w9[i];
           u[i] = keep + __shfl_xor_sync(0xffffffffu, send, 2);
         }
-        // ---- subsample sigmoid and this lane's share of the FC (the table row of an empty slot is zero) --
+        // ---- subsample sigmoid into the image's slot ----------------------------------------------------
 #pragma unroll
         for (int i = 0; i < 5; ++i) {
           const float zs = u[i] + bs_eff;
           const float as = kPrecise ? sigmoidf<SIG>(zs) : fmaf(0.5f, tanh_approx(0.5f * zs), 0.5f);
-          const float* wr = wblock + (xb * 5 + i) * 12;
-          const float4 w0 = *reinterpret_cast<const float4*>(wr);
-          const float4 w1 = *reinterpret_cast<const float4*>(wr + 4);
-          const float4 w2 = *reinterpret_cast<const float4*>(wr + 8);
-          fc[0] = fmaf(w0.x, as, fc[0]); fc[1] = fmaf(w0.y, as, fc[1]); fc[2] = fmaf(w0.z, as, fc[2]);
-          fc[3] = fmaf(w0.w, as, fc[3]); fc[4] = fmaf(w1.x, as, fc[4]); fc[5] = fmaf(w1.y, as, fc[5]);
-          fc[6] = fmaf(w1.z, as, fc[6]); fc[7] = fmaf(w1.w, as, fc[7]); fc[8] = fmaf(w2.x, as, fc[8]);
-          fc[9] = fmaf(w2.y, as, fc[9]);
+          if (valid && (i < 4 || !b1)) as_dst[18 * xb + i] = as;
         }
-        if (xb == 0) CNN_PHASE(3); else CNN_PHASE(5);
+        if (xb == 0) CNN_PHASE(4); else CNN_PHASE(7);
       }
-#pragma unroll
-      for (int kk = 0; kk < kOut; ++kk) {
-        fc[kk] += __shfl_xor_sync(0xffffffffu, fc[kk], 1);
-        fc[kk] += __shfl_xor_sync(0xffffffffu, fc[kk], 2);
-      }
-      CNN_PHASE(6);
-      // ---- hand the window row's ten sums to the image (the finisher warp waits for all six) ----------
-      if (valid && rsub == 0) {
-        const int slot = img_l & (kTfSlots - 1);
-        wait_counter_bounded(&sm.finished, img_l - kTfSlots + 1, status, gave_up);   // the slot's previous image is out
-        float* dst = &sm.part[slot][p][0];
-        *reinterpret_cast<float4*>(dst) = make_float4(fc[0], fc[1], fc[2], fc[3]);
-        *reinterpret_cast<float4*>(dst + 4) = make_float4(fc[4], fc[5], fc[6], fc[7]);
-        *reinterpret_cast<float2*>(dst + 8) = make_float2(fc[8], fc[9]);
-        mbar_arrive(&sm.img_done[slot]);   // release: the stores above are visible to whoever sees the phase complete
-      }
-      CNN_PHASE(7);
+      __syncwarp();
+      if (valid && rsub == 0) mbar_arrive(&sm.img_done[slot]);   // one of the image's six window rows (release)
+      CNN_PHASE(8);
     }
   }
   CNN_PHASE_END(g_phase_clocks_tc);
-  if (warp == 0) TC_CTA_TIME(2);    // the finisher is the last warp with work
 
   tc::fence_before_sync();
   __syncthreads();
-  if (warp == 1) tc::tmem_dealloc(tmem_base, 512);
-  TC_CTA_TIME(3);
+  if (warp == kTfMmaWarp) tc::tmem_dealloc(tmem_base, 512);
 }
 
-template <int PATH, int SIG>
-static int launch_forward_tc(cnn_net* net, const float* d_images, long n, float* d_out, int* d_argmax,
+template <int PATH, int SIG, bool U8>
+static int launch_forward_tc(cnn_net* net, const void* d_images, long n, float* d_out, int* d_argmax,
                              cudaStream_t stream) {
   // Every CTA owns a contiguous range of whole images (an image's window rows meet in shared memory).
   long grid = sm_count();
@@ -530,32 +669,34 @@ static int launch_forward_tc(cnn_net* net, const float* d_images, long n, float*
   const long per_cta = (n + grid - 1) / grid;
   grid = (n + per_cta - 1) / per_cta;
   const size_t smem = sizeof(TfSmem) + 128;
-  CNN_CUDA(cudaFuncSetAttribute(k_forward_tc<PATH, SIG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  k_forward_tc<PATH, SIG><<<(unsigned)grid, kTfThreads, smem, stream>>>(d_images, n, per_cta, net->d_params, d_out,
-                                                                       d_argmax, net->d_status);
-  cudaError_t e = cudaGetLastError();
+  CNN_CUDA(cudaFuncSetAttribute(k_forward_tc<PATH, SIG, U8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  cudaError_t e = launch_pdl(k_forward_tc<PATH, SIG, U8>, dim3((unsigned)grid), dim3(kTfThreads), smem, stream, d_images, n,
+                             per_cta, (const float*)net->d_params, d_out, d_argmax, net->d_status);
+  if (e == cudaSuccess) e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e, "k_forward_tc launch");
   return CNN_OK;
 }
 
 int forward_device_tc(cnn_net* net, int path, const float* d_images, long n, float* d_out, int* d_argmax,
                       cudaStream_t stream) {
-  if (path == 2) return launch_forward_tc<2, 2>(net, d_images, n, d_out, d_argmax, stream);
-  // Path 1 with fast_sigmoid set uses the short sigmoid form (ex2.approx, rcp.approx): the epilogue is
-  // bound by instruction issue and the special-function unit, and over the 65,536 images of benchmark
-  // configuration 2 the outputs are as close to the oracle with it (3.8e-6) as with the refined form (4.3e-6).
-  return net->fast_sigmoid ? launch_forward_tc<1, 1>(net, d_images, n, d_out, d_argmax, stream)
-                           : launch_forward_tc<1, 0>(net, d_images, n, d_out, d_argmax, stream);
+  if (path == 2) return launch_forward_tc<2, 2, false>(net, d_images, n, d_out, d_argmax, stream);
+  // Path 1 with fast_sigmoid set uses the short sigmoid form (ex2.approx, rcp.approx): over the 65,536 images of
+  // benchmark configuration 2 the outputs are as close to the oracle with it as with the refined form.
+  return net->fast_sigmoid ? launch_forward_tc<1, 1, false>(net, d_images, n, d_out, d_argmax, stream)
+                           : launch_forward_tc<1, 0, false>(net, d_images, n, d_out, d_argmax, stream);
+}
+
+int forward_device_tc_u8(cnn_net* net, const unsigned char* d_pixels, long n, float* d_out, int* d_argmax,
+                         cudaStream_t stream) {
+  return net->fast_sigmoid ? launch_forward_tc<1, 1, true>(net, d_pixels, n, d_out, d_argmax, stream)
+                           : launch_forward_tc<1, 0, true>(net, d_pixels, n, d_out, d_argmax, stream);
 }
 
 }  // namespace cnn
 
 #ifdef CNN_PHASE_CLOCKS
-extern "C" int cnn_debug_cta_times_tc(long long* out /* [160][4] */) {
-  return cudaMemcpyFromSymbol(out, cnn::g_tc_cta_times, sizeof(cnn::g_tc_cta_times)) == cudaSuccess ? 0 : 2;
-}
-// Sums of the SM clock at each stamp for the 16 warps of CTA 0 of the last launch (tuning builds only).
-extern "C" int cnn_debug_phase_clocks_tc(long long* out /* [16][16] */) {
+// Sums of the SM clock at each stamp for the 20 warps of CTA 0 of the last launch (tuning builds only).
+extern "C" int cnn_debug_phase_clocks_tc(long long* out /* [20][16] */) {
   return cudaMemcpyFromSymbol(out, cnn::g_phase_clocks_tc, sizeof(cnn::g_phase_clocks_tc)) == cudaSuccess ? 0 : 2;
 }
 #endif

@@ -236,13 +236,13 @@ static int launch_variant(cnn_net* net, const void* d_images, long n, float* d_o
 // fast_sigmoid set (the default): the short sigmoid form, 0.321 ms per 65,536 images; over that batch it
 // is as close to the fp64 oracle as the reference expression (2.1e-6; the fp32 oracle itself is 4.0e-6 away).
 // The kernel a call over n_total images uses (0 = this file's, 1 / 2 = forward_tc.cu).  Default (-1): the
-// three-pass tensor-core kernel from the batch size at which it overtakes this one (measured on a B200:
-// 22 us for anything up to 2,368 images against 10-20 us here, 41 against 47 us at 8,192 images, 203 against
-// 333 us at 65,536).  Both keep the 1e-5 parity bar.  With the reference's sigmoid expression asked for
-// (fast_sigmoid = 0) the default stays on this kernel.
-int forward_kernel_for(const cnn_net* net, long n_total) {
+// three-pass tensor-core kernel for batches of kTcMinBatch images and more, where it is the faster one, this
+// kernel below.  uint8 pixels follow the same rule, so that they give the same bits as the fp32
+// images they stand for (the reduced-precision path 2 is for fp32 images only).  Both keep the 1e-5 parity bar.
+// With the reference's sigmoid expression asked for (fast_sigmoid = 0) the default stays on this kernel.
+int forward_kernel_for(const cnn_net* net, long n_total, bool u8) {
   constexpr long kTcMinBatch = 6144;
-  if (net->forward_path >= 0) return net->forward_path;
+  if (net->forward_path >= 0 && !(u8 && net->forward_path == 2)) return net->forward_path;
   return (net->fast_sigmoid && n_total >= kTcMinBatch) ? 1 : 0;
 }
 
@@ -255,8 +255,9 @@ int forward_device(cnn_net* net, int path, const float* d_images, long n, float*
                            : launch_variant<0, false, 1>(net, d_images, n, d_out, d_argmax, stream);
 }
 
-int forward_device_u8(cnn_net* net, const unsigned char* d_pixels, long n, float* d_out, int* d_argmax,
+int forward_device_u8(cnn_net* net, int path, const unsigned char* d_pixels, long n, float* d_out, int* d_argmax,
                       cudaStream_t stream) {
+  if (path != 0) return forward_device_tc_u8(net, d_pixels, n, d_out, d_argmax, stream);
   return net->fast_sigmoid ? launch_variant<1, true, 1>(net, d_pixels, n, d_out, d_argmax, stream)
                            : launch_variant<0, true, 1>(net, d_pixels, n, d_out, d_argmax, stream);
 }
@@ -271,7 +272,7 @@ extern "C" int cnn_forward_batched(cnn_net* net, const float* d_images, long n, 
   CNN_REQUIRE(d_images != nullptr, "cnn_forward_batched: NULL images");
   CNN_REQUIRE((reinterpret_cast<uintptr_t>(d_images) & 15u) == 0,
               "cnn_forward_batched: image batch must start on a 16-byte boundary");
-  return cnn::forward_device(net, cnn::forward_kernel_for(net, n), d_images, n, d_out, d_argmax, cnn::as_stream(stream));
+  return cnn::forward_device(net, cnn::forward_kernel_for(net, n, false), d_images, n, d_out, d_argmax, cnn::as_stream(stream));
 }
 
 extern "C" int cnn_forward_batched_u8(cnn_net* net, const unsigned char* d_pixels, long n, float* d_out,
@@ -282,5 +283,5 @@ extern "C" int cnn_forward_batched_u8(cnn_net* net, const unsigned char* d_pixel
   CNN_REQUIRE(d_pixels != nullptr, "cnn_forward_batched_u8: NULL pixels");
   CNN_REQUIRE((reinterpret_cast<uintptr_t>(d_pixels) & 15u) == 0,
               "cnn_forward_batched_u8: pixel batch must start on a 16-byte boundary");
-  return cnn::forward_device_u8(net, d_pixels, n, d_out, d_argmax, cnn::as_stream(stream));
+  return cnn::forward_device_u8(net, cnn::forward_kernel_for(net, n, true), d_pixels, n, d_out, d_argmax, cnn::as_stream(stream));
 }

@@ -7,10 +7,10 @@
 #include "net.cuh"
 
 namespace cnn {
-int forward_kernel_for(const cnn_net* net, long n_total);
+int forward_kernel_for(const cnn_net* net, long n_total, bool u8);
 int forward_device(cnn_net* net, int path, const float* d_images, long n, float* d_out, int* d_argmax,
                    cudaStream_t stream);
-int forward_device_u8(cnn_net* net, const unsigned char* d_pixels, long n, float* d_out, int* d_argmax,
+int forward_device_u8(cnn_net* net, int path, const unsigned char* d_pixels, long n, float* d_out, int* d_argmax,
                       cudaStream_t stream);
 
 int ensure_train_scratch(cnn_net* net, int rows) {
@@ -189,14 +189,14 @@ static int forward_host_impl(cnn_net* net, const void* h_images, bool u8, long n
   // D2H of chunk c).
   long done = 0;
   int slot = 0;
-  const int path = forward_kernel_for(net, n);     // one kernel for the whole request, whatever the chunking
+  const int path = forward_kernel_for(net, n, u8);     // one kernel for the whole request, whatever the chunking
   while (done < n) {
     const long cnt = (n - done) < net->stage_images ? (n - done) : net->stage_images;
     cudaStream_t st = net->copy_stream[slot];
     CNN_CUDA(cudaMemcpyAsync(net->d_stage_img[slot],
                              static_cast<const unsigned char*>(h_images) + (size_t)done * image_bytes,
                              (size_t)cnt * image_bytes, cudaMemcpyHostToDevice, st));
-    rc = u8 ? forward_device_u8(net, reinterpret_cast<const unsigned char*>(net->d_stage_img[slot]), cnt,
+    rc = u8 ? forward_device_u8(net, path, reinterpret_cast<const unsigned char*>(net->d_stage_img[slot]), cnt,
                                 net->d_stage_out[slot], net->d_stage_arg[slot], st)
             : forward_device(net, path, net->d_stage_img[slot], cnt, net->d_stage_out[slot],
                              net->d_stage_arg[slot], st);

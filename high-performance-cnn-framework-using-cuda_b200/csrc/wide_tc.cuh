@@ -4,6 +4,8 @@
 // (cta_group::1), operands in shared memory, fp32 accumulators in tensor memory.
 #pragma once
 
+#include <cuda_fp16.h>
+
 #include "net.cuh"
 
 namespace cnn {
@@ -38,6 +40,11 @@ __device__ __forceinline__ unsigned long long smem_desc(unsigned smem_addr, unsi
 __host__ __device__ constexpr unsigned idesc_tf32(int M, int N, int a_mn_major, int b_mn_major) {
   return (1u << 4) | (2u << 7) | (2u << 10) | ((unsigned)a_mn_major << 15) | ((unsigned)b_mn_major << 16) |
          ((unsigned)(N >> 3) << 17) | ((unsigned)(M >> 4) << 24);
+}
+
+// The same for kind::f16 with both operands in fp16 (formats 0) and K-major, fp32 accumulation.
+__host__ __device__ constexpr unsigned idesc_f16(int M, int N) {
+  return (1u << 4) | ((unsigned)(N >> 3) << 17) | ((unsigned)(M >> 4) << 24);
 }
 
 __device__ __forceinline__ void tmem_alloc(unsigned* smem_dst, unsigned cols) {   // whole warp
@@ -75,6 +82,16 @@ __device__ __forceinline__ void mma_tf32_elect(unsigned tmem_d, unsigned long lo
       ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
+// kind::f16: K = 16 fp16 values per instruction, the same operand bytes as eight tf32 values.
+__device__ __forceinline__ void mma_f16_elect(unsigned tmem_d, unsigned long long adesc, unsigned long long bdesc,
+                                              unsigned idesc, unsigned accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+      "elect.sync _|q, 0xffffffff;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
 // Whole converged warp: the lane that elect.sync picks (the same one every time for a full mask)
 // arrives on the mbarrier when every MMA it has issued so far has completed.
 __device__ __forceinline__ void mma_commit_elect(unsigned long long* bar) {
@@ -104,6 +121,18 @@ __device__ __forceinline__ void tmem_ld16(unsigned taddr, float (&v)[16]) {
                :: "memory");
 #pragma unroll
   for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
+}
+
+// Split two fp32 values, times a power of two, into fp16 high parts (round to nearest) and fp16 remainders: hi + lo to
+// about 2^-23 relative, or to 2^-25 absolute where lo is an fp16 subnormal.  From 65,520 on hi is infinite.
+__device__ __forceinline__ void split_f16x2(float x, float y, float scale, __half2& hi, __half2& lo) {
+  const f32x2 s = pack2(scale, scale), v = pack2(x, y);
+  float sx, sy;
+  unpack2(mul2(v, s), sx, sy);
+  hi = __floats2half2_rn(sx, sy);
+  const float2 b = __half22float2(hi);
+  unpack2(fma2(v, s, pack2(-b.x, -b.y)), sx, sy);
+  lo = __floats2half2_rn(sx, sy);
 }
 
 // Split an fp32 value into a tf32-exact high part and the remainder (for the three-pass product

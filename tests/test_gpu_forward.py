@@ -351,3 +351,45 @@ def test_default_kernel_choice_follows_batch_size(cuda, pkg, params0):
         net.set_option("forward_path", path)
         ref[path] = run_forward(cuda, net, images)
     assert np.array_equal(ref[-1][0], ref[0][0])
+
+
+@pytest.mark.parametrize("what", ["largest", "out of range", "not a number", "uint8", "tiny weights", "huge weights"])
+@pytest.mark.parametrize("n", [3, 148 * 16 + 21])
+def test_tensor_core_forward_operand_range(cuda, pkg, params0, what, n):
+    """The tensor-core kernel's operands are fp16 parts of scaled values: pixels up to 65,519 / scale go through them, an
+    image with a larger pixel or a NaN is computed in fp32 (its neighbours are not touched), weights of any magnitude
+    are scaled with the pixels, and uint8 pixels give the bits of the fp32 images they stand for.  Reference: the fp32
+    CUDA-core kernel."""
+    pix = pkg.synth.synth_pixels_u8(41, n)
+    images = pkg.synth.u8_to_float(pix)
+    params = params0.copy()
+    spots = [0, n // 2, n - 1]
+    limit = 65520.0 / 2.0 ** (5 + np.floor(np.log2(np.abs(params[:150]).max() * 1.442695)))
+    if what == "largest":
+        images[spots, 5, 7] = limit * (1 - 1e-4)
+    elif what == "out of range":
+        images[spots, 27, 27] = limit
+        images[spots, 0, 0] = -3e6
+    elif what == "not a number":
+        images[spots, 11, 12] = np.nan
+    elif what.endswith("weights"):
+        params[:150] *= np.float32(1e-6 if what == "tiny weights" else 1e6)
+        images *= np.float32(1e4 if what == "tiny weights" else 1e-6)
+    net = pkg.Net(0)
+    net.set_params(params)
+    outs = {}
+    for path in (0, 1):
+        net.set_option("forward_path", path)
+        outs[path] = run_forward(cuda, net, images)
+        assert net.status() == 0
+    if what == "uint8":
+        d_pix = cuda.from_numpy(pix).cuda()
+        d_out = cuda.empty((n, 10), dtype=cuda.float32, device="cuda")
+        d_arg = cuda.empty((n,), dtype=cuda.int32, device="cuda")
+        net.forward_u8(d_pix, n, d_out, d_arg)
+        cuda.cuda.synchronize()
+        assert np.array_equal(d_out.cpu().numpy(), outs[1][0]) and np.array_equal(d_arg.cpu().numpy(), outs[1][1])
+    assert np.array_equal(np.isnan(outs[0][0]), np.isnan(outs[1][0]))
+    keep = ~np.isnan(outs[0][0]).any(axis=1)
+    assert keep.sum() == n - (len(set(spots)) if what == "not a number" else 0)
+    assert rel_err(outs[1][0][keep], outs[0][0][keep]) < 1e-5
