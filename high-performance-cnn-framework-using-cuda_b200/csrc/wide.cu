@@ -5,55 +5,150 @@
 // The reference's own kernels cannot run this shape (fixed array types; N * thread_index overflows
 // int), so its check is the generalised oracle.
 //
-// This file is the fp32 SIMT path: batch-level kernels with the conv activations and conv deltas
-// kept in HBM between them (at 56x56 / 64 maps one image's activations are 692 KB, more than an
-// SM's shared memory).  All reductions are fixed-order (no atomics).
+// This file is the fp32 SIMT path and the FC layer of all paths.  Between the forward and the backward pass the conv
+// activations are kept in HBM (at 56x56 / 64 maps one image's activations are 692 KB, more than an
+// SM's shared memory); inference does not write them.  All reductions are fixed-order (no atomics).
+#include <cooperative_groups.h>
+
 #include <cstring>
 #include <new>
 #include <vector>
 
+#include "cluster_exchange.cuh"
 #include "wide.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace cnn {
 
-constexpr int kWideFg = 8;       // filters per block in the forward conv
-constexpr int kWideGg = 4;       // filters per block in the conv weight gradient
-
 // ---- forward ---------------------------------------------------------------------------------
-// Block (image b, group of 8 maps): image in shared memory, thread = output position, 8 maps per
-// patch read.  Writes the conv ACTIVATIONS (sigmoid applied); pre-activations are never needed again
-// because sigmoid' = a (1 - a).
-template <int FLAVOR>
-__global__ void __launch_bounds__(256)
-k_wide_conv_fwd(WideDims d, const float* __restrict__ images, const float* __restrict__ params,
-                float* __restrict__ ac) {
-  extern __shared__ float sh[];
-  float* img = sh;                       // H*H
-  float* w = sh + d.H * d.H;             // 8 * 25
-  float* bias = w + kWideFg * 25;        // 8
-  const int b = blockIdx.x, f0 = blockIdx.y * kWideFg;
-  for (int i = threadIdx.x; i < d.H * d.H; i += blockDim.x) img[i] = images[(size_t)b * d.H * d.H + i];
-  for (int i = threadIdx.x; i < kWideFg * 25; i += blockDim.x)
-    w[i] = (f0 + i / 25 < d.F) ? params[d.o_wc + f0 * 25 + i] : 0.f;
-  if (threadIdx.x < kWideFg) bias[threadIdx.x] = (f0 + threadIdx.x < d.F) ? params[d.o_bc + f0 + threadIdx.x] : 0.f;
+// Convolution, bias, sigmoid and the subsample layer of one 4x4 window for a group of maps, two maps at a time: thread =
+// window (of any image: windows are numbered through the batch), the two maps in the halves of packed fp32 registers.
+// The 8x8 patch goes by row by row (eight pixels, each copied into both halves: 64 moves for 400 packed FMAs), so a
+// thread holds 16 accumulators, the 25 tap pairs and one row.  Bound by the fp32 FMA pipe: 400 FMAs per window and map
+// = 40 us for 333 images of 56x56 with 64 maps; 55 us measured (a block per image and 8 maps with one output per thread,
+// then the subsample layer from memory: 287 + 53 us).
+// Writes the subsample activations and, with STORE, the conv activations (what the backward pass reads; pre-activations
+// are never needed again because sigmoid' = a (1 - a)).  Positions outside the windows (C not a multiple of 4) reach
+// nothing and are not computed.
+constexpr int kWideWinThreads = 128;
+constexpr int kWideTapStride = 26;      // 25 tap pairs, padded to an even number for 128-bit loads
+
+// Eight pixels of a patch row; VEC: rows are 16-byte aligned (H a multiple of 4).
+template <bool VEC>
+__device__ __forceinline__ void load_row8(const float* __restrict__ src, float (&v)[8]) {
+  if (VEC) {
+    const float4 a = __ldg(reinterpret_cast<const float4*>(src)), b = __ldg(reinterpret_cast<const float4*>(src) + 1);
+    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+  } else {
+#pragma unroll
+    for (int c = 0; c < 8; ++c) v[c] = __ldg(src + c);
+  }
+}
+
+template <int FLAVOR, bool STORE, bool VEC>
+__global__ void __launch_bounds__(kWideWinThreads, 4)
+k_wide_conv_s1(WideDims d, long n, int maps_per_block, const float* __restrict__ images, const float* __restrict__ params,
+               float* __restrict__ ac, float* __restrict__ as) {
+  extern __shared__ __align__(16) float sh[];
+  // tap pairs [pair][26][2] | subsample taps, doubled [16][2] | bias pairs [pair][2]   (the first two are read 16 bytes at a time)
+  // (the short sigmoid form's factor -log2(e) is folded into taps and bias)
+  constexpr float kPre = (FLAVOR == 1) ? -1.4426950408889634f : 1.0f;
+  const int f0 = blockIdx.y * maps_per_block;
+  const int maps = min(maps_per_block, d.F - f0), pairs = (maps + 1) / 2;
+  float* tap = sh;
+  float* ws = tap + (maps_per_block + 1) / 2 * kWideTapStride * 2;
+  float* bias = ws + 32;
+  for (int i = threadIdx.x; i < pairs * kWideTapStride * 2; i += blockDim.x) {
+    const int pr = i / (kWideTapStride * 2), t = (i % (kWideTapStride * 2)) >> 1, f = 2 * pr + (i & 1);
+    tap[i] = (t < 25 && f < maps) ? kPre * params[d.o_wc + (f0 + f) * 25 + t] : 0.f;
+  }
+  for (int i = threadIdx.x; i < pairs * 2; i += blockDim.x) bias[i] = (i < maps) ? kPre * params[d.o_bc + f0 + i] : 0.f;
+  if (threadIdx.x < 32) ws[threadIdx.x] = params[d.o_ws + (threadIdx.x >> 1)];
+  const float bs = params[d.o_bs];
   __syncthreads();
-  const int CC = d.C * d.C;
-  for (int o = threadIdx.x; o < CC; o += blockDim.x) {
-    const int y = o / d.C, x = o % d.C;
-    float acc[kWideFg];
+  const int W = d.P * d.P;
+  const long t = (long)blockIdx.x * kWideWinThreads + threadIdx.x;
+  if (t >= n * W) return;
+  const long b = t / W;
+  const int w = (int)(t - b * W), p = w / d.P, q = w - p * d.P;
+  const float* src = images + ((size_t)b * d.H + 4 * p) * d.H + 4 * q;
+#pragma unroll 1
+  for (int pr = 0; pr < pairs; ++pr) {
+    f32x2 acc[4][4], wt[kWideTapStride];
+    const ulonglong2* tp = reinterpret_cast<const ulonglong2*>(tap + pr * kWideTapStride * 2);
 #pragma unroll
-    for (int g = 0; g < kWideFg; ++g) acc[g] = 0.f;
+    for (int i = 0; i < kWideTapStride / 2; ++i) {
+      const ulonglong2 v = tp[i];
+      wt[2 * i] = v.x; wt[2 * i + 1] = v.y;
+    }
+    const f32x2 bp = reinterpret_cast<const f32x2*>(bias)[pr];
 #pragma unroll
-    for (int j = 0; j < 5; ++j)
+    for (int y = 0; y < 4; ++y)
 #pragma unroll
-      for (int i = 0; i < 5; ++i) {
-        const float v = img[(y + i) * d.H + x + j];
+      for (int x = 0; x < 4; ++x) acc[y][x] = bp;
 #pragma unroll
-        for (int g = 0; g < kWideFg; ++g) acc[g] = fmaf(w[g * 25 + i * 5 + j], v, acc[g]);
+    for (int r = 0; r < 8; ++r) {
+      float v[8];
+      load_row8<VEC>(src + r * d.H, v);
+      f32x2 v2[8];
+#pragma unroll
+      for (int c = 0; c < 8; ++c) v2[c] = pack2(v[c], v[c]);
+#pragma unroll
+      for (int y = 0; y < 4; ++y) {
+        const int i = r - y;                 // tap row
+        if (i < 0 || i > 4) continue;
+#pragma unroll
+        for (int j = 0; j < 5; ++j)
+#pragma unroll
+          for (int x = 0; x < 4; ++x) acc[y][x] = fma2(wt[i * 5 + j], v2[x + j], acc[y][x]);
+      }
+    }
+    f32x2 z = pack2(0.f, 0.f);
+    const ulonglong2* wsp = reinterpret_cast<const ulonglong2*>(ws);
+    const int f = f0 + 2 * pr;
+    const bool second = 2 * pr + 1 < maps;
+    const size_t ac_at = STORE ? ((size_t)(b * d.F + f) * d.C + 4 * p) * d.C + 4 * q : 0;
+#pragma unroll
+    for (int y = 0; y < 4; ++y) {
+      float a0[4], a1[4];
+#pragma unroll
+      for (int x = 0; x < 4; ++x) {
+        float u0, u1;
+        unpack2(acc[y][x], u0, u1);
+        if (FLAVOR == 1) {
+          a0[x] = rcp_approx(1.0f + exp2f_approx(u0));
+          a1[x] = rcp_approx(1.0f + exp2f_approx(u1));
+        } else {
+          a0[x] = sigmoidf<FLAVOR>(u0);
+          a1[x] = sigmoidf<FLAVOR>(u1);
+        }
       }
 #pragma unroll
-    for (int g = 0; g < kWideFg; ++g)
-      if (f0 + g < d.F) ac[((size_t)b * d.F + f0 + g) * CC + o] = sigmoidf<FLAVOR>(acc[g] + bias[g]);
+      for (int x = 0; x < 4; x += 2) {
+        const ulonglong2 w2 = wsp[(4 * y + x) / 2];
+        z = fma2(w2.x, pack2(a0[x], a1[x]), z);
+        z = fma2(w2.y, pack2(a0[x + 1], a1[x + 1]), z);
+      }
+      if (STORE) {
+        float* dst = ac + ac_at + (size_t)y * d.C;
+        float* dst1 = dst + (size_t)d.C * d.C;
+        if (VEC) {
+          *reinterpret_cast<float4*>(dst) = make_float4(a0[0], a0[1], a0[2], a0[3]);
+          if (second) *reinterpret_cast<float4*>(dst1) = make_float4(a1[0], a1[1], a1[2], a1[3]);
+        } else {
+#pragma unroll
+          for (int x = 0; x < 4; ++x) {
+            dst[x] = a0[x];
+            if (second) dst1[x] = a1[x];
+          }
+        }
+      }
+    }
+    float z0, z1;
+    unpack2(z, z0, z1);
+    as[(size_t)(b * d.F + f) * W + w] = sigmoidf<FLAVOR>(z0 + bs);
+    if (second) as[(size_t)(b * d.F + f + 1) * W + w] = sigmoidf<FLAVOR>(z1 + bs);
   }
 }
 
@@ -74,53 +169,72 @@ __global__ void k_wide_s1_fwd(WideDims d, long n, const float* __restrict__ ac,
   as[idx] = sigmoidf<FLAVOR>(z + params[d.o_bs]);
 }
 
-// Block = kWideFcImgs images: FC, sigmoid, argmax, makeError, error norm.  (One image per block read the
-// 433 KB of FC weights from L2 once per image: 62 us for 1,024 images; four images share them.)
-constexpr int kWideFcImgs = 4;
+// FC, sigmoid, argmax, makeError, error norm for kWideFcImgs images by a cluster of kWideFcSlices blocks, each of which
+// adds up one slice of the S inputs; the partial sums meet in the first block's shared memory.  The FC weights
+// (433 KB at S = 10,816) are read from L2 once per kWideFcImgs images, and a thread's walk over its slice is five or six
+// steps long.  (One block per four images walked all S inputs, 42 dependent rounds of L2 loads: 49 us whatever the
+// batch; this takes 6 us for 333 images.)
+constexpr int kWideFcImgs = 8;
+constexpr int kWideFcSlices = 8;
+constexpr int kWideFcVals = 96;          // kWideFcImgs * kOut sums, padded to whole warps
 
 template <int FLAVOR>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256) __cluster_dims__(kWideFcSlices, 1, 1)
 k_wide_fc_fwd(WideDims d, long n, const float* __restrict__ as, const float* __restrict__ params,
               const unsigned* __restrict__ labels, float* __restrict__ out, int* __restrict__ argmax,
               float* __restrict__ delta_f, float* __restrict__ err) {
-  __shared__ float red[8][kWideFcImgs][kOut];
+  __shared__ float red[8][kWideFcVals];
+  __shared__ float part[kWideFcSlices][kWideFcVals];       // the first block's: one row per slice
   __shared__ float o_s[kWideFcImgs][kOut];
-  const long b0 = (long)blockIdx.x * kWideFcImgs;
+  cg::cluster_group cluster = cg::this_cluster();
+  const int slice = (int)cluster.block_rank();
+  const long b0 = (long)(blockIdx.x / kWideFcSlices) * kWideFcImgs;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int imgs = (int)((n - b0) < kWideFcImgs ? (n - b0) : kWideFcImgs);
-  float acc[kWideFcImgs][kOut];
+  const int s_end = (int)((long)d.S * (slice + 1) / kWideFcSlices);
+  f32x2 acc[kWideFcImgs][kOut / 2];
 #pragma unroll
   for (int g = 0; g < kWideFcImgs; ++g)
 #pragma unroll
-    for (int k = 0; k < kOut; ++k) acc[g][k] = 0.f;
-  for (int s = threadIdx.x; s < d.S; s += blockDim.x) {
-    float wv[kOut];
+    for (int k = 0; k < kOut / 2; ++k) acc[g][k] = pack2(0.f, 0.f);
+  for (int s = (int)((long)d.S * slice / kWideFcSlices) + threadIdx.x; s < s_end; s += blockDim.x) {
+    f32x2 wv[kOut / 2];
 #pragma unroll
-    for (int k = 0; k < kOut; ++k) wv[k] = params[d.o_wf + (size_t)k * d.S + s];
+    for (int k = 0; k < kOut / 2; ++k)
+      wv[k] = pack2(params[d.o_wf + (size_t)(2 * k) * d.S + s], params[d.o_wf + (size_t)(2 * k + 1) * d.S + s]);
 #pragma unroll
     for (int g = 0; g < kWideFcImgs; ++g) {
-      const float v = (g < imgs) ? as[(size_t)(b0 + g) * d.S + s] : 0.f;
+      const float v = as[(size_t)(b0 + (g < imgs ? g : 0)) * d.S + s];       // (sums of images past the batch are not used)
+      const f32x2 v2 = pack2(v, v);
 #pragma unroll
-      for (int k = 0; k < kOut; ++k) acc[g][k] = fmaf(wv[k], v, acc[g][k]);
+      for (int k = 0; k < kOut / 2; ++k) acc[g][k] = fma2(wv[k], v2, acc[g][k]);
     }
   }
 #pragma unroll
-  for (int m = 16; m > 0; m >>= 1)
+  for (int c = 0; c < kWideFcVals / 32; ++c) {       // 32 sums at a time: lane l ends with sum 32 c + l = image * 10 + k
+    float v[32];
 #pragma unroll
-    for (int g = 0; g < kWideFcImgs; ++g)
-#pragma unroll
-      for (int k = 0; k < kOut; ++k) acc[g][k] += __shfl_xor_sync(0xffffffffu, acc[g][k], m);
-  if (lane == 0) {
-#pragma unroll
-    for (int g = 0; g < kWideFcImgs; ++g)
-#pragma unroll
-      for (int k = 0; k < kOut; ++k) red[warp][g][k] = acc[g][k];
+    for (int i = 0; i < 32; i += 2) {
+      const int e = 32 * c + i;
+      if (e < kWideFcImgs * kOut) unpack2(acc[e / kOut][(e % kOut) / 2], v[i], v[i + 1]);
+      else v[i] = v[i + 1] = 0.f;
+    }
+    red[warp][32 * c + lane] = warp_reduce_scatter32(v, lane);
   }
   __syncthreads();
+  if (threadIdx.x < kWideFcVals) {
+    float z = 0.f;
+#pragma unroll
+    for (int ww = 0; ww < 8; ++ww) z += red[ww][threadIdx.x];
+    cluster.map_shared_rank(&part[0][0], 0)[slice * kWideFcVals + threadIdx.x] = z;
+  }
+  cluster.sync();
+  if (slice != 0) return;
   if (threadIdx.x < kWideFcImgs * kOut) {
     const int g = threadIdx.x / kOut, k = threadIdx.x % kOut;
     float z = 0.f;
-    for (int ww = 0; ww < 8; ++ww) z += red[ww][g][k];
+#pragma unroll
+    for (int c = 0; c < kWideFcSlices; ++c) z += part[c][threadIdx.x];
     const float o = sigmoidf<FLAVOR>(z + params[d.o_bf + k]);
     o_s[g][k] = o;
     if (g < imgs) {
@@ -149,205 +263,199 @@ k_wide_fc_fwd(WideDims d, long n, const float* __restrict__ as, const float* __r
 }
 
 // ---- backward --------------------------------------------------------------------------------
-// delta_s[b][s] = (sum_k Wf[k][s] delta_f[b][k]) * as (1 - as).  Thread = one s for kWideBpImgs images: the ten
-// weights of s stay in registers, the images' output deltas come from shared memory.
-constexpr int kWideBpImgs = 8;
-
-__global__ void __launch_bounds__(256)
-k_wide_bp_s1(WideDims d, long n, const float* __restrict__ as, const float* __restrict__ delta_f,
-             const float* __restrict__ params, float* __restrict__ ds) {
-  __shared__ float dlt[kWideBpImgs][kOut];
-  const long b0 = (long)blockIdx.x * kWideBpImgs;     // images along x (no 65,535 limit), the S range along y
-  const int imgs = (int)((n - b0) < kWideBpImgs ? (n - b0) : kWideBpImgs);
-  if (threadIdx.x < kWideBpImgs * kOut) {
-    const int g = threadIdx.x / kOut, k = threadIdx.x % kOut;
-    dlt[g][k] = (g < imgs) ? delta_f[(b0 + g) * kOut + k] : 0.f;
-  }
-  __syncthreads();
-  const int s = blockIdx.y * blockDim.x + threadIdx.x;
-  if (s >= d.S) return;
-  float wv[kOut];
-#pragma unroll
-  for (int k = 0; k < kOut; ++k) wv[k] = params[d.o_wf + (size_t)k * d.S + s];
-#pragma unroll
-  for (int g = 0; g < kWideBpImgs; ++g) {
-    if (g < imgs) {
-      float acc = 0.f;
-#pragma unroll
-      for (int k = 0; k < kOut; ++k) acc = fmaf(wv[k], dlt[g][k], acc);
-      const size_t idx = (size_t)(b0 + g) * d.S + s;
-      const float a = as[idx];
-      ds[idx] = acc * a * (1.f - a);
-    }
-  }
-}
-
-// G_wf[k][s] = sum_b delta_f[b][k] as[b][s].  The batch is cut into kWideFcSplit contiguous slices
-// (blockIdx.y); each thread owns one s for one slice and writes a partial, and k_wide_grad_fc_sum adds
-// the slices in order, so the result does not depend on scheduling.  Also G_bf.
+// The FC layer's part of the backward pass in one pass over the subsample activations:
+//   delta_s[b][s] = (sum_k Wf[k][s] delta_f[b][k]) * as (1 - as)      (bp_output_s1, bp_preact_s1)
+//   G_wf[k][s]    = sum_b delta_f[b][k] as[b][s]                      (bp_weight_f)
+// Thread = one s; the batch is cut into kWideFcSplit contiguous slices (blockIdx.y), each of which writes partial sums of
+// G_wf that k_wide_reduce adds in order, so the result does not depend on scheduling.  The ten weights and ten sums stay
+// in registers, the images' output deltas come from shared memory.  Bound by memory: as in, ds out (88 MB for 1,024 images of
+// S = 10,816; two kernels that each read as took 65 us, this one 30).
 constexpr int kWideFcSplit = 16;
+constexpr int kWideBpImgs = 64;          // images whose output deltas are staged at a time
 
-__global__ void k_wide_grad_fc(WideDims d, long n, const float* __restrict__ as, const float* __restrict__ delta_f,
-                               float* __restrict__ part_f) {
+__global__ void __launch_bounds__(128)
+k_wide_bp_fc(WideDims d, long n, const float* __restrict__ as, const float* __restrict__ delta_f,
+             const float* __restrict__ params, float* __restrict__ ds, float* __restrict__ part_f) {
+  __shared__ __align__(16) float dlt[kWideBpImgs][12];
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
+  const bool live = s < d.S;
   const long b0 = (n * blockIdx.y) / kWideFcSplit, b1 = (n * (blockIdx.y + 1)) / kWideFcSplit;
-  if (s >= d.S) return;
-  float acc[kOut];
+  f32x2 acc[kOut / 2], wv[kOut / 2];
 #pragma unroll
-  for (int k = 0; k < kOut; ++k) acc[k] = 0.f;
-  for (long b = b0; b < b1; ++b) {
-    const float v = as[b * d.S + s];
-#pragma unroll
-    for (int k = 0; k < kOut; ++k) acc[k] = fmaf(delta_f[b * kOut + k], v, acc[k]);
+  for (int k = 0; k < kOut / 2; ++k) {
+    acc[k] = pack2(0.f, 0.f);
+    wv[k] = live ? pack2(params[d.o_wf + (size_t)(2 * k) * d.S + s], params[d.o_wf + (size_t)(2 * k + 1) * d.S + s]) : pack2(0.f, 0.f);
   }
+  for (long c0 = b0; c0 < b1; c0 += kWideBpImgs) {
+    const int imgs = (int)((b1 - c0) < kWideBpImgs ? (b1 - c0) : kWideBpImgs);
+    __syncthreads();
+    for (int i = threadIdx.x; i < imgs * kOut; i += blockDim.x) dlt[i / kOut][i % kOut] = delta_f[c0 * kOut + i];
+    __syncthreads();
+    if (!live) continue;
+    const float* src = as + (size_t)c0 * d.S + s;
+    float* dst = ds + (size_t)c0 * d.S + s;
+#pragma unroll 4
+    for (int g = 0; g < imgs; ++g) {
+      const float a = src[(size_t)g * d.S];
+      const f32x2 a2 = pack2(a, a);
+      const ulonglong2 d0 = *reinterpret_cast<const ulonglong2*>(&dlt[g][0]), d1 = *reinterpret_cast<const ulonglong2*>(&dlt[g][4]);
+      const f32x2 dk[kOut / 2] = {d0.x, d0.y, d1.x, d1.y, *reinterpret_cast<const f32x2*>(&dlt[g][8])};
+      f32x2 sum = mul2(wv[0], dk[0]);
 #pragma unroll
-  for (int k = 0; k < kOut; ++k) part_f[((size_t)blockIdx.y * kOut + k) * d.S + s] = acc[k];
-}
-
-__global__ void k_wide_grad_fc_sum(WideDims d, long n, const float* __restrict__ part_f,
-                                   const float* __restrict__ delta_f, float* __restrict__ G) {
-  const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;   // over kOut * S
-  if (i < (long)kOut * d.S) {
-    float sum = 0.f;
+      for (int k = 1; k < kOut / 2; ++k) sum = fma2(wv[k], dk[k], sum);
 #pragma unroll
-    for (int c = 0; c < kWideFcSplit; ++c) sum += part_f[(size_t)c * kOut * d.S + i];
-    G[d.o_wf + i] = sum;
-  }
-  // G_bf: the warps of the last block add delta_f[.][k] for k = warp, warp + warps, ... (lane l takes images
-  // l, l + 32, ...; fixed shuffle tree)
-  if (blockIdx.x == gridDim.x - 1) {
-    const int lane = threadIdx.x & 31;
-    for (int k = threadIdx.x >> 5; k < kOut; k += (int)(blockDim.x >> 5)) {
-      float acc = 0.f;
-      for (long b = lane; b < n; b += 32) acc += delta_f[b * kOut + k];
-#pragma unroll
-      for (int m = 16; m > 0; m >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, m);
-      if (lane == 0) G[d.o_bf + k] = acc;
+      for (int k = 0; k < kOut / 2; ++k) acc[k] = fma2(dk[k], a2, acc[k]);
+      float lo, hi;
+      unpack2(sum, lo, hi);
+      dst[(size_t)g * d.S] = (lo + hi) * a * (1.f - a);
     }
   }
-}
-
-// Per image: 16 subsample-filter gradient partials + bias partial -> part[b][17]; also writes the
-// conv deltas dc = Ws[i][j] * delta_s * a (1 - a) / (C*C).  Block = one image, thread strides over
-// (f, p, q).
-__global__ void __launch_bounds__(256)
-k_wide_bp_c1(WideDims d, const float* __restrict__ ac, const float* __restrict__ ds,
-             const float* __restrict__ params, float* __restrict__ dc, float* __restrict__ part) {
-  __shared__ float red[8][17];
-  const int b = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const float inv_c = 1.0f / (float)(d.C * d.C), inv_s = 1.0f / (float)d.S;
-  float ws[16];
+  if (!live) return;
 #pragma unroll
-  for (int t = 0; t < 16; ++t) ws[t] = params[d.o_ws + t];
-  float acc[17];
-#pragma unroll
-  for (int t = 0; t < 17; ++t) acc[t] = 0.f;
-  for (int s = threadIdx.x; s < d.S; s += blockDim.x) {
-    const int q = s % d.P, p = (s / d.P) % d.P, f = s / (d.P * d.P);
-    const float dlt = ds[(size_t)b * d.S + s];
-    const size_t base = ((size_t)b * d.F + f) * d.C * d.C + (4 * p) * d.C + 4 * q;
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float a = ac[base + i * d.C + j];
-        acc[i * 4 + j] = fmaf(dlt, a, acc[i * 4 + j]);
-        dc[base + i * d.C + j] = (ws[i * 4 + j] * dlt) * a * (1.f - a) * inv_c;
-      }
-    acc[16] += dlt * inv_s;
-  }
-#pragma unroll
-  for (int m = 16; m > 0; m >>= 1)
-#pragma unroll
-    for (int t = 0; t < 17; ++t) acc[t] += __shfl_xor_sync(0xffffffffu, acc[t], m);
-  if (lane == 0) {
-#pragma unroll
-    for (int t = 0; t < 17; ++t) red[warp][t] = acc[t];
-  }
-  __syncthreads();
-  if (threadIdx.x < 17) {
-    float sum = 0.f;
-    for (int ww = 0; ww < 8; ++ww) sum += red[ww][threadIdx.x];
-    part[(size_t)b * 17 + threadIdx.x] = sum;
-  }
-  // positions outside the 4P x 4P area (only when C is not a multiple of 4) get no delta
-  if (4 * d.P != d.C) {
-    for (int o = threadIdx.x; o < d.F * d.C * d.C; o += blockDim.x) {
-      const int x = o % d.C, y = (o / d.C) % d.C;
-      if (y >= 4 * d.P || x >= 4 * d.P) dc[(size_t)b * d.F * d.C * d.C + o] = 0.f;
-    }
+  for (int k = 0; k < kOut / 2; ++k) {
+    float lo, hi;
+    unpack2(acc[k], lo, hi);
+    part_f[((size_t)blockIdx.y * kOut + 2 * k) * d.S + s] = lo;
+    part_f[((size_t)blockIdx.y * kOut + 2 * k + 1) * d.S + s] = hi;
   }
 }
 
-// Conv weight gradient partial of one image for 4 maps: part[b][f][26] (25 taps + bias term).
-__global__ void __launch_bounds__(256)
-k_wide_grad_c1(WideDims d, const float* __restrict__ images, const float* __restrict__ dc,
-               float* __restrict__ part) {
-  extern __shared__ float sh[];
-  float* img = sh;                                  // H*H
-  float* red = sh + d.H * d.H;                      // 8 warps * 4 maps * 26
-  const int b = blockIdx.x, f0 = blockIdx.y * kWideGg;
+// Conv deltas, conv weight and bias gradient and subsample-filter gradient of two maps for a slice of the batch (fp32 SIMT):
+//   dc = Ws[i][j] * delta_s * a (1 - a) / (C*C)       (bp_output_s1, bp_preact_c1)
+//   G_wc[f][u][v] = sum dc[y][x] * image[y + u][x + v], G_bc[f] = sum dc, G_ws[i][j] = sum delta_s * a
+// Thread = one window after another of the slice's images, the two maps in the halves of packed registers, all sums in
+// registers until the end: the deltas never exist in memory.  The patch goes by row by row as in the forward kernel.
+// Bound by the FMA pipe (400 FMAs per window and map for the weight gradient alone); 128 images of 56x56 with 64 maps: 62 us
+// (a kernel that wrote the deltas and one that read them back per map and image: 108 + 200 us).
+// Partial rows: part_c[slice][F][26], part_s[slice * pairs + pair][17].
+template <bool VEC>
+__global__ void __launch_bounds__(kWideWinThreads, 3)
+k_wide_grad_win(WideDims d, long n, const float* __restrict__ images, const float* __restrict__ ac,
+                const float* __restrict__ ds, const float* __restrict__ params, float* __restrict__ part_c,
+                float* __restrict__ part_s) {
+  __shared__ __align__(16) f32x2 ws2[16];
+  __shared__ float red[kWideWinThreads / 32][3][32];
+  const int f = 2 * blockIdx.x, slices = gridDim.y;
+  const bool second = f + 1 < d.F;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (int i = threadIdx.x; i < d.H * d.H; i += blockDim.x) img[i] = images[(size_t)b * d.H * d.H + i];
+  const float inv_c = 1.0f / (float)(d.C * d.C), inv_s = 1.0f / (float)d.S;
+  if (threadIdx.x < 16) ws2[threadIdx.x] = pack2(params[d.o_ws + threadIdx.x], params[d.o_ws + threadIdx.x]);
   __syncthreads();
-  const int CC = d.C * d.C;
-  float acc[kWideGg][26];
+  const int W = d.P * d.P;
+  const size_t CC = (size_t)d.C * d.C;
+  const long b0 = (n * blockIdx.y) / slices, b1 = (n * (blockIdx.y + 1)) / slices;
+  const long units = (b1 - b0) * W;
+  f32x2 acc[26];
+  float gs[17];
 #pragma unroll
-  for (int g = 0; g < kWideGg; ++g)
+  for (int t = 0; t < 26; ++t) acc[t] = pack2(0.f, 0.f);
 #pragma unroll
-    for (int t = 0; t < 26; ++t) acc[g][t] = 0.f;
-  for (int o = threadIdx.x; o < CC; o += blockDim.x) {
-    const int y = o / d.C, x = o % d.C;
-    float dv[kWideGg];
+  for (int t = 0; t < 17; ++t) gs[t] = 0.f;
+  const f32x2 one2 = pack2(1.f, 1.f), minus2 = pack2(-1.f, -1.f);
+#pragma unroll 1
+  for (long t = threadIdx.x; t < units; t += kWideWinThreads) {
+    const long bl = t / W;
+    const int w = (int)(t - bl * W), p = w / d.P, q = w - p * d.P;
+    const long b = b0 + bl;
+    const float dl0 = ds[(size_t)(b * d.F + f) * W + w], dl1 = second ? ds[(size_t)(b * d.F + f + 1) * W + w] : 0.f;
+    const f32x2 dl2 = pack2(dl0 * inv_c, dl1 * inv_c);
+    const float* a_at = ac + (size_t)(b * d.F + f) * CC + (size_t)(4 * p) * d.C + 4 * q;
+    const size_t to_second = second ? CC : 0;      // (without a second map the first is read twice: its delta is zero)
+    f32x2 dc[4][4];
 #pragma unroll
-    for (int g = 0; g < kWideGg; ++g) {
-      dv[g] = (f0 + g < d.F) ? dc[((size_t)b * d.F + f0 + g) * CC + o] : 0.f;
-      acc[g][25] += dv[g];
-    }
+    for (int y = 0; y < 4; ++y) {
+      float a0[4], a1[4];
+      const float* s0 = a_at + (size_t)y * d.C;
+      if (VEC) {
+        const float4 u = *reinterpret_cast<const float4*>(s0), v = *reinterpret_cast<const float4*>(s0 + to_second);
+        a0[0] = u.x; a0[1] = u.y; a0[2] = u.z; a0[3] = u.w;
+        a1[0] = v.x; a1[1] = v.y; a1[2] = v.z; a1[3] = v.w;
+      } else {
 #pragma unroll
-    for (int i = 0; i < 5; ++i)
-#pragma unroll
-      for (int j = 0; j < 5; ++j) {
-        const float v = img[(y + i) * d.H + x + j];
-#pragma unroll
-        for (int g = 0; g < kWideGg; ++g) acc[g][i * 5 + j] = fmaf(dv[g], v, acc[g][i * 5 + j]);
+        for (int x = 0; x < 4; ++x) { a0[x] = s0[x]; a1[x] = s0[to_second + x]; }
       }
-  }
 #pragma unroll
-  for (int g = 0; g < kWideGg; ++g)
-#pragma unroll
-    for (int t = 0; t < 26; ++t) {
-      float v = acc[g][t];
-#pragma unroll
-      for (int m = 16; m > 0; m >>= 1) v += __shfl_xor_sync(0xffffffffu, v, m);
-      if (lane == 0) red[(warp * kWideGg + g) * 26 + t] = v;
+      for (int x = 0; x < 4; ++x) {
+        const f32x2 a2 = pack2(a0[x], a1[x]);
+        gs[4 * y + x] = fmaf(dl1, a1[x], fmaf(dl0, a0[x], gs[4 * y + x]));
+        dc[y][x] = mul2(mul2(ws2[4 * y + x], dl2), mul2(a2, fma2(a2, minus2, one2)));
+        acc[25] = add2(acc[25], dc[y][x]);
+      }
     }
+    gs[16] += (dl0 + dl1) * inv_s;
+    const float* src = images + ((size_t)b * d.H + 4 * p) * d.H + 4 * q;
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+      float v[8];
+      load_row8<VEC>(src + r * d.H, v);
+      f32x2 v2[8];
+#pragma unroll
+      for (int c = 0; c < 8; ++c) v2[c] = pack2(v[c], v[c]);
+#pragma unroll
+      for (int y = 0; y < 4; ++y) {
+        const int i = r - y;                 // tap row
+        if (i < 0 || i > 4) continue;
+#pragma unroll
+        for (int x = 0; x < 4; ++x)
+#pragma unroll
+          for (int j = 0; j < 5; ++j) acc[i * 5 + j] = fma2(dc[y][x], v2[x + j], acc[i * 5 + j]);
+      }
+    }
+  }
+  // block sums, in a fixed order: lane t ends with value t of map f, of map f + 1 and of the filter gradient
+  float v0[32], v1[32], vs[32];
+#pragma unroll
+  for (int t = 0; t < 32; ++t) {
+    v0[t] = v1[t] = 0.f;
+    if (t < 26) unpack2(acc[t < 26 ? t : 0], v0[t], v1[t]);
+    vs[t] = t < 17 ? gs[t < 17 ? t : 0] : 0.f;
+  }
+  red[warp][0][lane] = warp_reduce_scatter32(v0, lane);
+  red[warp][1][lane] = warp_reduce_scatter32(v1, lane);
+  red[warp][2][lane] = warp_reduce_scatter32(vs, lane);
   __syncthreads();
-  if (threadIdx.x < kWideGg * 26) {
-    const int g = threadIdx.x / 26, t = threadIdx.x % 26;
-    float sum = 0.f;
-    for (int ww = 0; ww < 8; ++ww) sum += red[(ww * kWideGg + g) * 26 + t];
-    if (f0 + g < d.F) part[((size_t)b * d.F + f0 + g) * 26 + t] = sum;
+  if (threadIdx.x < 96) {
+    const int m = warp;
+    const float sum = (red[0][m][lane] + red[1][m][lane]) + (red[2][m][lane] + red[3][m][lane]);
+    if (m < 2) {
+      if (lane < 26 && f + m < d.F) part_c[((size_t)blockIdx.y * d.F + f + m) * 26 + lane] = sum;
+    } else if (lane < 17) {
+      part_s[((size_t)blockIdx.y * gridDim.x + blockIdx.x) * 17 + lane] = sum;
+    }
   }
 }
 
-// Sum the partials into the arena-ordered gradient; G[n_params+1] = sum of the per-image error norms;
-// padding zeroed.  One warp per output value: lane l adds rows l, l + 32, ... in order, then the lanes
+// The gradient vector from the partials; G[n_params+1] = sum of the per-image error norms;
+// padding zeroed.  First `value_blocks` blocks: one warp per output value (conv filters and biases, subsample filter and bias,
+// FC biases, error): lane l adds rows l, l + 32, ... in order, then the lanes
 // are combined by a fixed shuffle tree (the same order every run).  (One thread per value walking up
-// to 1,024 rows took 79 us of a 1.3 ms step.)
+// to 1,024 rows took 79 us of a 1.3 ms step.)  The other blocks: one thread per FC weight adds the batch slices.
 __global__ void __launch_bounds__(256)
 k_wide_reduce(WideDims d, long n, long rows_c, long rows_s, const float* __restrict__ part_c,
-              const float* __restrict__ part_s, const float* __restrict__ err, float* __restrict__ G) {
+              const float* __restrict__ part_s, const float* __restrict__ part_f, const float* __restrict__ delta_f,
+              const float* __restrict__ err, int value_blocks, float* __restrict__ G) {
+  if ((int)blockIdx.x >= value_blocks) {
+    const long i = (long)(blockIdx.x - value_blocks) * blockDim.x + threadIdx.x;   // over kOut * S
+    if (i < (long)kOut * d.S) {
+      float sum = 0.f;
+#pragma unroll
+      for (int c = 0; c < kWideFcSplit; ++c) sum += part_f[(size_t)c * kOut * d.S + i];
+      G[d.o_wf + i] = sum;
+    }
+    return;
+  }
   const int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   const int n_c = d.F * 26;
-  if (t > n_c + 17) return;
+  if (t > n_c + 17 + kOut) return;
   const float* src;
   long rows, stride;
   if (t < n_c) { src = part_c + t; rows = rows_c; stride = n_c; }
   else if (t < n_c + 17) { src = part_s + (t - n_c); rows = rows_s; stride = 17; }
+  else if (t < n_c + 17 + kOut) { src = delta_f + (t - n_c - 17); rows = n; stride = kOut; }
   else { src = err; rows = n; stride = 1; }
   float sum = 0.f;
+#pragma unroll 4
   for (long b = lane; b < rows; b += 32) sum += src[(size_t)b * stride];
 #pragma unroll
   for (int m = 16; m > 0; m >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, m);
@@ -358,6 +466,8 @@ k_wide_reduce(WideDims d, long n, long rows_c, long rows_s, const float* __restr
   } else if (t < n_c + 17) {
     const int k = t - n_c;
     if (k < 16) G[d.o_ws + k] = sum; else G[d.o_bs] = sum;
+  } else if (t < n_c + 17 + kOut) {
+    G[d.o_bf + t - n_c - 17] = sum;
   } else {
     G[d.n_params + 1] = sum;
     G[d.n_params] = 0.f;
@@ -376,23 +486,38 @@ using namespace cnn;
 
 static int wide_reserve(cnn_wide* w, long n) {
   if (n <= w->cap) return CNN_OK;
-  float** bufs[] = {&w->ac, &w->dc, &w->as, &w->ds, &w->delta_f, &w->err, &w->part_c, &w->part_s, &w->img_shift};
+  float** bufs[] = {&w->ac, &w->as, &w->ds, &w->delta_f, &w->err, &w->part_c, &w->part_s, &w->img_shift};
   for (float** p : bufs) { cudaFree(*p); *p = nullptr; }
   w->cap = 0;
   const WideDims& d = w->d;
   const size_t fcc = (size_t)d.F * d.C * d.C;
   CNN_CUDA(cudaMalloc(&w->ac, sizeof(float) * fcc * n));
-  CNN_CUDA(cudaMalloc(&w->dc, sizeof(float) * fcc * n));
   CNN_CUDA(cudaMalloc(&w->as, sizeof(float) * (size_t)d.S * n));
   CNN_CUDA(cudaMalloc(&w->ds, sizeof(float) * (size_t)d.S * n));
   CNN_CUDA(cudaMalloc(&w->delta_f, sizeof(float) * kOut * n));
   CNN_CUDA(cudaMalloc(&w->err, sizeof(float) * n));
   w->part_rows = n > 4096 ? n : 4096;
   CNN_CUDA(cudaMalloc(&w->part_c, sizeof(float) * (size_t)d.F * 26 * w->part_rows));
-  CNN_CUDA(cudaMalloc(&w->part_s, sizeof(float) * 17 * w->part_rows));   // one row per image, or per CTA of the fused kernel
+  CNN_CUDA(cudaMalloc(&w->part_s, sizeof(float) * 17 * w->part_rows));   // one row per block of the backward kernels
   if (wide_grad_tc_supported(d)) CNN_CUDA(cudaMalloc(&w->img_shift, sizeof(float) * 4 * (size_t)d.H * d.H * n));
   if (!w->part_f) CNN_CUDA(cudaMalloc(&w->part_f, sizeof(float) * (size_t)kWideFcSplit * kOut * d.S));
   w->cap = n;
+  return CNN_OK;
+}
+
+template <int FL, bool STORE, bool VEC>
+static int launch_conv_s1(cnn_wide* w, const float* d_images, long n, cudaStream_t st) {
+  const WideDims& d = w->d;
+  const long blocks = (n * d.P * d.P + kWideWinThreads - 1) / kWideWinThreads;
+  // Maps per block: as many as keep four waves of four blocks per SM, so that a block's set-up (its taps) is shared and the
+  // last wave is short; at least two (a packed pair).
+  int maps = d.F;
+  while (maps > 2 && blocks * ((d.F + maps - 1) / maps) < 16L * sm_count()) maps = (maps / 2 + 1) / 2 * 2;
+  const int pairs = (maps + 1) / 2;
+  const size_t smem = sizeof(float) * (size_t)(pairs * (kWideTapStride * 2 + 2) + 32);
+  CNN_CUDA(cudaFuncSetAttribute(k_wide_conv_s1<FL, STORE, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  k_wide_conv_s1<FL, STORE, VEC><<<dim3((unsigned)blocks, (unsigned)((d.F + maps - 1) / maps)), kWideWinThreads, smem, st>>>(
+      d, n, maps, d_images, w->d_params, w->ac, w->as);
   return CNN_OK;
 }
 
@@ -400,18 +525,19 @@ template <int FL>
 static int wide_forward_impl(cnn_wide* w, const float* d_images, const unsigned* d_labels, long n, float* d_out,
                              int* d_argmax, bool training, cudaStream_t st) {
   const WideDims& d = w->d;
-  const size_t smem = sizeof(float) * ((size_t)d.H * d.H + kWideFg * 25 + kWideFg);
-  CNN_CUDA(cudaFuncSetAttribute(k_wide_conv_fwd<FL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  int rc;
   if (w->conv_mode > 0 && wide_conv_tc_supported(d)) {
-    const int rc = wide_conv_fwd_tc(w, d_images, n, st);
-    if (rc != CNN_OK) return rc;
+    if ((rc = wide_conv_fwd_tc(w, d_images, n, st)) != CNN_OK) return rc;
+    const long ns = n * d.S;
+    k_wide_s1_fwd<FL><<<(unsigned)((ns + 255) / 256), 256, 0, st>>>(d, n, w->ac, w->d_params, w->as);
   } else {
-    k_wide_conv_fwd<FL><<<dim3((unsigned)n, (d.F + kWideFg - 1) / kWideFg), 256, smem, st>>>(d, d_images, w->d_params, w->ac);
+    const bool vec = d.H % 4 == 0 && (reinterpret_cast<uintptr_t>(d_images) & 15u) == 0;
+    if (vec) rc = training ? launch_conv_s1<FL, true, true>(w, d_images, n, st) : launch_conv_s1<FL, false, true>(w, d_images, n, st);
+    else rc = training ? launch_conv_s1<FL, true, false>(w, d_images, n, st) : launch_conv_s1<FL, false, false>(w, d_images, n, st);
+    if (rc != CNN_OK) return rc;
   }
-  const long ns = n * d.S;
-  k_wide_s1_fwd<FL><<<(unsigned)((ns + 255) / 256), 256, 0, st>>>(d, n, w->ac, w->d_params, w->as);
-  k_wide_fc_fwd<FL><<<(unsigned)((n + kWideFcImgs - 1) / kWideFcImgs), 256, 0, st>>>(d, n, w->as, w->d_params, d_labels, d_out, d_argmax,
-                                                 training ? w->delta_f : nullptr, training ? w->err : nullptr);
+  k_wide_fc_fwd<FL><<<(unsigned)((n + kWideFcImgs - 1) / kWideFcImgs * kWideFcSlices), 256, 0, st>>>(
+      d, n, w->as, w->d_params, d_labels, d_out, d_argmax, training ? w->delta_f : nullptr, training ? w->err : nullptr);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e, "wide forward launch");
   return CNN_OK;
@@ -452,7 +578,7 @@ int cnn_wide_create(int H, int F, cnn_wide** out) {
 
 int cnn_wide_destroy(cnn_wide* w) {
   if (!w) return CNN_OK;
-  float* bufs[] = {w->d_params, w->ac, w->dc, w->as, w->ds, w->delta_f, w->err, w->part_c, w->part_s, w->img_shift};
+  float* bufs[] = {w->d_params, w->ac, w->as, w->ds, w->delta_f, w->err, w->part_c, w->part_s, w->img_shift};
   for (float* p : bufs) cudaFree(p);
   cudaFree(w->d_status);
   cudaFree(w->part_f);
@@ -525,24 +651,32 @@ int cnn_wide_grad_batch(cnn_wide* w, const float* d_images, const unsigned int* 
   int rc = wide_reserve(w, n);
   if (rc != CNN_OK) return rc;
   if ((rc = wide_forward_dispatch(w, d_images, d_labels, n, nullptr, nullptr, true, st)) != CNN_OK) return rc;
-  k_wide_bp_s1<<<dim3((unsigned)((n + kWideBpImgs - 1) / kWideBpImgs), (unsigned)((d.S + 255) / 256)), 256, 0, st>>>(
-      d, n, w->as, w->delta_f, w->d_params, w->ds);
-  k_wide_grad_fc<<<dim3((d.S + 127) / 128, kWideFcSplit), 128, 0, st>>>(d, n, w->as, w->delta_f, w->part_f);
-  k_wide_grad_fc_sum<<<(unsigned)(((long)kOut * d.S + 255) / 256), 256, 0, st>>>(d, n, w->part_f, w->delta_f, d_grad);
-  long rows_c = n, rows_s = n;
+  k_wide_bp_fc<<<dim3((d.S + 127) / 128, kWideFcSplit), 128, 0, st>>>(d, n, w->as, w->delta_f, w->d_params, w->ds, w->part_f);
+  long rows_c, rows_s;
   if (w->conv_mode > 0 && wide_grad_tc_supported(d)) {
     // conv deltas, conv weight gradient and subsample-filter gradient in one kernel; the deltas stay on chip
     int rows = 0;
     if ((rc = wide_grad_c1_tc(w, d_images, n, &rows, st)) != CNN_OK) return rc;
     rows_c = rows_s = rows;
   } else {
-    k_wide_bp_c1<<<(unsigned)n, 256, 0, st>>>(d, w->ac, w->ds, w->d_params, w->dc, w->part_s);
-    const size_t smem = sizeof(float) * ((size_t)d.H * d.H + 8 * kWideGg * 26);
-    CNN_CUDA(cudaFuncSetAttribute(k_wide_grad_c1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k_wide_grad_c1<<<dim3((unsigned)n, (d.F + kWideGg - 1) / kWideGg), 256, smem, st>>>(d, d_images, w->dc, w->part_c);
+    // slices of the batch: three blocks per SM and map pair would fit; two waves of them
+    const int pairs = (d.F + 1) / 2;
+    long slices = (6L * sm_count() + pairs - 1) / pairs;
+    if (slices > n) slices = n;
+    if (slices * pairs > w->part_rows) slices = w->part_rows / pairs;
+    if (d.H % 4 == 0 && (reinterpret_cast<uintptr_t>(d_images) & 15u) == 0)
+      k_wide_grad_win<true><<<dim3(pairs, (unsigned)slices), kWideWinThreads, 0, st>>>(d, n, d_images, w->ac, w->ds, w->d_params,
+                                                                                      w->part_c, w->part_s);
+    else
+      k_wide_grad_win<false><<<dim3(pairs, (unsigned)slices), kWideWinThreads, 0, st>>>(d, n, d_images, w->ac, w->ds, w->d_params,
+                                                                                       w->part_c, w->part_s);
+    rows_c = slices;
+    rows_s = slices * pairs;
   }
-  const int n_red = d.F * 26 + 18;       // one warp each
-  k_wide_reduce<<<(n_red + 7) / 8, 256, 0, st>>>(d, n, rows_c, rows_s, w->part_c, w->part_s, w->err, d_grad);
+  const int value_blocks = (d.F * 26 + 18 + kOut + 7) / 8;       // one warp each
+  const int weight_blocks = (kOut * d.S + 255) / 256;
+  k_wide_reduce<<<value_blocks + weight_blocks, 256, 0, st>>>(d, n, rows_c, rows_s, w->part_c, w->part_s, w->part_f, w->delta_f,
+                                                              w->err, value_blocks, d_grad);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e, "wide backward launch");
   return CNN_OK;

@@ -26,7 +26,7 @@ struct cnn_wide {
   cnn::WideDims d;
   float* d_params = nullptr;
   long cap = 0;                 // images the workspace holds
-  float *ac = nullptr, *dc = nullptr, *as = nullptr, *ds = nullptr, *delta_f = nullptr, *err = nullptr;
+  float *ac = nullptr, *as = nullptr, *ds = nullptr, *delta_f = nullptr, *err = nullptr;
   float *part_c = nullptr, *part_s = nullptr;
   float* img_shift = nullptr;   // [cap][4][H][H]: every image shifted left by 0..3 columns (16-byte aligned tap windows)
   float* part_f = nullptr;      // FC weight-gradient partials of the batch slices
