@@ -165,13 +165,15 @@ def _check(rc: int) -> None:
 
 
 def _ptr(x) -> Optional[int]:
-    """Device/host address of a torch tensor, numpy array, int or None."""
+    """Device/host address of a torch tensor, numpy array, int or None.  (Tensors first, by one attribute
+    look-up: a call with three of them spends less time here than in the launch it makes.)"""
     if x is None:
         return None
+    data_ptr = getattr(x, "data_ptr", None)
+    if data_ptr is not None:
+        return data_ptr()
     if isinstance(x, int):
         return x
-    if hasattr(x, "data_ptr"):
-        return int(x.data_ptr())
     if isinstance(x, np.ndarray):
         return int(x.ctypes.data)
     if isinstance(x, C.c_void_p):
@@ -315,6 +317,9 @@ class Net:
         h = _P()
         _check(lib.cnn_net_create(seed, C.byref(h)))
         self._h = h
+        # the entry points that are called per batch, looked up once
+        self._forward, self._forward_u8 = lib.cnn_forward_batched, lib.cnn_forward_batched_u8
+        self._grad_batch, self._apply_update = lib.cnn_grad_batch, lib.cnn_apply_update
 
     # -- parameters ---------------------------------------------------------------------------
     def set_params(self, params) -> None:
@@ -358,8 +363,9 @@ class Net:
     def forward(self, d_images, n: int, d_out=None, d_argmax=None, stream=None) -> None:
         """Fused batched forward on device buffers: images [n,28,28] fp32 -> out [n,10] fp32,
         argmax [n] int32."""
-        _check(load_library().cnn_forward_batched(self._h, _ptr(d_images), int(n), _ptr(d_out),
-                                                  _ptr(d_argmax), _stream(stream)))
+        rc = self._forward(self._h, _ptr(d_images), int(n), _ptr(d_out), _ptr(d_argmax), _stream(stream))
+        if rc:
+            _check(rc)
 
     def forward_host(self, h_images, n: int, h_out=None, h_argmax=None) -> None:
         """Same through host buffers (pinned memory gives asynchronous copies)."""
@@ -369,8 +375,9 @@ class Net:
     def forward_u8(self, d_pixels, n: int, d_out=None, d_argmax=None, stream=None) -> None:
         """Fused forward on uint8 pixels [n,28,28] (IDX storage); same results as ``forward`` on
         ``pixels / 255.0``."""
-        _check(load_library().cnn_forward_batched_u8(self._h, _ptr(d_pixels), int(n), _ptr(d_out),
-                                                     _ptr(d_argmax), _stream(stream)))
+        rc = self._forward_u8(self._h, _ptr(d_pixels), int(n), _ptr(d_out), _ptr(d_argmax), _stream(stream))
+        if rc:
+            _check(rc)
 
     def forward_u8_host(self, h_pixels, n: int, h_out=None, h_argmax=None) -> None:
         _check(load_library().cnn_forward_batched_u8_host(self._h, _ptr(h_pixels), int(n), _ptr(h_out),
@@ -380,12 +387,15 @@ class Net:
     def grad_batch(self, d_images, d_labels, n: int, d_grad, stream=None) -> None:
         """Summed per-sample gradients of n images at the current parameters into d_grad
         (2368 floats: arena order, then zero padding; d_grad[2344] = sum of ||delta_f||_2)."""
-        _check(load_library().cnn_grad_batch(self._h, _ptr(d_images), _ptr(d_labels), int(n),
-                                             _ptr(d_grad), _stream(stream)))
+        rc = self._grad_batch(self._h, _ptr(d_images), _ptr(d_labels), int(n), _ptr(d_grad), _stream(stream))
+        if rc:
+            _check(rc)
 
     def apply_update(self, d_grad, scale: float, stream=None) -> None:
         """params += scale * d_grad[0:2343]."""
-        _check(load_library().cnn_apply_update(self._h, _ptr(d_grad), float(scale), _stream(stream)))
+        rc = self._apply_update(self._h, _ptr(d_grad), float(scale), _stream(stream))
+        if rc:
+            _check(rc)
 
     def train_minibatch(self, d_images, d_labels, n: int, batch: int, epochs: int, dt: float = 0.1,
                         d_mean_err=None, stream=None) -> None:

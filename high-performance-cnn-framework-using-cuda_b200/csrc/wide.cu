@@ -87,6 +87,11 @@ k_wide_conv_s1(WideDims d, long n, int maps_per_block, const float* __restrict__
     for (int y = 0; y < 4; ++y)
 #pragma unroll
       for (int x = 0; x < 4; ++x) acc[y][x] = bp;
+    f32x2 z = pack2(0.f, 0.f);
+    const ulonglong2* wsp = reinterpret_cast<const ulonglong2*>(ws);
+    const int f = f0 + 2 * pr;
+    const bool second = 2 * pr + 1 < maps;
+    const size_t ac_at = STORE ? ((size_t)(b * d.F + f) * d.C + 4 * p) * d.C + 4 * q : 0;
 #pragma unroll
     for (int r = 0; r < 8; ++r) {
       float v[8];
@@ -103,44 +108,40 @@ k_wide_conv_s1(WideDims d, long n, int maps_per_block, const float* __restrict__
 #pragma unroll
           for (int x = 0; x < 4; ++x) acc[y][x] = fma2(wt[i * 5 + j], v2[x + j], acc[y][x]);
       }
-    }
-    f32x2 z = pack2(0.f, 0.f);
-    const ulonglong2* wsp = reinterpret_cast<const ulonglong2*>(ws);
-    const int f = f0 + 2 * pr;
-    const bool second = 2 * pr + 1 < maps;
-    const size_t ac_at = STORE ? ((size_t)(b * d.F + f) * d.C + 4 * p) * d.C + 4 * q : 0;
+      // output row r - 4 is complete: its sigmoids (special-function unit) go under the next rows' FMAs
+      if (r >= 4) {
+        const int y = r - 4;
+        float a0[4], a1[4];
 #pragma unroll
-    for (int y = 0; y < 4; ++y) {
-      float a0[4], a1[4];
-#pragma unroll
-      for (int x = 0; x < 4; ++x) {
-        float u0, u1;
-        unpack2(acc[y][x], u0, u1);
-        if (FLAVOR == 1) {
-          a0[x] = rcp_approx(1.0f + exp2f_approx(u0));
-          a1[x] = rcp_approx(1.0f + exp2f_approx(u1));
-        } else {
-          a0[x] = sigmoidf<FLAVOR>(u0);
-          a1[x] = sigmoidf<FLAVOR>(u1);
+        for (int x = 0; x < 4; ++x) {
+          float u0, u1;
+          unpack2(acc[y][x], u0, u1);
+          if (FLAVOR == 1) {
+            a0[x] = rcp_approx(1.0f + exp2f_approx(u0));
+            a1[x] = rcp_approx(1.0f + exp2f_approx(u1));
+          } else {
+            a0[x] = sigmoidf<FLAVOR>(u0);
+            a1[x] = sigmoidf<FLAVOR>(u1);
+          }
         }
-      }
 #pragma unroll
-      for (int x = 0; x < 4; x += 2) {
-        const ulonglong2 w2 = wsp[(4 * y + x) / 2];
-        z = fma2(w2.x, pack2(a0[x], a1[x]), z);
-        z = fma2(w2.y, pack2(a0[x + 1], a1[x + 1]), z);
-      }
-      if (STORE) {
-        float* dst = ac + ac_at + (size_t)y * d.C;
-        float* dst1 = dst + (size_t)d.C * d.C;
-        if (VEC) {
-          *reinterpret_cast<float4*>(dst) = make_float4(a0[0], a0[1], a0[2], a0[3]);
-          if (second) *reinterpret_cast<float4*>(dst1) = make_float4(a1[0], a1[1], a1[2], a1[3]);
-        } else {
+        for (int x = 0; x < 4; x += 2) {
+          const ulonglong2 w2 = wsp[(4 * y + x) / 2];
+          z = fma2(w2.x, pack2(a0[x], a1[x]), z);
+          z = fma2(w2.y, pack2(a0[x + 1], a1[x + 1]), z);
+        }
+        if (STORE) {
+          float* dst = ac + ac_at + (size_t)y * d.C;
+          float* dst1 = dst + (size_t)d.C * d.C;
+          if (VEC) {
+            *reinterpret_cast<float4*>(dst) = make_float4(a0[0], a0[1], a0[2], a0[3]);
+            if (second) *reinterpret_cast<float4*>(dst1) = make_float4(a1[0], a1[1], a1[2], a1[3]);
+          } else {
 #pragma unroll
-          for (int x = 0; x < 4; ++x) {
-            dst[x] = a0[x];
-            if (second) dst1[x] = a1[x];
+            for (int x = 0; x < 4; ++x) {
+              dst[x] = a0[x];
+              if (second) dst1[x] = a1[x];
+            }
           }
         }
       }

@@ -393,3 +393,26 @@ def test_tensor_core_forward_operand_range(cuda, pkg, params0, what, n):
     keep = ~np.isnan(outs[0][0]).any(axis=1)
     assert keep.sum() == n - (len(set(spots)) if what == "not a number" else 0)
     assert rel_err(outs[1][0][keep], outs[0][0][keep]) < 1e-5
+
+
+@pytest.mark.parametrize("fast", [0, 1])
+@pytest.mark.parametrize("n", [2, 297, 888, 889, 895, 2073])
+def test_cuda_core_forward_around_its_dispatch(cuda, pkg, params0, n, fast):
+    """The one-image kernel (up to six images per SM) and the tile kernel above it, at one image more than the resident
+    blocks, at the dispatch line, at a ragged last tile and at one tile more than a round, fp32 and uint8.  Reference: the
+    tensor-core kernel, which is checked against the oracle."""
+    pix = pkg.synth.synth_pixels_u8(43, n)
+    images = pkg.synth.u8_to_float(pix)
+    net = pkg.Net(0)
+    net.set_params(params0)
+    net.set_fast_sigmoid(fast)
+    net.set_option("forward_path", 1)
+    ref, _ = run_forward(cuda, net, images)
+    net.set_option("forward_path", 0)
+    out, arg = run_forward(cuda, net, images)
+    assert rel_err(out, ref) < 1e-5 and np.array_equal(arg, np.argmax(out, axis=1).astype(np.int32))
+    d_pix = cuda.from_numpy(pix).cuda()
+    d_out = cuda.empty((n, 10), dtype=cuda.float32, device="cuda")
+    net.forward_u8(d_pix, n, d_out, None)
+    cuda.cuda.synchronize()
+    assert net.status() == 0 and np.array_equal(d_out.cpu().numpy(), out)
