@@ -12,7 +12,7 @@
 //    semantics (output delta without sigmoid derivative, every backward product from pre-update
 //    weights, biases and weights stepped by dt), per-epoch mean of ||delta_f||_2, early stop.
 //
-// Decomposition (both kernels): thread (f, window) owns one 4x4 subsample window of one feature
+// Decomposition of k_train_persample: thread (f, window) owns one 4x4 subsample window of one feature
 // map: 16 conv outputs (400 FMA forward, 400 FMA for the conv weight gradient), so conv
 // activations, their deltas and the 25 weight-gradient partials stay in registers.  216 threads
 // are live in a 224-thread block.
@@ -158,176 +158,330 @@ __device__ __forceinline__ void thread_backward(const TrSmem& sm, const FwdRegs&
     }
 }
 
+// After the call lane l holds, for the index scatter8_index(l), the sum of v[index] over the lanes that agree with it in bit 0
+// (lane bits 4, 3 and 2 pick the index, bit 1 is summed last; lanes that differ in bit 1 hold the same sum).
+__device__ __forceinline__ float reduce_scatter8(float (&v)[8], int lane) {
+#pragma unroll
+  for (int keep = 4; keep >= 1; keep >>= 1) {
+    const int mask = keep << 2;          // 16, 8, 4
+    const bool upper = (lane & mask) != 0;
+#pragma unroll
+    for (int i = 0; i < keep; ++i) {
+      const float send = upper ? v[i] : v[i + keep], stay = upper ? v[i + keep] : v[i];
+      v[i] = stay + __shfl_xor_sync(0xffffffffu, send, mask);
+    }
+  }
+  return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 2);
+}
+__device__ __forceinline__ int scatter8_index(int lane) { return ((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1); }
+
 // ----------------------------------------------------------------------------------------------
 // Minibatch gradient: one partial row per block.
 // Row layout (kRowStride floats): arena-ordered gradient [0, 2343), zero padding, and at
 // kRowErr the sum over the block's images of ||delta_f||_2.
+//
+// One or two teams of seven warps per block, an image each at a time.  Thread (window, map pair, half) of a team owns two
+// rows of a 4x4 subsample window for two maps, which sit in the halves of packed fp32 registers: 8 x 2 conv outputs on a
+// 6x8 patch (200 packed FMAs forward, 200 for the conv weight gradient), half of the window's ten FC terms.  One barrier
+// per image: the FC sums of the team's warps meet in shared memory, and every warp computes the output layer for itself.
+// The gradient of a team's images stays in registers (26 pairs of conv taps and bias, five pairs of FC weights, eight
+// subsample taps) until the block's reduction at the end (shuffles and shared memory, fixed order, no atomics).
+//
+// Small batches are a chain of latencies, large ones are bound by the FMA pipe (852 cycles of it per warp and image; 318 us for
+// 60,000 images).  Measured: a step of 256 images in a training loop 15.5 -> XXX us, the gradient of 60,000
+// images 1,030 -> XXX us.  (Before: a thread per window and map, scalar, two blocks of seven warps per SM at 128 registers
+// with the patch and all gradient terms in registers, two barriers per image, a row per image up to 296.)
 // ----------------------------------------------------------------------------------------------
+constexpr int kGrThreads = 224;                 // threads of a team: 216 with work
+constexpr int kGrWarps = kGrThreads / 32;
+constexpr int kGrStages = 3;                    // image buffers of a team
+constexpr int kGrRed = 27;                      // pairs per thread in the reduction: 25 taps + bias, padded to an odd number
 
-// MINB = 1: one block per SM, no register cap -- lowest latency, used for small batches.
-// MINB = 2: two blocks per SM at 128 registers -- higher throughput on large batches.
-// EARLY = true (used when every block has one image -- a training step of a few hundred images -- and the
-// predecessor on the stream is this library's own reduce + update kernel of the previous step, which does
-// not touch the images): the first image copies are issued before the wait for the predecessor kernel.  With many images per block that order
-// of the prologue compiles to a slower loop (1.06 against 0.985 ms for 57,344 images), so it is a variant.
-template <int FAST, int MINB, bool EARLY>
-__global__ void __launch_bounds__(kTrThreads, MINB)
+template <int TEAMS>
+struct GrSmem {
+  alignas(16) float img[TEAMS][kGrStages][kImg];
+  alignas(16) float ws[16];
+  alignas(16) f32x2 red[TEAMS * kS][kGrRed];    // conv gradient of every thread
+  alignas(8) float wf[kOut][36][kF];            // FC weights as [k][window][map]
+  alignas(8) float wc[25][kF];                  // taps as [tap][map]
+  alignas(8) float bc[8];
+  float bs[4], bf[12];
+  float part[TEAMS][2][kGrWarps][12];           // FC sums of a warp, by parity of the turn: outputs 0..4 at 0..4, 5..9 at 6..10
+  float red_s[TEAMS * kGrWarps][20];            // subsample-filter gradient of a warp: 16 taps and the bias term
+  float red_f[kS][kOut];                        // two teams: FC gradient of the second
+  float red_b[TEAMS][12];                       // FC bias gradient and error sum of a team
+  unsigned long long full[TEAMS][kGrStages];
+};
+
+// Barrier of one team's threads.
+template <int TEAMS>
+__device__ __forceinline__ void team_sync(int team) {
+  if (TEAMS == 1) __syncthreads();
+  else asm volatile("bar.sync %0, %1;" ::"r"(team + 1), "n"(kGrThreads) : "memory");
+}
+
+template <int FAST, int TEAMS>
+__global__ void __launch_bounds__(kGrThreads * TEAMS, 1)
 k_grad_partials(const float* __restrict__ images, const unsigned* __restrict__ labels, long n,
-                const float* __restrict__ params, float* __restrict__ rows, int* __restrict__ status) {
+                const float* __restrict__ params, float* __restrict__ rows, int* __restrict__ status, int chained) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  TrSmem& sm = *reinterpret_cast<TrSmem*>(smem_raw);
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const bool live = tid < kS;
-  const int s = live ? tid : kS - 1;
-  const int f = s / 36, w = s % 36, p = w / 6, q = w % 6;
+  GrSmem<TEAMS>& sm = *reinterpret_cast<GrSmem<TEAMS>*>(smem_raw);
+  const int team = TEAMS == 1 ? 0 : threadIdx.x / kGrThreads;
+  const int tid = threadIdx.x - team * kGrThreads, warp = tid >> 5, lane = threadIdx.x & 31;
+  constexpr float kPre = (FAST == 1) ? -1.4426950408889634f : 1.0f;   // the short sigmoid form's factor, folded into the conv weights
 
-  // In a training loop this kernel follows the previous step's reduce + update kernel.  Launched with
-  // launch_pdl() it starts while that kernel still runs: the barriers and the first two image copies (the
-  // images are nobody's output) are under way when the parameters become readable.
-  auto issue = [&](int stage, long img) {
-    mbar_expect_tx(&sm.full[stage], kImg * sizeof(float));
-    bulk_g2s(&sm.img[stage][0], images + img * kImg, kImg * sizeof(float), &sm.full[stage]);
+  // Image i of this team is first + i * step.
+  const long first = (long)blockIdx.x + (long)team * gridDim.x, step = (long)TEAMS * gridDim.x;
+  auto issue = [&](int i) {
+    const long im = first + (long)i * step;
+    if (im >= n) return;
+    unsigned long long* bar = &sm.full[team][i % kGrStages];
+    mbar_expect_tx(bar, kImg * sizeof(float));
+    bulk_g2s(&sm.img[team][i % kGrStages][0], images + im * kImg, kImg * sizeof(float), bar);
   };
-  if (EARLY) {
-    pdl_launch_dependents();   // one short-lived block per image: the reduce kernel's blocks may come on board at once
-    if (tid == 0) {
-      mbar_init(&sm.full[0], 1);
-      mbar_init(&sm.full[1], 1);
-      mbar_fence_init();
-      for (int st = 0; st < 2; ++st) {
-        const long im = (long)blockIdx.x + (long)st * gridDim.x;
-        if (im < n) issue(st, im);
-      }
-    }
-    pdl_wait();      // the parameters (and the row buffer this kernel writes at its end) belong to the predecessor until here
-    load_params_to_smem(sm, params, tid);
-    __syncthreads();
-  } else {
-    pdl_wait();
-    load_params_to_smem(sm, params, tid);
-    if (tid == 0) {
-      mbar_init(&sm.full[0], 1);
-      mbar_init(&sm.full[1], 1);
-      mbar_fence_init();
-    }
-    __syncthreads();
-    if (tid == 0) {
-      for (int st = 0; st < 2; ++st) {
-        const long im = (long)blockIdx.x + (long)st * gridDim.x;
-        if (im < n) issue(st, im);
-      }
-    }
+  pdl_launch_dependents();
+  if (tid == 0) {
+    for (int s = 0; s < kGrStages; ++s) mbar_init(&sm.full[team][s], 1);
+    mbar_fence_init();
+    // In a training loop the kernel before this one is the previous step's reduce + update kernel, which does not touch
+    // the images: their copies may leave while it still runs.
+    if (chained)
+      for (int i = 0; i < kGrStages; ++i) issue(i);
   }
+  pdl_wait();      // the parameters (and the row buffer this kernel writes at its end) belong to the predecessor until here
+  if (tid == 0 && !chained)
+    for (int i = 0; i < kGrStages; ++i) issue(i);
+  for (int i = threadIdx.x; i < kOut * kS; i += kGrThreads * TEAMS) {
+    const int k = i / kS, s = i % kS;
+    sm.wf[k][s % 36][s / 36] = params[kOffWf + i];
+  }
+  if (threadIdx.x < kF * 25) sm.wc[threadIdx.x % 25][threadIdx.x / 25] = kPre * params[kOffWc + threadIdx.x];
+  else if (threadIdx.x < 156) sm.bc[threadIdx.x - 150] = kPre * params[kOffBc + threadIdx.x - 150];
+  else if (threadIdx.x < 172) sm.ws[threadIdx.x - 156] = params[kOffWs + threadIdx.x - 156];
+  else if (threadIdx.x == 172) sm.bs[0] = params[kOffBs];
+  else if (threadIdx.x < 183) sm.bf[threadIdx.x - 173] = params[kOffBf + threadIdx.x - 173];
+  __syncthreads();
 
-  float acc_wc[25], acc_ws[16], acc_wf[kOut];
-  float acc_bc = 0.f, acc_bs = 0.f, acc_bf = 0.f, acc_err = 0.f;
+  const bool live = tid < kS;
+  const int half = tid & 1, unit = (live ? tid : 0) >> 1;      // (the eight idle threads shadow thread 0 and add zeros)
+  const int pr = unit / 36, w = unit % 36;
+  const int p = w / 6, q = w % 6;
+  const int at = (4 * p + 2 * half) * kH + 4 * q;
+
+  f32x2 g[26], gf[5];
+  float gs[8], g_bs = 0.f, g_bf = 0.f, err = 0.f;
 #pragma unroll
-  for (int i = 0; i < 25; ++i) acc_wc[i] = 0.f;
+  for (int t = 0; t < 26; ++t) g[t] = pack2(0.f, 0.f);
 #pragma unroll
-  for (int i = 0; i < 16; ++i) acc_ws[i] = 0.f;
+  for (int t = 0; t < 5; ++t) gf[t] = pack2(0.f, 0.f);
 #pragma unroll
-  for (int i = 0; i < kOut; ++i) acc_wf[i] = 0.f;
+  for (int t = 0; t < 8; ++t) gs[t] = 0.f;
+  const f32x2 one2 = pack2(1.f, 1.f), minus2 = pack2(-1.f, -1.f);
+  const float inv_c = 1.0f / (float)(kC * kC);
 
   bool gave_up = false;
   int it = 0;
-  for (long im = blockIdx.x; im < n; im += gridDim.x, ++it) {
-    const int stage = it & 1;
-    mbar_wait_bounded(&sm.full[stage], (unsigned)(it >> 1) & 1u, status, gave_up);
+  for (long im = first; im < n; im += step, ++it) {
     unsigned label = 0;
-    if (warp == 0 && lane < kOut) label = labels[im];
+    if (lane < kOut) label = labels[im];
+    mbar_wait_bounded(&sm.full[team][it % kGrStages], (unsigned)(it / kGrStages) & 1u, status, gave_up);
+    const float* patch = &sm.img[team][it % kGrStages][0] + at;
 
-    FwdRegs r;
-    float pk[kOut];
-    thread_forward<FAST>(sm, &sm.img[stage][0], f, p, q, s, live, r, pk);
-    warp_sum(pk);
-    if (lane == 0) {
+    // ---- forward ------------------------------------------------------------------------------
+    f32x2 a[2][4];
+    {
+      const f32x2 bias2 = *reinterpret_cast<const f32x2*>(&sm.bc[2 * pr]);
 #pragma unroll
-      for (int k = 0; k < kOut; ++k) sm.fc_part[warp][k] = pk[k];
+      for (int x = 0; x < 4; ++x) a[0][x] = a[1][x] = bias2;
     }
-    __syncthreads();  // (A) FC partials visible; every thread has taken its patch
-    if (tid == 0) {
-      const long nx = im + 2L * gridDim.x;
-      if (nx < n) issue(stage, nx);
+#pragma unroll
+    for (int r = 0; r < 6; ++r) {          // patch rows: eight pixels, each in both halves of a register pair
+      const float4 lo = *reinterpret_cast<const float4*>(patch + r * kH), hi = *reinterpret_cast<const float4*>(patch + r * kH + 4);
+      const f32x2 v[8] = {pack2(lo.x, lo.x), pack2(lo.y, lo.y), pack2(lo.z, lo.z), pack2(lo.w, lo.w),
+                          pack2(hi.x, hi.x), pack2(hi.y, hi.y), pack2(hi.z, hi.z), pack2(hi.w, hi.w)};
+#pragma unroll
+      for (int y = 0; y < 2; ++y) {
+        const int i = r - y;               // tap row
+        if (i < 0 || i > 4) continue;
+#pragma unroll
+        for (int j = 0; j < 5; ++j) {
+          const f32x2 wt = *reinterpret_cast<const f32x2*>(&sm.wc[i * 5 + j][2 * pr]);
+#pragma unroll
+          for (int x = 0; x < 4; ++x) a[y][x] = fma2(wt, v[x + j], a[y][x]);
+        }
+      }
+    }
+    f32x2 z2 = pack2(0.f, 0.f);
+#pragma unroll
+    for (int y = 0; y < 2; ++y) {
+      const float4 wrow = *reinterpret_cast<const float4*>(&sm.ws[4 * (2 * half + y)]);
+      const float ws[4] = {wrow.x, wrow.y, wrow.z, wrow.w};
+#pragma unroll
+      for (int x = 0; x < 4; ++x) {
+        float u0, u1;
+        unpack2(a[y][x], u0, u1);
+        a[y][x] = (FAST == 1) ? pack2(rcp_approx(1.0f + exp2f_approx(u0)), rcp_approx(1.0f + exp2f_approx(u1)))
+                              : pack2(sigmoidf<FAST>(u0), sigmoidf<FAST>(u1));
+        z2 = fma2(pack2(ws[x], ws[x]), a[y][x], z2);
+      }
+    }
+    float z0, z1;
+    unpack2(z2, z0, z1);
+    z0 += __shfl_xor_sync(0xffffffffu, z0, 1);
+    z1 += __shfl_xor_sync(0xffffffffu, z1, 1);
+    const float as0 = live ? sigmoidf<FAST>(z0 + sm.bs[0]) : 0.f, as1 = live ? sigmoidf<FAST>(z1 + sm.bs[0]) : 0.f;
+    // FC: output 5 half + j of this window and pair, added over the warp (lane bits 4, 3 and 2 pick one of eight values)
+    float v[8];
+    float2 wk[5];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      v[j] = 0.f;
+      if (j < 5) {
+        wk[j] = *reinterpret_cast<const float2*>(&sm.wf[5 * half + j][w][2 * pr]);
+        v[j] = fmaf(wk[j].x, as0, wk[j].y * as1);
+      }
+    }
+    float (&part)[kGrWarps][12] = sm.part[team][it & 1];
+    const float mine = reduce_scatter8(v, lane);
+    const int idx = scatter8_index(lane);
+    if ((lane & 2) == 0 && idx < 5) part[warp][6 * half + idx] = mine;
+    team_sync<TEAMS>(team);       // the team's sums are in shared memory; every thread is done with the previous image
+    if (tid == 0 && it > 0) issue(it + kGrStages - 1);
+
+    // ---- output layer on lanes 0..9 of every warp -------------------------------------------------
+    float delta = 0.f;
+    if (lane < kOut) {
+      float z = 0.f;
+#pragma unroll
+      for (int ww = 0; ww < kGrWarps; ++ww) z += part[ww][lane < 5 ? lane : lane + 1];
+      const float o = sigmoidf<FAST>(z + sm.bf[lane]);
+      delta = ((label == (unsigned)lane) ? 1.0f : 0.0f) - o;       // makeError
     }
     if (warp == 0) {
-      float d = 0.f;
-      if (lane < kOut) {
-        float z = 0.f;
-#pragma unroll
-        for (int ww = 0; ww < kTrWarps; ++ww) z += sm.fc_part[ww][lane];
-        z += sm.bf[lane];
-        const float o = sigmoidf<FAST>(z);
-        d = ((label == (unsigned)lane) ? 1.0f : 0.0f) - o;
-        sm.delta_f[lane] = d;
-        acc_bf += d;
-      }
-      float sq = d * d;
+      g_bf += delta;
+      float sq = delta * delta;                                    // zero on lanes >= 10
 #pragma unroll
       for (int m = 8; m > 0; m >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, m);
-      // lanes 0..15 hold the sum over lanes 0..15 (lanes 10..15 contributed zero)
-      if (lane == 0) acc_err += sqrtf(sq);
+      err += sqrtf(sq);                                            // (lane 0's is used)
     }
-    __syncthreads();  // (B) delta_f visible
-    float df[kOut];
+
+    // ---- backward -------------------------------------------------------------------------------
+    float das0 = 0.f, das1 = 0.f;
+    const f32x2 as2 = pack2(as0, as1);
 #pragma unroll
-    for (int k = 0; k < kOut; ++k) df[k] = sm.delta_f[k];
-    float delta_s, gws[16], gwc[25], gbc;
-    thread_backward(sm, r, live, df, delta_s, gws, gwc, gbc);
+    for (int j = 0; j < 5; ++j) {
+      const float d = __shfl_sync(0xffffffffu, delta, 5 * half + j);
+      das0 = fmaf(wk[j].x, d, das0);
+      das1 = fmaf(wk[j].y, d, das1);
+      gf[j] = fma2(pack2(d, d), as2, gf[j]);
+    }
+    das0 += __shfl_xor_sync(0xffffffffu, das0, 1);
+    das1 += __shfl_xor_sync(0xffffffffu, das1, 1);
+    const float ds0 = das0 * as0 * (1.f - as0), ds1 = das1 * as1 * (1.f - as1);      // zero in idle threads (as = 0)
+    if (half == 0) g_bs += ds0 + ds1;
+    const f32x2 dsc = pack2(ds0 * inv_c, ds1 * inv_c);
 #pragma unroll
-    for (int k = 0; k < kOut; ++k) acc_wf[k] = fmaf(df[k], live ? r.as : 0.f, acc_wf[k]);
+    for (int y = 0; y < 2; ++y) {
+      const float4 wrow = *reinterpret_cast<const float4*>(&sm.ws[4 * (2 * half + y)]);
+      const float ws[4] = {wrow.x, wrow.y, wrow.z, wrow.w};
 #pragma unroll
-    for (int i = 0; i < 16; ++i) acc_ws[i] += gws[i];
+      for (int x = 0; x < 4; ++x) {
+        float a0, a1;
+        unpack2(a[y][x], a0, a1);
+        gs[4 * y + x] = fmaf(ds1, a1, fmaf(ds0, a0, gs[4 * y + x]));
+        a[y][x] = mul2(mul2(pack2(ws[x], ws[x]), dsc), mul2(a[y][x], fma2(a[y][x], minus2, one2)));    // the conv delta / 576
+        g[25] = add2(g[25], a[y][x]);
+      }
+    }
 #pragma unroll
-    for (int i = 0; i < 25; ++i) acc_wc[i] += gwc[i];
-    acc_bc += gbc;
-    acc_bs += delta_s * (1.0f / (float)kS);
-    // No barrier needed here: the next iteration writes fc_part only after its own forward, and
-    // delta_f only after barrier (A) of the next iteration, which every thread reaches after this
-    // point.
+    for (int r = 0; r < 6; ++r) {
+      const float4 lo = *reinterpret_cast<const float4*>(patch + r * kH), hi = *reinterpret_cast<const float4*>(patch + r * kH + 4);
+      const f32x2 u[8] = {pack2(lo.x, lo.x), pack2(lo.y, lo.y), pack2(lo.z, lo.z), pack2(lo.w, lo.w),
+                          pack2(hi.x, hi.x), pack2(hi.y, hi.y), pack2(hi.z, hi.z), pack2(hi.w, hi.w)};
+#pragma unroll
+      for (int y = 0; y < 2; ++y) {
+        const int i = r - y;               // tap row
+        if (i < 0 || i > 4) continue;
+#pragma unroll
+        for (int x = 0; x < 4; ++x)
+#pragma unroll
+          for (int j = 0; j < 5; ++j) g[i * 5 + j] = fma2(a[y][x], u[x + j], g[i * 5 + j]);
+      }
+    }
   }
-  // With many images per block the reduce kernel is only brought onto the SMs from here on: its blocks wait
-  // for this grid to finish, and while they wait they hold registers that a second gradient block per SM needs.
-  if (!EARLY) pdl_launch_dependents();
 
   // ---- block-level reduction, fixed order ----------------------------------------------------
   float* row = rows + (size_t)blockIdx.x * kRowStride;
   if (live) {
 #pragma unroll
-    for (int k = 0; k < kOut; ++k) row[kOffWf + k * kS + s] = acc_wf[k];
-#pragma unroll
-    for (int i = 0; i < 25; ++i) sm.red_c[s][i] = acc_wc[i];
-    sm.red_c[s][25] = acc_bc;
+    for (int t = 0; t < 26; ++t) sm.red[team * kS + tid][t] = g[t];
   }
   {
-    float v[17];
+    const float mine = reduce_scatter8(gs, lane);
+    if ((lane & 2) == 0) sm.red_s[team * kGrWarps + warp][8 * half + scatter8_index(lane)] = mine;
 #pragma unroll
-    for (int i = 0; i < 16; ++i) v[i] = live ? acc_ws[i] : 0.f;
-    v[16] = live ? acc_bs : 0.f;
-    warp_sum(v);
-    if (lane == 0) {
+    for (int m = 16; m > 0; m >>= 1) g_bs += __shfl_xor_sync(0xffffffffu, g_bs, m);
+    if (lane == 0) sm.red_s[team * kGrWarps + warp][16] = g_bs * (1.0f / (float)kS);
+  }
+  if (warp == 0 && lane < kOut) sm.red_b[team][lane] = g_bf;
+  if (tid == 0) sm.red_b[team][10] = err;
+  if (TEAMS == 2 && team == 1 && live) {
 #pragma unroll
-      for (int i = 0; i < 17; ++i) sm.red_s[warp][i] = v[i];
+    for (int j = 0; j < 5; ++j) unpack2(gf[j], sm.red_f[tid][2 * j], sm.red_f[tid][2 * j + 1]);
+  }
+  __syncthreads();
+  if (team == 0 && live) {
+#pragma unroll
+    for (int j = 0; j < 5; ++j) {
+      float f0, f1;
+      unpack2(gf[j], f0, f1);
+      if (TEAMS == 2) { f0 += sm.red_f[tid][2 * j]; f1 += sm.red_f[tid][2 * j + 1]; }
+      float* dst = row + kOffWf + (5 * half + j) * kS + 2 * pr * 36 + w;
+      dst[0] = f0;
+      dst[36] = f1;
     }
   }
-  if (warp == 0 && lane < kOut) row[kOffBf + lane] = acc_bf;
-  if (tid == 0) row[kRowErr] = acc_err;
-  __syncthreads();
-  if (tid < kF * 26) {
-    const int ff = tid / 26, t = tid % 26;
-    float sum = 0.f;
-    for (int ww = 0; ww < 36; ++ww) sum += sm.red_c[ff * 36 + ww][t];
-    if (t < 25) row[kOffWc + ff * 25 + t] = sum;
-    else row[kOffBc + ff] = sum;
-  } else if (tid >= 192 && tid < 192 + 17) {
-    const int t = tid - 192;
-    float sum = 0.f;
+  // conv taps and biases: 78 pair columns, 2 TEAMS neighbouring threads each, 36 rows per thread
+  constexpr int kPer = 2 * TEAMS;
+  const unsigned group = __ballot_sync(0xffffffffu, threadIdx.x < 3 * 26 * kPer);
+  if (threadIdx.x < 3 * 26 * kPer) {        // (whole warps or none of the shuffled groups: 3 * 26 * kPer is a multiple of kPer)
+    const int col = threadIdx.x / kPer, part = threadIdx.x % kPer;
+    const int cp = col / 26, t = col % 26;
+    const int r0 = (part / 2) * kS + cp * 72 + (part % 2) * 36;      // 72 threads of a team share a pair
+    f32x2 s0 = pack2(0.f, 0.f), s1 = s0, s2 = s0, s3 = s0;
 #pragma unroll
-    for (int ww = 0; ww < kTrWarps; ++ww) sum += sm.red_s[ww][t];
-    if (t < 16) row[kOffWs + t] = sum;
-    else row[kOffBs] = sum;
+    for (int r = 0; r < 36; r += 4) {
+      s0 = add2(s0, sm.red[r0 + r][t]);
+      s1 = add2(s1, sm.red[r0 + r + 1][t]);
+      s2 = add2(s2, sm.red[r0 + r + 2][t]);
+      s3 = add2(s3, sm.red[r0 + r + 3][t]);
+    }
+    float lo, hi;
+    unpack2(add2(add2(s0, s1), add2(s2, s3)), lo, hi);
+#pragma unroll
+    for (int m = kPer / 2; m > 0; m >>= 1) {
+      lo += __shfl_xor_sync(group, lo, m);
+      hi += __shfl_xor_sync(group, hi, m);
+    }
+    if (part == 0) {
+      float* dst = t < 25 ? row + kOffWc + 2 * cp * 25 + t : row + kOffBc + 2 * cp;
+      dst[0] = lo;
+      dst[t < 25 ? 25 : 1] = hi;
+    }
+  } else if (threadIdx.x >= kGrThreads * TEAMS - 32) {      // the last warp: subsample filter and bias, FC biases, error sum, padding
+    if (lane < 17) {
+      float sum = 0.f;
+#pragma unroll
+      for (int ww = 0; ww < TEAMS * kGrWarps; ++ww) sum += sm.red_s[ww][lane];
+      row[lane < 16 ? kOffWs + lane : kOffBs] = sum;
+    } else if (lane < 28) {
+      const float sum = TEAMS == 2 ? sm.red_b[0][lane - 17] + sm.red_b[1][lane - 17] : sm.red_b[0][lane - 17];
+      row[lane < 27 ? kOffBf + lane - 17 : kRowErr] = sum;
+    }
+    // zero the padding so that reductions and collectives over the padded row stay finite
+    for (int i = kNParams + lane; i < kRowStride; i += 32)
+      if (i != kRowErr) row[i] = 0.f;
   }
-  // zero the padding so that reductions and collectives over the padded row stay finite
-  if (tid < kRowStride - kNParams && kNParams + tid != kRowErr) row[kNParams + tid] = 0.f;
 }
 
 // G[i] = sum over rows (fixed order: thirty-two interleaved row groups, then a fixed tree over the
@@ -365,6 +519,8 @@ k_reduce_rows(const float* __restrict__ rows, int n_rows, float* __restrict__ G,
 
 __global__ void k_apply_update(float* __restrict__ params, const float* __restrict__ G, float scale) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  pdl_launch_dependents();
+  pdl_wait();
   if (i < kNParams) params[i] = fmaf(scale, G[i], params[i]);
 }
 
@@ -520,46 +676,39 @@ static int set_smem_attr(K kernel, size_t bytes) {
   return CNN_OK;
 }
 
-int launch_grad_partials(cnn_net* net, const float* d_images, const unsigned* d_labels, long n,
-                                int grid, cudaStream_t st, bool chained) {
-  const size_t smem = sizeof(TrSmem);
+// `grid` blocks (one partial row each) over n images; up to one image per block a block has one team of warps, above two.
+static int launch_grad(const float* d_params, float* rows, int* status, int fast, const float* d_images, const unsigned* d_labels,
+                       long n, int grid, cudaStream_t st, bool chained) {
   int rc;
   cudaError_t le = cudaSuccess;
-#define CNN_LAUNCH_GRAD3(FL, MB, EA)                                                                          \
+#define CNN_LAUNCH_GRAD(FL, TEAMS)                                                                            \
   do {                                                                                                       \
-    if ((rc = set_smem_attr(k_grad_partials<FL, MB, EA>, smem)) != CNN_OK) return rc;                        \
-    le = launch_pdl(k_grad_partials<FL, MB, EA>, dim3(grid), dim3(kTrThreads), smem, st, d_images, d_labels, n, \
-                    (const float*)net->d_params, net->d_partials, net->d_status);                            \
+    if ((rc = set_smem_attr(k_grad_partials<FL, TEAMS>, sizeof(GrSmem<TEAMS>))) != CNN_OK) return rc;         \
+    le = launch_pdl(k_grad_partials<FL, TEAMS>, dim3(grid), dim3(kGrThreads * TEAMS), sizeof(GrSmem<TEAMS>), st, \
+                    d_images, d_labels, n, d_params, rows, status, chained ? 1 : 0);                         \
   } while (0)
-#define CNN_LAUNCH_GRAD(FL)                                   \
-  do {                                                        \
-    const bool early = chained && ((long)grid == n);          \
-    if (grid > sm_count()) {                                  \
-      if (early) CNN_LAUNCH_GRAD3(FL, 2, true);               \
-      else CNN_LAUNCH_GRAD3(FL, 2, false);                    \
-    } else {                                                  \
-      if (early) CNN_LAUNCH_GRAD3(FL, 1, true);               \
-      else CNN_LAUNCH_GRAD3(FL, 1, false);                    \
-    }                                                         \
-  } while (0)
-  if (net->fast_sigmoid) CNN_LAUNCH_GRAD(1);
-  else CNN_LAUNCH_GRAD(0);
+  if (n <= grid) {
+    if (fast) CNN_LAUNCH_GRAD(1, 1);
+    else CNN_LAUNCH_GRAD(0, 1);
+  } else {
+    if (fast) CNN_LAUNCH_GRAD(1, 2);
+    else CNN_LAUNCH_GRAD(0, 2);
+  }
 #undef CNN_LAUNCH_GRAD
-#undef CNN_LAUNCH_GRAD3
+  if (le == cudaSuccess) le = cudaGetLastError();
   if (le != cudaSuccess) return cuda_fail(le, "k_grad_partials launch");
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return cuda_fail(e, "k_grad_partials launch");
   return CNN_OK;
 }
 
-// Blocks of the gradient kernel.  Up to two blocks per SM there is one image per block (a training
-// step of a few hundred images is pure latency: one image per block halves it against two images
-// in sequence on half as many blocks); from 8 images per SM on, two blocks per SM walk the batch.
+int launch_grad_partials(cnn_net* net, const float* d_images, const unsigned* d_labels, long n, int grid, cudaStream_t st,
+                         bool chained) {
+  return launch_grad(net->d_params, net->d_partials, net->d_status, net->fast_sigmoid, d_images, d_labels, n, grid, st, chained);
+}
+
+// Blocks of the gradient kernel: one per SM at most (a block holds two images at a time), so that few rows are left to add.
 int grid_for_batch(long n) {
   const long sms = sm_count();
-  if (n <= 2 * sms) return (int)n;
-  const long cap = (n >= 8 * sms) ? 2 * sms : sms;
-  return (int)cap;
+  return (int)(n < sms ? n : sms);
 }
 
 }  // namespace cnn
@@ -581,20 +730,20 @@ int cnn_grad_batch(cnn_net* net, const float* d_images, const unsigned int* d_la
   CNN_REQUIRE((reinterpret_cast<uintptr_t>(d_images) & 15u) == 0,
               "cnn_grad_batch: image batch must start on a 16-byte boundary");
   const int grid = grid_for_batch(n);
-  int rc = ensure_train_scratch(net, 2 * sm_count());
+  int rc = ensure_train_scratch(net, sm_count());
   if (rc != CNN_OK) return rc;
   if ((rc = launch_grad_partials(net, d_images, d_labels, n, grid, st)) != CNN_OK) return rc;
-  k_reduce_rows<<<(kNParamsPadded + 31) / 32, 32 * kRedGroups, 0, st>>>(net->d_partials, grid, d_grad, nullptr, 0.f,
-                                                           nullptr, 0.f);
-  cudaError_t e = cudaGetLastError();
+  cudaError_t e = launch_pdl(k_reduce_rows, dim3((kNParamsPadded + 31) / 32), dim3(32 * kRedGroups), 0, st,
+                             (const float*)net->d_partials, grid, d_grad, (float*)nullptr, 0.f, (float*)nullptr, 0.f);
+  if (e == cudaSuccess) e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e, "k_reduce_rows launch");
   return CNN_OK;
 }
 
 int cnn_apply_update(cnn_net* net, const float* d_grad, float scale, void* stream) {
   CNN_REQUIRE(net && d_grad, "cnn_apply_update: NULL argument");
-  k_apply_update<<<(kNParams + 255) / 256, 256, 0, as_stream(stream)>>>(net->d_params, d_grad, scale);
-  cudaError_t e = cudaGetLastError();
+  cudaError_t e = launch_pdl(k_apply_update, dim3((kNParams + 255) / 256), dim3(256), 0, as_stream(stream), net->d_params, d_grad, scale);
+  if (e == cudaSuccess) e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e, "k_apply_update launch");
   return CNN_OK;
 }
@@ -608,7 +757,7 @@ int cnn_train_minibatch(cnn_net* net, const float* d_images, const unsigned int*
   CNN_REQUIRE((reinterpret_cast<uintptr_t>(d_images) & 15u) == 0,
               "cnn_train_minibatch: image batch must start on a 16-byte boundary");
   cudaStream_t st = as_stream(stream);
-  int rc = ensure_train_scratch(net, 2 * sm_count());
+  int rc = ensure_train_scratch(net, sm_count());
   if (rc != CNN_OK) return rc;
   if (d_mean_err) CNN_CUDA(cudaMemsetAsync(d_mean_err, 0, sizeof(float) * (size_t)epochs, st));
   for (int e = 0; e < epochs; ++e) {
@@ -638,7 +787,7 @@ int cnn_train_sgd_persample(cnn_net* net, const float* d_images, const unsigned 
   CNN_REQUIRE((reinterpret_cast<uintptr_t>(d_images) & 15u) == 0,
               "cnn_train_sgd_persample: image batch must start on a 16-byte boundary");
   cudaStream_t st = as_stream(stream);
-  int rc = ensure_train_scratch(net, 2 * sm_count());
+  int rc = ensure_train_scratch(net, sm_count());
   if (rc != CNN_OK) return rc;
   // Scratch reuse: d_grad holds the per-epoch means (epochs <= kNParamsPadded) and the epoch count.
   CNN_REQUIRE(epochs <= kNParamsPadded, "cnn_train_sgd_persample: too many epochs");
@@ -697,7 +846,7 @@ constexpr size_t kNoAllocFloats = (size_t)kNoAllocMaxRows * kRowStride + 64;
 static __device__ __align__(256) float g_noalloc_scratch[kNoAllocFloats];
 
 // Set-up, once per device, with that device current: in host code the array's name is only a
-// handle, its device address has to be asked for.  Also raises the kernel's shared-memory limit.
+// handle, its device address has to be asked for.
 static int noalloc_scratch(float** rows) {
   static float* scratch_of_device[64] = {nullptr};
   int dev = -1;
@@ -707,8 +856,6 @@ static int noalloc_scratch(float** rows) {
     float* ptr = nullptr;
     CNN_CUDA(cudaGetSymbolAddress(reinterpret_cast<void**>(&ptr), g_noalloc_scratch));
     CNN_REQUIRE(ptr != nullptr, "cnn_grad_batch_noalloc: no device address for the scratch array");
-    CNN_CUDA(cudaFuncSetAttribute(k_grad_partials<0, 1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)sizeof(TrSmem)));
     scratch_of_device[dev] = ptr;
   }
   *rows = scratch_of_device[dev];
@@ -746,11 +893,10 @@ int cnn_grad_batch_noalloc(const float* d_params, const float* d_images, const u
   // by its block, padding included, so no row needs clearing.  The status word starts at zero when
   // the library is loaded, is only ever set by a wait that ran out, and stays set until
   // cnn_grad_batch_noalloc_status reads and clears it.
-  k_grad_partials<0, 1, false><<<grid, kTrThreads, sizeof(TrSmem), st>>>(d_images, d_labels, n, d_params, rows, status);
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return cuda_fail(e, "k_grad_partials launch (no-alloc)");
-  k_reduce_rows<<<(kNParamsPadded + 31) / 32, 32 * kRedGroups, 0, st>>>(rows, grid, d_grad, nullptr, 0.f, nullptr, 0.f);
-  e = cudaGetLastError();
+  if ((rc = launch_grad(d_params, rows, status, 0, d_images, d_labels, n, grid, st, false)) != CNN_OK) return rc;
+  cudaError_t e = launch_pdl(k_reduce_rows, dim3((kNParamsPadded + 31) / 32), dim3(32 * kRedGroups), 0, st, (const float*)rows, grid,
+                             d_grad, (float*)nullptr, 0.f, (float*)nullptr, 0.f);
+  if (e == cudaSuccess) e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e, "k_reduce_rows launch (no-alloc)");
   return CNN_OK;
 }

@@ -230,8 +230,8 @@ int cnn_train_sgd_persample(cnn_net* net, const float* d_images, const unsigned 
  * (160 rows; every GPU that loads the library holds that memory until the process exits).
  *   - at most 65,536 images per call; larger batches are rejected with CNN_ERR_INVALID (split them:
  *     gradients of sub-batches add);
- *   - the first call on each device looks up the array's device address and raises the kernel's
- *     shared-memory limit; make that first call outside any stream capture;
+ *   - the first call on each device looks up the array's device address; make that first
+ *     call outside any stream capture;
  *   - all calls on one device share the one array (it still holds the previous call's rows), so two
  *     calls whose kernels can overlap on the GPU -- different streams, or different host threads --
  *     race; serialise them on one stream or with events;
