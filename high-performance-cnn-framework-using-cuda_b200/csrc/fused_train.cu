@@ -188,8 +188,9 @@ __device__ __forceinline__ int scatter8_index(int lane) { return ((lane >> 4) & 
 // subsample taps) until the block's reduction at the end (shuffles and shared memory, fixed order, no atomics).
 //
 // Small batches are a chain of latencies, large ones are bound by the FMA pipe (852 cycles of it per warp and image; 318 us for
-// 60,000 images).  Measured: a step of 256 images in a training loop 15.5 -> XXX us, the gradient of 60,000
-// images 1,030 -> XXX us.  (Before: a thread per window and map, scalar, two blocks of seven warps per SM at 128 registers
+// 60,000 images).  Measured: a step of 256 images in a training loop 15.4 -> 9.6 us (of which the
+// parameters 0.7, forward 2.5, backward 1.5, this kernel's reduction 1.2, the row sums 1.2 and the two hand-overs 1.5 us),
+// the gradient of 60,000 images 1,030 -> 640 us.  (Before: a thread per window and map, scalar, two blocks of seven warps per SM at 128 registers
 // with the patch and all gradient terms in registers, two barriers per image, a row per image up to 296.)
 // ----------------------------------------------------------------------------------------------
 constexpr int kGrThreads = 224;                 // threads of a team: 216 with work
@@ -251,22 +252,39 @@ k_grad_partials(const float* __restrict__ images, const unsigned* __restrict__ l
   pdl_wait();      // the parameters (and the row buffer this kernel writes at its end) belong to the predecessor until here
   if (tid == 0 && !chained)
     for (int i = 0; i < kGrStages; ++i) issue(i);
-  for (int i = threadIdx.x; i < kOut * kS; i += kGrThreads * TEAMS) {
-    const int k = i / kS, s = i % kS;
-    sm.wf[k][s % 36][s / 36] = params[kOffWf + i];
+  // Parameters: every load of a thread is under way before the first of them is stored (one L2 latency, not one per
+  // group of loads: 2.4 -> 0.75 us of a step).
+  const bool live = tid < kS;
+  {
+    float wf[kOut / TEAMS], small;
+    const int k0 = team * (kOut / TEAMS);
+#pragma unroll
+    for (int k = 0; k < kOut / TEAMS; ++k) wf[k] = params[kOffWf + (k0 + k) * kS + (live ? tid : 0)];
+    if (team == 0) small = params[tid < kOffWf ? tid : kOffBf + (tid - kOffWf < kOut ? tid - kOffWf : 0)];
+    if (live) {
+#pragma unroll
+      for (int k = 0; k < kOut / TEAMS; ++k) sm.wf[k0 + k][tid % 36][tid / 36] = wf[k];
+    }
+    if (team == 0) {
+      if (tid < kOffBc) sm.wc[tid % 25][tid / 25] = kPre * small;
+      else if (tid < kOffWs) sm.bc[tid - kOffBc] = kPre * small;
+      else if (tid < kOffBs) sm.ws[tid - kOffWs] = small;
+      else if (tid == kOffBs) sm.bs[0] = small;
+      else if (tid < kOffWf + kOut) sm.bf[tid - kOffWf] = small;
+    }
   }
-  if (threadIdx.x < kF * 25) sm.wc[threadIdx.x % 25][threadIdx.x / 25] = kPre * params[kOffWc + threadIdx.x];
-  else if (threadIdx.x < 156) sm.bc[threadIdx.x - 150] = kPre * params[kOffBc + threadIdx.x - 150];
-  else if (threadIdx.x < 172) sm.ws[threadIdx.x - 156] = params[kOffWs + threadIdx.x - 156];
-  else if (threadIdx.x == 172) sm.bs[0] = params[kOffBs];
-  else if (threadIdx.x < 183) sm.bf[threadIdx.x - 173] = params[kOffBf + threadIdx.x - 173];
   __syncthreads();
 
-  const bool live = tid < kS;
   const int half = tid & 1, unit = (live ? tid : 0) >> 1;      // (the eight idle threads shadow thread 0 and add zeros)
   const int pr = unit / 36, w = unit % 36;
   const int p = w / 6, q = w % 6;
   const int at = (4 * p + 2 * half) * kH + 4 * q;
+  // With one team there are registers enough to keep the taps.
+  f32x2 wt[TEAMS == 1 ? 25 : 1];
+  if (TEAMS == 1) {
+#pragma unroll
+    for (int t = 0; t < 25; ++t) wt[TEAMS == 1 ? t : 0] = *reinterpret_cast<const f32x2*>(&sm.wc[t][2 * pr]);
+  }
 
   f32x2 g[26], gf[5];
   float gs[8], g_bs = 0.f, g_bf = 0.f, err = 0.f;
@@ -305,28 +323,29 @@ k_grad_partials(const float* __restrict__ images, const unsigned* __restrict__ l
         if (i < 0 || i > 4) continue;
 #pragma unroll
         for (int j = 0; j < 5; ++j) {
-          const f32x2 wt = *reinterpret_cast<const f32x2*>(&sm.wc[i * 5 + j][2 * pr]);
+          const f32x2 tap = TEAMS == 1 ? wt[TEAMS == 1 ? i * 5 + j : 0] : *reinterpret_cast<const f32x2*>(&sm.wc[i * 5 + j][2 * pr]);
 #pragma unroll
-          for (int x = 0; x < 4; ++x) a[y][x] = fma2(wt, v[x + j], a[y][x]);
+          for (int x = 0; x < 4; ++x) a[y][x] = fma2(tap, v[x + j], a[y][x]);
         }
       }
     }
-    f32x2 z2 = pack2(0.f, 0.f);
+    f32x2 zy[2];
 #pragma unroll
     for (int y = 0; y < 2; ++y) {
       const float4 wrow = *reinterpret_cast<const float4*>(&sm.ws[4 * (2 * half + y)]);
       const float ws[4] = {wrow.x, wrow.y, wrow.z, wrow.w};
+      zy[y] = pack2(0.f, 0.f);
 #pragma unroll
       for (int x = 0; x < 4; ++x) {
         float u0, u1;
         unpack2(a[y][x], u0, u1);
         a[y][x] = (FAST == 1) ? pack2(rcp_approx(1.0f + exp2f_approx(u0)), rcp_approx(1.0f + exp2f_approx(u1)))
                               : pack2(sigmoidf<FAST>(u0), sigmoidf<FAST>(u1));
-        z2 = fma2(pack2(ws[x], ws[x]), a[y][x], z2);
+        zy[y] = fma2(pack2(ws[x], ws[x]), a[y][x], zy[y]);
       }
     }
     float z0, z1;
-    unpack2(z2, z0, z1);
+    unpack2(add2(zy[0], zy[1]), z0, z1);
     z0 += __shfl_xor_sync(0xffffffffu, z0, 1);
     z1 += __shfl_xor_sync(0xffffffffu, z1, 1);
     const float as0 = live ? sigmoidf<FAST>(z0 + sm.bs[0]) : 0.f, as1 = live ? sigmoidf<FAST>(z1 + sm.bs[0]) : 0.f;
@@ -498,10 +517,10 @@ k_reduce_rows(const float* __restrict__ rows, int n_rows, float* __restrict__ G,
   const int col = blockIdx.x * 32 + lane;
   pdl_launch_dependents();   // the next step's gradient kernel may set itself up now
   pdl_wait();                // the rows are complete
-  float acc = 0.f;
+  float acc = 0.f, p_old = 0.f;
   if (col < kRowStride) {
-#pragma unroll 4
-    for (int r = g; r < n_rows; r += kRedGroups) acc += rows[(size_t)r * kRowStride + col];
+    if (params && g == 0 && col < kNParams) p_old = params[col];      // under the row loads
+    acc = sum_rows<kRedGroups>(rows, n_rows, col, g);
   }
   part[g][lane] = acc;
   __syncthreads();
@@ -512,7 +531,7 @@ k_reduce_rows(const float* __restrict__ rows, int n_rows, float* __restrict__ G,
       q[i] = (part[4 * i][lane] + part[4 * i + 1][lane]) + (part[4 * i + 2][lane] + part[4 * i + 3][lane]);
     const float total = ((q[0] + q[1]) + (q[2] + q[3])) + ((q[4] + q[5]) + (q[6] + q[7]));
     if (G) G[col] = total;
-    if (params && col < kNParams) params[col] = fmaf(scale, total, params[col]);
+    if (params && col < kNParams) params[col] = fmaf(scale, total, p_old);
     if (mean_err && col == kRowErr) *mean_err += err_scale * total;
   }
 }

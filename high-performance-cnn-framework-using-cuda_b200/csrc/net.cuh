@@ -111,6 +111,25 @@ __device__ __forceinline__ bool mbar_wait_bounded(unsigned long long* bar, unsig
 constexpr int kRowStride = kNParamsPadded + 8;
 constexpr int kRowErr = kNParams + 1;  // 2344
 
+// Column `col` of rows g, g + GROUPS, g + 2 GROUPS, ... added in that order; five loads at a time are under way (with one
+// row per SM and 32 groups that is all of them).
+template <int GROUPS>
+__device__ __forceinline__ float sum_rows(const float* __restrict__ rows, int n_rows, int col, int g) {
+  float acc = 0.f;
+  for (int r0 = g; r0 < n_rows; r0 += 5 * GROUPS) {
+    float v[5];
+#pragma unroll
+    for (int i = 0; i < 5; ++i) {
+      const int r = r0 + i * GROUPS;
+      v[i] = rows[(size_t)(r < n_rows ? r : g) * kRowStride + col];
+    }
+#pragma unroll
+    for (int i = 0; i < 5; ++i)
+      if (r0 + i * GROUPS < n_rows) acc += v[i];
+  }
+  return acc;
+}
+
 // Batched forward with the convolution on the tensor cores (forward_tc.cu): path 1 or 2; uint8 pixels, path 1.
 int forward_device_tc(cnn_net* net, int path, const float* d_images, long n, float* d_out, int* d_argmax,
                       cudaStream_t stream);

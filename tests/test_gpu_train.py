@@ -339,3 +339,17 @@ def test_reference_trajectory_spread(cuda, pkg, ob, params0):
     drift = scaled_err(net.get_params(), runs[0])
     print("reference-vs-reference spread %.3e, library-vs-reference drift %.3e" % (spread, drift))
     assert drift < max(20 * spread, 1e-4)
+
+
+@pytest.mark.parametrize("n", [295, 296, 297, 1185])
+def test_grad_batch_around_full_rounds(cuda, pkg, ob, params0, n):
+    """Two images per block and turn, three image buffers per team: one image short of a full round, a full one, one image
+    into the next, and a batch whose last turn reuses the buffers with a single live team."""
+    images, labels = pkg.synth.synth_images(37, n)
+    net = pkg.Net(0)
+    net.set_params(params0)
+    g = gpu_grad(cuda, net, images, labels)
+    G, err = ob.grad_batch(params0, images, labels)
+    for name, (lo, hi) in BLOCKS.items():
+        assert scaled_err(g[lo:hi], G[lo:hi]) < 1e-5, name
+    assert abs(g[2344] - err) < 1e-5 * err and g[2343] == 0 and not g[2345:].any()
