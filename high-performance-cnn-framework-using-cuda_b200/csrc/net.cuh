@@ -3,6 +3,10 @@
 
 #include "cnn_common.cuh"
 
+namespace cnn {
+struct HostPipeline;
+}
+
 struct cnn_net {
   int device = 0;
   unsigned seed = 0;               // what cnn_net_create drew the initial parameters from (kept for checkpoints)
@@ -18,13 +22,7 @@ struct cnn_net {
   float* d_partials = nullptr;     // [partial_rows][kNParamsPadded]
   int partial_rows = 0;
   float* d_grad = nullptr;         // kNParamsPadded floats + 8 floats of statistics
-  // Host pipeline staging (allocated on first use).
-  float* d_stage_img[2] = {nullptr, nullptr};
-  float* d_stage_out[2] = {nullptr, nullptr};
-  int* d_stage_arg[2] = {nullptr, nullptr};
-  long stage_images = 0;
-  cudaStream_t copy_stream[2] = {nullptr, nullptr};
-  cudaEvent_t order_event = nullptr;   // host pipeline: ties the two copy streams behind the legacy stream
+  cnn::HostPipeline* host = nullptr;   // host_pipeline.cu (created on first use)
 };
 
 namespace cnn {

@@ -150,12 +150,14 @@ int cnn_net_status(cnn_net* net, int* status);
 int cnn_forward_batched(cnn_net* net, const float* d_images, long n, float* d_out, int* d_argmax,
                         void* stream);
 
-/* Same through host buffers: pipelined pinned-or-pageable H2D of the images in chunks, the fused
+/* Same through host buffers: the images go to the device in chunks (pinned ones from where they lie, pageable ones through
+ * a pinned ring that a few host threads of the library fill), the fused
  * kernel per chunk, D2H of the results; returns after everything has landed.  The pipeline runs on
- * two private streams which are first ordered behind all work queued so far on the legacy default
+ * private streams which are first ordered behind all work queued so far on the legacy default
  * stream (stream NULL: a cnn_apply_update, cnn_train_minibatch or cnn_grad_batch issued there is
  * seen).  Work that updates the parameters on a caller's own non-blocking stream is not waited for:
- * synchronise that stream before this call. */
+ * synchronise that stream before this call.  The threads and the ring (8 MB) are shared by all nets of the process that
+ * have used pageable buffers and go with the last of them. */
 int cnn_forward_batched_host(cnn_net* net, const float* h_images, long n, float* h_out,
                              int* h_argmax);
 

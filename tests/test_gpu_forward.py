@@ -416,3 +416,52 @@ def test_cuda_core_forward_around_its_dispatch(cuda, pkg, params0, n, fast):
     net.forward_u8(d_pix, n, d_out, None)
     cuda.cuda.synchronize()
     assert net.status() == 0 and np.array_equal(d_out.cpu().numpy(), out)
+
+
+@pytest.mark.parametrize("u8", [False, True])
+@pytest.mark.parametrize("n", [41, 200, 1024, 1025, 9001, 17000])
+def test_forward_host_buffers_pageable_and_pinned(cuda, pkg, params0, n, u8):
+    """The host pipeline around its sizes: below and above staging, one and two chunks, pieces that wrap around the ring, a
+    ragged end; pageable and pinned images, pageable and pinned results, either result left out -- always the bits of the
+    device call.  A second net runs the same request from another thread (one of the two finds the copy threads busy)."""
+    import threading
+    pix = pkg.synth.synth_pixels_u8(44, n)
+    images = pix if u8 else pkg.synth.u8_to_float(pix)
+    nets = [pkg.Net(0), pkg.Net(0)]
+    for net in nets:
+        net.set_params(params0)
+    d_img = cuda.from_numpy(images).cuda()
+    d_out = cuda.empty((n, 10), dtype=cuda.float32, device="cuda")
+    d_arg = cuda.empty((n,), dtype=cuda.int32, device="cuda")
+    (nets[0].forward_u8 if u8 else nets[0].forward)(d_img, n, d_out, d_arg)
+    cuda.cuda.synchronize()
+    want, want_arg = d_out.cpu().numpy(), d_arg.cpu().numpy()
+
+    def check(net, img, out, arg):
+        (net.forward_u8_host if u8 else net.forward_host)(img, n, out, arg)
+        assert out is None or np.array_equal(np.asarray(out), want)
+        assert arg is None or np.array_equal(np.asarray(arg), want_arg)
+
+    def pageable():
+        return np.full((n, 10), -1, np.float32), np.full(n, -1, np.int32)
+
+    pinned_img = cuda.from_numpy(images).pin_memory()
+    check(nets[0], images, *pageable())
+    check(nets[0], images, pageable()[0], None)
+    check(nets[0], images, None, pageable()[1])
+    check(nets[0], pinned_img, *pageable())
+    check(nets[0], pinned_img, cuda.empty((n, 10)).pin_memory(), cuda.empty(n, dtype=cuda.int32).pin_memory())
+    failed = []
+
+    def other():
+        try:
+            for _ in range(3):
+                check(nets[1], images, *pageable())
+        except Exception as e:      # reported by the main thread
+            failed.append(e)
+    t = threading.Thread(target=other)
+    t.start()
+    for _ in range(3):
+        check(nets[0], images, *pageable())
+    t.join()
+    assert not failed
