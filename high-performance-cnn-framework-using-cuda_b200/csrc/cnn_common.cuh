@@ -45,6 +45,13 @@ __device__ __forceinline__ float rcp_approx(float x) {
   return y;
 }
 
+// Smaller of two floats; a NaN stays one (fminf returns the other operand).
+__device__ __forceinline__ float min_nan(float a, float b) {
+  float y;
+  asm("min.NaN.f32 %0, %1, %2;" : "=f"(y) : "f"(a), "f"(b));
+  return y;
+}
+
 // Two floats in one 64-bit register pair and the packed fp32 instructions on them (sm_100): one issue slot for two
 // lanes' worth of arithmetic, each half rounded like the scalar instruction.
 typedef unsigned long long f32x2;

@@ -110,20 +110,6 @@ struct TfSmem {
 
 CNN_PHASE_TABLE(g_phase_clocks_tc, 20)
 
-// Eight consecutive fp32 columns of this warp's 32 tensor-memory lanes; not waited for.
-__device__ __forceinline__ void tmem_ld8_nowait(unsigned taddr, unsigned (&r)[8]) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-               : "r"(taddr));
-}
-// Wait for this warp's outstanding tensor-memory loads; the registers are listed as in/out operands
-// so that their uses cannot be scheduled above the wait.
-__device__ __forceinline__ void tmem_wait8(unsigned (&a)[8]) {
-  asm volatile("tcgen05.wait::ld.sync.aligned;"
-               : "+r"(a[0]), "+r"(a[1]), "+r"(a[2]), "+r"(a[3]), "+r"(a[4]), "+r"(a[5]), "+r"(a[6]), "+r"(a[7])
-               :: "memory");
-}
-
 __device__ __forceinline__ float tanh_approx(float x) {
   float y;
   asm("tanh.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -566,8 +552,8 @@ k_forward_tc(const void* __restrict__ images, long n, long imgs_per_cta, const f
         __syncwarp();
         tc::fence_after_sync();
         unsigned nxt[8];
-        tmem_ld8_nowait(t0 + (unsigned)(xb * kTfBN), nxt);
-        tmem_wait8(nxt);
+        tc::tmem_ld8_nowait(t0 + (unsigned)(xb * kTfBN), nxt);
+        tc::tmem_wait8(nxt);
         float z[18];
         f32x2 d2[4];               // the row's four activations before the reciprocal (of two maps), one step behind
         // Step ch turns 8 accumulator columns (window column ch / 3, maps 2 * (ch % 3) + {0, 1}) into exponentials and
@@ -576,13 +562,13 @@ k_forward_tc(const void* __restrict__ images, long n, long imgs_per_cta, const f
         for (int ch = 0; ch < 10; ++ch) {
           f32x2 e2[4];
           if (ch < 9) {
-            if (ch > 0) tmem_wait8(nxt);
+            if (ch > 0) tc::tmem_wait8(nxt);
             // the window row's four columns of two maps: t = unscale * acc + bias
 #pragma unroll
             for (int j = 0; j < 4; ++j)
               e2[j] = fma2(pack2(__uint_as_float(nxt[2 * j]), __uint_as_float(nxt[2 * j + 1])), unscale2, bc2[ch % 3]);
             if (ch < 8) {
-              tmem_ld8_nowait(t0 + (unsigned)(xb * kTfBN + (ch + 1) * 8), nxt);
+              tc::tmem_ld8_nowait(t0 + (unsigned)(xb * kTfBN + (ch + 1) * 8), nxt);
             } else {
               // the last columns of this block are in registers: hand it back to the MMA warp
               tc::fence_before_sync();

@@ -59,6 +59,8 @@ k_wide_conv_s1(WideDims d, long n, int maps_per_block, const float* __restrict__
   float* tap = sh;
   float* ws = tap + (maps_per_block + 1) / 2 * kWideTapStride * 2;
   float* bias = ws + 32;
+  pdl_launch_dependents();
+  pdl_wait();
   for (int i = threadIdx.x; i < pairs * kWideTapStride * 2; i += blockDim.x) {
     const int pr = i / (kWideTapStride * 2), t = (i % (kWideTapStride * 2)) >> 1, f = 2 * pr + (i & 1);
     tap[i] = (t < 25 && f < maps) ? kPre * params[d.o_wc + (f0 + f) * 25 + t] : 0.f;
@@ -153,62 +155,52 @@ k_wide_conv_s1(WideDims d, long n, int maps_per_block, const float* __restrict__
   }
 }
 
-// Thread = one subsample output (b, f, p, q).
-template <int FLAVOR>
-__global__ void k_wide_s1_fwd(WideDims d, long n, const float* __restrict__ ac,
-                              const float* __restrict__ params, float* __restrict__ as) {
-  const long idx = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= n * d.S) return;
-  const int q = (int)(idx % d.P), p = (int)((idx / d.P) % d.P);
-  const long bf = idx / (d.P * d.P);
-  const float* src = ac + (size_t)bf * d.C * d.C + (4 * p) * d.C + 4 * q;
-  float z = 0.f;
-#pragma unroll
-  for (int j = 0; j < 4; ++j)
-#pragma unroll
-    for (int i = 0; i < 4; ++i) z = fmaf(params[d.o_ws + i * 4 + j], src[i * d.C + j], z);
-  as[idx] = sigmoidf<FLAVOR>(z + params[d.o_bs]);
-}
-
-// FC, sigmoid, argmax, makeError, error norm for kWideFcImgs images by a cluster of kWideFcSlices blocks, each of which
-// adds up one slice of the S inputs; the partial sums meet in the first block's shared memory.  The FC weights
-// (433 KB at S = 10,816) are read from L2 once per kWideFcImgs images, and a thread's walk over its slice is five or six
-// steps long.  (One block per four images walked all S inputs, 42 dependent rounds of L2 loads: 49 us whatever the
-// batch; this takes 6 us for 333 images.)
+// FC, sigmoid, argmax, makeError, error norm by clusters of kWideFcSlices blocks, each of which adds up one slice of the S
+// inputs for the cluster's images; the partial sums meet in the first block's shared memory.  A warp has kWideFcImgs
+// images and 8 * 10 sums in registers.  `sets` (1, 2 or 4): groups of images in a block, each of 8 / sets warps that share
+// the slice; the groups walk it at the same time, so the weights (433 KB at S = 10,816) come from L2 once for all of them and
+// from L1 for the others.  One group is the shortest walk (five or six steps): right while the clusters of one group fit the
+// chip at once; four groups have the least traffic.  Bound by L2 latency.
 constexpr int kWideFcImgs = 8;
 constexpr int kWideFcSlices = 8;
 constexpr int kWideFcVals = 96;          // kWideFcImgs * kOut sums, padded to whole warps
+constexpr int kWideFcSets = 4;
 
 template <int FLAVOR>
-__global__ void __launch_bounds__(256) __cluster_dims__(kWideFcSlices, 1, 1)
-k_wide_fc_fwd(WideDims d, long n, const float* __restrict__ as, const float* __restrict__ params,
+__global__ void __launch_bounds__(256, 2) __cluster_dims__(kWideFcSlices, 1, 1)
+k_wide_fc_fwd(WideDims d, long n, int sets, const float* __restrict__ as, const float* __restrict__ wf, const float* __restrict__ params,
               const unsigned* __restrict__ labels, float* __restrict__ out, int* __restrict__ argmax,
               float* __restrict__ delta_f, float* __restrict__ err) {
   __shared__ float red[8][kWideFcVals];
-  __shared__ float part[kWideFcSlices][kWideFcVals];       // the first block's: one row per slice
-  __shared__ float o_s[kWideFcImgs][kOut];
+  __shared__ float part[kWideFcSlices][kWideFcSets * kWideFcVals];       // the first block's: one row per slice
+  __shared__ float o_s[kWideFcSets * kWideFcImgs][kOut];
   cg::cluster_group cluster = cg::this_cluster();
   const int slice = (int)cluster.block_rank();
-  const long b0 = (long)(blockIdx.x / kWideFcSlices) * kWideFcImgs;
+  const long b0 = (long)(blockIdx.x / kWideFcSlices) * sets * kWideFcImgs;     // the cluster's images
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int imgs = (int)((n - b0) < kWideFcImgs ? (n - b0) : kWideFcImgs);
+  const int set = warp % sets, parts = 8 / sets, part_of = warp / sets;
+  const long first = b0 + set * kWideFcImgs;                                   // the warp's images
+  const int imgs = (int)((n - first) < kWideFcImgs ? (n - first) : kWideFcImgs);
   const int s_end = (int)((long)d.S * (slice + 1) / kWideFcSlices);
   f32x2 acc[kWideFcImgs][kOut / 2];
 #pragma unroll
   for (int g = 0; g < kWideFcImgs; ++g)
 #pragma unroll
     for (int k = 0; k < kOut / 2; ++k) acc[g][k] = pack2(0.f, 0.f);
-  for (int s = (int)((long)d.S * slice / kWideFcSlices) + threadIdx.x; s < s_end; s += blockDim.x) {
-    f32x2 wv[kOut / 2];
+  pdl_launch_dependents();
+  pdl_wait();
+  if (imgs > 0) {
+    for (int s = (int)((long)d.S * slice / kWideFcSlices) + part_of * 32 + lane; s < s_end; s += parts * 32) {
+      f32x2 wv[kOut / 2];
 #pragma unroll
-    for (int k = 0; k < kOut / 2; ++k)
-      wv[k] = pack2(params[d.o_wf + (size_t)(2 * k) * d.S + s], params[d.o_wf + (size_t)(2 * k + 1) * d.S + s]);
+      for (int k = 0; k < kOut / 2; ++k) wv[k] = pack2(wf[(size_t)(2 * k) * d.S + s], wf[(size_t)(2 * k + 1) * d.S + s]);
 #pragma unroll
-    for (int g = 0; g < kWideFcImgs; ++g) {
-      const float v = as[(size_t)(b0 + (g < imgs ? g : 0)) * d.S + s];       // (sums of images past the batch are not used)
-      const f32x2 v2 = pack2(v, v);
+      for (int g = 0; g < kWideFcImgs; ++g) {
+        const float v = as[(size_t)(first + (g < imgs ? g : 0)) * d.S + s];       // (sums of images past the batch are not used)
+        const f32x2 v2 = pack2(v, v);
 #pragma unroll
-      for (int k = 0; k < kOut / 2; ++k) acc[g][k] = fma2(wv[k], v2, acc[g][k]);
+        for (int k = 0; k < kOut / 2; ++k) acc[g][k] = fma2(wv[k], v2, acc[g][k]);
+      }
     }
   }
 #pragma unroll
@@ -223,29 +215,28 @@ k_wide_fc_fwd(WideDims d, long n, const float* __restrict__ as, const float* __r
     red[warp][32 * c + lane] = warp_reduce_scatter32(v, lane);
   }
   __syncthreads();
-  if (threadIdx.x < kWideFcVals) {
+  for (int e = threadIdx.x; e < sets * kWideFcVals; e += 256) {
+    const int g = e / kWideFcVals, v = e - g * kWideFcVals;
     float z = 0.f;
-#pragma unroll
-    for (int ww = 0; ww < 8; ++ww) z += red[ww][threadIdx.x];
-    cluster.map_shared_rank(&part[0][0], 0)[slice * kWideFcVals + threadIdx.x] = z;
+    for (int ww = g; ww < 8; ww += sets) z += red[ww][v];
+    cluster.map_shared_rank(&part[0][0], 0)[slice * (kWideFcSets * kWideFcVals) + e] = z;
   }
   cluster.sync();
   if (slice != 0) return;
-  if (threadIdx.x < kWideFcImgs * kOut) {
-    const int g = threadIdx.x / kOut, k = threadIdx.x % kOut;
+  const int total = (int)((n - b0) < sets * kWideFcImgs ? (n - b0) : sets * kWideFcImgs);
+  for (int e = threadIdx.x; e < total * kOut; e += 256) {
+    const int g = e / kOut, k = e % kOut;
     float z = 0.f;
 #pragma unroll
-    for (int c = 0; c < kWideFcSlices; ++c) z += part[c][threadIdx.x];
+    for (int c = 0; c < kWideFcSlices; ++c) z += part[c][g / kWideFcImgs * kWideFcVals + g % kWideFcImgs * kOut + k];
     const float o = sigmoidf<FLAVOR>(z + params[d.o_bf + k]);
     o_s[g][k] = o;
-    if (g < imgs) {
-      const long b = b0 + g;
-      if (out) out[(size_t)b * kOut + k] = o;
-      if (delta_f) delta_f[(size_t)b * kOut + k] = ((labels[b] == (unsigned)k) ? 1.0f : 0.0f) - o;
-    }
+    const long b = b0 + g;
+    if (out) out[(size_t)b * kOut + k] = o;
+    if (delta_f) delta_f[(size_t)b * kOut + k] = ((labels[b] == (unsigned)k) ? 1.0f : 0.0f) - o;
   }
   __syncthreads();
-  if (threadIdx.x < imgs) {
+  if (threadIdx.x < total) {
     const int g = threadIdx.x;
     const long b = b0 + g;
     int best = 0;
@@ -267,6 +258,7 @@ k_wide_fc_fwd(WideDims d, long n, const float* __restrict__ as, const float* __r
 // The FC layer's part of the backward pass in one pass over the subsample activations:
 //   delta_s[b][s] = (sum_k Wf[k][s] delta_f[b][k]) * as (1 - as)      (bp_output_s1, bp_preact_s1)
 //   G_wf[k][s]    = sum_b delta_f[b][k] as[b][s]                      (bp_weight_f)
+// (ds_max, if given: the largest finite |delta_s| of each block.)
 // Thread = one s; the batch is cut into kWideFcSplit contiguous slices (blockIdx.y), each of which writes partial sums of
 // G_wf that k_wide_reduce adds in order, so the result does not depend on scheduling.  The ten weights and ten sums stay
 // in registers, the images' output deltas come from shared memory.  Bound by memory: as in, ds out (88 MB for 1,024 images of
@@ -276,16 +268,20 @@ constexpr int kWideBpImgs = 64;          // images whose output deltas are stage
 
 __global__ void __launch_bounds__(128)
 k_wide_bp_fc(WideDims d, long n, const float* __restrict__ as, const float* __restrict__ delta_f,
-             const float* __restrict__ params, float* __restrict__ ds, float* __restrict__ part_f) {
+             const float* __restrict__ wf, float* __restrict__ ds, float* __restrict__ part_f, float* __restrict__ ds_max) {
   __shared__ __align__(16) float dlt[kWideBpImgs][12];
+  __shared__ float red[4];
+  float most = 0.f;
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   const bool live = s < d.S;
   const long b0 = (n * blockIdx.y) / kWideFcSplit, b1 = (n * (blockIdx.y + 1)) / kWideFcSplit;
   f32x2 acc[kOut / 2], wv[kOut / 2];
+  pdl_launch_dependents();
+  pdl_wait();
 #pragma unroll
   for (int k = 0; k < kOut / 2; ++k) {
     acc[k] = pack2(0.f, 0.f);
-    wv[k] = live ? pack2(params[d.o_wf + (size_t)(2 * k) * d.S + s], params[d.o_wf + (size_t)(2 * k + 1) * d.S + s]) : pack2(0.f, 0.f);
+    wv[k] = live ? pack2(wf[(size_t)(2 * k) * d.S + s], wf[(size_t)(2 * k + 1) * d.S + s]) : pack2(0.f, 0.f);
   }
   for (long c0 = b0; c0 < b1; c0 += kWideBpImgs) {
     const int imgs = (int)((b1 - c0) < kWideBpImgs ? (b1 - c0) : kWideBpImgs);
@@ -308,8 +304,17 @@ k_wide_bp_fc(WideDims d, long n, const float* __restrict__ as, const float* __re
       for (int k = 0; k < kOut / 2; ++k) acc[k] = fma2(dk[k], a2, acc[k]);
       float lo, hi;
       unpack2(sum, lo, hi);
-      dst[(size_t)g * d.S] = (lo + hi) * a * (1.f - a);
+      const float v = (lo + hi) * a * (1.f - a);
+      dst[(size_t)g * d.S] = v;
+      most = fabsf(v) <= 3.4e38f ? fmaxf(most, fabsf(v)) : most;
     }
+  }
+  if (ds_max) {
+#pragma unroll
+    for (int m = 16; m > 0; m >>= 1) most = fmaxf(most, __shfl_xor_sync(0xffffffffu, most, m));
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = most;
+    __syncthreads();
+    if (threadIdx.x == 0) ds_max[blockIdx.y * gridDim.x + blockIdx.x] = fmaxf(fmaxf(red[0], red[1]), fmaxf(red[2], red[3]));
   }
   if (!live) return;
 #pragma unroll
@@ -340,6 +345,8 @@ k_wide_grad_win(WideDims d, long n, const float* __restrict__ images, const floa
   const bool second = f + 1 < d.F;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const float inv_c = 1.0f / (float)(d.C * d.C), inv_s = 1.0f / (float)d.S;
+  pdl_launch_dependents();
+  pdl_wait();
   if (threadIdx.x < 16) ws2[threadIdx.x] = pack2(params[d.o_ws + threadIdx.x], params[d.o_ws + threadIdx.x]);
   __syncthreads();
   const int W = d.P * d.P;
@@ -426,43 +433,88 @@ k_wide_grad_win(WideDims d, long n, const float* __restrict__ images, const floa
   }
 }
 
-// The gradient vector from the partials; G[n_params+1] = sum of the per-image error norms;
-// padding zeroed.  First `value_blocks` blocks: one warp per output value (conv filters and biases, subsample filter and bias,
-// FC biases, error): lane l adds rows l, l + 32, ... in order, then the lanes
-// are combined by a fixed shuffle tree (the same order every run).  (One thread per value walking up
-// to 1,024 rows took 79 us of a 1.3 ms step.)  The other blocks: one thread per FC weight adds the batch slices.
+// The gradient vector from the partials; G[n_params+1] = sum of the per-image error norms; padding zeroed; everything added in a
+// fixed order.  Blocks, in this order:
+//   value_blocks: a warp per output value (SIMT path: conv filters; both: conv biases, subsample filter and bias, FC biases,
+//     error): lane l adds rows l, l + 32, ..., then the lanes are combined by a fixed shuffle tree.  (One thread per value
+//     walking up to 1,024 rows took 79 us of a 1.3 ms step.)
+//   filter_blocks, tensor-core path: (map group, kernel row i, four maps).  The CTAs' D[(x, f)][(i, c)] are added first, 16 bytes
+//     per thread and CTA, eight threads taking every eighth CTA; then G[f][i][j] = sum_x D[(x, f)][(i, x + j)].
+//   the rest: a thread per FC weight adds the batch slices; on the tensor-core path the sums are in [window][map] order.
+template <bool TC>
 __global__ void __launch_bounds__(256)
-k_wide_reduce(WideDims d, long n, long rows_c, long rows_s, const float* __restrict__ part_c,
-              const float* __restrict__ part_s, const float* __restrict__ part_f, const float* __restrict__ delta_f,
-              const float* __restrict__ err, int value_blocks, float* __restrict__ G) {
-  if ((int)blockIdx.x >= value_blocks) {
-    const long i = (long)(blockIdx.x - value_blocks) * blockDim.x + threadIdx.x;   // over kOut * S
+k_wide_reduce(WideDims d, long n, long rows_c, long rows_s, const float* __restrict__ part_c, const float* __restrict__ part_s,
+              const float* __restrict__ part_f, const float* __restrict__ delta_f, const float* __restrict__ err, int value_blocks,
+              int filter_blocks, float* __restrict__ G) {
+  constexpr int kSlices = 8, kTile = 8 * 16;      // of a filter block: CTA slices; 8 c x 16 columns (x, f)
+  __shared__ __align__(16) float sums[TC ? kSlices : 1][TC ? kTile : 1];
+  pdl_launch_dependents();
+  pdl_wait();
+  const int block = blockIdx.x;
+  if (block >= value_blocks + filter_blocks) {
+    const long i = (long)(block - value_blocks - filter_blocks) * blockDim.x + threadIdx.x;   // over kOut * S
     if (i < (long)kOut * d.S) {
       float sum = 0.f;
 #pragma unroll
       for (int c = 0; c < kWideFcSplit; ++c) sum += part_f[(size_t)c * kOut * d.S + i];
-      G[d.o_wf + i] = sum;
+      if (TC) {
+        const int k = (int)(i / d.S), s = (int)(i - (long)k * d.S), w = s / d.F;
+        G[d.o_wf + (size_t)k * d.S + (size_t)(s - w * d.F) * (d.P * d.P) + w] = sum;
+      } else {
+        G[d.o_wf + i] = sum;
+      }
     }
     return;
   }
-  const int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (TC && block >= value_blocks) {
+    const int e = block - value_blocks, quads = kTwF / 4, group = e / (5 * quads), i = e / quads % 5, fq = e % quads;   // maps 4 fq ..
+    const int tile = threadIdx.x % (kTile / 4), slice = threadIdx.x / (kTile / 4);         // tile: four columns of row c = tile / 4
+    const float* src = part_c + (size_t)(group * rows_c) * kTwGradN * kTwGradCols + (size_t)(i * 8 + tile / 4) * kTwGradCols + 16 * fq +
+                       4 * (tile % 4);
+    float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 8
+    for (long c = slice; c < rows_c; c += kSlices) {
+      const float4 v = *reinterpret_cast<const float4*>(src + (size_t)c * kTwGradN * kTwGradCols);
+      sum.x += v.x; sum.y += v.y; sum.z += v.z; sum.w += v.w;
+    }
+    *reinterpret_cast<float4*>(&sums[slice][tile * 4]) = sum;
+    __syncthreads();
+    if (threadIdx.x < 20) {
+      const int m = threadIdx.x / 5, j = threadIdx.x % 5;
+      float g = 0.f;
+#pragma unroll
+      for (int x = 0; x < 4; ++x) {
+        const int at = (x + j) * 16 + 8 * (m >> 1) + 2 * x + (m & 1);
+        for (int c = 0; c < kSlices; ++c) g += sums[c][at];
+      }
+      G[d.o_wc + (group * kTwF + 4 * fq + m) * 25 + i * 5 + j] = g;
+    }
+    return;
+  }
+  const int t = block * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
-  const int n_c = d.F * 26;
+  const int n_c = TC ? d.F : d.F * 26;
   if (t > n_c + 17 + kOut) return;
   const float* src;
   long rows, stride;
-  if (t < n_c) { src = part_c + t; rows = rows_c; stride = n_c; }
-  else if (t < n_c + 17) { src = part_s + (t - n_c); rows = rows_s; stride = 17; }
+  if (t < n_c && TC) { src = part_s + (size_t)(t / kTwF) * rows_c * kTwPartB + t % kTwF; rows = 4 * rows_c; stride = kTwPartB; }
+  else if (t < n_c) { src = part_c + t; rows = rows_c; stride = n_c; }
+  else if (t < n_c + 17) { src = part_s + (TC ? 4 * kTwF : 0) + (t - n_c); rows = rows_s; stride = TC ? kTwPartB : 17; }
   else if (t < n_c + 17 + kOut) { src = delta_f + (t - n_c - 17); rows = n; stride = kOut; }
   else { src = err; rows = n; stride = 1; }
   float sum = 0.f;
+  if (TC && t < n_c) {        // a CTA's conv bias sums: a row for each quarter of its rows
 #pragma unroll 4
-  for (long b = lane; b < rows; b += 32) sum += src[(size_t)b * stride];
+    for (long b = lane; b < rows; b += 32) sum += src[(size_t)(b >> 2) * stride + (b & 3) * kTwF];
+  } else {
+#pragma unroll 4
+    for (long b = lane; b < rows; b += 32) sum += src[(size_t)b * stride];
+  }
 #pragma unroll
   for (int m = 16; m > 0; m >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, m);
   if (lane != 0) return;
   if (t < n_c) {
-    const int f = t / 26, k = t % 26;
+    const int f = TC ? t : t / 26, k = TC ? 25 : t % 26;
     if (k < 25) G[d.o_wc + f * 25 + k] = sum; else G[d.o_bc + f] = sum;
   } else if (t < n_c + 17) {
     const int k = t - n_c;
@@ -485,29 +537,67 @@ __global__ void k_wide_update(int n_params, float* __restrict__ params, const fl
 
 using namespace cnn;
 
-static int wide_reserve(cnn_wide* w, long n) {
-  if (n <= w->cap) return CNN_OK;
-  float** bufs[] = {&w->ac, &w->as, &w->ds, &w->delta_f, &w->err, &w->part_c, &w->part_s, &w->img_shift};
-  for (float** p : bufs) { cudaFree(*p); *p = nullptr; }
-  w->cap = 0;
+// Which kernels a call takes.  The tensor-core path wants whole groups of 64 maps, rows of whole 16-byte pieces (one thread loads
+// eight pixels of a row as two float4) and windows without a remainder; everything else runs on the fp32 path.
+static bool wide_on_tc(const cnn_wide* w, const float* d_images) {
+  return w->conv_mode > 0 && wide_tc_supported(w->d) && (reinterpret_cast<uintptr_t>(d_images) & 15u) == 0;
+}
+
+// Slices of the batch for k_wide_grad_win: three blocks per SM and map pair would fit; two waves of them.
+static long wide_grad_slices(const WideDims& d, long n) {
+  const int pairs = (d.F + 1) / 2;
+  const long slices = (6L * sm_count() + pairs - 1) / pairs;
+  return slices < n ? slices : n;
+}
+
+static int wide_bp_fc_blocks(const WideDims& d) { return (d.S + 127) / 128; }
+
+// Lays the arena out for a call, growing it if it is too small.  One allocation (a cudaMalloc costs about 0.36 ms) of what this
+// call's kernels use: inference keeps no deltas, the tensor-core path no conv activations (2.8 GB for 4,096 images of 56x56 / 64).
+static int wide_reserve(cnn_wide* w, long n, bool training, bool tc, WideWork& k) {
   const WideDims& d = w->d;
-  const size_t fcc = (size_t)d.F * d.C * d.C;
-  CNN_CUDA(cudaMalloc(&w->ac, sizeof(float) * fcc * n));
-  CNN_CUDA(cudaMalloc(&w->as, sizeof(float) * (size_t)d.S * n));
-  CNN_CUDA(cudaMalloc(&w->ds, sizeof(float) * (size_t)d.S * n));
-  CNN_CUDA(cudaMalloc(&w->delta_f, sizeof(float) * kOut * n));
-  CNN_CUDA(cudaMalloc(&w->err, sizeof(float) * n));
-  w->part_rows = n > 4096 ? n : 4096;
-  CNN_CUDA(cudaMalloc(&w->part_c, sizeof(float) * (size_t)d.F * 26 * w->part_rows));
-  CNN_CUDA(cudaMalloc(&w->part_s, sizeof(float) * 17 * w->part_rows));   // one row per block of the backward kernels
-  if (wide_grad_tc_supported(d)) CNN_CUDA(cudaMalloc(&w->img_shift, sizeof(float) * 4 * (size_t)d.H * d.H * n));
-  if (!w->part_f) CNN_CUDA(cudaMalloc(&w->part_f, sizeof(float) * (size_t)kWideFcSplit * kOut * d.S));
-  w->cap = n;
+  for (int pass = 0; pass < 2; ++pass) {          // sizes, then pointers
+    size_t at = 0;
+    auto take = [&](float*& p, size_t floats) {
+      p = pass ? w->arena + at : nullptr;
+      at += (floats + 63) & ~(size_t)63;
+    };
+    take(k.as, (size_t)d.S * n);
+    if (tc) {
+      take(k.pixel_max, kTwPrepBlocks);
+      take(k.wf_t, (size_t)kOut * d.S);
+    }
+    if (training) {
+      take(k.ds, (size_t)d.S * n);
+      take(k.delta_f, (size_t)kOut * n);
+      take(k.err, n);
+      take(k.part_f, (size_t)kWideFcSplit * kOut * d.S);
+      if (tc) {
+        const size_t ctas = (size_t)wide_tc_max_ctas() * (d.F / kTwF);
+        take(k.ds_max, (size_t)wide_bp_fc_blocks(d) * kWideFcSplit);
+        take(k.part_g, ctas * kTwGradN * kTwGradCols);
+        take(k.part_b, ctas * kTwPartB);
+      } else {
+        const size_t slices = wide_grad_slices(d, n);
+        take(k.ac, (size_t)d.F * d.C * d.C * n);
+        take(k.part_c, slices * d.F * 26);
+        take(k.part_s, slices * ((d.F + 1) / 2) * 17);
+      }
+    }
+    k.floats = at;
+    if (!pass && at > w->arena_floats) {
+      cudaFree(w->arena);
+      w->arena = nullptr;
+      w->arena_floats = 0;
+      CNN_CUDA(cudaMalloc(&w->arena, sizeof(float) * at));
+      w->arena_floats = at;
+    }
+  }
   return CNN_OK;
 }
 
 template <int FL, bool STORE, bool VEC>
-static int launch_conv_s1(cnn_wide* w, const float* d_images, long n, cudaStream_t st) {
+static int launch_conv_s1(cnn_wide* w, const WideWork& k, const float* d_images, long n, cudaStream_t st) {
   const WideDims& d = w->d;
   const long blocks = (n * d.P * d.P + kWideWinThreads - 1) / kWideWinThreads;
   // Maps per block: as many as keep four waves of four blocks per SM, so that a block's set-up (its taps) is shared and the
@@ -517,39 +607,42 @@ static int launch_conv_s1(cnn_wide* w, const float* d_images, long n, cudaStream
   const int pairs = (maps + 1) / 2;
   const size_t smem = sizeof(float) * (size_t)(pairs * (kWideTapStride * 2 + 2) + 32);
   CNN_CUDA(cudaFuncSetAttribute(k_wide_conv_s1<FL, STORE, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  k_wide_conv_s1<FL, STORE, VEC><<<dim3((unsigned)blocks, (unsigned)((d.F + maps - 1) / maps)), kWideWinThreads, smem, st>>>(
-      d, n, maps, d_images, w->d_params, w->ac, w->as);
+  cudaError_t e = launch_pdl(k_wide_conv_s1<FL, STORE, VEC>, dim3((unsigned)blocks, (unsigned)((d.F + maps - 1) / maps)),
+                             dim3(kWideWinThreads), smem, st, d, n, maps, d_images, (const float*)w->d_params, k.ac, k.as);
+  if (e != cudaSuccess) return cuda_fail(e, "k_wide_conv_s1 launch");
   return CNN_OK;
 }
 
 template <int FL>
-static int wide_forward_impl(cnn_wide* w, const float* d_images, const unsigned* d_labels, long n, float* d_out,
-                             int* d_argmax, bool training, cudaStream_t st) {
+static int wide_forward_impl(cnn_wide* w, const WideWork& k, bool tc, const float* d_images, const unsigned* d_labels, long n,
+                             float* d_out, int* d_argmax, bool training, cudaStream_t st) {
   const WideDims& d = w->d;
   int rc;
-  if (w->conv_mode > 0 && wide_conv_tc_supported(d)) {
-    if ((rc = wide_conv_fwd_tc(w, d_images, n, st)) != CNN_OK) return rc;
-    const long ns = n * d.S;
-    k_wide_s1_fwd<FL><<<(unsigned)((ns + 255) / 256), 256, 0, st>>>(d, n, w->ac, w->d_params, w->as);
+  if (tc) {
+    rc = wide_tc_forward(w, k, d_images, n, st);
   } else {
     const bool vec = d.H % 4 == 0 && (reinterpret_cast<uintptr_t>(d_images) & 15u) == 0;
-    if (vec) rc = training ? launch_conv_s1<FL, true, true>(w, d_images, n, st) : launch_conv_s1<FL, false, true>(w, d_images, n, st);
-    else rc = training ? launch_conv_s1<FL, true, false>(w, d_images, n, st) : launch_conv_s1<FL, false, false>(w, d_images, n, st);
-    if (rc != CNN_OK) return rc;
+    if (vec) rc = training ? launch_conv_s1<FL, true, true>(w, k, d_images, n, st) : launch_conv_s1<FL, false, true>(w, k, d_images, n, st);
+    else rc = training ? launch_conv_s1<FL, true, false>(w, k, d_images, n, st) : launch_conv_s1<FL, false, false>(w, k, d_images, n, st);
   }
-  k_wide_fc_fwd<FL><<<(unsigned)((n + kWideFcImgs - 1) / kWideFcImgs * kWideFcSlices), 256, 0, st>>>(
-      d, n, w->as, w->d_params, d_labels, d_out, d_argmax, training ? w->delta_f : nullptr, training ? w->err : nullptr);
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return cuda_fail(e, "wide forward launch");
+  if (rc != CNN_OK) return rc;
+  // Groups of images per FC cluster: as few as let all clusters be on the chip at once (two blocks per SM).
+  int sets = 1;
+  while (sets < kWideFcSets && (n + kWideFcImgs * sets - 1) / (kWideFcImgs * sets) * kWideFcSlices > 2L * sm_count()) sets *= 2;
+  const long clusters = (n + kWideFcImgs * sets - 1) / (kWideFcImgs * sets);
+  cudaError_t e = launch_pdl(k_wide_fc_fwd<FL>, dim3((unsigned)(clusters * kWideFcSlices)), dim3(256), 0, st, d, n, sets,
+                             (const float*)k.as, (const float*)(tc ? k.wf_t : w->d_params + d.o_wf), (const float*)w->d_params, d_labels,
+                             d_out, d_argmax, training ? k.delta_f : nullptr, training ? k.err : nullptr);
+  if (e != cudaSuccess) return cuda_fail(e, "k_wide_fc_fwd launch");
   return CNN_OK;
 }
 
-static int wide_forward_dispatch(cnn_wide* w, const float* d_images, const unsigned* d_labels, long n, float* d_out,
-                                 int* d_argmax, bool training, cudaStream_t st) {
+static int wide_forward_dispatch(cnn_wide* w, const WideWork& k, bool tc, const float* d_images, const unsigned* d_labels, long n,
+                                 float* d_out, int* d_argmax, bool training, cudaStream_t st) {
   switch (w->flavour) {
-    case 1: return wide_forward_impl<1>(w, d_images, d_labels, n, d_out, d_argmax, training, st);
-    case 2: return wide_forward_impl<2>(w, d_images, d_labels, n, d_out, d_argmax, training, st);
-    default: return wide_forward_impl<0>(w, d_images, d_labels, n, d_out, d_argmax, training, st);
+    case 1: return wide_forward_impl<1>(w, k, tc, d_images, d_labels, n, d_out, d_argmax, training, st);
+    case 2: return wide_forward_impl<2>(w, k, tc, d_images, d_labels, n, d_out, d_argmax, training, st);
+    default: return wide_forward_impl<0>(w, k, tc, d_images, d_labels, n, d_out, d_argmax, training, st);
   }
 }
 
@@ -579,10 +672,9 @@ int cnn_wide_create(int H, int F, cnn_wide** out) {
 
 int cnn_wide_destroy(cnn_wide* w) {
   if (!w) return CNN_OK;
-  float* bufs[] = {w->d_params, w->ac, w->as, w->ds, w->delta_f, w->err, w->part_c, w->part_s, w->img_shift};
-  for (float* p : bufs) cudaFree(p);
+  cudaFree(w->d_params);
+  cudaFree(w->arena);
   cudaFree(w->d_status);
-  cudaFree(w->part_f);
   delete w;
   return CNN_OK;
 }
@@ -607,7 +699,7 @@ int cnn_wide_set_option(cnn_wide* w, const char* key, int value) {
   CNN_REQUIRE(w && key, "cnn_wide_set_option: NULL argument");
   if (std::strcmp(key, "fast_sigmoid") == 0) { w->flavour = (value == 2) ? 2 : (value ? 1 : 0); return CNN_OK; }
   if (std::strcmp(key, "conv") == 0) {
-    CNN_REQUIRE(value >= 0 && value <= 2, "cnn_wide_set_option: conv is 0 (fp32 SIMT), 1 (tf32 tensor cores) or 2 (3 x tf32)");
+    CNN_REQUIRE(value >= 0 && value <= 2, "cnn_wide_set_option: conv is 0 (fp32 SIMT), 1 (tensor cores, one fp16 pass) or 2 (three passes)");
     w->conv_mode = value;
     return CNN_OK;
   }
@@ -633,9 +725,11 @@ int cnn_wide_forward(cnn_wide* w, const float* d_images, long n, float* d_out, i
   CNN_REQUIRE(n >= 0 && n <= 65535L * 32, "cnn_wide_forward: bad image count");
   if (n == 0) return CNN_OK;
   CNN_REQUIRE(d_images != nullptr, "cnn_wide_forward: NULL images");
-  int rc = wide_reserve(w, n);
+  WideWork k;
+  const bool tc = wide_on_tc(w, d_images);
+  int rc = wide_reserve(w, n, false, tc, k);
   if (rc != CNN_OK) return rc;
-  return wide_forward_dispatch(w, d_images, nullptr, n, d_out, d_argmax, false, as_stream(stream));
+  return wide_forward_dispatch(w, k, tc, d_images, nullptr, n, d_out, d_argmax, false, as_stream(stream));
 }
 
 int cnn_wide_grad_batch(cnn_wide* w, const float* d_images, const unsigned int* d_labels, long n, float* d_grad,
@@ -649,36 +743,35 @@ int cnn_wide_grad_batch(cnn_wide* w, const float* d_images, const unsigned int* 
     return CNN_OK;
   }
   CNN_REQUIRE(d_images && d_labels, "cnn_wide_grad_batch: NULL images or labels");
-  int rc = wide_reserve(w, n);
+  WideWork k;
+  const bool tc = wide_on_tc(w, d_images);
+  int rc = wide_reserve(w, n, true, tc, k);
   if (rc != CNN_OK) return rc;
-  if ((rc = wide_forward_dispatch(w, d_images, d_labels, n, nullptr, nullptr, true, st)) != CNN_OK) return rc;
-  k_wide_bp_fc<<<dim3((d.S + 127) / 128, kWideFcSplit), 128, 0, st>>>(d, n, w->as, w->delta_f, w->d_params, w->ds, w->part_f);
-  long rows_c, rows_s;
-  if (w->conv_mode > 0 && wide_grad_tc_supported(d)) {
-    // conv deltas, conv weight gradient and subsample-filter gradient in one kernel; the deltas stay on chip
-    int rows = 0;
-    if ((rc = wide_grad_c1_tc(w, d_images, n, &rows, st)) != CNN_OK) return rc;
-    rows_c = rows_s = rows;
-  } else {
-    // slices of the batch: three blocks per SM and map pair would fit; two waves of them
-    const int pairs = (d.F + 1) / 2;
-    long slices = (6L * sm_count() + pairs - 1) / pairs;
-    if (slices > n) slices = n;
-    if (slices * pairs > w->part_rows) slices = w->part_rows / pairs;
-    if (d.H % 4 == 0 && (reinterpret_cast<uintptr_t>(d_images) & 15u) == 0)
-      k_wide_grad_win<true><<<dim3(pairs, (unsigned)slices), kWideWinThreads, 0, st>>>(d, n, d_images, w->ac, w->ds, w->d_params,
-                                                                                      w->part_c, w->part_s);
-    else
-      k_wide_grad_win<false><<<dim3(pairs, (unsigned)slices), kWideWinThreads, 0, st>>>(d, n, d_images, w->ac, w->ds, w->d_params,
-                                                                                       w->part_c, w->part_s);
-    rows_c = slices;
-    rows_s = slices * pairs;
-  }
-  const int value_blocks = (d.F * 26 + 18 + kOut + 7) / 8;       // one warp each
+  if ((rc = wide_forward_dispatch(w, k, tc, d_images, d_labels, n, nullptr, nullptr, true, st)) != CNN_OK) return rc;
+  const int bp_blocks = wide_bp_fc_blocks(d);
+  cudaError_t e = launch_pdl(k_wide_bp_fc, dim3(bp_blocks, kWideFcSplit), dim3(128), 0, st, d, n, (const float*)k.as,
+                             (const float*)k.delta_f, (const float*)(tc ? k.wf_t : w->d_params + d.o_wf), k.ds, k.part_f, k.ds_max);
+  if (e != cudaSuccess) return cuda_fail(e, "k_wide_bp_fc launch");
   const int weight_blocks = (kOut * d.S + 255) / 256;
-  k_wide_reduce<<<value_blocks + weight_blocks, 256, 0, st>>>(d, n, rows_c, rows_s, w->part_c, w->part_s, w->part_f, w->delta_f,
-                                                              w->err, value_blocks, d_grad);
-  cudaError_t e = cudaGetLastError();
+  if (tc) {
+    int ctas = 0;
+    if ((rc = wide_tc_backward(w, k, d_images, n, bp_blocks * kWideFcSplit, &ctas, st)) != CNN_OK) return rc;
+    const int groups = d.F / kTwF, filter_blocks = groups * 5 * (kTwF / 4), value_blocks = (d.F + 18 + kOut + 7) / 8;
+    e = launch_pdl(k_wide_reduce<true>, dim3(value_blocks + filter_blocks + weight_blocks), dim3(256), 0, st, d, n, (long)ctas,
+                   (long)ctas * groups, (const float*)k.part_g, (const float*)k.part_b, (const float*)k.part_f, (const float*)k.delta_f,
+                   (const float*)k.err, value_blocks, filter_blocks, d_grad);
+  } else {
+    const int pairs = (d.F + 1) / 2;
+    const long slices = wide_grad_slices(d, n);
+    const bool vec = d.H % 4 == 0 && (reinterpret_cast<uintptr_t>(d_images) & 15u) == 0;
+    e = launch_pdl(vec ? k_wide_grad_win<true> : k_wide_grad_win<false>, dim3(pairs, (unsigned)slices), dim3(kWideWinThreads), 0, st, d, n,
+                   d_images, (const float*)k.ac, (const float*)k.ds, (const float*)w->d_params, k.part_c, k.part_s);
+    if (e != cudaSuccess) return cuda_fail(e, "k_wide_grad_win launch");
+    const int value_blocks = (d.F * 26 + 18 + kOut + 7) / 8;       // one warp each
+    e = launch_pdl(k_wide_reduce<false>, dim3(value_blocks + weight_blocks), dim3(256), 0, st, d, n, slices, slices * pairs,
+                   (const float*)k.part_c, (const float*)k.part_s, (const float*)k.part_f, (const float*)k.delta_f, (const float*)k.err,
+                   value_blocks, 0, d_grad);
+  }
   if (e != cudaSuccess) return cuda_fail(e, "wide backward launch");
   return CNN_OK;
 }

@@ -1,5 +1,5 @@
 // Shared definitions of the widened configuration (wide.cu: fp32 SIMT kernels and the C ABI;
-// wide_tc.cu: tcgen05 tensor-core convolution).
+// wide_tc.cu: the tensor-core kernels).
 #pragma once
 
 #include "net.cuh"
@@ -25,29 +25,37 @@ inline WideDims make_wide_dims(int H, int F) {
 struct cnn_wide {
   cnn::WideDims d;
   float* d_params = nullptr;
-  long cap = 0;                 // images the workspace holds
-  float *ac = nullptr, *as = nullptr, *ds = nullptr, *delta_f = nullptr, *err = nullptr;
-  float *part_c = nullptr, *part_s = nullptr;
-  float* img_shift = nullptr;   // [cap][4][H][H]: every image shifted left by 0..3 columns (16-byte aligned tap windows)
-  float* part_f = nullptr;      // FC weight-gradient partials of the batch slices
+  // Workspace: one allocation, laid out anew by each call for its images and kernels; it only grows.
+  float* arena = nullptr;
+  size_t arena_floats = 0;
   int flavour = 1;              // sigmoid flavour (cnn_common.cuh): 1 = the short form (default, as cnn_net), 2 = refined, 0 = reference expression
-  int conv_mode = 0;            // 0 fp32 SIMT, 1 tf32 tcgen05 (one pass), 2 tf32 tcgen05 (three passes)
+  int conv_mode = 0;            // 0 fp32 SIMT, 1 fp16 tensor-core operands (one pass), 2 two fp16 parts each (three passes)
   int* d_status = nullptr;      // bounded-wait status word
-  long part_rows = 0;           // rows of [F][26] that part_c holds
-  // Tensor map (a CUtensorMap, kept opaque here) through which the fused delta + weight-gradient kernel reads the
-  // conv activations, and what it was encoded for.
-  alignas(64) unsigned char ac_map[128] = {};
-  const float* ac_map_ptr = nullptr;
-  long ac_map_cap = 0;
 };
 
-
 namespace cnn {
-bool wide_conv_tc_supported(const WideDims& d);
-// Conv + bias + sigmoid on the tensor cores: writes w->ac for n images.
-int wide_conv_fwd_tc(cnn_wide* w, const float* d_images, long n, cudaStream_t st);
-bool wide_grad_tc_supported(const WideDims& d);
-// Conv deltas, conv weight + bias gradient partials and subsample-filter gradient partials on the tensor cores,
-// from w->ac and w->ds: fills w->part_c with *rows_out rows of [F][26] and w->part_s with as many rows of [17].
-int wide_grad_c1_tc(cnn_wide* w, const float* d_images, long n, int* rows_out, cudaStream_t st);
+// What a call's kernels keep between them.  SIMT path: as, ds [image][map][window]; tensor-core path: [image][window][map].
+struct WideWork {
+  float *ac = nullptr;          // SIMT training: conv activations [image][map][C][C]
+  float *as = nullptr, *ds = nullptr, *delta_f = nullptr, *err = nullptr;
+  float *part_c = nullptr, *part_s = nullptr;            // SIMT training: rows of [F][26] and of [17]
+  float *part_f = nullptr;      // FC weight-gradient partials of the batch slices
+  float *ds_max = nullptr;      // tensor-core training: largest |ds| per block of the kernel that writes it
+  float *pixel_max = nullptr, *wf_t = nullptr;           // tensor-core path: largest pixels per block; FC weights [output][window][map]
+  float *part_g = nullptr, *part_b = nullptr;            // tensor-core training: see k_wide_tc
+  size_t floats = 0;
+};
+
+constexpr int kTwPrepBlocks = 256;
+constexpr int kTwF = 64;                       // maps of a tensor-core CTA (more maps: more CTAs)
+constexpr int kTwGradN = 48;                   // (i, c): six kernel rows of eight columns
+constexpr int kTwGradCols = 4 * kTwF;          // (x, f)
+constexpr int kTwPartB = 4 * kTwF + 20;        // floats of a CTA's bias and subsample-filter sums
+
+// Tensor-core path (wide_tc.cu).  Forward: w.pixel_max, w.wf_t, w.as from the images.  Backward: from the images, w.ds and w.ds_max
+// to w.part_g and w.part_b, of *ctas CTAs for each kTwF maps.
+bool wide_tc_supported(const WideDims& d);
+int wide_tc_max_ctas();
+int wide_tc_forward(cnn_wide* w, const WideWork& k, const float* d_images, long n, cudaStream_t st);
+int wide_tc_backward(cnn_wide* w, const WideWork& k, const float* d_images, long n, int ds_blocks, int* ctas, cudaStream_t st);
 }  // namespace cnn

@@ -310,10 +310,10 @@ int cnn_wide_set_params(cnn_wide* w, const float* h_params);
 int cnn_wide_get_params(cnn_wide* w, float* h_params);
 /* "fast_sigmoid": 0 = the reference's expression, 1 = the short form (default, as for cnn_net), 2 = a
  * refined form (two-step argument reduction, Newton-refined reciprocal); "conv": 0 = fp32 SIMT
- * convolution, 1 = implicit GEMM on the tf32 tensor cores (tcgen05, about 1e-3 relative), 2 = the same
- * in three tf32 passes (hi*hi + lo*hi + hi*lo, fp32-level accuracy).  The tensor-core forward needs F to
- * be a multiple of 16, at most 256; the fused tensor-core backward (conv deltas + weight gradients in one
- * TMA-fed kernel) needs F = 64 and H a multiple of 4, otherwise the fp32 SIMT backward runs. */
+ * convolution, 1 = tensor cores (tcgen05), fp16 operands with 11 significant bits in one pass (about 1e-3
+ * relative), 2 = the same with both operands in two fp16 parts and three passes (hi*hi + lo*hi + hi*lo, fp32-level
+ * accuracy).  The tensor-core kernels take F a multiple of 64, H a multiple of 4 and images that start on a
+ * 16-byte boundary; the fp32 kernels run everything else. */
 int cnn_wide_set_option(cnn_wide* w, const char* key, int value);
 /* As cnn_net_status. */
 int cnn_wide_status(cnn_wide* w, int* status);

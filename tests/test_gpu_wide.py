@@ -139,6 +139,43 @@ def test_tensor_core_conv_matches_oracle(cuda, pkg, ob, H, F, n, mode, tol):
         assert scaled_err(g[lo:hi], G[lo:hi]) < tol * (1 if mode == 2 else 10), name
 
 
+@pytest.mark.parametrize("H,F,n,mode,sigmoid,offset", [
+    (8, 64, 1, 2, 1, 0),        # one window per image: half a row group is empty
+    (8, 64, 300, 2, 0, 0),      # two image groups per FC cluster
+    (12, 64, 601, 1, 1, 0),     # four, the last one ragged
+    (28, 64, 33, 2, 2, 0),      # row groups of an image end in the middle of a group set
+    (56, 128, 3, 2, 1, 0),      # two groups of maps
+    (56, 64, 70, 2, 1, 0),      # units of a CTA: several hand-overs of the gradient accumulators and a rest
+    (28, 64, 9, 2, 1, 1),       # images not 16-byte aligned: the fp32 path
+    (30, 64, 9, 2, 1, 0),       # a height that is not a multiple of 4: the fp32 path
+])
+def test_tensor_core_edges_match_oracle(cuda, pkg, ob, H, F, n, mode, sigmoid, offset):
+    x, labels = wide_inputs(n, H, 9)
+    params = wide_params(ob, H, F, 10)
+    net = pkg.WideNet(H, F)
+    net.set_params(params)
+    net.set_option("conv", mode)
+    net.set_option("fast_sigmoid", sigmoid)
+    d_x = cuda.zeros((n * H * H + offset,), dtype=cuda.float32, device="cuda")[offset:]
+    d_x.copy_(cuda.from_numpy(x.reshape(-1)))
+    d_lab = cuda.from_numpy(labels.astype(np.int32)).cuda()
+    d_out = cuda.empty((n, 10), dtype=cuda.float32, device="cuda")
+    d_g = cuda.full((net.n_padded,), 9.0, dtype=cuda.float32, device="cuda")
+    net.forward(d_x, n, d_out, None)
+    net.grad_batch(d_x, d_lab, n, d_g)
+    cuda.cuda.synchronize()
+    assert net.status() == 0
+    tol = 1e-5 if mode == 2 else 3e-3
+    ref_out, _ = ob.forward_batch(params, x, H=H, F=F)
+    assert rel_err(d_out.cpu().numpy(), ref_out) < tol
+    G, err = ob.grad_batch(params, x, labels, H=H, F=F)
+    g = d_g.cpu().numpy()
+    for name, (lo, hi) in blocks(H, F).items():
+        assert scaled_err(g[lo:hi], G[lo:hi]) < tol * (1 if mode == 2 else 10), name
+    assert abs(g[net.n_params + 1] - err) < tol * max(err, 1.0)
+    assert g[net.n_params] == 0 and not g[net.n_params + 2:].any()
+
+
 @pytest.mark.parametrize("mode", [0, 2])
 def test_wide_full_batch_matches_oracle(cuda, pkg, ob, mode):
     """Benchmark configuration 5 at its full size (batch 1,024 of 56x56 images, 64 maps) against the
