@@ -309,7 +309,8 @@ k_wide_bp_fc(WideDims d, long n, const float* __restrict__ as, const float* __re
       most = fabsf(v) <= 3.4e38f ? fmaxf(most, fabsf(v)) : most;
     }
   }
-  if (ds_max) {
+  if (ds_max) {                            // tensor-core path
+    if (blockIdx.y == 0 && s < d.F) ds[(size_t)n * d.S + s] = 0.f;
 #pragma unroll
     for (int m = 16; m > 0; m >>= 1) most = fmaxf(most, __shfl_xor_sync(0xffffffffu, most, m));
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = most;
@@ -568,7 +569,7 @@ static int wide_reserve(cnn_wide* w, long n, bool training, bool tc, WideWork& k
       take(k.wf_t, (size_t)kOut * d.S);
     }
     if (training) {
-      take(k.ds, (size_t)d.S * n);
+      take(k.ds, (size_t)d.S * n + (tc ? d.F : 0));         // (behind it zeros for windows that do not exist: k_wide_bp_fc)
       take(k.delta_f, (size_t)kOut * n);
       take(k.err, n);
       take(k.part_f, (size_t)kWideFcSplit * kOut * d.S);

@@ -56,12 +56,12 @@ constexpr int kTwLoadWarps = 7, kTwMmaWarp = 7, kTwEpiWarp0 = 8, kTwEpiWarps = 1
 constexpr int kTwRows = kTwGroups * kTwGroupRows;                   // 208 loader threads with work
 constexpr float kTwMaxExp = 31.f;                                   // (1 + 2^31)^4 is still finite
 constexpr int kTwHalf = kTwN / 2;                                   // columns of a half (32 maps): what an accumulator holds
-constexpr int kTwAcc = 3;                                           // accumulators
+constexpr int kTwAccMax = 4;                                        // accumulators in the forward kernel; the backward kernel has two
 // backward
 constexpr unsigned kTwDcChunk = 128 * 16;                           // 8 values of (x, f) for 128 rows
 constexpr unsigned kTwDcPart = (kTwHalf / 8) * kTwDcChunk;          // 32 KB: one part of a half's deltas
-constexpr int kTwGradCol = kTwAcc * kTwHalf;                        // the two halves' gradient accumulators behind the others
-constexpr int kTwFlush = 4;                                         // units per hand-over of the gradient accumulators
+constexpr int kTwGradCol = 2 * kTwHalf;                             // two sets of gradient accumulators (a set: both halves) behind the others
+constexpr int kTwFlush = 4;                                         // units between two hand-overs of a set
 
 struct TwSmem {
   alignas(128) unsigned char slab[kTwSlabs][2][kTwPlane];           // [high, low]
@@ -69,8 +69,8 @@ struct TwSmem {
   alignas(16) float bias[kTwF];
   alignas(16) float ws[16];
   float bs;
-  unsigned long long a_full[kTwSlabs], a_free[kTwSlabs], d_full[kTwAcc], d_free[kTwAcc];
-  unsigned long long dc_full[2], dc_free[2], g_full, g_free;        // backward: deltas of a half, gradient accumulators
+  unsigned long long a_full[kTwSlabs], a_free[kTwSlabs], d_full[kTwAccMax], d_free[kTwAccMax];
+  unsigned long long dc_full[2], dc_free[2], g_full[2], g_free[2];  // backward: deltas of a half, sets of gradient accumulators
   float max_of[3][kTwThreads / 32];                                 // largest tap, pixel, subsample delta by warp
   unsigned tmem_base;
   long long clock_base;                                             // phase clocks only
@@ -95,6 +95,8 @@ __device__ __forceinline__ int exponent_of(float v) {
   const int e = (int)((__float_as_uint(v) >> 23) & 255u) - 127;
   return e > 60 ? 60 : (e < -60 ? -60 : e);
 }
+// *p += v, not waited for.
+__device__ __forceinline__ void red_add(float* p, float v) { asm volatile("red.global.add.f32 [%0], %1;" ::"l"(p), "f"(v) : "memory"); }
 __device__ __forceinline__ float pow2i(int e) { return __int_as_float((127 + e) << 23); }
 
 // What the tensor-core kernels need of a batch beforehand: per-block maxima of the (finite) pixel magnitudes, and the FC weights
@@ -141,28 +143,31 @@ k_wide_tc(WideDims d, long n, const float* __restrict__ images, const float* __r
   TwBwdSmem& sb = *reinterpret_cast<TwBwdSmem*>(smem_base);        // backward only
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   constexpr bool kShort = (FL == 1);
+  constexpr int kAcc = BWD ? 2 : kTwAccMax;
   constexpr float kPre = kShort ? -1.4426950408889634f : 1.0f;     // the short sigmoid form's factor, folded into taps and bias
   const int f0 = blockIdx.y * kTwF;
   const int gi = (d.C + 7) / 8;                                    // groups per image
+  // (at most 2,097,120 images: group and unit numbers fit in 32 bits, and a unit's place is advanced, not divided out)
   const long n_units = (n * gi + kTwGroups - 1) / kTwGroups * d.P;
-  const long u0 = n_units * blockIdx.x / gridDim.x;
+  const unsigned u0 = (unsigned)(n_units * blockIdx.x / gridDim.x);
   const int units = (int)(n_units * (blockIdx.x + 1) / gridDim.x - u0);
+  const unsigned set0 = u0 / (unsigned)d.P, q0 = u0 - set0 * (unsigned)d.P;      // group set and window column of the first unit
 
   if (tid == 0) {
     for (int s = 0; s < kTwSlabs; ++s) {
       mbar_init(&sm.a_full[s], kTwLoadWarps);
       mbar_init(&sm.a_free[s], 1);
     }
-    for (int s = 0; s < kTwAcc; ++s) {
+    for (int s = 0; s < kAcc; ++s) {
       mbar_init(&sm.d_full[s], 1);
       mbar_init(&sm.d_free[s], kTwEpiWarps);
     }
     for (int h = 0; h < 2; ++h) {
       mbar_init(&sm.dc_full[h], kTwEpiWarps);
       mbar_init(&sm.dc_free[h], 1);
+      mbar_init(&sm.g_full[h], 1);
+      mbar_init(&sm.g_free[h], 4);
     }
-    mbar_init(&sm.g_full, 1);
-    mbar_init(&sm.g_free, kTwEpiWarps);
     mbar_fence_init();
   }
   if (warp == kTwMmaWarp) tc::tmem_alloc(&sm.tmem_base, 512);
@@ -244,23 +249,55 @@ k_wide_tc(WideDims d, long n, const float* __restrict__ images, const float* __r
     const bool mine = tid < kTwRows;
     float4 v0, v1;
     bool have;
-    auto load = [&](int k) {           // (clamped, not conditional: a load under a condition is waited for on the spot)
-      const long u = u0 + (k < units ? k : units - 1);
-      const long t = u / d.P;
-      const int q = (int)(u - t * d.P);
-      const long G = t * kTwGroups + (mine ? g : 0), b = G / gi;
-      const int y = 8 * (int)(G - b * gi) + row;
+    const float* src;
+    unsigned G = set0 * kTwGroups + (mine ? g : 0);
+    auto place = [&]() {
+      const unsigned b = G / (unsigned)gi;
+      const int y = 8 * (int)(G - b * (unsigned)gi) + row;
       have = mine && b < n && y < d.H;
-      const float* src = images + ((size_t)(have ? b : 0) * d.H + (have ? y : 0)) * d.H + 4 * q;
-      v0 = __ldg(reinterpret_cast<const float4*>(src));
-      v1 = __ldg(reinterpret_cast<const float4*>(src) + 1);
+      src = images + ((size_t)(have ? b : 0) * d.H + (have ? y : 0)) * d.H;
     };
-    load(0);
+    auto load = [&](int q) {           // (clamped, not conditional: a load under a condition is waited for on the spot)
+      v0 = __ldg(reinterpret_cast<const float4*>(src + 4 * q));
+      v1 = __ldg(reinterpret_cast<const float4*>(src + 4 * q) + 1);
+    };
+    int q = (int)q0;
+    place();
+    load(q);
+    // Backward, warps 0-3: adds (or, the first time, puts) a complete set of gradient accumulators, a warp its quarter of the rows (x, f),
+    // to the CTA's sums -- every address has one thread that adds to it, in order; as a reduction, which needs no answer.
+    auto flush = [&](int set) {
+      if (warp >= 4) return;
+      mbar_wait_bounded(&sm.g_full[set & 1], (unsigned)(set >> 1) & 1u, status, gave_up);
+      __syncwarp();
+      tc::fence_after_sync();
+      const unsigned t0 = tmem_base + ((unsigned)(warp * 32) << 16) + (unsigned)(kTwGradCol + (set & 1) * 2 * kTwGradN);
+      float* dst = part_g + (size_t)(blockIdx.y * gridDim.x + blockIdx.x) * kTwGradN * kTwGradCols + warp * 32 + lane;
+      const float s1 = pow2i(-dc_exp), s2 = pow2i(-pe);
+#pragma unroll 1
+      for (int c = 0; c < 2 * kTwGradN; c += 8) {
+        unsigned r[8];
+        tc::tmem_ld8_nowait(t0 + (unsigned)c, r);
+        tc::tmem_wait8(r);
+        float* to = dst + (c < kTwGradN ? c * kTwGradCols : (c - kTwGradN) * kTwGradCols + 128);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+          const float v = __uint_as_float(r[e]) * s1 * s2;
+          if (set > 0) red_add(to + e * kTwGradCols, v);
+          else to[e * kTwGradCols] = v;
+        }
+      }
+      tc::fence_before_sync();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&sm.g_free[set & 1]);
+    };
     for (int k = 0; k < units; ++k) {
       const int s = k % kTwSlabs;
       CNN_PHASE(0);
       mbar_wait_bounded(&sm.a_free[s], ((unsigned)(k / kTwSlabs) & 1u) ^ 1u, status, gave_up);
       CNN_PHASE(1);
+      // (the slab is free: the gradients of the unit that had it are complete, and with the last unit of a set the set)
+      if (BWD && k >= kTwSlabs && (k - kTwSlabs) % kTwFlush == kTwFlush - 1) flush((k - kTwSlabs) / kTwFlush);
       __half2 hi[4], lo[4];
       tc::split_f16x2(have ? v0.x : 0.f, have ? v0.y : 0.f, px_scale, hi[0], lo[0]);
       tc::split_f16x2(have ? v0.z : 0.f, have ? v0.w : 0.f, px_scale, hi[1], lo[1]);
@@ -270,12 +307,19 @@ k_wide_tc(WideDims d, long n, const float* __restrict__ images, const float* __r
         *reinterpret_cast<uint4*>(sm.slab[s][0] + tid * 16) = *reinterpret_cast<uint4*>(hi);
         if (PASSES == 3) *reinterpret_cast<uint4*>(sm.slab[s][1] + tid * 16) = *reinterpret_cast<uint4*>(lo);
       }
-      load(k + 1);
+      if (++q == d.P) {
+        q = 0;
+        G += kTwGroups;
+        place();
+      }
+      load(q);                         // (after the last unit: a group past the range, or the first rows)
       tc::fence_async_smem();
       __syncwarp();
       if (lane == 0) mbar_arrive(&sm.a_full[s]);
       CNN_PHASE(2);
     }
+    if (BWD)
+      for (int set = units > kTwSlabs ? (units - kTwSlabs) / kTwFlush : 0; set <= (units - 1) / kTwFlush; ++set) flush(set);
   } else if (warp == kTwMmaWarp) {
     // ================= MMA issue: the whole warp runs the loop, one elected lane issues =============
     const unsigned idesc = tc::idesc_f16(128, kTwHalf);
@@ -284,11 +328,11 @@ k_wide_tc(WideDims d, long n, const float* __restrict__ images, const float* __r
     const int halves = 2 * units;
     for (int v = 0; v < halves + (BWD ? 2 : 0); ++v) {
       if (v < halves) {
-        const int k = v >> 1, h = v & 1, s = k % kTwSlabs, acc = v % kTwAcc;
+        const int k = v >> 1, h = v & 1, s = k % kTwSlabs, acc = v % kAcc;
         CNN_PHASE(0);
         if (h == 0) mbar_wait_bounded(&sm.a_full[s], (unsigned)(k / kTwSlabs) & 1u, status, gave_up);
         CNN_PHASE(1);
-        mbar_wait_bounded(&sm.d_free[acc], ((unsigned)(v / kTwAcc) & 1u) ^ 1u, status, gave_up);
+        mbar_wait_bounded(&sm.d_free[acc], ((unsigned)(v / kAcc) & 1u) ^ 1u, status, gave_up);
         CNN_PHASE(2);
         __syncwarp();
         tc::fence_after_sync();
@@ -309,11 +353,12 @@ k_wide_tc(WideDims d, long n, const float* __restrict__ images, const float* __r
       if (BWD && v >= 2) {
         // the gradient of the half two steps back: its deltas were made while the convolutions since then ran
         const int gv = v - 2, k = gv >> 1, h = gv & 1, s = k % kTwSlabs;
+        const int set = k / kTwFlush;
         const bool first = k % kTwFlush == 0;
         CNN_PHASE(4);
         mbar_wait_bounded(&sm.dc_full[h], (unsigned)k & 1u, status, gave_up);
         CNN_PHASE(5);
-        if (first && h == 0) mbar_wait_bounded(&sm.g_free, ((unsigned)(k / kTwFlush) & 1u) ^ 1u, status, gave_up);
+        if (first && h == 0) mbar_wait_bounded(&sm.g_free[set & 1], ((unsigned)(set >> 1) & 1u) ^ 1u, status, gave_up);
         CNN_PHASE(6);
         __syncwarp();
         tc::fence_after_sync();
@@ -326,13 +371,13 @@ k_wide_tc(WideDims d, long n, const float* __restrict__ images, const float* __r
           const unsigned long long a = pass == 1 ? dc_d[1] : dc_d[0], b = pass == 2 ? x_d[1] : x_d[0];
 #pragma unroll
           for (int ks = 0; ks < 8; ++ks)       // 16 rows = two groups
-            tc::mma_f16_elect(tmem_base + (unsigned)(kTwGradCol + h * kTwGradN), a + (unsigned)(ks * 256 >> 4),
+            tc::mma_f16_elect(tmem_base + (unsigned)(kTwGradCol + (2 * (set & 1) + h) * kTwGradN), a + (unsigned)(ks * 256 >> 4),
                               b + (unsigned)(ks * 2 * kTwGroupStride >> 4), idesc_g, (first && pass == 0 && ks == 0) ? 0u : 1u);
         }
         tc::mma_commit_elect(&sm.dc_free[h]);
         if (h == 1) {
           tc::mma_commit_elect(&sm.a_free[s]);
-          if (k % kTwFlush == kTwFlush - 1 || k == units - 1) tc::mma_commit_elect(&sm.g_full);
+          if (k % kTwFlush == kTwFlush - 1 || k == units - 1) tc::mma_commit_elect(&sm.g_full[set & 1]);
         }
         CNN_PHASE(7);
       }
@@ -344,67 +389,51 @@ k_wide_tc(WideDims d, long n, const float* __restrict__ images, const float* __r
     const bool b0 = (lane & 1) != 0, b1 = (lane & 2) != 0;
     const f32x2 one2 = pack2(1.f, 1.f), minus2 = pack2(-1.f, -1.f), unscale2 = pack2(unscale, unscale);
     const float inv_c = 1.0f / (float)(d.C * d.C);
-    f32x2 k2[4];                                   // forward: the row's subsample taps; backward: times 2^dc_exp / (C*C)
+    f32x2 k2[4];                                   // forward: the row's subsample taps; backward: times -2^dc_exp / (C*C)
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      const float w = BWD ? sm.ws[rsub * 4 + j] * inv_c * pow2i(dc_exp) : sm.ws[rsub * 4 + j];
+      const float w = BWD ? -sm.ws[rsub * 4 + j] * inv_c * pow2i(dc_exp) : sm.ws[rsub * 4 + j];
       k2[j] = pack2(w, w);
     }
     const unsigned lane_base = tmem_base + ((unsigned)(quarter * 32) << 16);
-    // backward: sums of this lane's row over units: subsample-filter taps (row rsub) and delta_s in halves by map parity, and the
-    // conv bias per map pair of either half
+    // backward: sums of this lane's row over units: subsample-filter taps (row rsub, negated) and delta_s in halves by map parity,
+    // and the conv bias per map pair of either half
     f32x2 gs2[4], gds2 = pack2(0.f, 0.f), gb2[2][4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) gs2[j] = gb2[0][j] = gb2[1][j] = pack2(0.f, 0.f);
-    float* my_g = BWD ? part_g + (size_t)(blockIdx.y * gridDim.x + blockIdx.x) * kTwGradN * 256 : nullptr;
-
-    // Adds (or, the first time, puts) the gradient accumulators to the CTA's sums: warp (group, quarter) takes columns 24 (group & 1)
-    // .. + 23 of half group / 2, rows 32 quarter ..
-    auto flush = [&](int j) {
-      mbar_wait_bounded(&sm.g_full, (unsigned)j & 1u, status, gave_up);
-      __syncwarp();
-      tc::fence_after_sync();
-      const unsigned t0 = lane_base + (unsigned)(kTwGradCol + (group >> 1) * kTwGradN + (group & 1) * 24);
-      float* dst = my_g + ((size_t)(group & 1) * 24) * 256 + (group >> 1) * 128 + quarter * 32 + lane;
-#pragma unroll 1
-      for (int c = 0; c < 24; c += 8) {
-        unsigned r[8];
-        tc::tmem_ld8_nowait(t0 + (unsigned)c, r);
-        tc::tmem_wait8(r);
-        float old[8];
-#pragma unroll
-        for (int e = 0; e < 8; ++e) old[e] = j > 0 ? dst[(size_t)(c + e) * 256] : 0.f;
-#pragma unroll
-        for (int e = 0; e < 8; ++e) dst[(size_t)(c + e) * 256] = old[e] + __uint_as_float(r[e]) * pow2i(-dc_exp) * pow2i(-pe);
-      }
-      tc::fence_before_sync();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&sm.g_free);
+    int q = (int)q0;
+    unsigned G = set0 * kTwGroups + quarter * 4 + (lane >> 3);
+    bool live;
+    float* at;                       // this lane's window and maps in as / ds; of a window that does not exist: the zeros behind ds
+    auto place = [&]() {
+      const unsigned b = G / (unsigned)gi;
+      const int p = (8 * (int)(G - b * (unsigned)gi) + (lane & 7)) >> 2;      // C is a multiple of 4: a window's rows are all in or all out
+      live = b < n && p < d.P;
+      const size_t window = live ? ((size_t)b * d.P + p) * d.P + q : (BWD ? (size_t)n * d.P * d.P : 0);
+      at = (BWD ? const_cast<float*>(ds) : as) + window * d.F + f0 + 8 * group;
     };
-
-    int flushed = 0;
+    place();
+    // Backward: the window's deltas of eight maps, the next half's taken as soon as this half's are used.
+    float4 dlo, dhi;
+    if (BWD) {
+      dlo = __ldg(reinterpret_cast<const float4*>(at));
+      dhi = __ldg(reinterpret_cast<const float4*>(at) + 1);
+    }
     for (int k = 0; k < units; ++k) {
-      const long u = u0 + k, t = u / d.P;
-      const int q = (int)(u - t * d.P);
-      const long G = t * kTwGroups + quarter * 4 + (lane >> 3), b = G / gi;
-      const int y = 8 * (int)(G - b * gi) + (lane & 7), p = y >> 2;      // C is a multiple of 4: a window's rows are all in or all out
-      const bool live = b < n && p < d.P;
-      const size_t at = ((size_t)(live ? b : 0) * d.P * d.P + (size_t)(live ? p : 0) * d.P + q) * d.F + f0 + 8 * group;
-#pragma unroll 1
+#pragma unroll
       for (int h = 0; h < 2; ++h) {
-        const int v = 2 * k + h, acc = v % kTwAcc;
-        float dsv[8];                              // backward: the window's deltas of this warp's eight maps
-        if (BWD) {
-          const float4 lo = __ldg(reinterpret_cast<const float4*>(ds + at + 32 * h)), hi = __ldg(reinterpret_cast<const float4*>(ds + at + 32 * h) + 1);
-          dsv[0] = lo.x; dsv[1] = lo.y; dsv[2] = lo.z; dsv[3] = lo.w; dsv[4] = hi.x; dsv[5] = hi.y; dsv[6] = hi.z; dsv[7] = hi.w;
-          // (one unit late: the accumulators of the last units are then complete or nearly so)
-          if (h == 0 && k >= kTwFlush && k % kTwFlush == 1) flush(flushed++);
+        const int v = 2 * k + h, acc = v % kAcc;
+        if (BWD && h == 1) {         // `at` is only for the loads ahead
+          if (live) at += d.F;
+          if (++q == d.P) {
+            q = 0;
+            G += kTwGroups;
+            place();
+          }
         }
         CNN_PHASE(0);
-        mbar_wait_bounded(&sm.d_full[acc], (unsigned)(v / kTwAcc) & 1u, status, gave_up);
+        mbar_wait_bounded(&sm.d_full[acc], (unsigned)(v / kAcc) & 1u, status, gave_up);
         CNN_PHASE(1);
-        if (BWD) mbar_wait_bounded(&sm.dc_free[h], ((unsigned)k & 1u) ^ 1u, status, gave_up);
-        CNN_PHASE(2);
         __syncwarp();
         tc::fence_after_sync();
         const unsigned t0 = lane_base + (unsigned)(acc * kTwHalf + 32 * group);
@@ -426,7 +455,16 @@ k_wide_tc(WideDims d, long n, const float* __restrict__ images, const float* __r
             __syncwarp();
             if (lane == 0) mbar_arrive(&sm.d_free[acc]);
           }
-          if constexpr (kShort) {
+          if constexpr (BWD && kShort) {
+            // -a = 1 / (-1 - 2^t): a reciprocal each, which costs fewer issue slots than sharing them as below
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              float x, yv;
+              unpack2(a2[j], x, yv);
+              unpack2(fma2(pack2(exp2f_approx(x), exp2f_approx(yv)), minus2, minus2), x, yv);
+              a2[j] = pack2(rcp_approx(x), rcp_approx(yv));
+            }
+          } else if constexpr (kShort) {
             // 1 / d_j with d_j = 1 + 2^t_j: one reciprocal for the row's four (t is capped so that their product stays finite: an
             // activation below 4.7e-10 counts as that)
             f32x2 dd[4];
@@ -440,32 +478,30 @@ k_wide_tc(WideDims d, long n, const float* __restrict__ images, const float* __r
             float x, yv;
             unpack2(mul2(d01, d23), x, yv);
             const f32x2 r = pack2(rcp_approx(x), rcp_approx(yv));
-            if constexpr (BWD) {
-              const f32x2 r23 = mul2(r, d23), r01 = mul2(r, d01);
-              a2[0] = mul2(r23, dd[1]); a2[1] = mul2(r23, dd[0]); a2[2] = mul2(r01, dd[3]); a2[3] = mul2(r01, dd[2]);
-            } else {
-              const f32x2 n01 = fma2(k2[0], dd[1], mul2(k2[1], dd[0])), n23 = fma2(k2[2], dd[3], mul2(k2[3], dd[2]));
-              unpack2(mul2(r, fma2(n01, d23, mul2(n23, d01))), z[2 * ch], z[2 * ch + 1]);
-            }
+            const f32x2 n01 = fma2(k2[0], dd[1], mul2(k2[1], dd[0])), n23 = fma2(k2[2], dd[3], mul2(k2[3], dd[2]));
+            unpack2(mul2(r, fma2(n01, d23, mul2(n23, d01))), z[2 * ch], z[2 * ch + 1]);
           } else {
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
               float x, yv;
               unpack2(a2[j], x, yv);
-              a2[j] = pack2(sigmoidf<FL>(x), sigmoidf<FL>(yv));
+              a2[j] = BWD ? pack2(-sigmoidf<FL>(x), -sigmoidf<FL>(yv)) : pack2(sigmoidf<FL>(x), sigmoidf<FL>(yv));
             }
             if constexpr (!BWD)
               unpack2(fma2(k2[3], a2[3], fma2(k2[2], a2[2], fma2(k2[1], a2[1], mul2(k2[0], a2[0])))), z[2 * ch], z[2 * ch + 1]);
           }
           if constexpr (BWD) {
-            const f32x2 dl = live ? pack2(dsv[2 * ch], dsv[2 * ch + 1]) : pack2(0.f, 0.f);
+            const float4 dq = ch < 2 ? dlo : dhi;
+            const f32x2 dl = ch % 2 ? pack2(dq.z, dq.w) : pack2(dq.x, dq.y);
             unsigned hi[4], lo[4];
-            f32x2 sum = pack2(0.f, 0.f);
+            f32x2 sum;
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-              gs2[j] = fma2(dl, a2[j], gs2[j]);
-              const f32x2 dcv = mul2(mul2(k2[j], dl), mul2(a2[j], fma2(a2[j], minus2, one2)));
-              sum = add2(sum, dcv);
+              // a2 is -a: m = -dl a, m - m a = -dl a (1 - a)
+              const f32x2 m = mul2(dl, a2[j]);
+              gs2[j] = add2(gs2[j], m);
+              const f32x2 dcv = mul2(k2[j], fma2(m, a2[j], m));
+              sum = j ? add2(sum, dcv) : dcv;
               float x, yv;
               unpack2(dcv, x, yv);
               const __half2 hv = __floats2half2_rn(x, yv);
@@ -479,14 +515,21 @@ k_wide_tc(WideDims d, long n, const float* __restrict__ images, const float* __r
             }
             if (h == 0) gb2[0][ch] = add2(gb2[0][ch], sum);
             else gb2[1][ch] = add2(gb2[1][ch], sum);
-            if (rsub == 0) gds2 = add2(gds2, dl);
+            gds2 = add2(gds2, dl);                 // (the window's four lanes have the same: lane 0's sum is used)
+            if (ch == 1) dlo = __ldg(reinterpret_cast<const float4*>(h ? at : at + 32));
+            if (ch == 3) dhi = __ldg(reinterpret_cast<const float4*>(h ? at : at + 32) + 1);
+            if (ch == 0) {
+              CNN_PHASE(2);
+              mbar_wait_bounded(&sm.dc_free[h], ((unsigned)k & 1u) ^ 1u, status, gave_up);
+              CNN_PHASE(3);
+            }
             unsigned char* dst = sb.dc[h][0] + (unsigned)(4 * group + ch) * kTwDcChunk + (unsigned)(quarter * 32 + lane) * 16u;
             *reinterpret_cast<uint4*>(dst) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
             if (PASSES == 3) *reinterpret_cast<uint4*>(dst + kTwDcPart) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
           }
           if (ch < 3) tc::tmem_wait8(nxt);
         }
-        CNN_PHASE(3);
+        CNN_PHASE(4);
         if constexpr (BWD) {
           tc::fence_async_smem();      // generic-proxy writes -> visible to the tensor core's operand reads
           __syncwarp();
@@ -505,14 +548,21 @@ k_wide_tc(WideDims d, long n, const float* __restrict__ images, const float* __r
             w2[i] = keep + __shfl_xor_sync(0xffffffffu, send, 2);
           }
           if (live)
-            *reinterpret_cast<float2*>(as + at + 32 * h + (b0 ? 4 : 0) + (b1 ? 2 : 0)) =
+            *reinterpret_cast<float2*>(at + 32 * h + (b0 ? 4 : 0) + (b1 ? 2 : 0)) =
                 make_float2(sigmoidf<FL>(w2[0] + sm.bs), sigmoidf<FL>(w2[1] + sm.bs));
         }
-        CNN_PHASE(4);
+        CNN_PHASE(5);
+      }
+      if (!BWD) {
+        at += d.F;
+        if (++q == d.P) {
+          q = 0;
+          G += kTwGroups;
+          place();
+        }
       }
     }
     if constexpr (BWD) {
-      while (flushed <= (units - 1) / kTwFlush) flush(flushed++);
       // conv bias: sum over the quarter's rows; lane 8 h + 2 ch + parity ends with that map's
       float v[32];
 #pragma unroll
@@ -528,7 +578,7 @@ k_wide_tc(WideDims d, long n, const float* __restrict__ images, const float* __r
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         unpack2(gs2[j], x, yv);
-        s5[j] = x + yv;
+        s5[j] = -(x + yv);
       }
       unpack2(gds2, x, yv);
       s5[4] = x + yv;
