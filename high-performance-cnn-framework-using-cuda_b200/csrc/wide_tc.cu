@@ -29,11 +29,16 @@
 //
 // One CTA per SM, 24 warps (80 registers), hand-overs by mbarriers with bounded waits:
 //   warps 0-6   load a unit's rows (32 bytes per thread, one unit ahead in registers), split them and store the slab;
+//               backward: warps 0-3 also drain the gradient accumulators, of which two sets alternate (374 us against 386 for a
+//               step of 1,024 images with one set drained by the epilogue);
 //   warp 7      issues the MMAs (an elected lane of the converged warp) and commits to mbarriers;
-//   warps 8-23  epilogue, a quarter of the rows and 8 maps of each half of a unit: tcgen05.ld of 8 columns at a time; bias,
-//               sigmoid; forward: the window row's four subsample taps, the four rows of a window by a shuffle
-//               reduce-scatter, sigmoid, out; backward: deltas, their fp16 parts into the A operand, subsample-filter
-//               gradient and bias sums in registers.
+//   warps 8-23  epilogue, a quarter of the rows and 16 maps: tcgen05.ld of 8 columns at a time; bias, sigmoid.
+//               Forward: the window row's four subsample taps, the four rows of a window by a shuffle reduce-scatter, sigmoid, out;
+//               all warps half by half, as the tensor core is ahead.  Backward: deltas, their fp16 parts into the A operand,
+//               subsample-filter gradient and bias sums in registers; eight warps for each half of a unit, so that one half's work
+//               while the other's wait for the tensor core (377 -> 363 us, with one pass 344 -> 325).
+// Bounds, for 1,024 images: forward 104 us of kernel, issue slots (53 % busy; MUFU and ALU pipes about a third each) and latencies
+// between hand-overs; backward 235 us, of which the packed fp32 pipe is busy 80 % in the epilogue's arithmetic.
 // Work is cut into equal ranges of units, so a CTA may begin and end in the middle of a group set.
 #include <type_traits>
 
@@ -160,10 +165,10 @@ k_wide_tc(WideDims d, long n, const float* __restrict__ images, const float* __r
     }
     for (int s = 0; s < kAcc; ++s) {
       mbar_init(&sm.d_full[s], 1);
-      mbar_init(&sm.d_free[s], kTwEpiWarps);
+      mbar_init(&sm.d_free[s], BWD ? kTwEpiWarps / 2 : kTwEpiWarps);
     }
     for (int h = 0; h < 2; ++h) {
-      mbar_init(&sm.dc_full[h], kTwEpiWarps);
+      mbar_init(&sm.dc_full[h], kTwEpiWarps / 2);
       mbar_init(&sm.dc_free[h], 1);
       mbar_init(&sm.g_full[h], 1);
       mbar_init(&sm.g_free[h], 4);
@@ -384,7 +389,10 @@ k_wide_tc(WideDims d, long n, const float* __restrict__ images, const float* __r
     }
   } else {
     // ================= epilogue ====================================================================
-    const int ew = warp - kTwEpiWarp0, group = ew >> 2, quarter = warp & 3;
+    const int ew = warp - kTwEpiWarp0, h = ew >> 3, quarter = warp & 3;
+    // The warp's 16 maps: backward 16 of its half h from m0 on, forward eight of each half, m0 .. and 32 + m0 ..
+    constexpr int kPartMaps = BWD ? 8 : 32;
+    const int m0 = BWD ? 32 * h + 16 * ((ew >> 2) & 1) : 8 * (ew >> 2);
     const int rsub = lane & 3;                     // row of the 4x4 window
     const bool b0 = (lane & 1) != 0, b1 = (lane & 2) != 0;
     const f32x2 one2 = pack2(1.f, 1.f), minus2 = pack2(-1.f, -1.f), unscale2 = pack2(unscale, unscale);
@@ -398,9 +406,9 @@ k_wide_tc(WideDims d, long n, const float* __restrict__ images, const float* __r
     const unsigned lane_base = tmem_base + ((unsigned)(quarter * 32) << 16);
     // backward: sums of this lane's row over units: subsample-filter taps (row rsub, negated) and delta_s in halves by map parity,
     // and the conv bias per map pair of either half
-    f32x2 gs2[4], gds2 = pack2(0.f, 0.f), gb2[2][4];
+    f32x2 gs2[4], gds2 = pack2(0.f, 0.f), gb2[8];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) gs2[j] = gb2[0][j] = gb2[1][j] = pack2(0.f, 0.f);
+    for (int j = 0; j < 4; ++j) gs2[j] = gb2[j] = gb2[4 + j] = pack2(0.f, 0.f);
     int q = (int)q0;
     unsigned G = set0 * kTwGroups + quarter * 4 + (lane >> 3);
     bool live;
@@ -410,20 +418,31 @@ k_wide_tc(WideDims d, long n, const float* __restrict__ images, const float* __r
       const int p = (8 * (int)(G - b * (unsigned)gi) + (lane & 7)) >> 2;      // C is a multiple of 4: a window's rows are all in or all out
       live = b < n && p < d.P;
       const size_t window = live ? ((size_t)b * d.P + p) * d.P + q : (BWD ? (size_t)n * d.P * d.P : 0);
-      at = (BWD ? const_cast<float*>(ds) : as) + window * d.F + f0 + 8 * group;
+      at = (BWD ? const_cast<float*>(ds) : as) + window * d.F + f0 + m0;
     };
     place();
-    // Backward: the window's deltas of eight maps, the next half's taken as soon as this half's are used.
+    // Backward: the window's deltas of eight maps, the next eight taken as soon as these are used.
     float4 dlo, dhi;
     if (BWD) {
       dlo = __ldg(reinterpret_cast<const float4*>(at));
       dhi = __ldg(reinterpret_cast<const float4*>(at) + 1);
     }
     for (int k = 0; k < units; ++k) {
+      unsigned nxt[8];
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int v = 2 * k + h, acc = v % kAcc;
-        if (BWD && h == 1) {         // `at` is only for the loads ahead
+      for (int part = 0; part < 2; ++part) {         // eight maps
+        const int acc = BWD ? h : 2 * (k & 1) + part;
+        const unsigned t0 = lane_base + (unsigned)(acc * kTwHalf + 4 * (m0 & 31) + (BWD ? 32 * part : 0));
+        if (!BWD || part == 0) {
+          CNN_PHASE(0);
+          mbar_wait_bounded(&sm.d_full[acc], (unsigned)(BWD ? k : k >> 1) & 1u, status, gave_up);
+          CNN_PHASE(1);
+          __syncwarp();
+          tc::fence_after_sync();
+          tc::tmem_ld8_nowait(t0, nxt);
+          tc::tmem_wait8(nxt);
+        }
+        if (BWD && part == 1) {      // `at` is only for the loads ahead
           if (live) at += d.F;
           if (++q == d.P) {
             q = 0;
@@ -431,24 +450,15 @@ k_wide_tc(WideDims d, long n, const float* __restrict__ images, const float* __r
             place();
           }
         }
-        CNN_PHASE(0);
-        mbar_wait_bounded(&sm.d_full[acc], (unsigned)(v / kAcc) & 1u, status, gave_up);
-        CNN_PHASE(1);
-        __syncwarp();
-        tc::fence_after_sync();
-        const unsigned t0 = lane_base + (unsigned)(acc * kTwHalf + 32 * group);
-        unsigned nxt[8];
-        tc::tmem_ld8_nowait(t0, nxt);
-        tc::tmem_wait8(nxt);
         float z[8];
 #pragma unroll
-        for (int ch = 0; ch < 4; ++ch) {           // a window row of maps 32 h + 8 group + 2 ch + {0, 1}
-          const f32x2 bias2 = *reinterpret_cast<const f32x2*>(&sm.bias[32 * h + 8 * group + 2 * ch]);
+        for (int ch = 0; ch < 4; ++ch) {           // a window row of maps m0 + kPartMaps * part + 2 ch + {0, 1}
+          const f32x2 bias2 = *reinterpret_cast<const f32x2*>(&sm.bias[m0 + kPartMaps * part + 2 * ch]);
           f32x2 a2[4];
 #pragma unroll
           for (int j = 0; j < 4; ++j)
             a2[j] = fma2(pack2(__uint_as_float(nxt[2 * j]), __uint_as_float(nxt[2 * j + 1])), unscale2, bias2);
-          if (ch < 3) {
+          if ((BWD && part == 0) || ch < 3) {
             tc::tmem_ld8_nowait(t0 + (unsigned)((ch + 1) * 8), nxt);
           } else {
             tc::fence_before_sync();
@@ -513,28 +523,22 @@ k_wide_tc(WideDims d, long n, const float* __restrict__ images, const float* __r
                 lo[j] = *reinterpret_cast<const unsigned*>(&lv);
               }
             }
-            if (h == 0) gb2[0][ch] = add2(gb2[0][ch], sum);
-            else gb2[1][ch] = add2(gb2[1][ch], sum);
+            gb2[4 * part + ch] = add2(gb2[4 * part + ch], sum);
             gds2 = add2(gds2, dl);                 // (the window's four lanes have the same: lane 0's sum is used)
-            if (ch == 1) dlo = __ldg(reinterpret_cast<const float4*>(h ? at : at + 32));
-            if (ch == 3) dhi = __ldg(reinterpret_cast<const float4*>(h ? at : at + 32) + 1);
-            if (ch == 0) {
+            if (ch == 1) dlo = __ldg(reinterpret_cast<const float4*>(part ? at : at + 8));
+            if (ch == 3) dhi = __ldg(reinterpret_cast<const float4*>(part ? at : at + 8) + 1);
+            if (part == 0 && ch == 0) {
               CNN_PHASE(2);
               mbar_wait_bounded(&sm.dc_free[h], ((unsigned)k & 1u) ^ 1u, status, gave_up);
               CNN_PHASE(3);
             }
-            unsigned char* dst = sb.dc[h][0] + (unsigned)(4 * group + ch) * kTwDcChunk + (unsigned)(quarter * 32 + lane) * 16u;
+            unsigned char* dst = sb.dc[h][0] + (unsigned)((m0 & 31) / 2 + 4 * part + ch) * kTwDcChunk + (unsigned)(quarter * 32 + lane) * 16u;
             *reinterpret_cast<uint4*>(dst) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
             if (PASSES == 3) *reinterpret_cast<uint4*>(dst + kTwDcPart) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
           }
-          if (ch < 3) tc::tmem_wait8(nxt);
+          if ((BWD && part == 0) || ch < 3) tc::tmem_wait8(nxt);
         }
-        CNN_PHASE(4);
-        if constexpr (BWD) {
-          tc::fence_async_smem();      // generic-proxy writes -> visible to the tensor core's operand reads
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&sm.dc_full[h]);
-        } else {
+        if constexpr (!BWD) {
           // the window's four rows are four neighbouring lanes: reduce-scatter, lane r ends with maps 4 (r & 1) + 2 (r >> 1) + {0, 1}
           float w4[4], w2[2];
 #pragma unroll
@@ -548,12 +552,16 @@ k_wide_tc(WideDims d, long n, const float* __restrict__ images, const float* __r
             w2[i] = keep + __shfl_xor_sync(0xffffffffu, send, 2);
           }
           if (live)
-            *reinterpret_cast<float2*>(at + 32 * h + (b0 ? 4 : 0) + (b1 ? 2 : 0)) =
+            *reinterpret_cast<float2*>(at + kPartMaps * part + (b0 ? 4 : 0) + (b1 ? 2 : 0)) =
                 make_float2(sigmoidf<FL>(w2[0] + sm.bs), sigmoidf<FL>(w2[1] + sm.bs));
         }
-        CNN_PHASE(5);
       }
-      if (!BWD) {
+      CNN_PHASE(4);
+      if (BWD) {
+        tc::fence_async_smem();        // generic-proxy writes -> visible to the tensor core's operand reads
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&sm.dc_full[h]);
+      } else {
         at += d.F;
         if (++q == d.P) {
           q = 0;
@@ -561,18 +569,19 @@ k_wide_tc(WideDims d, long n, const float* __restrict__ images, const float* __r
           place();
         }
       }
+      CNN_PHASE(5);
     }
     if constexpr (BWD) {
-      // conv bias: sum over the quarter's rows; lane 8 h + 2 ch + parity ends with that map's
+      // conv bias: sum over the quarter's rows; lane i ends with map m0 + i's
       float v[32];
 #pragma unroll
       for (int i = 0; i < 16; i += 2) {
-        unpack2(gb2[i >> 3][(i & 7) >> 1], v[i], v[i + 1]);
+        unpack2(gb2[i >> 1], v[i], v[i + 1]);
         v[16 + i] = v[17 + i] = 0.f;
       }
       const float mine = warp_reduce_scatter32(v, lane) * pow2i(-dc_exp);
       const size_t cta = (size_t)(blockIdx.y * gridDim.x + blockIdx.x) * kTwPartB;
-      if (lane < 16) part_b[cta + quarter * kTwF + 32 * (lane >> 3) + 8 * group + (lane & 7)] = mine;
+      if (lane < 16) part_b[cta + quarter * kTwF + m0 + lane] = mine;
       // subsample filter: taps of row rsub, then the sum of delta_s
       float s5[5], x, yv;
 #pragma unroll
