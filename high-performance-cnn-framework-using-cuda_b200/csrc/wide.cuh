@@ -46,7 +46,7 @@ struct WideWork {
   size_t floats = 0;
 };
 
-constexpr int kTwPrepBlocks = 256;
+constexpr int kTwPrepBlocks = 592;             // four per SM: the pixels of a large batch are read with enough loads under way
 constexpr int kTwF = 64;                       // maps of a tensor-core CTA (more maps: more CTAs)
 constexpr int kTwGradN = 48;                   // (i, c): six kernel rows of eight columns
 constexpr int kTwGradCols = 4 * kTwF;          // (x, f)

@@ -114,6 +114,7 @@ k_wide_prep(WideDims d, const float4* __restrict__ images, long quads, const flo
   float m = 0.f;
   pdl_launch_dependents();
   pdl_wait();
+#pragma unroll 4
   for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < quads; i += (long)gridDim.x * blockDim.x) {
     const float4 v = __ldg(images + i);
     const float a[4] = {fabsf(v.x), fabsf(v.y), fabsf(v.z), fabsf(v.w)};
