@@ -57,7 +57,7 @@ SIGMOID_NAMES = {0: "reference expression (expf + IEEE divide)",
                  1: "short form: ex2.approx + rcp.approx (~1e-6 rel per evaluation)"}
 
 # dram__bytes_read.sum + dram__bytes_write.sum of one launch over 65,536 images, per forward path,
-# from the ncu captures summarised under profiles/ (k_fused_forward_*, k_forward_tc_*).
+# from the ncu captures summarised under profiles/ (kernels_per_case.md).
 TRAFFIC_BYTES_PER_LAUNCH = {0: 210611456, 1: 211582976, 2: 211068160}
 
 
