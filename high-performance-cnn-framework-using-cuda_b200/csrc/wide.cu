@@ -262,11 +262,12 @@ k_wide_fc_fwd(WideDims d, long n, int sets, const float* __restrict__ as, const 
 // Thread = one s; the batch is cut into kWideFcSplit contiguous slices (blockIdx.y), each of which writes partial sums of
 // G_wf that k_wide_reduce adds in order, so the result does not depend on scheduling.  The ten weights and ten sums stay
 // in registers, the images' output deltas come from shared memory.  Bound by memory: as in, ds out (88 MB for 1,024 images of
-// S = 10,816; two kernels that each read as took 65 us, this one 30).
+// S = 10,816; two kernels that each read as took 65 us, this one 28 with four
+// images' loads under way and about 24 with eight, for which it needs more than the 48 registers that the compiler would take).
 constexpr int kWideFcSplit = 16;
 constexpr int kWideBpImgs = 64;          // images whose output deltas are staged at a time
 
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(128, 6)
 k_wide_bp_fc(WideDims d, long n, const float* __restrict__ as, const float* __restrict__ delta_f,
              const float* __restrict__ wf, float* __restrict__ ds, float* __restrict__ part_f, float* __restrict__ ds_max) {
   __shared__ __align__(16) float dlt[kWideBpImgs][12];
@@ -291,7 +292,7 @@ k_wide_bp_fc(WideDims d, long n, const float* __restrict__ as, const float* __re
     if (!live) continue;
     const float* src = as + (size_t)c0 * d.S + s;
     float* dst = ds + (size_t)c0 * d.S + s;
-#pragma unroll 4
+#pragma unroll 8
     for (int g = 0; g < imgs; ++g) {
       const float a = src[(size_t)g * d.S];
       const f32x2 a2 = pack2(a, a);
