@@ -568,7 +568,8 @@ static int wide_reserve(cnn_wide* w, long n, bool training, bool tc, WideWork& k
     };
     take(k.as, (size_t)d.S * n);
     if (tc) {
-      take(k.pixel_max, kTwPrepBlocks);
+      take(k.img_max, n);
+      take(k.scale_of, 4 * (d.F / kTwF));
       take(k.wf_t, (size_t)kOut * d.S);
     }
     if (training) {

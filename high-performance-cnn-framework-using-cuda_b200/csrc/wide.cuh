@@ -11,7 +11,7 @@ struct WideDims {
   int o_wc, o_bc, o_ws, o_bs, o_wf, o_bf, n_params, n_padded;
 };
 
-inline WideDims make_wide_dims(int H, int F) {
+__host__ __device__ inline WideDims make_wide_dims(int H, int F) {
   WideDims d;
   d.H = H; d.F = F; d.C = H - 4; d.P = d.C / 4; d.S = F * d.P * d.P;
   d.o_wc = 0; d.o_bc = d.o_wc + F * 25; d.o_ws = d.o_bc + F; d.o_bs = d.o_ws + 16;
@@ -41,7 +41,8 @@ struct WideWork {
   float *part_c = nullptr, *part_s = nullptr;            // SIMT training: rows of [F][26] and of [17]
   float *part_f = nullptr;      // FC weight-gradient partials of the batch slices
   float *ds_max = nullptr;      // tensor-core training: largest |ds| per block of the kernel that writes it
-  float *pixel_max = nullptr, *wf_t = nullptr;           // tensor-core path: largest pixels per block; FC weights [output][window][map]
+  float *img_max = nullptr, *scale_of = nullptr;         // tensor-core path: largest pixel of each image; what the scales follow (k_wide_tc)
+  float *wf_t = nullptr;                                 // tensor-core path: FC weights [output][window][map]
   float *part_g = nullptr, *part_b = nullptr;            // tensor-core training: see k_wide_tc
   size_t floats = 0;
 };
@@ -52,7 +53,7 @@ constexpr int kTwGradN = 48;                   // (i, c): six kernel rows of eig
 constexpr int kTwGradCols = 4 * kTwF;          // (x, f)
 constexpr int kTwPartB = 4 * kTwF + 20;        // floats of a CTA's bias and subsample-filter sums
 
-// Tensor-core path (wide_tc.cu).  Forward: w.pixel_max, w.wf_t, w.as from the images.  Backward: from the images, w.ds and w.ds_max
+// Tensor-core path (wide_tc.cu).  Forward: w.img_max, w.scale_of, w.wf_t, w.as from the images.  Backward: from these, w.ds and w.ds_max
 // to w.part_g and w.part_b, of *ctas CTAs for each kTwF maps.
 bool wide_tc_supported(const WideDims& d);
 int wide_tc_max_ctas();

@@ -27,6 +27,16 @@
 // the batch's subsample deltas (k_wide_bp_fc); they are undone exactly.  (tf32 operands need twice the MMAs, and deltas
 // in a layout that costs one 4-byte store per value and part.)
 //
+// One scale serves all images of a call, so an image may not be so bright that it takes the others' pixels out of fp16's
+// range.  What the parts of a scaled pixel lose is 2^-25, and the largest is scaled to 2^14 at least; so an image takes part if its
+// largest pixel is at most
+//   * 2^(10 - E), 2^E <= the largest weight (with the short sigmoid's factor) < 2^(E + 1): then the scale is 2^(E + 4) at least, and what any
+//     pixel loses is below 2^-23 in any pre-activation; or
+//   * 2^12 times the smallest (non-zero) largest pixel of an image: then no image's pixels lose more than 2^-27 of its own largest.
+// Every other image -- and one with a pixel that is not finite; all images, if a weight or delta is 2^60 or more -- is left out
+// by loaders and epilogue and computed in plain fp32 at the end of the kernel, by the CTAs in turn (wide_plain_image; 56x56 with 64 maps: 60 us
+// forward, 220 us for a gradient, per CTA and image; 1,024 images of which 1,023 go that way 1.8 ms, against 0.34 ms and the fp32 kernels' 0.69).
+//
 // One CTA per SM, 24 warps (80 registers), hand-overs by mbarriers with bounded waits:
 //   warps 0-6   load a unit's rows (32 bytes per thread, one unit ahead in registers), split them and store the slab;
 //               backward: warps 0-3 also drain the gradient accumulators, of which two sets alternate (374 us against 386 for a
@@ -77,7 +87,9 @@ struct TwSmem {
   float bs;
   unsigned long long a_full[kTwSlabs], a_free[kTwSlabs], d_full[kTwAccMax], d_free[kTwAccMax];
   unsigned long long dc_full[2], dc_free[2], g_full[2], g_free[2];  // backward: deltas of a half, sets of gradient accumulators
-  float max_of[3][kTwThreads / 32];                                 // largest tap, pixel, subsample delta by warp
+  float max_of[4][kTwThreads / 32];                                 // largest tap, pixel, subsample delta, by warp; smallest pixel maximum
+  float limit;                                                      // images with larger pixels are computed in plain fp32 ...
+  int any_plain;                                                    // ... and there are some
   unsigned tmem_base;
   long long clock_base;                                             // phase clocks only
 };
@@ -105,44 +117,163 @@ __device__ __forceinline__ int exponent_of(float v) {
 __device__ __forceinline__ void red_add(float* p, float v) { asm volatile("red.global.add.f32 [%0], %1;" ::"l"(p), "f"(v) : "memory"); }
 __device__ __forceinline__ float pow2i(int e) { return __int_as_float((127 + e) << 23); }
 
-// What the tensor-core kernels need of a batch beforehand: per-block maxima of the (finite) pixel magnitudes, and the FC weights
-// in the order in which those kernels have the subsample activations, [window][map] instead of [map][window].
+// What the tensor-core kernels need of a batch beforehand: every image's largest pixel magnitude (not a number, if it has such a
+// pixel), and the FC weights in the order in which those kernels have the subsample activations, [window][map] instead of
+// [map][window].  A team of threads per image, as many as make its pixels eight loads of 16 bytes per thread at most, all under way at once.
 __global__ void __launch_bounds__(256)
-k_wide_prep(WideDims d, const float4* __restrict__ images, long quads, const float* __restrict__ params, float* __restrict__ pixel_max,
-            float* __restrict__ wf_t) {
-  __shared__ float red[8];
-  float m = 0.f;
+k_wide_prep(WideDims d, long n, int team, const float4* images, const float* params, float* __restrict__ img_max, float* __restrict__ wf_t) {
+  __shared__ unsigned red[8];
   pdl_launch_dependents();
   pdl_wait();
-#pragma unroll 4
-  for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < quads; i += (long)gridDim.x * blockDim.x) {
-    const float4 v = __ldg(images + i);
-    const float a[4] = {fabsf(v.x), fabsf(v.y), fabsf(v.z), fabsf(v.w)};
+  const int quads = d.H * d.H / 4, teams = 256 / team, mine = threadIdx.x / team, at = threadIdx.x % team;
+  for (long b0 = (long)blockIdx.x * teams; b0 < n; b0 += (long)gridDim.x * teams) {
+    const long b = b0 + mine;
+    const float4* src = images + (size_t)(b < n ? b : 0) * quads;
+    unsigned m = 0;                    // magnitudes compared as integers: what is not a number is above infinity
+    for (int i0 = at; i0 < quads; i0 += 8 * team) {
+      float4 v[8];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) m = (a[k] <= 3.4e38f) ? fmaxf(m, a[k]) : m;
+      for (int j = 0; j < 8; ++j) v[j] = src[i0 + j * team < quads ? i0 + j * team : i0];
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        m = max(max(m, max(__float_as_uint(v[j].x) & 0x7fffffffu, __float_as_uint(v[j].y) & 0x7fffffffu)),
+                max(__float_as_uint(v[j].z) & 0x7fffffffu, __float_as_uint(v[j].w) & 0x7fffffffu));
+    }
+    m = __reduce_max_sync(0xffffffffu, m);
+    if (team > 32) {
+      if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
+      __syncthreads();
+      if (at == 0)
+        for (int k = 1; k < team / 32; ++k) m = max(m, red[(threadIdx.x >> 5) + k]);
+      __syncthreads();
+    }
+    if (at == 0 && b < n) img_max[b] = __uint_as_float(m);
   }
-  m = warp_max(m);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
   const int W = d.P * d.P;
   for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < (long)kOut * d.S; i += (long)gridDim.x * blockDim.x) {
     const int k = (int)(i / d.S), s = (int)(i - (long)k * d.S);
     wf_t[i] = params[d.o_wf + (size_t)k * d.S + (size_t)(s % d.F) * W + s / d.F];
   }
+}
+
+// The way out for an image whose pixels do not fit the batch's scale: plain fp32 by all threads of a CTA, for its 64 maps from f0 on.  Out of
+// line and with rolled loops: what it needs of registers and stack the hot code would pay for.  Thread = map and every twelfth window of a row of
+// windows, taps from shared memory.  Forward: the image's subsample activations as[window][map].  Backward: reads ds[window][map] and adds the image's
+// share to the CTA's sums, in a fixed order and their layouts (a filter tap (i, j) goes to x = 0, c = j of D).  The deltas of a row of windows go through
+// shared memory, where a thread has a map, a tap row (or the bias) and every other row of deltas.
+constexpr int kTwPlainTeams = kTwThreads / kTwF;                    // 12 = 2 halves of 5 tap rows and the bias
+constexpr int kTwPlainMaxP = 31;                                    // H = 128
+struct TwPlain {
+  float tap[25][kTwF];
+  float filter[kTwThreads / 32][17];                                // backward only from here on
+  alignas(16) float4 dc[kTwPlainMaxP * 4][kTwF];                    // [window column, its row][map]
+};
+static_assert(sizeof(TwPlain::tap) <= offsetof(TwSmem, bias) && sizeof(TwPlain) <= sizeof(TwBwdSmem), "space for wide_plain_image");
+
+template <int FL, bool BWD>
+__device__ __noinline__ void wide_plain_image(int H, int F, int f0, TwPlain& sm, const float* image, const float* params, float* as_or_ds,
+                                              float* part_g, float* part_b) {
+  const WideDims d = make_wide_dims(H, F);
+  const int tid = threadIdx.x, m = tid % kTwF, team = tid / kTwF;
+  __syncthreads();                     // (whatever was in sm has been used)
+  for (int e = tid; e < 25 * kTwF; e += kTwThreads) sm.tap[e / kTwF][e % kTwF] = params[d.o_wc + (f0 + e % kTwF) * 25 + e / kTwF];
   __syncthreads();
-  if (threadIdx.x == 0) {
+  const int half = team & 1, row = team >> 1;
+  float gs[17], g[5];
 #pragma unroll
-    for (int k = 1; k < 8; ++k) m = fmaxf(m, red[k]);
-    pixel_max[blockIdx.x] = m;
+  for (int t = 0; t < 17; ++t) gs[t] = 0.f;
+#pragma unroll
+  for (int j = 0; j < 5; ++j) g[j] = 0.f;
+  auto pixels = [&](int y, int q, float (&v)[8]) {
+    const float4* src = reinterpret_cast<const float4*>(image + y * H + 4 * q);
+    const float4 lo = src[0], hi = src[1];
+    v[0] = lo.x; v[1] = lo.y; v[2] = lo.z; v[3] = lo.w;
+    v[4] = hi.x; v[5] = hi.y; v[6] = hi.z; v[7] = hi.w;
+  };
+#pragma unroll 1
+  for (int p = 0; p < d.P; ++p) {
+#pragma unroll 1
+    for (int q = team; q < d.P; q += kTwPlainTeams) {
+      float* at = as_or_ds + (size_t)(p * d.P + q) * F + f0 + m;
+      float z = params[d.o_bs];
+      const float dl = BWD ? *at : 0.f, dlc = dl / (float)(d.C * d.C), bias = params[d.o_bc + f0 + m];
+      gs[16] += dl;
+      float a[4][4], v[8];
+#pragma unroll
+      for (int o = 0; o < 16; ++o) a[o / 4][o % 4] = bias;
+#pragma unroll 1
+      for (int i = 0; i < 5; ++i)
+#pragma unroll
+        for (int y = 0; y < 4; ++y) {
+          pixels(4 * p + y + i, q, v);
+#pragma unroll
+          for (int j = 0; j < 5; ++j)
+#pragma unroll
+            for (int x = 0; x < 4; ++x) a[y][x] = fmaf(sm.tap[i * 5 + j][m], v[x + j], a[y][x]);
+        }
+#pragma unroll
+      for (int y = 0; y < 4; ++y) {
+        float dc[4];
+#pragma unroll
+        for (int x = 0; x < 4; ++x) {
+          const float av = sigmoidf<FL>(a[y][x]), w = params[d.o_ws + 4 * y + x];
+          z = fmaf(w, av, z);
+          gs[4 * y + x] = fmaf(dl, av, gs[4 * y + x]);
+          dc[x] = w * dlc * (av * (1.f - av));
+        }
+        if (BWD) sm.dc[4 * q + y][m] = make_float4(dc[0], dc[1], dc[2], dc[3]);
+      }
+      if (!BWD) *at = sigmoidf<FL>(z);
+    }
+    if (!BWD) continue;
+    __syncthreads();
+#pragma unroll 1
+    for (int e = half; e < 4 * d.P; e += 2) {
+      const float4 dc = sm.dc[e][m];
+      if (row == 5) {
+        g[0] += (dc.x + dc.y) + (dc.z + dc.w);
+      } else {
+        float v[8];
+        pixels(4 * p + e % 4 + row, e / 4, v);
+#pragma unroll
+        for (int j = 0; j < 5; ++j) g[j] = fmaf(dc.w, v[j + 3], fmaf(dc.z, v[j + 2], fmaf(dc.y, v[j + 1], fmaf(dc.x, v[j], g[j]))));
+      }
+    }
+    __syncthreads();
+  }
+  if (!BWD) return;
+#pragma unroll 1
+  for (int h = 0; h < 2; ++h) {        // one half after the other: the same addresses
+    if (h == half) {
+      if (row == 5) part_b[m] += g[0];
+      else
+#pragma unroll
+        for (int j = 0; j < 5; ++j) red_add(part_g + (row * 8 + j) * kTwGradCols + 8 * (m >> 1) + (m & 1), g[j]);
+    }
+    __syncthreads();
+  }
+#pragma unroll
+  for (int t = 0; t < 17; ++t) {
+#pragma unroll
+    for (int k = 16; k > 0; k >>= 1) gs[t] += __shfl_xor_sync(0xffffffffu, gs[t], k);
+    if ((tid & 31) == 0) sm.filter[tid >> 5][t] = gs[t];
+  }
+  __syncthreads();
+  if (tid < 17) {
+    float sum = 0.f;
+    for (int k = 0; k < kTwThreads / 32; ++k) sum += sm.filter[k][tid];
+    part_b[4 * kTwF + tid] += tid == 16 ? sum / (float)d.S : sum;
   }
 }
 
 // FL: sigmoid flavour.  PASSES: 3 or 1.  BWD: false = forward (writes as), true = backward (reads ds, writes the partial gradients).
 // as, ds: [image][window][map].  part_g: per CTA (of all map groups) [kTwGradN][256] sums of D; part_b: per CTA [4][64] conv bias
-// sums (a row per quarter of the rows) and the 17 subsample-filter sums behind them.
+// sums (a row per quarter of the rows) and the 17 subsample-filter sums behind them.  scale_of: of each map group {limit, largest
+// pixel within it, largest of all}, from the forward kernel for the backward kernel.
 template <int FL, int PASSES, bool BWD>
 __global__ void __launch_bounds__(kTwThreads, 1)
-k_wide_tc(WideDims d, long n, const float* __restrict__ images, const float* __restrict__ params, const float* __restrict__ pixel_max,
-          float* __restrict__ as, const float* __restrict__ ds, const float* __restrict__ ds_max, int ds_blocks,
+k_wide_tc(WideDims d, long n, const float* __restrict__ images, const float* __restrict__ params, const float* img_max,
+          float* scale_of, float* __restrict__ as, const float* __restrict__ ds, const float* __restrict__ ds_max, int ds_blocks,
           float* __restrict__ part_g, float* __restrict__ part_b, int* __restrict__ status) {
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem_base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~(uintptr_t)127);
@@ -182,27 +313,57 @@ k_wide_tc(WideDims d, long n, const float* __restrict__ images, const float* __r
   pdl_wait();
 
   // ---- scales: taps to 256..512, pixels to 2^14..2^15 at most ------------------------------------------------
-  float wmax = 0.f, pmax = 0.f, dmax = 0.f;
+  float wmax = 0.f, dmax = 0.f, pmax = 0.f, pmin = INFINITY;       // (pmax: what is not finite counts as infinite)
   for (int i = tid; i < kTwF * 25; i += kTwThreads) {
     const float a = fabsf(kPre * params[d.o_wc + f0 * 25 + i]);
-    wmax = (a <= 3.4e38f) ? fmaxf(wmax, a) : wmax;
+    wmax = (a <= 3.4e38f) ? fmaxf(wmax, a) : INFINITY;
   }
-  if (tid < kTwPrepBlocks) pmax = pixel_max[tid];
-  if (BWD)
+  if (BWD) {
     for (int i = tid; i < ds_blocks; i += kTwThreads) dmax = fmaxf(dmax, ds_max[i]);
+  } else {
+#pragma unroll 4
+    for (long b = tid; b < n; b += kTwThreads) {
+      const float m = img_max[b];
+      pmax = m <= 3.4e38f ? fmaxf(pmax, m) : INFINITY;
+      pmin = m > 0.f ? fminf(pmin, m) : pmin;
+    }
+  }
   wmax = warp_max(wmax);
-  pmax = warp_max(pmax);
   dmax = warp_max(dmax);
+  pmax = warp_max(pmax);
+  pmin = -warp_max(-pmin);
   if (lane == 0) {
     sm.max_of[0][warp] = wmax;
     sm.max_of[1][warp] = pmax;
     sm.max_of[2][warp] = dmax;
+    sm.max_of[3][warp] = pmin;
   }
   __syncthreads();
   const int mine_at = lane < kTwThreads / 32 ? lane : 0;
   wmax = warp_max(sm.max_of[0][mine_at]);
-  pmax = warp_max(sm.max_of[1][mine_at]);
   dmax = warp_max(sm.max_of[2][mine_at]);
+  // The images that take part (see above), and the largest pixel among them.
+  constexpr float kHuge = 1152921504606846976.f;                   // 2^60
+  float limit, all;
+  if (BWD) {
+    limit = scale_of[4 * blockIdx.y];
+    pmax = scale_of[4 * blockIdx.y + 1];
+    all = scale_of[4 * blockIdx.y + 2];
+  } else {
+    all = pmax = warp_max(sm.max_of[1][mine_at]);
+    pmin = -warp_max(-sm.max_of[3][mine_at]);
+    limit = wmax < kHuge ? fminf(fmaxf(pow2i(10 - exponent_of(wmax)), 4096.f * pmin), kHuge) : -1.f;
+    if (!(all <= limit)) {
+      pmax = 0.f;
+      for (long b = tid; b < n; b += kTwThreads) pmax = img_max[b] <= limit ? fmaxf(pmax, img_max[b]) : pmax;
+      pmax = warp_max(pmax);
+      __syncthreads();
+      if (lane == 0) sm.max_of[1][warp] = pmax;
+      __syncthreads();
+      pmax = warp_max(sm.max_of[1][mine_at]);
+    }
+    if (blockIdx.x == 0 && tid < 3) scale_of[4 * blockIdx.y + tid] = tid == 0 ? limit : (tid == 1 ? pmax : all);
+  }
   const int we = 8 - exponent_of(wmax), pe = 14 - exponent_of(pmax);
   const int back = -(we + pe);
   const float w_scale = pow2i(we), px_scale = pow2i(pe), unscale = pow2i(back < -126 ? -126 : (back > 126 ? 126 : back));
@@ -214,6 +375,14 @@ k_wide_tc(WideDims d, long n, const float* __restrict__ images, const float* __r
     for (int k = 8; k > 0; k >>= 1) ws_max = fmaxf(ws_max, __shfl_xor_sync(0xffffffffu, ws_max, k));
     dc_exp = 14 - exponent_of(ws_max / (float)(d.C * d.C)) - exponent_of(dmax);
     dc_exp = dc_exp > 100 ? 100 : (dc_exp < -100 ? -100 : dc_exp);
+    if (!(dmax < kHuge && ws_max < kHuge)) {
+      limit = -1.f;
+      dc_exp = 0;
+    }
+  }
+  if (tid == 0) {
+    sm.limit = limit;
+    sm.any_plain = !(all <= limit);
   }
 
   // ---- weights: step s holds kernel rows 2 s and 2 s + 1, chunk = kernel row, row = accumulator column -----------
@@ -222,7 +391,7 @@ k_wide_tc(WideDims d, long n, const float* __restrict__ images, const float* __r
     const int f = 2 * (col >> 3) + (col & 1), x = (col & 7) >> 1;
     float w[5];
 #pragma unroll
-    for (int t = 0; t < 5; ++t) w[t] = i < 5 ? kPre * params[d.o_wc + (f0 + f) * 25 + (i < 5 ? i : 0) * 5 + t] : 0.f;
+    for (int t = 0; t < 5; ++t) w[t] = i < 5 && wmax < kHuge ? kPre * params[d.o_wc + (f0 + f) * 25 + (i < 5 ? i : 0) * 5 + t] : 0.f;
     __half2 hi[4], lo[4];
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
@@ -256,12 +425,14 @@ k_wide_tc(WideDims d, long n, const float* __restrict__ images, const float* __r
     const bool mine = tid < kTwRows;
     float4 v0, v1;
     bool have;
+    float most;                        // the image's largest pixel
     const float* src;
     unsigned G = set0 * kTwGroups + (mine ? g : 0);
     auto place = [&]() {
       const unsigned b = G / (unsigned)gi;
       const int y = 8 * (int)(G - b * (unsigned)gi) + row;
       have = mine && b < n && y < d.H;
+      most = img_max[have ? b : 0];
       src = images + ((size_t)(have ? b : 0) * d.H + (have ? y : 0)) * d.H;
     };
     auto load = [&](int q) {           // (clamped, not conditional: a load under a condition is waited for on the spot)
@@ -306,10 +477,11 @@ k_wide_tc(WideDims d, long n, const float* __restrict__ images, const float* __r
       // (the slab is free: the gradients of the unit that had it are complete, and with the last unit of a set the set)
       if (BWD && k >= kTwSlabs && (k - kTwSlabs) % kTwFlush == kTwFlush - 1) flush((k - kTwSlabs) / kTwFlush);
       __half2 hi[4], lo[4];
-      tc::split_f16x2(have ? v0.x : 0.f, have ? v0.y : 0.f, px_scale, hi[0], lo[0]);
-      tc::split_f16x2(have ? v0.z : 0.f, have ? v0.w : 0.f, px_scale, hi[1], lo[1]);
-      tc::split_f16x2(have ? v1.x : 0.f, have ? v1.y : 0.f, px_scale, hi[2], lo[2]);
-      tc::split_f16x2(have ? v1.z : 0.f, have ? v1.w : 0.f, px_scale, hi[3], lo[3]);
+      const bool in = have && most <= limit;
+      tc::split_f16x2(in ? v0.x : 0.f, in ? v0.y : 0.f, px_scale, hi[0], lo[0]);
+      tc::split_f16x2(in ? v0.z : 0.f, in ? v0.w : 0.f, px_scale, hi[1], lo[1]);
+      tc::split_f16x2(in ? v1.x : 0.f, in ? v1.y : 0.f, px_scale, hi[2], lo[2]);
+      tc::split_f16x2(in ? v1.z : 0.f, in ? v1.w : 0.f, px_scale, hi[3], lo[3]);
       if (mine) {
         *reinterpret_cast<uint4*>(sm.slab[s][0] + tid * 16) = *reinterpret_cast<uint4*>(hi);
         if (PASSES == 3) *reinterpret_cast<uint4*>(sm.slab[s][1] + tid * 16) = *reinterpret_cast<uint4*>(lo);
@@ -414,11 +586,11 @@ k_wide_tc(WideDims d, long n, const float* __restrict__ images, const float* __r
     int q = (int)q0;
     unsigned G = set0 * kTwGroups + quarter * 4 + (lane >> 3);
     bool live;
-    float* at;                       // this lane's window and maps in as / ds; of a window that does not exist: the zeros behind ds
+    float* at;                       // this lane's window and maps in as / ds; of one that does not take part: the zeros behind ds
     auto place = [&]() {
       const unsigned b = G / (unsigned)gi;
       const int p = (8 * (int)(G - b * (unsigned)gi) + (lane & 7)) >> 2;      // C is a multiple of 4: a window's rows are all in or all out
-      live = b < n && p < d.P;
+      live = b < n && p < d.P && img_max[b < n ? b : 0] <= sm.limit;
       const size_t window = live ? ((size_t)b * d.P + p) * d.P + q : (BWD ? (size_t)n * d.P * d.P : 0);
       at = (BWD ? const_cast<float*>(ds) : as) + window * d.F + f0 + m0;
     };
@@ -608,11 +780,22 @@ k_wide_tc(WideDims d, long n, const float* __restrict__ images, const float* __r
   tc::fence_before_sync();
   __syncthreads();
   if (warp == kTwMmaWarp) tc::tmem_dealloc(tmem_base, 512);
+  const size_t cta = blockIdx.y * gridDim.x + blockIdx.x;
   if (BWD && tid < 17) {
     float sum = 0.f;
 #pragma unroll
     for (int w = 0; w < kTwEpiWarps; ++w) sum += sb.red[w][tid];
-    part_b[(size_t)(blockIdx.y * gridDim.x + blockIdx.x) * kTwPartB + 4 * kTwF + tid] = tid == 16 ? sum / (float)d.S : sum;
+    part_b[cta * kTwPartB + 4 * kTwF + tid] = tid == 16 ? sum / (float)d.S : sum;
+  }
+  if (sm.any_plain) {
+    const float top = sm.limit;
+#pragma unroll 1
+    for (long b = blockIdx.x; b < n; b += gridDim.x) {
+      if (img_max[b] <= top) continue;
+      wide_plain_image<FL, BWD>(d.H, d.F, f0, *reinterpret_cast<TwPlain*>(smem_base), images + (size_t)b * d.H * d.H, params,
+                                (BWD ? const_cast<float*>(ds) : as) + (size_t)b * d.P * d.P * d.F, part_g + cta * kTwGradN * kTwGradCols,
+                                part_b + cta * kTwPartB);
+    }
   }
 }
 
@@ -629,7 +812,7 @@ static int launch_wide_tc(cnn_wide* w, const WideWork& k, const float* d_images,
   const size_t smem = (BWD ? sizeof(TwBwdSmem) : sizeof(TwSmem)) + 128;
   CNN_CUDA(cudaFuncSetAttribute(k_wide_tc<FL, PASSES, BWD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   cudaError_t e = launch_pdl(k_wide_tc<FL, PASSES, BWD>, dim3((unsigned)wide_tc_grid(d, n), (unsigned)(d.F / kTwF)), dim3(kTwThreads), smem, st, d, n,
-                             d_images, (const float*)w->d_params, (const float*)k.pixel_max, k.as, (const float*)k.ds,
+                             d_images, (const float*)w->d_params, (const float*)k.img_max, k.scale_of, k.as, (const float*)k.ds,
                              (const float*)k.ds_max, ds_blocks, k.part_g, k.part_b, w->d_status);
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e, "k_wide_tc launch");
@@ -650,8 +833,10 @@ static int launch_wide_tc(cnn_wide* w, const WideWork& k, const float* d_images,
 
 int wide_tc_forward(cnn_wide* w, const WideWork& k, const float* d_images, long n, cudaStream_t st) {
   const WideDims& d = w->d;
-  cudaError_t e = launch_pdl(k_wide_prep, dim3(kTwPrepBlocks), dim3(256), 0, st, d, reinterpret_cast<const float4*>(d_images),
-                             n * d.H * d.H / 4, (const float*)w->d_params, k.pixel_max, k.wf_t);
+  int team = 32;
+  while (team < 256 && 8 * team < d.H * d.H / 4) team *= 2;
+  cudaError_t e = launch_pdl(k_wide_prep, dim3(kTwPrepBlocks), dim3(256), 0, st, d, n, team, reinterpret_cast<const float4*>(d_images),
+                             (const float*)w->d_params, k.img_max, k.wf_t);
   if (e != cudaSuccess) return cuda_fail(e, "k_wide_prep launch");
   CNN_WIDE_TC(false, w, k, d_images, n, 0, st);
 }

@@ -219,3 +219,64 @@ def test_wide_full_batch_matches_oracle(cuda, pkg, ob, mode):
         print("  %s: library %.3e, fp32 oracle %.3e (against the fp64 oracle)" % (name, e_lib, e_or))
         assert e_lib < max(1e-5, 2 * e_or), name
     assert abs(g[net.n_params + 1] - err64) < 1e-5 * max(err64, 1.0)
+
+
+@pytest.mark.parametrize("what", ["bright images", "all but one bright", "not finite", "huge filter", "huge FC weights", "dim"])
+@pytest.mark.parametrize("mode", [1, 2])
+@pytest.mark.parametrize("H,F,n", [(56, 64, 40), (8, 128, 301)])
+def test_tensor_core_images_do_not_depend_on_their_neighbours(cuda, pkg, ob, H, F, n, mode, what):
+    """One power of two scales the pixels of a call, so an image much brighter than others (or not finite) has to leave them
+    untouched and come out right itself: both for the outputs, image by image, and for the gradient.  Weights of any magnitude
+    too.  Yardstick: the fp64 oracle, which computes each image by itself, within the tolerance of the mode or four times the fp32
+    kernels' own distance from it (pixels of 30,000 leave few bits to sums that a sigmoid does not saturate); where its values
+    are not finite, the fp32 kernels."""
+    x, labels = wide_inputs(n, H, 11)
+    params = wide_params(ob, H, F, 12)
+    S = F * ((H - 4) // 4) ** 2
+    fc = slice(F * 26 + 17, F * 26 + 17 + 10 * S)
+    spots = [0, n // 2, n - 1]
+    if what == "bright images":
+        x[spots[0], 3, 3], x[spots[1], H - 1, H - 1], x[spots[2], 4, 5] = 1e6, 1e30, -4e5
+    elif what == "all but one bright":
+        x[1:] *= np.float32(3e4)
+    elif what == "not finite":
+        x[spots[0], 3, 3], x[spots[1], 2, 2], x[spots[2], 4, 5] = np.nan, np.inf, -np.inf
+    elif what == "huge filter":
+        params[:F * 25] *= np.float32(1e25)
+        x *= np.float32(1e-25)
+    elif what == "huge FC weights":
+        params[fc] *= np.float32(1e22)
+    elif what == "dim":
+        x[1:] *= np.float32(1e-3)
+        x[spots[1]] = 0
+    net = pkg.WideNet(H, F)
+    net.set_params(params)
+    d_x = cuda.from_numpy(x).cuda()
+    d_lab = cuda.from_numpy(labels.astype(np.int32)).cuda()
+    outs, grads = {}, {}
+    for conv in (0, mode):
+        net.set_option("conv", conv)
+        d_out = cuda.empty((n, 10), dtype=cuda.float32, device="cuda")
+        d_g = cuda.zeros(net.n_padded, dtype=cuda.float32, device="cuda")
+        net.forward(d_x, n, d_out, None)
+        net.grad_batch(d_x, d_lab, n, d_g)
+        cuda.cuda.synchronize()
+        assert net.status() == 0
+        outs[conv], grads[conv] = d_out.cpu().numpy(), d_g.cpu().numpy()
+    tol = 1e-5 if mode == 2 else 3e-3
+    if what in ("not finite", "huge FC weights"):
+        ref, G = outs[0], grads[0]
+    else:
+        ref, _ = ob.forward_batch(params, x, H=H, F=F, dtype=np.float64)
+        G, _ = ob.grad_batch(params, x, labels, H=H, F=F, dtype=np.float64)
+    assert np.array_equal(np.isnan(outs[mode]), np.isnan(ref))
+    ok = ~np.isnan(ref).any(axis=1)
+    assert ok.sum() >= n - 3
+    e_tc, e_fp32 = (float(np.max(np.abs(outs[c][ok].astype(np.float64) - ref[ok]))) for c in (mode, 0))
+    assert e_tc < max(tol, 4 * e_fp32)
+    if what == "not finite":
+        return
+    for name, (lo, hi) in blocks(H, F).items():
+        e_tc, e_fp32 = scaled_err(grads[mode][lo:hi], G[lo:hi]), scaled_err(grads[0][lo:hi], G[lo:hi])
+        print("%s: tensor cores %.3e, fp32 kernels %.3e" % (name, e_tc, e_fp32))
+        assert e_tc < max(tol * (1 if mode == 2 else 10), 4 * e_fp32), name
