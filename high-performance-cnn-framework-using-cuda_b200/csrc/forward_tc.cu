@@ -27,8 +27,9 @@
 // epilogue's bias FMA): weights so that w lies between 256 and 512, pixels by more than 25 w, which keeps what a pixel's
 // parts lose (2^-25 of the scaled value, absolute) below 2^-24 in any pre-activation, whatever the pixels.  An image
 // with a scaled pixel of 65,520 or more (a pixel of 1,000 to 2,000 where w = 1: its pre-activations are no longer
-// of order one) is noticed by the loader, and a finisher warp computes it in plain fp32 instead (slow, 0.1 ms
-// per image; no image data is expected there).
+// of order one) is noticed by the loader, and a finisher warp computes it in plain fp32 instead (slow, 0.1 ms per image; no
+// image data is expected there).  uint8 pixels reach that limit only where w is above 1,000: the finishers look for themselves
+// then.  With a weight or a conv bias of 1e27 or more, or one that is not finite, all images go that way.
 // Path 2 uses the high parts only (11 significant bits, as tf32) and one special-function operation
 // per activation: outputs within about 1e-4, argmax equal wherever the top-two margin is clear of that.
 //
@@ -116,6 +117,9 @@ __device__ __forceinline__ float tanh_approx(float x) {
   return y;
 }
 
+// Group g of a CTA starts 224 g + 112 (g / 3) pixels into its images: 8 rows further per group, 12 more per image.
+__device__ __forceinline__ int group_pixel(int g) { return 8 * kH * g + 4 * kH * (g / kTfGroupsImg); }
+
 // Bounded spin on a counter in shared memory (same limit and status convention as mbar_wait_bounded).
 __device__ __forceinline__ void wait_counter_bounded(const int* counter, int at_least, int* status, bool& gave_up) {
   if (gave_up) return;
@@ -132,14 +136,15 @@ __device__ __forceinline__ void wait_counter_bounded(const int* counter, int at_
 
 // FC sums (without bias) of one image in plain fp32 by one warp, lane k < 10 returns sum k: the way out for images whose
 // pixels do not fit fp16.  Lanes own windows; kept out of line and rolled so that it costs the hot code nothing.
-template <int SIG>
-__device__ __noinline__ float image_fc_plain(const float* __restrict__ image, const float* __restrict__ params, int lane) {
+template <int SIG, typename Pixel>
+__device__ __noinline__ float image_fc_plain(const Pixel* image, const float* params, int lane) {
+  auto pixel = [](Pixel v) { return sizeof(Pixel) == 1 ? (float)((double)v / 255.0) : (float)v; };
   float mine = 0.f;
 #pragma unroll 1
   for (int w0 = 0; w0 < 36; w0 += 32) {
     const int w = w0 + lane;
     const bool live = w < 36;
-    const float* base = image + (live ? (4 * (w / 6)) * kH + 4 * (w % 6) : 0);
+    const Pixel* base = image + (live ? (4 * (w / 6)) * kH + 4 * (w % 6) : 0);
 #pragma unroll 1
     for (int f = 0; f < kF; ++f) {
       float zs = params[kOffBs];
@@ -148,7 +153,7 @@ __device__ __noinline__ float image_fc_plain(const float* __restrict__ image, co
         float acc = params[kOffBc + f];
 #pragma unroll 1
         for (int t = 0; t < 25; ++t)
-          acc = fmaf(params[kOffWc + f * 25 + t], base[(o / 4 + t / 5) * kH + o % 4 + t % 5], acc);
+          acc = fmaf(params[kOffWc + f * 25 + t], pixel(base[(o / 4 + t / 5) * kH + o % 4 + t % 5]), acc);
         zs = fmaf(params[kOffWs + o], sigmoidf<SIG>(acc), zs);
       }
       const float as = live ? sigmoidf<SIG>(zs) : 0.f;
@@ -162,6 +167,28 @@ __device__ __noinline__ float image_fc_plain(const float* __restrict__ image, co
     }
   }
   return mine;
+}
+
+// uint8 pixels where the parameters ask for the way out: white, at the scale that the weights set, is beyond fp16 (weights above 1,000), or, `all`,
+// the parameters are.  FC sums of the three images from `base` on (of a CTA's images; lane 10 j + k: sum k), `z` where the tensor core's
+// are right.  As the fp32 images' loader does, all images of a tile with a pixel out of range are taken -- noticed here, because in the
+// loader it cost 5 % of every call.
+template <int SIG>
+__device__ __noinline__ float finish_plain_u8(const unsigned char* pixels, const float* params, const unsigned* lut, int base, int imgs, bool all,
+                                              float z, int lane) {
+  for (int j = 0; j < 3 && base + j < imgs; ++j) {
+    const int g = (base + j) * kTfGroupsImg, end = imgs * kTfGroupsImg;
+    const int g0 = g / kTfGroups * kTfGroups, g1 = min(((g + kTfGroupsImg - 1) / kTfGroups + 1) * kTfGroups, end) - 1;      // of its tiles
+    unsigned most = 0;
+    for (int i = group_pixel(g0) / 4 + lane; i < (group_pixel(g1) + kTfGroupRows * kH) / 4; i += 32)
+      most = __vmaxu4(most, reinterpret_cast<const unsigned*>(pixels)[i]);
+    most = __reduce_max_sync(0xffffffffu, max(max(most & 255u, (most >> 8) & 255u), max((most >> 16) & 255u, most >> 24)));
+    if (!all && (lut[most] & 0xffffu) != 0x7c00u) continue;      // its high part is finite
+    const float s = image_fc_plain<SIG>(pixels + (size_t)(base + j) * kImg, params, lane);
+    const float sk = __shfl_sync(0xffffffffu, s, lane % 10);
+    if (lane / 10 == j) z = sk;
+  }
+  return z;
 }
 
 // PATH 1: three passes, sigmoid flavour SIG (0 or 1).  PATH 2: one pass, tanh sigmoid.  U8: `images` points at
@@ -213,8 +240,6 @@ k_forward_tc(const void* __restrict__ images, long n, long imgs_per_cta, const f
   // ---- loaders: the first copies leave now ------------------------------------------------------------------
   const int lt = tid - 32 * kTfLoadWarp0;
   const bool loader = lt >= 0 && lt < kTfLoaders;
-  // group g of this CTA starts 224 g + 112 (g / 3) pixels into its images: 8 rows further per group, 12 more per image
-  auto group_pixel = [](int g) { return 8 * kH * g + 4 * kH * (g / kTfGroupsImg); };
   auto fetch = [&](int k) {       // one thread: the rows of tile k, from its first group's first to its last group's twelfth
     constexpr unsigned kBytes = U8 ? 1u : 4u;
     const int g0 = k * kTfGroups, g1 = min(g0 + kTfGroups, n_groups) - 1;
@@ -236,7 +261,7 @@ k_forward_tc(const void* __restrict__ images, long n, long imgs_per_cta, const f
     const int e = lane + 32 * j;      // the 150 weights and 6 biases
     if (e < kOffBc + kF) {
       const float a = fabsf(params[e]);
-      finite = finite && (a <= 3.402823466e38f);
+      finite = finite && (a <= 1e27f);      // (below 2^90: the weights' exponent is not clamped)
       if (e < kOffBc) wmax = fmaxf(wmax, a);
     }
   }
@@ -345,18 +370,17 @@ k_forward_tc(const void* __restrict__ images, long n, long imgs_per_cta, const f
 #pragma unroll
         for (int kk = 0; kk < kOut / 2; ++kk) unpack2(fc2[j][kk], sums[10 * j + 2 * kk], sums[10 * j + 2 * kk + 1]);
       float z = warp_reduce_scatter32(sums, lane);      // lane 10 li + k: sum k of image base + li
-      bool bad = !U8 && active && (plain || sm.out_of_range[img & (kTfRange - 1)] != 0);
-      if (U8 && plain) bad = active;
-      if (__any_sync(0xffffffffu, bad)) {
-        if constexpr (!U8) {
-          for (int j = 0; j < 3; ++j) {
-            if (!__shfl_sync(0xffffffffu, (int)bad, 10 * j)) continue;
-            const float s = image_fc_plain<kPrecise ? SIG : 1>(static_cast<const float*>(images) + (img0 + base + j) * kImg, params, lane);
-            const float sk = __shfl_sync(0xffffffffu, s, k);
-            if (li == j) z = sk;
-          }
-        } else {
-          z = active ? __int_as_float(0x7fffffff) : 0.f;    // parameters that are not finite
+      if constexpr (U8) {
+        if (plain || px_scale >= 65536.f)
+          z = finish_plain_u8<SIG>(static_cast<const unsigned char*>(images) + img0 * kImg, params, sm.lut, base, imgs_here, plain, z, lane);
+      }
+      const bool bad = !U8 && active && (plain || sm.out_of_range[img & (kTfRange - 1)] != 0);
+      if (!U8 && __any_sync(0xffffffffu, bad)) {
+        for (int j = 0; j < 3; ++j) {
+          if (!__shfl_sync(0xffffffffu, (int)bad, 10 * j)) continue;
+          const float s = image_fc_plain<kPrecise ? SIG : 1>(static_cast<const float*>(images) + (img0 + base + j) * kImg, params, lane);
+          const float sk = __shfl_sync(0xffffffffu, s, k);
+          if (li == j) z = sk;
         }
         if (bad && k == 0) sm.out_of_range[img & (kTfRange - 1)] = 0;
       }

@@ -395,6 +395,45 @@ def test_tensor_core_forward_operand_range(cuda, pkg, params0, what, n):
     assert rel_err(outs[1][0][keep], outs[0][0][keep]) < 1e-5
 
 
+@pytest.mark.parametrize("what,tol", [("weights x 4000", 2e-3), ("weights x 1e5", 5e-2), ("infinite bias", 1e-5), ("not a number", 0),
+                                      ("blank image, weights x 1e32", 1e-5)])
+@pytest.mark.parametrize("n", [3, 148 * 16 + 21])
+def test_tensor_core_forward_uint8_parameter_range(cuda, pkg, params0, what, tol, n):
+    """uint8 pixels meet the same limits as the fp32 images they stand for: with weights whose pixel scale takes them out of fp16's
+    range, or with parameters that are not finite, the tensor-core kernel computes them in fp32, to the fp32 images' bits.  Yardstick:
+    the CUDA-core kernel; a pre-activation of 25 terms up to 0.5 * factor is only known to 25 * 0.5 * factor * 2^-24 in fp32,
+    3e-3 and 7e-2 here, and a sigmoid's slope is at most 1/4 at the windows that it does not saturate."""
+    pix = pkg.synth.synth_pixels_u8(47, n)
+    params = params0.copy()
+    if "weights" in what:
+        params[:150] *= np.float32(what.split()[-1])
+    if what.startswith("blank"):
+        pix[:] = 0
+    elif what == "infinite bias":
+        params[150] = np.inf
+    elif what == "not a number":
+        params[77] = np.nan
+    images = pkg.synth.u8_to_float(pix)
+    d_pix = cuda.from_numpy(pix).cuda()
+    outs = {}
+    for path in (0, 1):
+        net = pkg.Net(0)
+        net.set_params(params)
+        net.set_option("forward_path", path)
+        d_out = cuda.empty((n, 10), dtype=cuda.float32, device="cuda")
+        d_arg = cuda.empty((n,), dtype=cuda.int32, device="cuda")
+        net.forward_u8(d_pix, n, d_out, d_arg)
+        cuda.cuda.synchronize()
+        outs[path] = d_out.cpu().numpy()
+        out, arg = run_forward(cuda, net, images)
+        assert net.status() == 0
+        assert np.array_equal(outs[path], out, equal_nan=True) and np.array_equal(d_arg.cpu().numpy(), arg)
+    if what == "not a number":
+        assert np.isnan(outs[0]).all() and np.isnan(outs[1]).all()
+    else:
+        assert float(np.max(np.abs(outs[1].astype(np.float64) - outs[0]))) < tol
+
+
 @pytest.mark.parametrize("fast", [0, 1])
 @pytest.mark.parametrize("n", [2, 297, 888, 889, 895, 2073])
 def test_cuda_core_forward_around_its_dispatch(cuda, pkg, params0, n, fast):
