@@ -103,11 +103,9 @@ CNN_PHASE_TABLE(g_phase_clocks_wg, 24)
 
 bool wide_tc_supported(const WideDims& d) { return d.F % kTwF == 0 && d.H % 4 == 0; }
 
-__device__ __forceinline__ float warp_max(float m) {
-#pragma unroll
-  for (int k = 16; k > 0; k >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, k));
-  return m;
-}
+// Largest and smallest over a warp of values that are not negative (whose bits are in the values' order).
+__device__ __forceinline__ float warp_max(float m) { return __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(m))); }
+__device__ __forceinline__ float warp_min(float m) { return __uint_as_float(__reduce_min_sync(0xffffffffu, __float_as_uint(m))); }
 // Exponent e with 2^e <= v < 2^(e+1), kept where scales built from it stay normal numbers.
 __device__ __forceinline__ int exponent_of(float v) {
   const int e = (int)((__float_as_uint(v) >> 23) & 255u) - 127;
@@ -126,7 +124,8 @@ k_wide_prep(WideDims d, long n, int team, const float4* images, const float* par
   pdl_launch_dependents();
   pdl_wait();
   const int quads = d.H * d.H / 4, teams = 256 / team, mine = threadIdx.x / team, at = threadIdx.x % team;
-  for (long b0 = (long)blockIdx.x * teams; b0 < n; b0 += (long)gridDim.x * teams) {
+  // (from the last block down: the first have the weights)
+  for (long b0 = (long)(gridDim.x - 1 - blockIdx.x) * teams; b0 < n; b0 += (long)gridDim.x * teams) {
     const long b = b0 + mine;
     const float4* src = images + (size_t)(b < n ? b : 0) * quads;
     unsigned m = 0;                    // magnitudes compared as integers: what is not a number is above infinity
@@ -156,9 +155,10 @@ k_wide_prep(WideDims d, long n, int team, const float4* images, const float* par
   }
 }
 
-// The way out for an image whose pixels do not fit the batch's scale: plain fp32 by all threads of a CTA, for its 64 maps from f0 on.  Out of
-// line and with rolled loops: what it needs of registers and stack the hot code would pay for.  Thread = map and every twelfth window of a row of
-// windows, taps from shared memory.  Forward: the image's subsample activations as[window][map].  Backward: reads ds[window][map] and adds the image's
+// The way out for an image whose pixels do not fit the batch's scale: plain fp32 by all threads of a CTA, for its 64 maps from f0 on.  With
+// rolled loops and in line: what it needs of registers and stack, or a call, the hot code pays for (1,024 images: forward 117.7 us without it, 120.3
+// this way; a gradient 333.3, 332.0 in line and 333.3 with a call).  Thread = map and every twelfth window of a row of windows, taps from shared
+// memory.  Forward: the image's subsample activations as[window][map].  Backward: reads ds[window][map] and adds the image's
 // share to the CTA's sums, in a fixed order and their layouts (a filter tap (i, j) goes to x = 0, c = j of D).  The deltas of a row of windows go through
 // shared memory, where a thread has a map, a tap row (or the bias) and every other row of deltas.
 constexpr int kTwPlainTeams = kTwThreads / kTwF;                    // 12 = 2 halves of 5 tap rows and the bias
@@ -171,7 +171,7 @@ struct TwPlain {
 static_assert(sizeof(TwPlain::tap) <= offsetof(TwSmem, bias) && sizeof(TwPlain) <= sizeof(TwBwdSmem), "space for wide_plain_image");
 
 template <int FL, bool BWD>
-__device__ __noinline__ void wide_plain_image(int H, int F, int f0, TwPlain& sm, const float* image, const float* params, float* as_or_ds,
+__device__ __forceinline__ void wide_plain_image(int H, int F, int f0, TwPlain& sm, const float* image, const float* params, float* as_or_ds,
                                               float* part_g, float* part_b) {
   const WideDims d = make_wide_dims(H, F);
   const int tid = threadIdx.x, m = tid % kTwF, team = tid / kTwF;
@@ -321,17 +321,21 @@ k_wide_tc(WideDims d, long n, const float* __restrict__ images, const float* __r
   if (BWD) {
     for (int i = tid; i < ds_blocks; i += kTwThreads) dmax = fmaxf(dmax, ds_max[i]);
   } else {
-#pragma unroll 4
-    for (long b = tid; b < n; b += kTwThreads) {
-      const float m = img_max[b];
-      pmax = m <= 3.4e38f ? fmaxf(pmax, m) : INFINITY;
-      pmin = m > 0.f ? fminf(pmin, m) : pmin;
+    for (long b0 = tid; b0 < n; b0 += 4 * kTwThreads) {
+      float m[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) m[j] = img_max[b0 + j * kTwThreads < n ? b0 + j * kTwThreads : b0];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        pmax = m[j] <= 3.4e38f ? fmaxf(pmax, m[j]) : INFINITY;
+        pmin = m[j] > 0.f ? fminf(pmin, m[j]) : pmin;
+      }
     }
   }
   wmax = warp_max(wmax);
   dmax = warp_max(dmax);
   pmax = warp_max(pmax);
-  pmin = -warp_max(-pmin);
+  pmin = warp_min(pmin);
   if (lane == 0) {
     sm.max_of[0][warp] = wmax;
     sm.max_of[1][warp] = pmax;
@@ -351,7 +355,7 @@ k_wide_tc(WideDims d, long n, const float* __restrict__ images, const float* __r
     all = scale_of[4 * blockIdx.y + 2];
   } else {
     all = pmax = warp_max(sm.max_of[1][mine_at]);
-    pmin = -warp_max(-sm.max_of[3][mine_at]);
+    pmin = warp_min(sm.max_of[3][mine_at]);
     limit = wmax < kHuge ? fminf(fmaxf(pow2i(10 - exponent_of(wmax)), 4096.f * pmin), kHuge) : -1.f;
     if (!(all <= limit)) {
       pmax = 0.f;
@@ -425,14 +429,13 @@ k_wide_tc(WideDims d, long n, const float* __restrict__ images, const float* __r
     const bool mine = tid < kTwRows;
     float4 v0, v1;
     bool have;
-    float most;                        // the image's largest pixel
     const float* src;
     unsigned G = set0 * kTwGroups + (mine ? g : 0);
     auto place = [&]() {
       const unsigned b = G / (unsigned)gi;
       const int y = 8 * (int)(G - b * (unsigned)gi) + row;
       have = mine && b < n && y < d.H;
-      most = img_max[have ? b : 0];
+      if (sm.any_plain) have = have && img_max[have ? b : 0] <= sm.limit;
       src = images + ((size_t)(have ? b : 0) * d.H + (have ? y : 0)) * d.H;
     };
     auto load = [&](int q) {           // (clamped, not conditional: a load under a condition is waited for on the spot)
@@ -477,11 +480,10 @@ k_wide_tc(WideDims d, long n, const float* __restrict__ images, const float* __r
       // (the slab is free: the gradients of the unit that had it are complete, and with the last unit of a set the set)
       if (BWD && k >= kTwSlabs && (k - kTwSlabs) % kTwFlush == kTwFlush - 1) flush((k - kTwSlabs) / kTwFlush);
       __half2 hi[4], lo[4];
-      const bool in = have && most <= limit;
-      tc::split_f16x2(in ? v0.x : 0.f, in ? v0.y : 0.f, px_scale, hi[0], lo[0]);
-      tc::split_f16x2(in ? v0.z : 0.f, in ? v0.w : 0.f, px_scale, hi[1], lo[1]);
-      tc::split_f16x2(in ? v1.x : 0.f, in ? v1.y : 0.f, px_scale, hi[2], lo[2]);
-      tc::split_f16x2(in ? v1.z : 0.f, in ? v1.w : 0.f, px_scale, hi[3], lo[3]);
+      tc::split_f16x2(have ? v0.x : 0.f, have ? v0.y : 0.f, px_scale, hi[0], lo[0]);
+      tc::split_f16x2(have ? v0.z : 0.f, have ? v0.w : 0.f, px_scale, hi[1], lo[1]);
+      tc::split_f16x2(have ? v1.x : 0.f, have ? v1.y : 0.f, px_scale, hi[2], lo[2]);
+      tc::split_f16x2(have ? v1.z : 0.f, have ? v1.w : 0.f, px_scale, hi[3], lo[3]);
       if (mine) {
         *reinterpret_cast<uint4*>(sm.slab[s][0] + tid * 16) = *reinterpret_cast<uint4*>(hi);
         if (PASSES == 3) *reinterpret_cast<uint4*>(sm.slab[s][1] + tid * 16) = *reinterpret_cast<uint4*>(lo);
@@ -590,7 +592,8 @@ k_wide_tc(WideDims d, long n, const float* __restrict__ images, const float* __r
     auto place = [&]() {
       const unsigned b = G / (unsigned)gi;
       const int p = (8 * (int)(G - b * (unsigned)gi) + (lane & 7)) >> 2;      // C is a multiple of 4: a window's rows are all in or all out
-      live = b < n && p < d.P && img_max[b < n ? b : 0] <= sm.limit;
+      live = b < n && p < d.P;
+      if (sm.any_plain) live = live && img_max[live ? b : 0] <= sm.limit;
       const size_t window = live ? ((size_t)b * d.P + p) * d.P + q : (BWD ? (size_t)n * d.P * d.P : 0);
       at = (BWD ? const_cast<float*>(ds) : as) + window * d.F + f0 + m0;
     };
