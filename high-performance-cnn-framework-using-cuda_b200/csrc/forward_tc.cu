@@ -195,7 +195,7 @@ __device__ __noinline__ float finish_plain_u8(const unsigned char* pixels, const
 // uint8 pixels and the kernel applies the reference's ingest, float(pixel / 255.0) (mnist.h:145, main.cu:57-65).
 template <int PATH, int SIG, bool U8>
 __global__ void __launch_bounds__(kTfThreads, 1)
-k_forward_tc(const void* __restrict__ images, long n, long imgs_per_cta, const float* __restrict__ params,
+k_forward_tc(const void* images, long n, long imgs_per_cta, const float* params,
              float* __restrict__ out, int* __restrict__ argmax, int* __restrict__ status) {
   extern __shared__ unsigned char smem_raw[];
   TfSmem& sm = *reinterpret_cast<TfSmem*>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~(uintptr_t)127);

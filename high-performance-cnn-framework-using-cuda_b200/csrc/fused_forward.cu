@@ -50,7 +50,7 @@ struct FwSmem {
 // float(pixel / 255.0) (mnist.h:145 then main.cu:57-65), through a 256-entry table.
 template <int FAST, bool U8>
 __global__ void __launch_bounds__(kFwThreads, kFwBlocksPerSm)
-k_forward_one(const void* __restrict__ images, long n, const float* __restrict__ params,
+k_forward_one(const void* images, long n, const float* params,
                 float* __restrict__ out, int* __restrict__ argmax, int* __restrict__ status) {
   __shared__ FwSmem sm;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -229,7 +229,7 @@ struct FtSmem {
 
 template <int FAST, bool U8>
 __global__ void __launch_bounds__(kFtThreads, kFtBlocksPerSm)
-k_forward_tiles(const void* __restrict__ images, long n, const float* __restrict__ params,
+k_forward_tiles(const void* images, long n, const float* params,
                 float* __restrict__ out, int* __restrict__ argmax, int* __restrict__ status) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   FtSmem& sm = *reinterpret_cast<FtSmem*>(smem_raw);

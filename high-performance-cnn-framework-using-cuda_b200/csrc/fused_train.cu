@@ -44,7 +44,7 @@ struct TrSmem {
   int flag[4];
 };
 
-__device__ __forceinline__ void load_params_to_smem(TrSmem& sm, const float* __restrict__ params, int tid) {
+__device__ __forceinline__ void load_params_to_smem(TrSmem& sm, const float* params, int tid) {
   for (int i = tid; i < kF * 28; i += kTrThreads) {
     const int f = i / 28, t = i % 28;
     sm.wc[f][t] = (t < 25) ? params[kOffWc + f * 25 + t] : 0.f;
@@ -223,8 +223,8 @@ __device__ __forceinline__ void team_sync(int team) {
 
 template <int FAST, int TEAMS>
 __global__ void __launch_bounds__(kGrThreads * TEAMS, 1)
-k_grad_partials(const float* __restrict__ images, const unsigned* __restrict__ labels, long n,
-                const float* __restrict__ params, float* __restrict__ rows, int* __restrict__ status, int chained) {
+k_grad_partials(const float* images, const unsigned* labels, long n,
+                const float* params, float* __restrict__ rows, int* __restrict__ status, int chained) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   GrSmem<TEAMS>& sm = *reinterpret_cast<GrSmem<TEAMS>*>(smem_raw);
   const int team = TEAMS == 1 ? 0 : threadIdx.x / kGrThreads;
@@ -510,7 +510,7 @@ k_grad_partials(const float* __restrict__ images, const unsigned* __restrict__ l
 constexpr int kRedGroups = 32;
 
 __global__ void __launch_bounds__(32 * kRedGroups)
-k_reduce_rows(const float* __restrict__ rows, int n_rows, float* __restrict__ G,
+k_reduce_rows(const float* rows, int n_rows, float* __restrict__ G,
               float* __restrict__ params, float scale, float* __restrict__ mean_err, float err_scale) {
   __shared__ float part[kRedGroups][33];
   const int lane = threadIdx.x & 31, g = threadIdx.x >> 5;
@@ -536,7 +536,7 @@ k_reduce_rows(const float* __restrict__ rows, int n_rows, float* __restrict__ G,
   }
 }
 
-__global__ void k_apply_update(float* __restrict__ params, const float* __restrict__ G, float scale) {
+__global__ void k_apply_update(float* __restrict__ params, const float* G, float scale) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   pdl_launch_dependents();
   pdl_wait();
@@ -548,7 +548,7 @@ __global__ void k_apply_update(float* __restrict__ params, const float* __restri
 // ----------------------------------------------------------------------------------------------
 template <int FAST>
 __global__ void __launch_bounds__(kTrThreads, 1)
-k_train_persample(const float* __restrict__ images, const unsigned* __restrict__ labels, long n,
+k_train_persample(const float* images, const unsigned* labels, long n,
                   int epochs, float dt, float threshold, float* __restrict__ params,
                   float* __restrict__ mean_err, int* __restrict__ epochs_run, int* __restrict__ status) {
   extern __shared__ __align__(128) unsigned char smem_raw[];

@@ -59,6 +59,9 @@ __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, unsigned by
 // stream is still running, once every block of the predecessor has called pdl_launch_dependents() (or
 // exited); whatever it reads of the predecessor's results must come after pdl_wait(), which returns when
 // the predecessor has completed and its writes are visible.  Both are no-ops in an ordinary launch.
+// Such a kernel reads global memory by ordinary loads only: neither __ldg nor `const T* __restrict__` parameters, which allow the
+// read-only path.  That path is for data that nobody writes during the kernel's lifetime (which begins before the wait), and its
+// loads may be moved in front of the wait.  Pointers that a kernel writes through may stay __restrict__.
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
@@ -112,7 +115,7 @@ constexpr int kRowErr = kNParams + 1;  // 2344
 // Column `col` of rows g, g + GROUPS, g + 2 GROUPS, ... added in that order; five loads at a time are under way (with one
 // row per SM and 32 groups that is all of them).
 template <int GROUPS>
-__device__ __forceinline__ float sum_rows(const float* __restrict__ rows, int n_rows, int col, int g) {
+__device__ __forceinline__ float sum_rows(const float* rows, int n_rows, int col, int g) {
   float acc = 0.f;
   for (int r0 = g; r0 < n_rows; r0 += 5 * GROUPS) {
     float v[5];

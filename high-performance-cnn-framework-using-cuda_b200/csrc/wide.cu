@@ -24,8 +24,9 @@ namespace cnn {
 // ---- forward ---------------------------------------------------------------------------------
 // Convolution, bias, sigmoid and the subsample layer of one 4x4 window for a group of maps, two maps at a time: thread =
 // window (of any image: windows are numbered through the batch), the two maps in the halves of packed fp32 registers.
-// The 8x8 patch goes by row by row (eight pixels, each copied into both halves: 64 moves for 400 packed FMAs), so a
-// thread holds 16 accumulators, the 25 tap pairs and one row.  Bound by the fp32 FMA pipe: 400 FMAs per window and map
+// The 8x8 patch stays in registers over the pairs (64, beside 32 of accumulators; each pixel copied into both halves: 64 moves for
+// 400 packed FMAs), the taps are read from shared memory where they are used: with the taps in registers too 58 instead of 55 us.  (Not with
+// unaligned rows where conv activations are stored: kept 198, loaded for each pair 167 us for 333 images of 57x57.)  Bound by the fp32 FMA pipe: 400 FMAs per window and map
 // = 40 us for 333 images of 56x56 with 64 maps; 55 us measured (a block per image and 8 maps with one output per thread,
 // then the subsample layer from memory: 287 + 53 us).
 // Writes the subsample activations and, with STORE, the conv activations (what the backward pass reads; pre-activations
@@ -36,19 +37,19 @@ constexpr int kWideTapStride = 26;      // 25 tap pairs, padded to an even numbe
 
 // Eight pixels of a patch row; VEC: rows are 16-byte aligned (H a multiple of 4).
 template <bool VEC>
-__device__ __forceinline__ void load_row8(const float* __restrict__ src, float (&v)[8]) {
+__device__ __forceinline__ void load_row8(const float* src, float (&v)[8]) {
   if (VEC) {
-    const float4 a = __ldg(reinterpret_cast<const float4*>(src)), b = __ldg(reinterpret_cast<const float4*>(src) + 1);
+    const float4 a = *reinterpret_cast<const float4*>(src), b = reinterpret_cast<const float4*>(src)[1];
     v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
   } else {
 #pragma unroll
-    for (int c = 0; c < 8; ++c) v[c] = __ldg(src + c);
+    for (int c = 0; c < 8; ++c) v[c] = src[c];
   }
 }
 
 template <int FLAVOR, bool STORE, bool VEC>
 __global__ void __launch_bounds__(kWideWinThreads, 4)
-k_wide_conv_s1(WideDims d, long n, int maps_per_block, const float* __restrict__ images, const float* __restrict__ params,
+k_wide_conv_s1(WideDims d, long n, int maps_per_block, const float* images, const float* params,
                float* __restrict__ ac, float* __restrict__ as) {
   extern __shared__ __align__(16) float sh[];
   // tap pairs [pair][26][2] | subsample taps, doubled [16][2] | bias pairs [pair][2]   (the first two are read 16 bytes at a time)
@@ -75,15 +76,17 @@ k_wide_conv_s1(WideDims d, long n, int maps_per_block, const float* __restrict__
   const long b = t / W;
   const int w = (int)(t - b * W), p = w / d.P, q = w - p * d.P;
   const float* src = images + ((size_t)b * d.H + 4 * p) * d.H + 4 * q;
+  constexpr bool kKeep = VEC || !STORE;
+  float patch[8][8];
+  if (kKeep) {
+#pragma unroll
+    for (int r = 0; r < 8; ++r) load_row8<VEC>(src + r * d.H, patch[r]);
+  }
 #pragma unroll 1
   for (int pr = 0; pr < pairs; ++pr) {
-    f32x2 acc[4][4], wt[kWideTapStride];
-    const ulonglong2* tp = reinterpret_cast<const ulonglong2*>(tap + pr * kWideTapStride * 2);
-#pragma unroll
-    for (int i = 0; i < kWideTapStride / 2; ++i) {
-      const ulonglong2 v = tp[i];
-      wt[2 * i] = v.x; wt[2 * i + 1] = v.y;
-    }
+    if (!kKeep) asm volatile("" : "+l"(src));      // (or the compiler moves the loads out of the loop)
+    f32x2 acc[4][4];
+    const f32x2* wt = reinterpret_cast<const f32x2*>(tap + pr * kWideTapStride * 2);
     const f32x2 bp = reinterpret_cast<const f32x2*>(bias)[pr];
 #pragma unroll
     for (int y = 0; y < 4; ++y)
@@ -96,8 +99,8 @@ k_wide_conv_s1(WideDims d, long n, int maps_per_block, const float* __restrict__
     const size_t ac_at = STORE ? ((size_t)(b * d.F + f) * d.C + 4 * p) * d.C + 4 * q : 0;
 #pragma unroll
     for (int r = 0; r < 8; ++r) {
-      float v[8];
-      load_row8<VEC>(src + r * d.H, v);
+      float (&v)[8] = patch[r];
+      if (!kKeep) load_row8<VEC>(src + r * d.H, v);
       f32x2 v2[8];
 #pragma unroll
       for (int c = 0; c < 8; ++c) v2[c] = pack2(v[c], v[c]);
@@ -168,8 +171,8 @@ constexpr int kWideFcSets = 4;
 
 template <int FLAVOR>
 __global__ void __launch_bounds__(256, 2) __cluster_dims__(kWideFcSlices, 1, 1)
-k_wide_fc_fwd(WideDims d, long n, int sets, const float* __restrict__ as, const float* __restrict__ wf, const float* __restrict__ params,
-              const unsigned* __restrict__ labels, float* __restrict__ out, int* __restrict__ argmax,
+k_wide_fc_fwd(WideDims d, long n, int sets, const float* as, const float* wf, const float* params,
+              const unsigned* labels, float* __restrict__ out, int* __restrict__ argmax,
               float* __restrict__ delta_f, float* __restrict__ err) {
   __shared__ float red[8][kWideFcVals];
   __shared__ float part[kWideFcSlices][kWideFcSets * kWideFcVals];       // the first block's: one row per slice
@@ -266,10 +269,11 @@ k_wide_fc_fwd(WideDims d, long n, int sets, const float* __restrict__ as, const 
 // images' loads under way and about 24 with eight, for which it needs more than the 48 registers that the compiler would take).
 constexpr int kWideFcSplit = 16;
 constexpr int kWideBpImgs = 64;          // images whose output deltas are staged at a time
+constexpr int kWideBpAhead = 8;          // images whose activations are under way at a time
 
 __global__ void __launch_bounds__(128, 6)
-k_wide_bp_fc(WideDims d, long n, const float* __restrict__ as, const float* __restrict__ delta_f,
-             const float* __restrict__ wf, float* __restrict__ ds, float* __restrict__ part_f, float* __restrict__ ds_max) {
+k_wide_bp_fc(WideDims d, long n, const float* as, const float* delta_f,
+             const float* wf, float* __restrict__ ds, float* __restrict__ part_f, float* __restrict__ ds_max) {
   __shared__ __align__(16) float dlt[kWideBpImgs][12];
   __shared__ float red[4];
   float most = 0.f;
@@ -292,9 +296,7 @@ k_wide_bp_fc(WideDims d, long n, const float* __restrict__ as, const float* __re
     if (!live) continue;
     const float* src = as + (size_t)c0 * d.S + s;
     float* dst = ds + (size_t)c0 * d.S + s;
-#pragma unroll 8
-    for (int g = 0; g < imgs; ++g) {
-      const float a = src[(size_t)g * d.S];
+    auto image = [&](int g, float a) {
       const f32x2 a2 = pack2(a, a);
       const ulonglong2 d0 = *reinterpret_cast<const ulonglong2*>(&dlt[g][0]), d1 = *reinterpret_cast<const ulonglong2*>(&dlt[g][4]);
       const f32x2 dk[kOut / 2] = {d0.x, d0.y, d1.x, d1.y, *reinterpret_cast<const f32x2*>(&dlt[g][8])};
@@ -308,6 +310,21 @@ k_wide_bp_fc(WideDims d, long n, const float* __restrict__ as, const float* __re
       const float v = (lo + hi) * a * (1.f - a);
       dst[(size_t)g * d.S] = v;
       most = fabsf(v) <= 3.4e38f ? fmaxf(most, fabsf(v)) : most;
+    };
+    float ahead[kWideBpAhead];               // (spelt out: a load may not move in front of the stores before it)
+    int g = 0;
+    for (; g + kWideBpAhead <= imgs; g += kWideBpAhead) {
+#pragma unroll
+      for (int i = 0; i < kWideBpAhead; ++i) ahead[i] = src[(size_t)(g + i) * d.S];
+#pragma unroll
+      for (int i = 0; i < kWideBpAhead; ++i) image(g + i, ahead[i]);
+    }
+    if (g < imgs) {
+#pragma unroll
+      for (int i = 0; i < kWideBpAhead - 1; ++i) ahead[i] = src[(size_t)(g + i < imgs ? g + i : g) * d.S];
+#pragma unroll
+      for (int i = 0; i < kWideBpAhead - 1; ++i)
+        if (g + i < imgs) image(g + i, ahead[i]);
     }
   }
   if (ds_max) {                            // tensor-core path
@@ -333,13 +350,13 @@ k_wide_bp_fc(WideDims d, long n, const float* __restrict__ as, const float* __re
 //   G_wc[f][u][v] = sum dc[y][x] * image[y + u][x + v], G_bc[f] = sum dc, G_ws[i][j] = sum delta_s * a
 // Thread = one window after another of the slice's images, the two maps in the halves of packed registers, all sums in
 // registers until the end: the deltas never exist in memory.  The patch goes by row by row as in the forward kernel.
-// Bound by the FMA pipe (400 FMAs per window and map for the weight gradient alone); 128 images of 56x56 with 64 maps: 62 us
-// (a kernel that wrote the deltas and one that read them back per map and image: 108 + 200 us).
+// Bound by the FMA pipe (400 FMAs per window and map for the weight gradient alone); 333 images of 56x56 with 64 maps: 134 us,
+// 154 us with the rows' loads wherever the compiler put them; 128 images: 62 us before that (a kernel that wrote the deltas and one that read them back per map and image: 108 + 200 us).
 // Partial rows: part_c[slice][F][26], part_s[slice * pairs + pair][17].
 template <bool VEC>
 __global__ void __launch_bounds__(kWideWinThreads, 3)
-k_wide_grad_win(WideDims d, long n, const float* __restrict__ images, const float* __restrict__ ac,
-                const float* __restrict__ ds, const float* __restrict__ params, float* __restrict__ part_c,
+k_wide_grad_win(WideDims d, long n, const float* images, const float* ac,
+                const float* ds, const float* params, float* __restrict__ part_c,
                 float* __restrict__ part_s) {
   __shared__ __align__(16) f32x2 ws2[16];
   __shared__ float red[kWideWinThreads / 32][3][32];
@@ -394,6 +411,7 @@ k_wide_grad_win(WideDims d, long n, const float* __restrict__ images, const floa
     }
     gs[16] += (dl0 + dl1) * inv_s;
     const float* src = images + ((size_t)b * d.H + 4 * p) * d.H + 4 * q;
+    asm volatile("" : "+l"(src));        // the rows' loads begin here, not beside the activations': 100 bytes of spills per unit less
 #pragma unroll
     for (int r = 0; r < 8; ++r) {
       float v[8];
@@ -447,8 +465,8 @@ k_wide_grad_win(WideDims d, long n, const float* __restrict__ images, const floa
 // A tensor-core step of 1,024 images 359 -> 343 us, of 128 images 92.9 -> 77.0; a fp32 step of 128 images 110 -> 108 us.)
 template <bool TC>
 __global__ void __launch_bounds__(256, 4)
-k_wide_reduce(WideDims d, long n, long rows_c, long rows_s, const float* __restrict__ part_c, const float* __restrict__ part_s,
-              const float* __restrict__ part_f, const float* __restrict__ delta_f, const float* __restrict__ err, int value_blocks,
+k_wide_reduce(WideDims d, long n, long rows_c, long rows_s, const float* part_c, const float* part_s,
+              const float* part_f, const float* delta_f, const float* err, int value_blocks,
               int filter_blocks, float* __restrict__ G) {
   constexpr int kSlices = 8, kTile = 8 * 16;      // of a filter block: CTA slices; 8 c x 16 columns (x, f)
   __shared__ __align__(16) float sums[TC ? kSlices : 1][TC ? kTile : 1];
@@ -532,7 +550,7 @@ k_wide_reduce(WideDims d, long n, long rows_c, long rows_s, const float* __restr
   }
 }
 
-__global__ void k_wide_update(int n_params, float* __restrict__ params, const float* __restrict__ G, float scale) {
+__global__ void k_wide_update(int n_params, float* __restrict__ params, const float* G, float scale) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n_params) params[i] = fmaf(scale, G[i], params[i]);
 }

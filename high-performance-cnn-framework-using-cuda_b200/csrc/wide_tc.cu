@@ -272,8 +272,8 @@ __device__ __forceinline__ void wide_plain_image(int H, int F, int f0, TwPlain& 
 // pixel within it, largest of all}, from the forward kernel for the backward kernel.
 template <int FL, int PASSES, bool BWD>
 __global__ void __launch_bounds__(kTwThreads, 1)
-k_wide_tc(WideDims d, long n, const float* __restrict__ images, const float* __restrict__ params, const float* img_max,
-          float* scale_of, float* __restrict__ as, const float* __restrict__ ds, const float* __restrict__ ds_max, int ds_blocks,
+k_wide_tc(WideDims d, long n, const float* images, const float* params, const float* img_max,
+          float* scale_of, float* __restrict__ as, const float* ds, const float* ds_max, int ds_blocks,
           float* __restrict__ part_g, float* __restrict__ part_b, int* __restrict__ status) {
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem_base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~(uintptr_t)127);
@@ -439,8 +439,8 @@ k_wide_tc(WideDims d, long n, const float* __restrict__ images, const float* __r
       src = images + ((size_t)(have ? b : 0) * d.H + (have ? y : 0)) * d.H;
     };
     auto load = [&](int q) {           // (clamped, not conditional: a load under a condition is waited for on the spot)
-      v0 = __ldg(reinterpret_cast<const float4*>(src + 4 * q));
-      v1 = __ldg(reinterpret_cast<const float4*>(src + 4 * q) + 1);
+      v0 = *reinterpret_cast<const float4*>(src + 4 * q);
+      v1 = reinterpret_cast<const float4*>(src + 4 * q)[1];
     };
     int q = (int)q0;
     place();
@@ -601,8 +601,8 @@ k_wide_tc(WideDims d, long n, const float* __restrict__ images, const float* __r
     // Backward: the window's deltas of eight maps, the next eight taken as soon as these are used.
     float4 dlo, dhi;
     if (BWD) {
-      dlo = __ldg(reinterpret_cast<const float4*>(at));
-      dhi = __ldg(reinterpret_cast<const float4*>(at) + 1);
+      dlo = *reinterpret_cast<const float4*>(at);
+      dhi = reinterpret_cast<const float4*>(at)[1];
     }
     for (int k = 0; k < units; ++k) {
       unsigned nxt[8];
@@ -702,8 +702,8 @@ k_wide_tc(WideDims d, long n, const float* __restrict__ images, const float* __r
             }
             gb2[4 * part + ch] = add2(gb2[4 * part + ch], sum);
             gds2 = add2(gds2, dl);                 // (the window's four lanes have the same: lane 0's sum is used)
-            if (ch == 1) dlo = __ldg(reinterpret_cast<const float4*>(part ? at : at + 8));
-            if (ch == 3) dhi = __ldg(reinterpret_cast<const float4*>(part ? at : at + 8) + 1);
+            if (ch == 1) dlo = *reinterpret_cast<const float4*>(part ? at : at + 8);
+            if (ch == 3) dhi = reinterpret_cast<const float4*>(part ? at : at + 8)[1];
             if (part == 0 && ch == 0) {
               CNN_PHASE(2);
               mbar_wait_bounded(&sm.dc_free[h], ((unsigned)k & 1u) ^ 1u, status, gave_up);
