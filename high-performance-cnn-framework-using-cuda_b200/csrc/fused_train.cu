@@ -240,16 +240,19 @@ k_grad_partials(const float* images, const unsigned* labels, long n,
     mbar_expect_tx(bar, kImg * sizeof(float));
     bulk_g2s(&sm.img[team][i % kGrStages][0], images + im * kImg, kImg * sizeof(float), bar);
   };
-  pdl_launch_dependents();
+  if (chained) pdl_launch_dependents();
   if (tid == 0) {
     for (int s = 0; s < kGrStages; ++s) mbar_init(&sm.full[team][s], 1);
     mbar_fence_init();
     // In a training loop the kernel before this one is the previous step's reduce + update kernel, which does not touch
-    // the images: their copies may leave while it still runs.
+    // the images: their copies may leave while it still runs.  Whatever wrote the images is complete by then, because the loop's
+    // first gradient kernel (the one that is not chained) lets its successors start only behind its own wait; kernels that
+    // triggered before their waits could otherwise all start while the writer still runs.
     if (chained)
       for (int i = 0; i < kGrStages; ++i) issue(i);
   }
   pdl_wait();      // the parameters (and the row buffer this kernel writes at its end) belong to the predecessor until here
+  if (!chained) pdl_launch_dependents();
   if (tid == 0 && !chained)
     for (int i = 0; i < kGrStages; ++i) issue(i);
   // Parameters: every load of a thread is under way before the first of them is stored (one L2 latency, not one per

@@ -50,3 +50,42 @@ def test_no_read_only_loads_beside_a_running_predecessor(name):
     if "pdl_wait(" not in text and name.endswith(".cu"):
         return
     assert not list(offences(text))
+
+
+def body_of(name, kernel):
+    with open(os.path.join(CSRC, name)) as f:
+        found = [body for signature, body in functions(f.read()) if re.search(r"\b%s\(" % kernel, signature)]
+    assert len(found) == 1
+    return found[0]
+
+
+def triggers_after_wait(body, chained):
+    """Whether a kernel lets its successor start only once its own wait is over (calls under `if (chained)` or `if (!chained)`
+    count in the one case or the other)."""
+    events = re.findall(r"(?:if \((!?chained)\) )?(pdl_launch_dependents|pdl_wait)\(\)", body)
+    order = [call for condition, call in events if condition in ("", "chained" if chained else "!chained")]
+    assert sorted(order) == ["pdl_launch_dependents", "pdl_wait"]
+    return order[0] == "pdl_wait"
+
+
+@pytest.mark.parametrize("exchange", ["k_reduce_rows", "k_reduce_exchange_update"])
+@pytest.mark.parametrize("empty_first_steps", [0, 2])
+def test_early_image_copies_follow_whatever_wrote_the_images(exchange, empty_first_steps):
+    """In a training loop the gradient kernel of a later step copies its first images before its wait.  A kernel may start when the
+    one before it has triggered, which says that the launches further back are complete only if that trigger came after a
+    wait; the kernel that wrote the images (launch 0, which may trigger as early as it likes) has to be among them."""
+    grad = body_of("fused_train.cu", "k_grad_partials")
+    reduce_after = triggers_after_wait(body_of("fused_train.cu" if exchange == "k_reduce_rows" else "dp_exchange.cu", exchange), False)
+    launches, trained = [("writer", False, False)], False
+    for step in range(empty_first_steps + 4):
+        if step >= empty_first_steps:          # (a rank without images of a global batch launches no gradient kernel)
+            launches.append(("grad", trained, triggers_after_wait(grad, trained)))
+            trained = True
+        launches.append(("reduce", False, reduce_after))
+    complete = -1                              # launches up to this one are complete when launch i starts
+    for i, (kind, chained, _) in enumerate(launches):
+        if i > 0 and launches[i - 1][2]:
+            complete = max(complete, i - 2)
+        assert not (kind == "grad" and chained) or complete >= 0, i
+    assert re.search(r"first > 0 \|\| e > 0|trained", open(os.path.join(CSRC, "fused_train.cu")).read())
+    assert re.search(r"stream, trained\);.*?trained = trained \|\| hi > lo;", open(os.path.join(CSRC, "dp_exchange.cu")).read(), re.S)
