@@ -752,7 +752,7 @@ int cnn_grad_batch(cnn_net* net, const float* d_images, const unsigned int* d_la
   CNN_REQUIRE((reinterpret_cast<uintptr_t>(d_images) & 15u) == 0,
               "cnn_grad_batch: image batch must start on a 16-byte boundary");
   const int grid = grid_for_batch(n);
-  int rc = ensure_train_scratch(net, sm_count());
+  int rc = ensure_train_scratch(net);
   if (rc != CNN_OK) return rc;
   if ((rc = launch_grad_partials(net, d_images, d_labels, n, grid, st)) != CNN_OK) return rc;
   cudaError_t e = launch_pdl(k_reduce_rows, dim3((kNParamsPadded + 31) / 32), dim3(32 * kRedGroups), 0, st,
@@ -779,7 +779,7 @@ int cnn_train_minibatch(cnn_net* net, const float* d_images, const unsigned int*
   CNN_REQUIRE((reinterpret_cast<uintptr_t>(d_images) & 15u) == 0,
               "cnn_train_minibatch: image batch must start on a 16-byte boundary");
   cudaStream_t st = as_stream(stream);
-  int rc = ensure_train_scratch(net, sm_count());
+  int rc = ensure_train_scratch(net);
   if (rc != CNN_OK) return rc;
   if (d_mean_err) CNN_CUDA(cudaMemsetAsync(d_mean_err, 0, sizeof(float) * (size_t)epochs, st));
   for (int e = 0; e < epochs; ++e) {
@@ -809,7 +809,7 @@ int cnn_train_sgd_persample(cnn_net* net, const float* d_images, const unsigned 
   CNN_REQUIRE((reinterpret_cast<uintptr_t>(d_images) & 15u) == 0,
               "cnn_train_sgd_persample: image batch must start on a 16-byte boundary");
   cudaStream_t st = as_stream(stream);
-  int rc = ensure_train_scratch(net, sm_count());
+  int rc = ensure_train_scratch(net);
   if (rc != CNN_OK) return rc;
   // Scratch reuse: d_grad holds the per-epoch means (epochs <= kNParamsPadded) and the epoch count.
   CNN_REQUIRE(epochs <= kNParamsPadded, "cnn_train_sgd_persample: too many epochs");

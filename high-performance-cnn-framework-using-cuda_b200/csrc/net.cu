@@ -9,15 +9,10 @@
 namespace cnn {
 void destroy_host_pipeline(HostPipeline* p);
 
-int ensure_train_scratch(cnn_net* net, int rows) {
+// (One row per SM: no launch of the gradient kernel has more blocks, see grid_for_batch.)
+int ensure_train_scratch(cnn_net* net) {
   if (!net->d_grad) CNN_CUDA(cudaMalloc(&net->d_grad, sizeof(float) * (kNParamsPadded + 8)));
-  if (rows > net->partial_rows) {
-    if (net->d_partials) CNN_CUDA(cudaFree(net->d_partials));
-    net->d_partials = nullptr;
-    net->partial_rows = 0;
-    CNN_CUDA(cudaMalloc(&net->d_partials, sizeof(float) * (size_t)rows * (kNParamsPadded + 8)));
-    net->partial_rows = rows;
-  }
+  if (!net->d_partials) CNN_CUDA(cudaMalloc(&net->d_partials, sizeof(float) * (size_t)sm_count() * kRowStride));
   return CNN_OK;
 }
 }  // namespace cnn

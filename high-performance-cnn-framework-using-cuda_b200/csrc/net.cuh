@@ -19,8 +19,7 @@ struct cnn_net {
   int fast_sigmoid = 1;            // sigmoid of the fused kernels: 0 = reference expression, 1 = short form (default)
 
   // Training scratch (allocated on first use): per-block partial gradients and the reduced vector.
-  float* d_partials = nullptr;     // [partial_rows][kNParamsPadded]
-  int partial_rows = 0;
+  float* d_partials = nullptr;     // one row of kRowStride floats per SM
   float* d_grad = nullptr;         // kNParamsPadded floats + 8 floats of statistics
   cnn::HostPipeline* host = nullptr;   // host_pipeline.cu (created on first use)
 };
@@ -136,7 +135,7 @@ int forward_device_tc(cnn_net* net, int path, const float* d_images, long n, flo
                       cudaStream_t stream);
 int forward_device_tc_u8(cnn_net* net, const unsigned char* d_pixels, long n, float* d_out, int* d_argmax,
                          cudaStream_t stream);
-int ensure_train_scratch(cnn_net* net, int rows);
+int ensure_train_scratch(cnn_net* net);
 // Blocks of the minibatch gradient kernel for a batch of n images (one partial row per block).
 int grid_for_batch(long n);
 // Fused forward + backward of n images at fixed parameters: `grid` partial rows into net->d_partials.

@@ -40,6 +40,27 @@ def test_single_rank_exchange_equals_minibatch_kernel(cuda, pkg, params0):
     dp.close()
 
 
+def test_exchange_uses_the_scratch_of_a_net_that_trained_alone(cuda, pkg, params0):
+    """A net keeps its training scratch: a data-parallel step behind ordinary ones allocates nothing (and frees nothing, which
+    would wait for the device)."""
+    n = 300
+    images, labels = pkg.synth.synth_images(82, n)
+    d_img = cuda.from_numpy(images).cuda()
+    d_lab = cuda.from_numpy(labels.astype(np.int32)).cuda()
+    nets = [pkg.Net(0) for _ in range(4)]          # (several: the driver hands out memory in larger pieces than one scratch)
+    for net in nets:
+        net.train_minibatch(d_img, d_lab, n, n, 1, 0.1, None)
+    dps = [pkg.DataParallel(net) for net in nets]
+    cuda.cuda.synchronize()
+    before = cuda.cuda.mem_get_info()[0]
+    for dp in dps:
+        dp.step(d_img, d_lab, n, 0.1 / n)
+    cuda.cuda.synchronize()
+    assert cuda.cuda.mem_get_info()[0] == before
+    for dp in dps:
+        dp.close()
+
+
 def test_dp_rejects_bad_arguments(cuda, pkg):
     net = pkg.Net(0)
     with pytest.raises(pkg.CnnError):
