@@ -23,6 +23,7 @@ int forward_device_u8(cnn_net* net, int path, const unsigned char* d_pixels, lon
 
 constexpr int kHpSlots = 3;
 constexpr long kHpMaxChunk = 8192, kHpMinChunk = 1024;      // images per chunk
+static_assert(kHpSlots * (sizeof(float) * (kOut + 1) * kHpMaxChunk + 256) + sizeof(int) * kHpSlots <= PinnedBlock::kPage, "results fit a lease");
 constexpr size_t kHpMinStaged = 128 * 1024;                 // below, the driver's own staging is as fast
 
 struct HostPipeline {
@@ -34,10 +35,10 @@ struct HostPipeline {
     long first = 0, count = 0;                 // the chunk whose results wait in h_res (count 0: none)
   } slot[kHpSlots];
   unsigned char* d_block = nullptr;            // all slots' images and results
-  float* h_block = nullptr;                    // pinned: all slots' results
-  size_t d_slot_bytes = 0, h_slot_bytes = 0;   // what a slot has of them
-  int d_slots = 0, h_slots = 0;
-  int* h_status = nullptr;                     // pinned: the net's status word after each slot's last kernel
+  size_t d_slot_bytes = 0;                     // what a slot has of it
+  int d_slots = 0;
+  PinnedHeap::Lease h_block;                   // all slots' results (for pageable ones), and behind them:
+  int* h_status = nullptr;                     // the net's status word after each slot's last kernel
   cudaEvent_t piece[CopyPool::kSlots] = {};    // a ring slot's copy to the device is done
   cudaEvent_t order_event = nullptr;           // ties the slots' streams behind the legacy stream
   std::unique_ptr<CopyPool::Ref> pool;
@@ -46,8 +47,6 @@ struct HostPipeline {
     for (Slot& s : slot)
       if (s.stream) cudaStreamDestroy(s.stream);
     cudaFree(d_block);
-    cudaFreeHost(h_block);
-    cudaFreeHost(h_status);
     for (cudaEvent_t e : piece)
       if (e) cudaEventDestroy(e);
     if (order_event) cudaEventDestroy(order_event);
@@ -56,8 +55,8 @@ struct HostPipeline {
   // One allocation each for all slots: a cudaMalloc costs 0.4 ms whatever its size.
   int reserve(int slots, long chunk, size_t image_bytes, bool pinned_results, bool staged) {
     if (!order_event) {
-      CNN_CUDA(cudaMallocHost(&h_status, sizeof(int) * kHpSlots));
-      for (Slot& s : slot) CNN_CUDA(cudaStreamCreateWithFlags(&s.stream, cudaStreamNonBlocking));
+      for (Slot& s : slot)
+        if (!s.stream) CNN_CUDA(cudaStreamCreateWithFlags(&s.stream, cudaStreamNonBlocking));
       CNN_CUDA(cudaEventCreateWithFlags(&order_event, cudaEventDisableTiming));
     }
     const size_t img = ((size_t)chunk * image_bytes + 255) & ~(size_t)255, res = (sizeof(float) * (kOut + 1) * (size_t)chunk + 255) & ~(size_t)255;
@@ -69,19 +68,17 @@ struct HostPipeline {
       d_slot_bytes = img + res;
       d_slots = slots;
     }
-    if (pinned_results && (h_slot_bytes < res || h_slots < slots)) {
-      cudaFreeHost(h_block);
-      h_block = nullptr;
-      h_slots = 0;
-      CNN_CUDA(cudaMallocHost(&h_block, res * slots));
-      h_slot_bytes = res;
-      h_slots = slots;
+    const size_t pinned = (pinned_results ? res * slots : 0) + sizeof(int) * kHpSlots;
+    if (h_block.bytes() < pinned && !h_block.take(pinned)) {
+      set_error("cnn_forward_batched_host: no pinned memory");
+      return CNN_ERR_CUDA;
     }
     for (int i = 0; i < slots; ++i) {
       slot[i].d_img = d_block + d_slot_bytes * i;
       slot[i].d_res = reinterpret_cast<float*>(slot[i].d_img + img);
-      slot[i].h_res = pinned_results ? h_block + h_slot_bytes / sizeof(float) * i : nullptr;
+      slot[i].h_res = pinned_results ? reinterpret_cast<float*>(h_block.get() + res * i) : nullptr;
     }
+    h_status = reinterpret_cast<int*>(h_block.get() + (pinned_results ? res * slots : 0));
     if (staged && !pool) {
       for (cudaEvent_t& e : piece)
         if (!e) CNN_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));

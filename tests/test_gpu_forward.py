@@ -504,3 +504,28 @@ def test_forward_host_buffers_pageable_and_pinned(cuda, pkg, params0, n, u8):
         check(nets[0], images, *pageable())
     t.join()
     assert not failed
+
+
+def test_forward_host_with_nets_that_come_and_go(cuda, pkg, params0):
+    """Each net sets the pipeline up and, as the last of them, takes the shared threads and ring down again: pageable requests, a
+    small one that is not staged first, results pinned or left out, always the bits of the device call."""
+    n = 3000
+    pix = pkg.synth.synth_pixels_u8(45, n)
+    d_pix = cuda.from_numpy(pix).cuda()
+    d_out = cuda.empty((n, 10), dtype=cuda.float32, device="cuda")
+    for turn in range(4):
+        net = pkg.Net(0)
+        net.set_params(params0)
+        net.forward_u8(d_pix, n, d_out, None)
+        cuda.cuda.synchronize()
+        want = d_out.cpu().numpy()
+        if turn % 2:
+            out = np.empty((20, 10), np.float32)
+            net.forward_u8_host(pix[:20], 20, out, None)
+            assert rel_err(out, want[:20]) < 1e-5      # (so few images go through another kernel)
+        if turn == 2:
+            net.forward_u8_host(pix, n, None, None)
+        out = cuda.empty((n, 10)).pin_memory() if turn == 3 else np.empty((n, 10), np.float32)
+        net.forward_u8_host(pix, n, out, None)
+        assert np.array_equal(np.asarray(out), want)
+        net.close()
