@@ -195,8 +195,8 @@ def test_device_generator_matches_host(cuda, pkg):
 
 @pytest.mark.parametrize("n", [1, 9, 1000, 8192 + 77])
 def test_uint8_input_is_bit_identical_to_fp32(cuda, pkg, params0, n):
-    """uint8 pixels through the in-kernel pixel/255.0 table == fp32 images through the fp32 kernel
-    (the CUDA-core kernel, which is the one that has the uint8 ingest)."""
+    """uint8 pixels through the in-kernel pixel/255.0 table == fp32 images, through the CUDA-core kernels (the
+    tensor-core kernel's ingest: test_tensor_core_forward_operand_range)."""
     pix = pkg.synth.synth_pixels_u8(26, n)
     images = pkg.synth.u8_to_float(pix)
     net = pkg.Net(0)
@@ -270,7 +270,7 @@ def test_forward_host_is_ordered_behind_legacy_stream_work(cuda, pkg, params0):
 @pytest.mark.parametrize("fast", [0, 1])
 @pytest.mark.parametrize("n", [1, 5, 16, 17, 100, 2368 + 5, 4099])
 def test_tensor_core_forward_three_passes_matches_oracle(cuda, pkg, ob, params0, n, fast):
-    """forward_path = 1: tcgen05 convolution in three tf32 passes keeps the 1e-5 bar of the fp32 path."""
+    """forward_path = 1: tcgen05 convolution in three passes of fp16 parts keeps the 1e-5 bar of the fp32 path."""
     images, _ = pkg.synth.synth_images(21, n)
     net = pkg.Net(0)
     net.set_params(params0)
@@ -285,7 +285,7 @@ def test_tensor_core_forward_three_passes_matches_oracle(cuda, pkg, ob, params0,
 
 def test_tensor_core_forward_full_size(cuda, pkg, ob, params0):
     """Benchmark configuration 2 at full size on both tensor-core paths.  Path 1 (three passes): 1e-5
-    on every sigmoid, argmax on every clear-margin row.  Path 2 (one tf32 pass, tanh.approx sigmoid) is
+    on every sigmoid, argmax on every clear-margin row.  Path 2 (one pass of the high parts, tanh.approx sigmoid) is
     a reduced-precision mode: its bar is 5e-3 absolute on the sigmoids and argmax equality on every
     row whose top-two margin is clear of that error (1e-2 relative); both counts are printed."""
     n = 65536

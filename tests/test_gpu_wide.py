@@ -113,9 +113,9 @@ def test_wide_full_batch_runs_and_is_deterministic(cuda, pkg, ob):
 
 
 @pytest.mark.parametrize("mode,tol", [(2, 1e-5), (1, 3e-3)])
-@pytest.mark.parametrize("H,F,n", [(56, 64, 1), (56, 64, 5), (28, 16, 33)])
+@pytest.mark.parametrize("H,F,n", [(56, 64, 1), (56, 64, 5), (28, 64, 33)])
 def test_tensor_core_conv_matches_oracle(cuda, pkg, ob, H, F, n, mode, tol):
-    """conv = 2: three tf32 passes on tcgen05 keep the 1e-5 bar; conv = 1: one pass, tf32 accuracy."""
+    """conv = 2: three passes of fp16 parts on tcgen05 keep the 1e-5 bar; conv = 1: one pass, 11 significant bits."""
     x, labels = wide_inputs(n, H, 5)
     params = wide_params(ob, H, F, 6)
     net = pkg.WideNet(H, F)
@@ -148,6 +148,8 @@ def test_tensor_core_conv_matches_oracle(cuda, pkg, ob, H, F, n, mode, tol):
     (56, 64, 70, 2, 1, 0),      # units of a CTA: several hand-overs of the gradient accumulators and a rest
     (28, 64, 9, 2, 1, 1),       # images not 16-byte aligned: the fp32 path
     (30, 64, 9, 2, 1, 0),       # a height that is not a multiple of 4: the fp32 path
+    (28, 16, 33, 2, 1, 0),      # maps that are not a multiple of 64: the fp32 path, in either mode
+    (28, 16, 33, 1, 1, 0),
 ])
 def test_tensor_core_edges_match_oracle(cuda, pkg, ob, H, F, n, mode, sigmoid, offset):
     x, labels = wide_inputs(n, H, 9)
@@ -180,7 +182,7 @@ def test_tensor_core_edges_match_oracle(cuda, pkg, ob, H, F, n, mode, sigmoid, o
 def test_wide_full_batch_matches_oracle(cuda, pkg, ob, mode):
     """Benchmark configuration 5 at its full size (batch 1,024 of 56x56 images, 64 maps) against the
     generalised oracle: forward outputs within 1e-5 relative, every gradient block within 1e-5 of its
-    largest magnitude, for the fp32 SIMT convolution (conv = 0) and the three-pass tf32 tensor-core
+    largest magnitude, for the fp32 SIMT convolution (conv = 0) and the three-pass tensor-core
     convolution (conv = 2)."""
     H, F, n = 56, 64, 1024
     x, labels = wide_inputs(n, H, 7)
