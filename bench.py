@@ -56,9 +56,9 @@ CONFIG4_IMAGES, CONFIG4_PER_GPU, CONFIG4_EPOCHS = 60000, 256, 10
 SIGMOID_NAMES = {0: "reference expression (expf + IEEE divide)",
                  1: "short form: ex2.approx + rcp.approx (~1e-6 rel per evaluation)"}
 
-# dram__bytes_read.sum + dram__bytes_write.sum of one launch over 65,536 images, per forward path,
-# from the ncu captures summarised under profiles/ (kernels_per_case.md).
-TRAFFIC_BYTES_PER_LAUNCH = {0: 210611456, 1: 211582976, 2: 211068160}
+# dram__bytes_read.sum + dram__bytes_write.sum of one launch over 65,536 images, per forward path (ncu; the captures are
+# summarised under profiles/).
+TRAFFIC_BYTES_PER_LAUNCH = {0: 210775296, 1: 211907584, 2: 210908160}
 
 
 def measured_peak_gbs():
@@ -802,7 +802,7 @@ def run_ours(args):
         if eff_path == 0:
             roof["fp32_fma_frac"] = FLOP_PER_IMAGE * BATCH / (kernel_ms * 1e-3) / fp32_peak
         if eff_path in (1, 2):
-            # tensor work actually issued (zeros of the banded operand included): MMAs per tile x 2*128*80*8 flop,
+            # tensor work actually issued (zeros of the banded operand included): MMAs per tile x 2*128*80*16 flop,
             # one tile = 16 groups of 8 output rows = 16/3 images; fp16 peak = the measured bf16 burst peak
             mma_flop_per_image = (30 if eff_path == 1 else 10) * 2 * 128 * 80 * 16 / (16.0 / 3.0)
             fp16_peak = measured_bf16_tflops() * 1e12
@@ -821,7 +821,7 @@ def run_ours(args):
             "roofline": roof,
             "e2e": {"value": e2e_value, "unit": "images/s", "h2d_bytes_per_step": BATCH * 3136,
                     "d2h_bytes_per_step": BATCH * 44, "steps": e2e_steps,
-                    "api": "cnn_forward_batched_host (pinned host buffers, 8,192-image chunks on two streams)"},
+                    "api": "cnn_forward_batched_host (pinned host buffers, chunks of at most 8,192 images over three slots)"},
             "e2e_u8": {"value": e2e_u8_value, "unit": "images/s", "h2d_bytes_per_step": BATCH * 784,
                        "d2h_bytes_per_step": BATCH * 44, "api": "cnn_forward_batched_u8_host (uint8 pixels, "
                        "pixel/255.0 applied in the kernel; bit-identical results)"},
