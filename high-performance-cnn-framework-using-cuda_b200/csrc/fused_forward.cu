@@ -430,11 +430,14 @@ static int launch_variant(cnn_net* net, int path, const void* d_images, long n, 
 }
 
 // The kernel a call over n_total images uses: 0 = k_forward_tiles, kForwardOne = k_forward_one, 1 / 2 = forward_tc.cu.
-// Default (-1): the three-pass tensor-core kernel for batches of kTcMinBatch images and more, this file's below.
+// Default (-1): the three-pass tensor-core kernel for batches of kTcMinBatch images and more, this file's below.  The line is the one
+// that the interface promises (the two sides differ in their last bits); it is not where the kernels meet.  That is at one round of
+// tiles, 14 images per SM: 2,072 images 10.9 us here, 11.1 on the tensor cores; 2,073 images 14.2 and 11.1; 4,144: 19.1 and 15.4; 6,143: 27.3 and
+// 18.8 (uint8: 11.5 / 10.9, 14.9 / 10.9, 21.0 / 14.9, 29.9 / 18.0).
 // uint8 pixels follow the same rule, so that they give the same bits as the fp32
 // images they stand for (the reduced-precision path 2 is for fp32 images only).  All keep the 1e-5 parity bar.
 // With the reference's sigmoid expression asked for (fast_sigmoid = 0) the default stays in this file.  Up to six images
-// per SM the one-image kernel is the faster one: 600 images 8.0 us, 1,000 images 11.0 us, against 10.5 us for a round of
+// per SM the one-image kernel is the faster one: 600 images 8.0 us, 1,000 images 11.0 us, against 10.6 us for a round of
 // tiles, which is what anything up to 2,072 images costs there.
 int forward_kernel_for(const cnn_net* net, long n_total, bool u8) {
   constexpr long kTcMinBatch = 6144;

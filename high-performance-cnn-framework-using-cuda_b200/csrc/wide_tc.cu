@@ -47,8 +47,8 @@
 //               all warps half by half, as the tensor core is ahead.  Backward: deltas, their fp16 parts into the A operand,
 //               subsample-filter gradient and bias sums in registers; eight warps for each half of a unit, so that one half's work
 //               while the other's wait for the tensor core (377 -> 363 us, with one pass 344 -> 325).
-// Bounds: forward 97 us for 1,024 images (before, with an im2col gather and a subsample kernel of its own: 174 + 152 us), the
-// special-function unit two thirds busy; backward 192 us (454 us, which did not have to compute the activations), special-function
+// Bounds: forward 98 us for 1,024 images (before, with an im2col gather and a subsample kernel of its own: 174 + 152 us), the
+// special-function unit two thirds busy; backward 184 us (454 us, which did not have to compute the activations), special-function
 // unit, fp32 pipe and issue slots about half busy each, the rest the hand-overs between tensor core and epilogue.
 // Work is cut into equal ranges of units, so a CTA may begin and end in the middle of a group set.
 #include <type_traits>

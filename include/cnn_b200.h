@@ -314,10 +314,10 @@ int cnn_wide_get_params(cnn_wide* w, float* h_params);
  * relative), 2 = the same with both operands in two fp16 parts and three passes (hi*hi + lo*hi + hi*lo, fp32-level
  * accuracy).  The tensor-core kernels take F a multiple of 64, H a multiple of 4 and images that start on a
  * 16-byte boundary; the fp32 kernels run everything else.  Their fp16 operands are scaled by powers of two, one for the pixels of a
- * call; an image that is too bright for the others' scale -- its largest pixel above 2^(10 - E), with 2^E the largest filter weight's power
- * of two, and above 4,096 times that of the dimmest image that is not blank -- or has a pixel that is not finite is computed in plain fp32 by the same
- * kernels (slower, and as exact): no image's result depends on what else is in the call.  Filter weights share a scale too: they
- * are exact to 2^-34 of the largest. */
+ * call.  An image that is too bright for the others' scale (its largest pixel above both 2^(10 - E), where 2^E is the largest
+ * power of two not above the largest filter weight, and 4,096 times the largest pixel of the dimmest image that is not
+ * blank), or that has a pixel that is not finite, is computed in plain fp32 by the same kernels: slower, and no image spoils
+ * another's result.  The filter weights share a scale too: they are exact to 2^-34 of the largest. */
 int cnn_wide_set_option(cnn_wide* w, const char* key, int value);
 /* As cnn_net_status. */
 int cnn_wide_status(cnn_wide* w, int* status);
