@@ -225,7 +225,7 @@ def test_wide_full_batch_matches_oracle(cuda, pkg, ob, mode):
 
 @pytest.mark.parametrize("what", ["bright images", "all but one bright", "not finite", "huge filter", "huge FC weights", "dim"])
 @pytest.mark.parametrize("mode", [1, 2])
-@pytest.mark.parametrize("H,F,n", [(56, 64, 40), (8, 128, 301)])
+@pytest.mark.parametrize("H,F,n", [(56, 64, 40), (8, 128, 301), (8, 64, 3500)])
 def test_tensor_core_images_do_not_depend_on_their_neighbours(cuda, pkg, ob, H, F, n, mode, what):
     """One power of two scales the pixels of a call, so an image much brighter than others (or not finite) has to leave them
     untouched and come out right itself: both for the outputs, image by image, and for the gradient.  Weights of any magnitude
