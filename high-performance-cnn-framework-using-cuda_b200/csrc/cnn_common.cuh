@@ -52,6 +52,13 @@ __device__ __forceinline__ float min_nan(float a, float b) {
   return y;
 }
 
+// Largest magnitude of three floats, NaN if one of them is.
+__device__ __forceinline__ float max_abs_nan(float a, float b, float c) {
+  float y;
+  asm("max.NaN.abs.f32 %0, %1, %2, %3;" : "=f"(y) : "f"(a), "f"(b), "f"(c));
+  return y;
+}
+
 // Two floats in one 64-bit register pair and the packed fp32 instructions on them (sm_100): one issue slot for two
 // lanes' worth of arithmetic, each half rounded like the scalar instruction.
 typedef unsigned long long f32x2;

@@ -19,14 +19,19 @@
 // Column chunks are kept at columns 0-7, 8-15, 12-19, 20-27, so that both blocks start on a chunk.
 // One tile of 16 groups (5.33 images) costs 10 MMAs of 128 x 80 x 16 per pass.
 //
-// Accuracy.  Path 1 splits both operands into an fp16 high part and an fp16 remainder and issues hi*hi + lo*hi +
-// hi*lo (fp32 accumulation): 22-23 significant bits of either operand take part, what is left out is lo*lo,
+// Accuracy.  Path 1 splits both operands into an fp16 high part and an fp16 remainder and issues hi*hi + hi*lo +
+// lo*hi (fp32 accumulation): 22-23 significant bits of either operand take part, what is left out is lo*lo,
 // about 2^-24 relative.  fp16 instead of tf32 halves the MMAs (K = 16 per instruction at the same operand bytes,
 // and operand bytes are what an MMA of this shape costs) at one more bit of mantissa.  Its range does not cover
-// fp32's, so weights and pixels are scaled by powers of two that follow the largest weight w (undone, exactly, in the
+// fp32's, so weights and pixels are scaled with powers of two that follow the largest weight w (undone, exactly, in the
 // epilogue's bias FMA): weights so that w lies between 256 and 512, pixels by more than 25 w, which keeps what a pixel's
-// parts lose (2^-25 of the scaled value, absolute) below 2^-24 in any pre-activation, whatever the pixels.  An image
-// with a scaled pixel of 65,520 or more (a pixel of 1,000 to 2,000 where w = 1: its pre-activations are no longer
+// parts lose (2^-25 of the scaled value, absolute) below 2^-24 in any pre-activation, whatever the pixels.
+// Besides the power of two a pixel is multiplied by 255, and the weights by 1 / 255 (in two parts, so that it costs them
+// nothing): a pixel that is a byte / 255, as image files have them, then is a whole number below 256 times a power of two, in fp32
+// arithmetic exactly, its high part all of it and its remainder zero.  A tile of such images takes two passes instead
+// of three; the third would add zeros, so what an image gives does not depend on its neighbours.  (65,536 images: 138 -> 115 us; images
+// of other numbers 134 -> 127 us, by the loader alone.)  Such a pixel kept as a byte needs no table: fp16(byte) is two instructions per pair.
+// An image with a scaled pixel of 65,520 or more (a pixel of 1,000 to 2,000 where w = 1: its pre-activations are no longer
 // of order one) is noticed by the loader, and a finisher warp computes it in plain fp32 instead (slow, 0.1 ms per image; no
 // image data is expected there).  uint8 pixels reach that limit only where w is above 1,000: the finishers look for themselves
 // then.  With a weight or a conv bias of 1e27 or more, or one that is not finite, all images go that way.
@@ -34,10 +39,9 @@
 // per activation: outputs within about 1e-4, argmax equal wherever the top-two margin is clear of that.
 //
 // Pipeline (one CTA per SM, 20 warps, everything handed over through mbarriers with bounded waits):
-//   warps 4-7   fetch the tile's rows -- consecutive in HBM -- by one bulk copy per tile, three tiles ahead, convert
-//               them to fp16 high and low parts and store them in the operand layout, 16 bytes per store (uint8
-//               pixels go through a 256-entry table of both parts of pixel / 255.0).  (Loads into registers one
-//               tile ahead left the copy's latency, 2,300 cycles per tile, in the path: cost 4 us of 136);
+//   warps 4-7   fetch the tile's rows -- consecutive in HBM -- by one bulk copy per tile, three tiles ahead (path 2: warp 3 does), convert
+//               them to fp16 high and low parts and store them in the operand layout, 16 bytes per store.  A copy into registers
+//               one tile ahead left its latency, 2,300 cycles per tile, in the path: cost 4 us of 136;
 //   warp 3      issues the tile's MMAs into one of three 160-column accumulators and commits to
 //               mbarriers (the whole warp runs the loop, an elected lane issues: see wide_tc.cuh);
 //   warps 8-19  three epilogue groups of four warps (one per 32-lane quarter of tensor memory), one
@@ -49,10 +53,10 @@
 //               output, so the weights are read once for three images), reduce-scatter, output
 //               sigmoid, argmax (lowest index wins ties), 44 bytes per image to HBM.
 //
-// Measured on a B200 (tf32 operands over stacked images before, now): 65,536 fp32 images 213 -> 137 us, 30,011 uint8 images
-// 151 us (CUDA-core kernel) -> 65 us, path 2 on 65,536 images 122 -> 98 us.  What bounds it now, per tile of 5.33 images
-// (2,900 cycles): the shared-memory data pipe (30 MMAs fetch 195 KB of operands, the other warps move 75 KB), and next
-// the special-function unit (1,600 cycles) and instruction issue (1,700); path 2: the special-function unit, 73 % busy.
+// Measured on a B200 (three passes whatever the pixels, a table for uint8 before, now): 65,536 fp32 images 138 -> 115 us, 30,011 uint8 images
+// 65 -> 54 us, path 2 on 65,536 images 98 -> 92 us (loader without bank conflicts).  What bounds it now, per tile of 5.33 images
+// (2,400 cycles): the shared-memory data pipe (20 MMAs fetch 130 KB of operands, 1,040 cycles, the other warps and the copies take 900),
+// and next the special-function unit (1,600 cycles) and instruction issue (1,400); path 2: the special-function unit, 75 % busy.
 #include <type_traits>
 
 #include "cluster_exchange.cuh"
@@ -71,9 +75,9 @@ constexpr int kTfGroups = 16;                // groups of 8 output rows per tile
 constexpr int kTfGroupsImg = 3;              // groups per image
 constexpr int kTfGroupRows = 12;             // input rows a group keeps: 8 + 4
 constexpr unsigned kTfGroupStride = kTfGroupRows * 16;                       // 192 B
-constexpr unsigned kTfChunkStride = kTfGroups * kTfGroupStride + 32;         // 3,104 B: the 32 B put the four chunks of a
-                                                                             // row into different banks for the loader
-constexpr int kTfSlabBytes = 4 * kTfChunkStride;                             // 12,416
+constexpr unsigned kTfChunkStride = kTfGroups * kTfGroupStride + 16;         // 3,088 B: the 16 B put the four chunks of the rows
+                                                                             // r and r + 4 into different banks for the loader
+constexpr int kTfSlabBytes = 4 * kTfChunkStride;                             // 12,352
 constexpr int kTfBN = 80;                    // MMA N of one 12-column block: 72 used, padded to 16n
 constexpr unsigned kTfBChunk = kTfBN * 16;   // 1,280 B between the two K chunks of a kernel row
 constexpr unsigned kTfBRow = 2 * kTfBChunk;  // 2,560 B per kernel row (K = 16)
@@ -99,11 +103,11 @@ struct TfSmem {
   alignas(128) unsigned char b_lo[kTfBBytes];                 // path 1 only
   alignas(16) float wf[kTfFcIn][3][32][4];    // FC weights of subsample output 32 j + lane: ten, padded to twelve
   alignas(16) float as[kTfSlots][kTfAsStride];   // subsample activations of an image: [window row][6 * window column + map]
-  unsigned lut[256];                          // uint8 pixels only: fp16 parts of pixel / 255.0, high part in the low half
   float bc[8], ws[16], bs[4], bf[12];
   unsigned long long raw_full[kTfRaw], raw_free[kTfRaw];
   unsigned long long a_full[kTfSlabsTotal], a_free[kTfSlabsTotal], d_full[2 * kTfAcc], d_free[2 * kTfAcc], img_done[kTfSlots];
   unsigned char out_of_range[kTfRange];
+  alignas(4) unsigned char has_low[kTfSlabsTotal][4];    // per slab and loader warp: some pixel of the tile has a remainder
   int finished[kTfFinishers];                            // image triples that each finisher warp has written out (slot reuse guard)
   unsigned tmem_base;
   long long clock_base;                       // phase clocks only
@@ -174,7 +178,7 @@ __device__ __noinline__ float image_fc_plain(const Pixel* image, const float* pa
 // are right.  As the fp32 images' loader does, all images of a tile with a pixel out of range are taken -- noticed here, because in the
 // loader it cost 5 % of every call.
 template <int SIG>
-__device__ __noinline__ float finish_plain_u8(const unsigned char* pixels, const float* params, const unsigned* lut, int base, int imgs, bool all,
+__device__ __noinline__ float finish_plain_u8(const unsigned char* pixels, const float* params, float level, int base, int imgs, bool all,
                                               float z, int lane) {
   for (int j = 0; j < 3 && base + j < imgs; ++j) {
     const int g = (base + j) * kTfGroupsImg, end = imgs * kTfGroupsImg;
@@ -183,7 +187,7 @@ __device__ __noinline__ float finish_plain_u8(const unsigned char* pixels, const
     for (int i = group_pixel(g0) / 4 + lane; i < (group_pixel(g1) + kTfGroupRows * kH) / 4; i += 32)
       most = __vmaxu4(most, reinterpret_cast<const unsigned*>(pixels)[i]);
     most = __reduce_max_sync(0xffffffffu, max(max(most & 255u, (most >> 8) & 255u), max((most >> 16) & 255u, most >> 24)));
-    if (!all && (lut[most] & 0xffffu) != 0x7c00u) continue;      // its high part is finite
+    if (!all && (float)most * level < 65520.f) continue;      // its high part is finite
     const float s = image_fc_plain<SIG>(pixels + (size_t)(base + j) * kImg, params, lane);
     const float sk = __shfl_sync(0xffffffffu, s, lane % 10);
     if (lane / 10 == j) z = sk;
@@ -201,7 +205,8 @@ k_forward_tc(const void* images, long n, long imgs_per_cta, const float* params,
   TfSmem& sm = *reinterpret_cast<TfSmem*>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~(uintptr_t)127);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   constexpr bool kPrecise = (PATH == 1);
-  constexpr int kTfSlabs = kPrecise ? kTfSlabsTotal / 2 : kTfSlabsTotal;   // slabs in flight
+  constexpr bool kLow = kPrecise && !U8;                                   // pixels may have a remainder
+  constexpr int kTfSlabs = kLow ? kTfSlabsTotal / 2 : kTfSlabsTotal;       // slabs in flight
   // Path 2 computes tanh(v / 2): conv weights and bias are halved.  Path 1 with the short sigmoid form folds
   // the form's multiplication by -log2(e) into them.
   constexpr bool kShort = kPrecise && (SIG == 1);
@@ -215,7 +220,7 @@ k_forward_tc(const void* images, long n, long imgs_per_cta, const float* params,
 
   // ---- set-up that touches nothing of the kernel before this one ------------------------------------
   pdl_launch_dependents();
-  if (tid == 0) {
+  if (tid == 32 * kTfMmaWarp) {
     for (int s = 0; s < kTfRaw; ++s) {
       mbar_init(&sm.raw_full[s], 1);
       mbar_init(&sm.raw_free[s], kTfLoaders / 32);
@@ -240,18 +245,26 @@ k_forward_tc(const void* images, long n, long imgs_per_cta, const float* params,
   // ---- loaders: the first copies leave now ------------------------------------------------------------------
   const int lt = tid - 32 * kTfLoadWarp0;
   const bool loader = lt >= 0 && lt < kTfLoaders;
-  auto fetch = [&](int k) {       // one thread: the rows of tile k, from its first group's first to its last group's twelfth
-    constexpr unsigned kBytes = U8 ? 1u : 4u;
+  // One thread: the rows of tile k, from its first group's first to its last group's twelfth (source offset, size), by one bulk copy.
+  constexpr unsigned kPixelBytes = U8 ? 1u : 4u;
+  auto fetch_extent = [&](int k, unsigned& bytes) {
     const int g0 = k * kTfGroups, g1 = min(g0 + kTfGroups, n_groups) - 1;
     const int first = group_pixel(g0);
-    const unsigned bytes = (unsigned)(group_pixel(g1) + kTfGroupRows * kH - first) * kBytes;
+    bytes = (unsigned)(group_pixel(g1) + kTfGroupRows * kH - first) * kPixelBytes;
+    return static_cast<const unsigned char*>(images) + (size_t)(img0 * kImg + first) * kPixelBytes;
+  };
+  auto fetch = [&](int k, const unsigned char* src, unsigned bytes) {
     unsigned long long* bar = &sm.raw_full[k % kTfRaw];
     mbar_expect_tx(bar, bytes);
-    bulk_g2s(sm.raw[k % kTfRaw], static_cast<const unsigned char*>(images) + (size_t)(img0 * kImg + first) * kBytes, bytes, bar);
+    bulk_g2s(sm.raw[k % kTfRaw], src, bytes, bar);
   };
 
-  if (tid == 0)        // the thread that initialised the barriers
-    for (int k = 0; k < kTfRaw - 1 && k < n_tiles; ++k) fetch(k);
+  if (tid == 32 * kTfMmaWarp)        // the thread that initialised the barriers
+    for (int k = 0; k < kTfRaw && k < n_tiles; ++k) {
+      unsigned bytes;
+      const unsigned char* src = fetch_extent(k, bytes);
+      fetch(k, src, bytes);
+    }
 
   // ---- set-up: weight scale, B operand (banded weights), FC table, small parameters -------------------------
   float wmax = 0.f;
@@ -268,17 +281,11 @@ k_forward_tc(const void* images, long n, long imgs_per_cta, const float* params,
 #pragma unroll
   for (int m = 16; m > 0; m >>= 1) wmax = fmaxf(wmax, __shfl_xor_sync(0xffffffffu, wmax, m));
   const bool plain = !__all_sync(0xffffffffu, finite);    // parameters that fp16 cannot stand in for: every image in plain fp32
-  // With 2^E <= max |kPre * w| < 2^(E+1) weights are scaled by 2^(8-E) and pixels by 2^(E+5): the accumulator carries 2^13.
+  // With 2^E <= max |kPre * w| < 2^(E+1) weights are scaled by 2^(16-E) / 255 and pixels by 255 * 2^(E-3): the accumulator carries 2^13.
   int wexp = (int)((__float_as_uint(fabsf(kPre) * wmax) >> 23) & 255u) - 127;
   wexp = wexp > 90 ? 90 : (wexp < -90 ? -90 : wexp);
-  const float w_scale = __int_as_float((127 + 8 - wexp) << 23), px_scale = __int_as_float((127 + 5 + wexp) << 23);
+  const float w_scale = __int_as_float((127 + 16 - wexp) << 23), px_scale = 255.f * __int_as_float((127 - 3 + wexp) << 23);
   constexpr float w_unscale = 1.0f / 8192.0f;
-  if (U8 && tid < 256) {
-    const float v = (float)((double)tid / 255.0) * px_scale;
-    const __half hi = __float2half_rn(v);
-    const __half lo = __float2half_rn(v - __half2float(hi));
-    sm.lut[tid] = (unsigned)__half_as_ushort(hi) | ((unsigned)__half_as_ushort(lo) << 16);
-  }
 
   for (int e = tid; e < 5 * 2 * kTfBN; e += kTfThreads) {     // one 16-byte row of a chunk: 8 columns of one accumulator column
     const int i = e / (2 * kTfBN), rem = e % (2 * kTfBN);
@@ -287,8 +294,10 @@ k_forward_tc(const void* images, long n, long imgs_per_cta, const float* params,
     const int qq = nn / 24, r = nn % 24, f = 2 * (r / 8) + (r & 1), x = 4 * qq + ((r & 7) >> 1);
     float w[5];
 #pragma unroll
-    for (int d = 0; d < 5; ++d) w[d] = (nn < 72) ? kPre * params[kOffWc + f * 25 + i * 5 + d] : 0.f;
+    for (int d = 0; d < 5; ++d) w[d] = (nn < 72) ? w_scale * params[kOffWc + f * 25 + i * 5 + d] : 0.f;
     __half2 hi[4], lo[4];
+    constexpr double kFactor = (double)kPre / 255.0;            // in two parts, so that the factor costs the weights no bit
+    constexpr float kFactorHi = (float)kFactor, kFactorLo = (float)(kFactor - (double)kFactorHi);
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
       float t[2];
@@ -299,7 +308,9 @@ k_forward_tc(const void* images, long n, long imgs_per_cta, const float* params,
 #pragma unroll
         for (int dd = 0; dd < 5; ++dd) t[h] = (d == dd) ? w[dd] : t[h];
       }
-      tc::split_f16x2(t[0], t[1], w_scale, hi[c], lo[c]);
+      hi[c] = __floats2half2_rn(t[0] * kFactorHi, t[1] * kFactorHi);
+      const float2 b = __half22float2(hi[c]);
+      lo[c] = __floats2half2_rn(fmaf(t[0], kFactorLo, fmaf(t[0], kFactorHi, -b.x)), fmaf(t[1], kFactorLo, fmaf(t[1], kFactorHi, -b.y)));
     }
     const unsigned off = (unsigned)i * kTfBRow + (unsigned)ch * kTfBChunk + (unsigned)nn * 16u;
     *reinterpret_cast<uint4*>(sm.b_hi + off) = *reinterpret_cast<uint4*>(hi);
@@ -371,8 +382,8 @@ k_forward_tc(const void* images, long n, long imgs_per_cta, const float* params,
         for (int kk = 0; kk < kOut / 2; ++kk) unpack2(fc2[j][kk], sums[10 * j + 2 * kk], sums[10 * j + 2 * kk + 1]);
       float z = warp_reduce_scatter32(sums, lane);      // lane 10 li + k: sum k of image base + li
       if constexpr (U8) {
-        if (plain || px_scale >= 65536.f)
-          z = finish_plain_u8<SIG>(static_cast<const unsigned char*>(images) + img0 * kImg, params, sm.lut, base, imgs_here, plain, z, lane);
+        if (plain || px_scale >= 65520.f)
+          z = finish_plain_u8<SIG>(static_cast<const unsigned char*>(images) + img0 * kImg, params, px_scale * (1.0f / 255.0f), base, imgs_here, plain, z, lane);
       }
       const bool bad = !U8 && active && (plain || sm.out_of_range[img & (kTfRange - 1)] != 0);
       if (!U8 && __any_sync(0xffffffffu, bad)) {
@@ -412,9 +423,16 @@ k_forward_tc(const void* images, long n, long imgs_per_cta, const float* params,
     for (int k = 0; k < n_tiles; ++k) {
       const int s = k % kTfSlabs, b = k % kTfAcc;
       CNN_PHASE(0);
+      unsigned bytes = 0;
+      const unsigned char* src = kPrecise ? nullptr : fetch_extent(k + kTfRaw, bytes);
       mbar_wait_bounded(&sm.a_full[s], (unsigned)(k / kTfSlabs) & 1u, status, gave_up);
       CNN_PHASE(1);
+      // Issuing a bulk copy takes 300 cycles.  With one pass this warp has them to spare, with two or three the loaders do (path 2 by the
+      // loaders: 94 instead of 91 us; path 1 by this warp: 118 instead of 116).
+      if (!kPrecise && lane == 0 && k + kTfRaw < n_tiles) fetch(k + kTfRaw, src, bytes);     // the loaders are done with tile k's buffer
+      __syncwarp();
       CNN_PHASE(2);
+      const bool low = kLow && *reinterpret_cast<const volatile unsigned*>(sm.has_low[s]) != 0;
       const unsigned long long ad_hi = tc::smem_desc(smem_u32(sm.slab[s]), kTfChunkStride, kTfGroupStride);
       const unsigned long long ad_lo = tc::smem_desc(smem_u32(sm.slab[(s + kTfSlabsTotal / 2) % kTfSlabsTotal]), kTfChunkStride, kTfGroupStride);
       const unsigned d_tile = tmem_base + (unsigned)(b * kTfDCols);
@@ -433,8 +451,9 @@ k_forward_tc(const void* images, long n, long imgs_per_cta, const float* params,
         const unsigned a_blk = ((unsigned)(2 * xb) * kTfChunkStride) >> 4;
 #pragma unroll
         for (int pass = 0; pass < (kPrecise ? 3 : 1); ++pass) {
-          const unsigned long long a_d = ((pass == 1) ? ad_lo : ad_hi) + a_blk;
-          const unsigned long long b_d = (pass == 2) ? bd_lo : bd_hi;
+          if (pass == 2 && !low) continue;
+          const unsigned long long a_d = ((pass == 2) ? ad_lo : ad_hi) + a_blk;
+          const unsigned long long b_d = (pass == 1) ? bd_lo : bd_hi;
 #pragma unroll
           for (int i = 0; i < 5; ++i)
             tc::mma_f16_elect(d_blk, a_d + (unsigned)i, b_d + (unsigned)i * (kTfBRow >> 4), idesc, (pass | i) ? 1u : 0u);
@@ -446,72 +465,102 @@ k_forward_tc(const void* images, long n, long imgs_per_cta, const float* params,
     }
   } else if (loader) {
     // ================= loaders: image rows -> operand slabs ==========================================
-    // Unit u = (group, row, chunk), chunk fastest: eight consecutive lanes store two rows of the four chunks without a bank
-    // conflict.  A thread's units u + 128 j repeat after three, eight groups further on.
+    // A thread converts eight pixels (one column chunk) of six rows of one group: rows j + 4 * sub (j < 4), j + 4 + 2 * sub (j = 4, 5).  Eight
+    // consecutive lanes are the four chunks of two rows, four rows apart as a rule: neither their 16-byte loads (rows of 28 floats) nor
+    // their stores meet in a bank then (two rows that are neighbours took two turns per load: 200 cycles per tile).
     typedef typename std::conditional<U8, unsigned, float4>::type Piece;     // four pixels
-    int ugroup[3], ugoff[3];
-    unsigned usoff[3];
-#pragma unroll
-    for (int j = 0; j < 3; ++j) {
-      const int u = lt + kTfLoaders * j;
-      const int r = u % (4 * kTfGroupRows), row = r >> 2, chunk = r & 3;
-      ugroup[j] = u / (4 * kTfGroupRows);
-      ugoff[j] = row * 7 + 2 * chunk - (chunk >> 1);                          // columns 0, 8, 12, 20
-      usoff[j] = (unsigned)chunk * kTfChunkStride + (unsigned)(ugroup[j] * kTfGroupRows + row) * 16u;
-    }
+    const int chunk = lane & 3, sub = (lane >> 2) & 1, group = 4 * (warp - kTfLoadWarp0) + (lane >> 3);
+    const int column = 2 * chunk - (chunk >> 1);                              // columns 0, 8, 12, 20
+    const unsigned slab_at = (unsigned)chunk * kTfChunkStride + (unsigned)(group * kTfGroupRows) * 16u;
+    auto row_of = [&](int j) { return j < 4 ? j + 4 * sub : j + 4 + 2 * sub; };
+    // uint8 pixels: fp16 1024 + pixel is the byte below 0x64; times 2^e1, minus 1024 * 2^e1, is exact; 2^e2 (as a rule 1) finishes the scale where
+    // fp16 could not hold its factors, and rounds, overflows or vanishes as the conversion of an fp32 image's scaled pixel does.
+    const int e1 = min(max(wexp - 3, -24), 5), e2 = min(max(wexp - 3 - e1, -25), 15);
+    const __half2 s1 = __float2half2_rn(__int_as_float((127 + e1) << 23)), s2 = __float2half2_rn(__int_as_float((127 + e2) << 23));
+    const __half2 base1 = __float2half2_rn(-1024.f * __int_as_float((127 + e1) << 23));
+    const f32x2 px_scale2 = pack2(px_scale, px_scale);
+    unsigned stale = (1u << kTfSlabs) - 1;      // slabs whose low part, this warp's share of it, is not all zeros
+    bool expect_low = true;
     for (int k = 0; k < n_tiles; ++k) {
       const int s = k % kTfSlabs, r = k % kTfRaw;
       CNN_PHASE(0);
-      if (lt == 0 && k + kTfRaw - 1 < n_tiles) {       // the buffer of tile k - 1 is next
-        if (k > 0) mbar_wait_bounded(&sm.raw_free[(k - 1) % kTfRaw], (unsigned)((k - 1) / kTfRaw) & 1u, status, gave_up);
-        fetch(k + kTfRaw - 1);
-      }
-      __syncwarp();
       mbar_wait_bounded(&sm.raw_full[r], (unsigned)(k / kTfRaw) & 1u, status, gave_up);
       CNN_PHASE(1);
-      // Groups past the last image read what the buffer held before: their output rows are never looked at.
-      const Piece* raw = reinterpret_cast<const Piece*>(sm.raw[r]) - group_pixel(k * kTfGroups) / 4;
-      Piece v[kTfUnits][2];
-#pragma unroll
-      for (int j = 0; j < kTfUnits; ++j) {
-        const Piece* p = raw + group_pixel(k * kTfGroups + ugroup[j % 3] + (kTfGroups / 2) * (j / 3)) / 4 + ugoff[j % 3];
-        v[j][0] = p[0];
-        v[j][1] = p[1];
-      }
       mbar_wait_bounded(&sm.a_free[s], ((unsigned)(k / kTfSlabs) & 1u) ^ 1u, status, gave_up);
       CNN_PHASE(2);
+      // Groups past the last image read what the buffer held before: their output rows are never looked at.
+      const Piece* raw = reinterpret_cast<const Piece*>(sm.raw[r]) + (group_pixel(k * kTfGroups + group) - group_pixel(k * kTfGroups)) / 4 + column;
+      const bool live = k * kTfGroups + group < n_groups;
       unsigned char* hi_s = sm.slab[s];
       unsigned char* lo_s = sm.slab[(s + kTfSlabsTotal / 2) % kTfSlabsTotal];
-      __half2 top = __floats2half2_rn(0.f, 0.f);
+      float top = 0.f;
+      // Stores the high parts and, LOW, the low parts; says whether some pixel of this thread's has (or, without LOW, may have) a remainder.
+      auto convert = [&](auto low_too) {
+        [[maybe_unused]] constexpr bool LOW = decltype(low_too)::value;
+        unsigned bits = 0;
+        Piece v[kTfUnits][2];
 #pragma unroll
-      for (int j = 0; j < kTfUnits; ++j) {
-        unsigned hi[4], lo[4];
-        const bool live = k * kTfGroups + ugroup[j % 3] + (kTfGroups / 2) * (j / 3) < n_groups;
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          if constexpr (U8) {
-            const unsigned b = v[j][h];
-            const unsigned e0 = sm.lut[b & 255u], e1 = sm.lut[(b >> 8) & 255u], e2 = sm.lut[(b >> 16) & 255u], e3 = sm.lut[b >> 24];
-            hi[2 * h] = __byte_perm(e0, e1, 0x5410); hi[2 * h + 1] = __byte_perm(e2, e3, 0x5410);
-            lo[2 * h] = __byte_perm(e0, e1, 0x7632); lo[2 * h + 1] = __byte_perm(e2, e3, 0x7632);
-          } else {
-            __half2 h0, h1, l0, l1;
-            tc::split_f16x2(v[j][h].x, v[j][h].y, px_scale, h0, l0);
-            tc::split_f16x2(v[j][h].z, v[j][h].w, px_scale, h1, l1);
-            if (live) top = __hmax2_nan(top, __hmax2_nan(__habs2(h0), __habs2(h1)));
-            hi[2 * h] = *reinterpret_cast<unsigned*>(&h0); hi[2 * h + 1] = *reinterpret_cast<unsigned*>(&h1);
-            lo[2 * h] = *reinterpret_cast<unsigned*>(&l0); lo[2 * h + 1] = *reinterpret_cast<unsigned*>(&l1);
-          }
+        for (int j = 0; j < kTfUnits; ++j) {
+          const Piece* p = raw + row_of(j) * (kH / 4);
+          v[j][0] = p[0];
+          v[j][1] = p[1];
         }
-        const unsigned o = usoff[j % 3] + (unsigned)(j / 3) * ((kTfGroups / 2) * kTfGroupStride);
-        *reinterpret_cast<uint4*>(hi_s + o) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-        if (kPrecise) *reinterpret_cast<uint4*>(lo_s + o) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+#pragma unroll
+        for (int j = 0; j < kTfUnits; ++j) {
+          unsigned hi[4];
+          const unsigned o = slab_at + (unsigned)row_of(j) * 16u;
+          if constexpr (U8) {
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+              const unsigned two = __byte_perm(v[j][c >> 1], 0x64646464u, (c & 1) ? 0x4342 : 0x4140);
+              __half2 x = __hfma2(*reinterpret_cast<const __half2*>(&two), s1, base1);
+              if (e2 != 0) x = __hmul2(x, s2);
+              hi[c] = *reinterpret_cast<unsigned*>(&x);
+            }
+          } else {
+            float x[8], big = 0.f;
+            unpack2(mul2(pack2(v[j][0].x, v[j][0].y), px_scale2), x[0], x[1]);
+            unpack2(mul2(pack2(v[j][0].z, v[j][0].w), px_scale2), x[2], x[3]);
+            unpack2(mul2(pack2(v[j][1].x, v[j][1].y), px_scale2), x[4], x[5]);
+            unpack2(mul2(pack2(v[j][1].z, v[j][1].w), px_scale2), x[6], x[7]);
+            [[maybe_unused]] unsigned lo[4];
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+              const __half2 h = __floats2half2_rn(x[2 * c], x[2 * c + 1]);
+              hi[c] = *reinterpret_cast<const unsigned*>(&h);
+              big = max_abs_nan(big, x[2 * c], x[2 * c + 1]);
+              if constexpr (LOW) {
+                const float2 b = __half22float2(h);
+                const __half2 l = __floats2half2_rn(x[2 * c] - b.x, x[2 * c + 1] - b.y);
+                lo[c] = *reinterpret_cast<const unsigned*>(&l);
+                bits |= lo[c];
+              } else {
+                bits |= (__float_as_uint(x[2 * c]) | __float_as_uint(x[2 * c + 1])) & 0x1fffu;      // eleven significant bits leave no remainder
+              }
+            }
+            if constexpr (LOW) *reinterpret_cast<uint4*>(lo_s + o) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+            if (live) top = max_abs_nan(top, big, big);
+          }
+          *reinterpret_cast<uint4*>(hi_s + o) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+        }
+        return bits != 0;
+      };
+      if constexpr (kLow) {
+        // Without remainders (uint8 / 255, as image files have them) the low part is not multiplied; it is written only where it was not all zeros
+        // before.  The tile before says which of the two conversions to try first.
+        bool low = expect_low || __any_sync(0xffffffffu, convert(std::false_type()));
+        if (low || ((stale >> s) & 1u)) {
+          low = __any_sync(0xffffffffu, convert(std::true_type()));
+          stale = (stale & ~(1u << s)) | ((unsigned)low << s);
+        }
+        expect_low = low;
+        if (lane == 0) *reinterpret_cast<volatile unsigned char*>(&sm.has_low[s][warp - kTfLoadWarp0]) = low;
+      } else {
+        convert(std::false_type());
       }
       if constexpr (!U8) {
-        const float2 t = __half22float2(top);
-        const float big = (t.x != t.x || t.y != t.y) ? 1e30f : fmaxf(t.x, t.y);
         // fp16 holds magnitudes below 65,520: a larger scaled pixel (or one that is not a number) marks the tile's images
-        if (!(big < 65536.f)) {
+        if (!(top < 65520.f)) {
           const int first = (k * kTfGroups) / kTfGroupsImg, last = (k * kTfGroups + kTfGroups - 1) / kTfGroupsImg;
           for (int im = first; im <= last; ++im)
             if (im < imgs_here) sm.out_of_range[im & (kTfRange - 1)] = 1;
@@ -523,6 +572,13 @@ k_forward_tc(const void* images, long n, long imgs_per_cta, const float* params,
         mbar_arrive(&sm.raw_free[r]);
         mbar_arrive(&sm.a_full[s]);
       }
+      if (kPrecise && lt == 0 && k + kTfRaw < n_tiles) {
+        unsigned bytes;
+        const unsigned char* src = fetch_extent(k + kTfRaw, bytes);
+        mbar_wait_bounded(&sm.raw_free[r], (unsigned)(k / kTfRaw) & 1u, status, gave_up);
+        fetch(k + kTfRaw, src, bytes);
+      }
+      __syncwarp();
       CNN_PHASE(3);
     }
   } else if (warp >= kTfEpiWarp0) {

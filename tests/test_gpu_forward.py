@@ -434,6 +434,38 @@ def test_tensor_core_forward_uint8_parameter_range(cuda, pkg, params0, what, tol
         assert float(np.max(np.abs(outs[1].astype(np.float64) - outs[0]))) < tol
 
 
+@pytest.mark.parametrize("factor", [1e-9, 1e-6, 1e-3, 1.0, 30.0, 900.0])
+@pytest.mark.parametrize("n", [5, 148 * 16 + 21])
+def test_tensor_core_forward_bytes_beside_other_pixels(cuda, pkg, params0, factor, n):
+    """Pixels that are bytes / 255 leave no fp16 remainder, and a tile of them skips the pass that multiplies remainders: they give the
+    same bits as uint8 pixels and beside images with remainders, at every weight scale (the pixels' scale follows it, and the byte conversion
+    has two ranges).  Yardstick for the others: the fp32 CUDA-core kernel; a pre-activation of 25 terms up to 0.5 * factor is
+    known to 25 * 0.5 * factor * 2^-23 in fp32, a sigmoid's slope is at most 1/4, and 216 of them meet weights up to 0.5."""
+    pix = pkg.synth.synth_pixels_u8(53, n)
+    images = pkg.synth.u8_to_float(pix)
+    params = params0.copy()
+    params[:150] *= np.float32(factor)
+    rng = np.random.default_rng(3)
+    mixed = images.copy()
+    mixed[2::7] *= rng.uniform(0.5, 1.0, mixed[2::7].shape).astype(np.float32)
+    net = pkg.Net(0)
+    net.set_params(params)
+    net.set_option("forward_path", 1)
+    out, arg = run_forward(cuda, net, images)
+    out_m, _ = run_forward(cuda, net, mixed)
+    d_out = cuda.empty((n, 10), dtype=cuda.float32, device="cuda")
+    net.forward_u8(cuda.from_numpy(pix).cuda(), n, d_out, None)
+    cuda.cuda.synchronize()
+    assert np.array_equal(d_out.cpu().numpy(), out)
+    same = np.arange(n) % 7 != 2
+    assert np.array_equal(out_m[same], out[same])
+    net.set_option("forward_path", 0)
+    ref, _ = run_forward(cuda, net, mixed)
+    assert net.status() == 0
+    tol = max(1e-5, 216 * 0.5 / 4 / 4 * 25 * 0.5 * factor * 2.0 ** -23)
+    assert rel_err(out_m, ref) < tol
+
+
 @pytest.mark.parametrize("fast", [0, 1])
 @pytest.mark.parametrize("n", [2, 297, 888, 889, 895, 2073])
 def test_cuda_core_forward_around_its_dispatch(cuda, pkg, params0, n, fast):
