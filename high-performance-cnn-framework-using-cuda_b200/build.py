@@ -21,7 +21,7 @@ CSRC = os.path.join(PKG_DIR, "csrc")
 LIB_PATH = os.path.join(PKG_DIR, "libcnn_b200.so")
 OBJ_DIR = os.path.join(PKG_DIR, "build")
 
-SOURCES = ["layer_abi.cu", "net.cu", "host_pipeline.cu", "checkpoint.cu", "fused_forward.cu", "forward_tc.cu", "fused_train.cu", "dp_exchange.cu",
+SOURCES = ["layer_abi.cu", "net.cu", "host_pipeline.cu", "checkpoint.cu", "fused_forward.cu", "forward_tc.cu", "fused_train.cu", "grad_tc.cu", "dp_exchange.cu",
            "persample_cluster8.cu", "wide.cu", "wide_tc.cu", "synth.cu"]
 
 NVCC_FLAGS = [

@@ -20,6 +20,8 @@
 // Arithmetic notes (all within fp32 rounding of the reference, which itself sums with atomics in
 // a run-dependent order): sums use FMA; the per-term divisions by 576 / 216 of layer.cu:379, 397,
 // 320 become one multiplication of the delta by the reciprocal constant.
+#include <type_traits>
+
 #include "net.cuh"
 
 namespace cnn {
@@ -187,8 +189,8 @@ __device__ __forceinline__ int scatter8_index(int lane) { return ((lane >> 4) & 
 // The gradient of a team's images stays in registers (26 pairs of conv taps and bias, five pairs of FC weights, eight
 // subsample taps) until the block's reduction at the end (shuffles and shared memory, fixed order, no atomics).
 //
-// Small batches are a chain of latencies, large ones are bound by the FMA pipe (852 cycles of it per warp and image; 318 us for
-// 60,000 images).  Measured: a step of 256 images in a training loop 15.4 -> 9.6 us (of which the
+// Batches of up to 2,047 images, and what grad_tc.cu leaves.  Small batches are a chain of latencies, large ones are bound by the FMA pipe (852 cycles
+// of it per warp and image; 318 us for 60,000 images).  Measured: a step of 256 images in a training loop 15.4 -> 9.6 us (of which the
 // parameters 0.7, forward 2.5, backward 1.5, this kernel's reduction 1.2, the row sums 1.2 and the two hand-overs 1.5 us),
 // the gradient of 60,000 images 1,030 -> 640 us.  (Before: a thread per window and map, scalar, two blocks of seven warps per SM at 128 registers
 // with the patch and all gradient terms in registers, two barriers per image, a row per image up to 296.)
@@ -197,6 +199,8 @@ constexpr int kGrThreads = 224;                 // threads of a team: 216 with w
 constexpr int kGrWarps = kGrThreads / 32;
 constexpr int kGrStages = 3;                    // image buffers of a team
 constexpr int kGrRed = 27;                      // pairs per thread in the reduction: 25 taps + bias, padded to an odd number
+
+constexpr int kGrShares = 256;                  // most blocks that may have left images (LEFT)
 
 template <int TEAMS>
 struct GrSmem {
@@ -212,6 +216,7 @@ struct GrSmem {
   float red_f[kS][kOut];                        // two teams: FC gradient of the second
   float red_b[TEAMS][12];                       // FC bias gradient and error sum of a team
   unsigned long long full[TEAMS][kGrStages];
+  int before[kGrShares + 1];                    // LEFT only: images left in the shares before this one
 };
 
 // Barrier of one team's threads.
@@ -221,21 +226,33 @@ __device__ __forceinline__ void team_sync(int team) {
   else asm volatile("bar.sync %0, %1;" ::"r"(team + 1), "n"(kGrThreads) : "memory");
 }
 
-template <int FAST, int TEAMS>
+// LEFT: the images that the tensor-core kernel (grad_tc.cu) has left, the last left[b] of each share b of per_cta images; no rows are
+// written if there are none.
+template <int FAST, int TEAMS, bool LEFT = false>
 __global__ void __launch_bounds__(kGrThreads * TEAMS, 1)
 k_grad_partials(const float* images, const unsigned* labels, long n,
-                const float* params, float* __restrict__ rows, int* __restrict__ status, int chained) {
+                const float* params, float* __restrict__ rows, int* __restrict__ status, int chained,
+                const int* left, int shares, int per_cta) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   GrSmem<TEAMS>& sm = *reinterpret_cast<GrSmem<TEAMS>*>(smem_raw);
   const int team = TEAMS == 1 ? 0 : threadIdx.x / kGrThreads;
   const int tid = threadIdx.x - team * kGrThreads, warp = tid >> 5, lane = threadIdx.x & 31;
   constexpr float kPre = (FAST == 1) ? -1.4426950408889634f : 1.0f;   // the short sigmoid form's factor, folded into the conv weights
 
+  // Number of the im-th image, one of share `share` or a later one.
+  const long n_all = n;
+  auto at = [&](long im, [[maybe_unused]] int& share) -> long {
+    while (im >= sm.before[share + 1]) ++share;
+    const long end = (long)(share + 1) * per_cta < n_all ? (long)(share + 1) * per_cta : n_all;
+    return end - sm.before[share + 1] + im;
+  };
+  [[maybe_unused]] int share_copied = 0, share_read = 0;
   // Image i of this team is first + i * step.
   const long first = (long)blockIdx.x + (long)team * gridDim.x, step = (long)TEAMS * gridDim.x;
-  auto issue = [&](int i) {
-    const long im = first + (long)i * step;
+  auto issue = [&](int i, auto mapped) {
+    long im = first + (long)i * step;
     if (im >= n) return;
+    if constexpr (decltype(mapped)::value) im = at(im, share_copied);
     unsigned long long* bar = &sm.full[team][i % kGrStages];
     mbar_expect_tx(bar, kImg * sizeof(float));
     bulk_g2s(&sm.img[team][i % kGrStages][0], images + im * kImg, kImg * sizeof(float), bar);
@@ -249,12 +266,38 @@ k_grad_partials(const float* images, const unsigned* labels, long n,
     // first gradient kernel (the one that is not chained) lets its successors start only behind its own wait; kernels that
     // triggered before their waits could otherwise all start while the writer still runs.
     if (chained)
-      for (int i = 0; i < kGrStages; ++i) issue(i);
+      for (int i = 0; i < kGrStages; ++i) issue(i, std::false_type());
   }
   pdl_wait();      // the parameters (and the row buffer this kernel writes at its end) belong to the predecessor until here
   if (!chained) pdl_launch_dependents();
+  if constexpr (LEFT) {
+    const int mine = (int)threadIdx.x < shares ? left[threadIdx.x] : 0;
+    if ((int)threadIdx.x < shares) sm.before[threadIdx.x + 1] = mine;
+    if (!__syncthreads_or(mine)) return;
+    if (threadIdx.x < 32) {        // running sums, kGrShares / 32 shares per lane
+      int upto[kGrShares / 32], sum = 0;
+#pragma unroll
+      for (int i = 0; i < kGrShares / 32; ++i) {
+        const int b = lane * (kGrShares / 32) + i;
+        sum += b < shares ? sm.before[b + 1] : 0;
+        upto[i] = sum;
+      }
+      int ahead = sum;
+#pragma unroll
+      for (int m = 1; m < 32; m <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, ahead, m);
+        if (lane >= m) ahead += v;
+      }
+      ahead -= sum;
+#pragma unroll
+      for (int i = 0; i < kGrShares / 32; ++i) sm.before[lane * (kGrShares / 32) + i + 1] = ahead + upto[i];
+      if (lane == 0) sm.before[0] = 0;
+    }
+    __syncthreads();
+    n = sm.before[shares];
+  }
   if (tid == 0 && !chained)
-    for (int i = 0; i < kGrStages; ++i) issue(i);
+    for (int i = 0; i < kGrStages; ++i) issue(i, std::integral_constant<bool, LEFT>());
   // Parameters: every load of a thread is under way before the first of them is stored (one L2 latency, not one per
   // group of loads: 2.4 -> 0.75 us of a step).
   const bool live = tid < kS;
@@ -281,7 +324,7 @@ k_grad_partials(const float* images, const unsigned* labels, long n,
   const int half = tid & 1, unit = (live ? tid : 0) >> 1;      // (the eight idle threads shadow thread 0 and add zeros)
   const int pr = unit / 36, w = unit % 36;
   const int p = w / 6, q = w % 6;
-  const int at = (4 * p + 2 * half) * kH + 4 * q;
+  const int patch_at = (4 * p + 2 * half) * kH + 4 * q;
   // With one team there are registers enough to keep the taps.
   f32x2 wt[TEAMS == 1 ? 25 : 1];
   if (TEAMS == 1) {
@@ -301,12 +344,16 @@ k_grad_partials(const float* images, const unsigned* labels, long n,
   const float inv_c = 1.0f / (float)(kC * kC);
 
   bool gave_up = false;
+  auto run = [&](auto mapped) {
   int it = 0;
   for (long im = first; im < n; im += step, ++it) {
     unsigned label = 0;
-    if (lane < kOut) label = labels[im];
+    if (lane < kOut) {
+      if constexpr (decltype(mapped)::value) label = labels[at(im, share_read)];
+      else label = labels[im];
+    }
     mbar_wait_bounded(&sm.full[team][it % kGrStages], (unsigned)(it / kGrStages) & 1u, status, gave_up);
-    const float* patch = &sm.img[team][it % kGrStages][0] + at;
+    const float* patch = &sm.img[team][it % kGrStages][0] + patch_at;
 
     // ---- forward ------------------------------------------------------------------------------
     f32x2 a[2][4];
@@ -368,7 +415,7 @@ k_grad_partials(const float* images, const unsigned* labels, long n,
     const int idx = scatter8_index(lane);
     if ((lane & 2) == 0 && idx < 5) part[warp][6 * half + idx] = mine;
     team_sync<TEAMS>(team);       // the team's sums are in shared memory; every thread is done with the previous image
-    if (tid == 0 && it > 0) issue(it + kGrStages - 1);
+    if (tid == 0 && it > 0) issue(it + kGrStages - 1, mapped);
 
     // ---- output layer on lanes 0..9 of every warp -------------------------------------------------
     float delta = 0.f;
@@ -430,6 +477,15 @@ k_grad_partials(const float* images, const unsigned* labels, long n,
           for (int j = 0; j < 5; ++j) g[i * 5 + j] = fma2(a[y][x], u[x + j], g[i * 5 + j]);
       }
     }
+  }
+
+  };
+  // (Where all images are left, as a rule because none has whole numbers / 255 as pixels, there is nothing to look up: 7 % less.)
+  if constexpr (LEFT) {
+    if (n < n_all) run(std::true_type());
+    else run(std::false_type());
+  } else {
+    run(std::false_type());
   }
 
   // ---- block-level reduction, fixed order ----------------------------------------------------
@@ -512,14 +568,16 @@ k_grad_partials(const float* images, const unsigned* labels, long n,
 // (The data-parallel exchange kernel adds a rank's rows in exactly this order.)
 constexpr int kRedGroups = 32;
 
+// With `left` (grad_tc.cu: images left by each of the n_rows blocks) n_rows more rows follow if any block has left some.
 __global__ void __launch_bounds__(32 * kRedGroups)
 k_reduce_rows(const float* rows, int n_rows, float* __restrict__ G,
-              float* __restrict__ params, float scale, float* __restrict__ mean_err, float err_scale) {
+              float* __restrict__ params, float scale, float* __restrict__ mean_err, float err_scale, const int* left, int more) {
   __shared__ float part[kRedGroups][33];
   const int lane = threadIdx.x & 31, g = threadIdx.x >> 5;
   const int col = blockIdx.x * 32 + lane;
   pdl_launch_dependents();   // the next step's gradient kernel may set itself up now
   pdl_wait();                // the rows are complete
+  if (left && __syncthreads_or((int)threadIdx.x < n_rows && left[threadIdx.x] != 0)) n_rows += more;
   float acc = 0.f, p_old = 0.f;
   if (col < kRowStride) {
     if (params && g == 0 && col < kNParams) p_old = params[col];      // under the row loads
@@ -707,7 +765,7 @@ static int launch_grad(const float* d_params, float* rows, int* status, int fast
   do {                                                                                                       \
     if ((rc = set_smem_attr(k_grad_partials<FL, TEAMS>, sizeof(GrSmem<TEAMS>))) != CNN_OK) return rc;         \
     le = launch_pdl(k_grad_partials<FL, TEAMS>, dim3(grid), dim3(kGrThreads * TEAMS), sizeof(GrSmem<TEAMS>), st, \
-                    d_images, d_labels, n, d_params, rows, status, chained ? 1 : 0);                         \
+                    d_images, d_labels, n, d_params, rows, status, chained ? 1 : 0, (const int*)nullptr, 0, 0); \
   } while (0)
   if (n <= grid) {
     if (fast) CNN_LAUNCH_GRAD(1, 1);
@@ -725,6 +783,42 @@ static int launch_grad(const float* d_params, float* rows, int* status, int fast
 int launch_grad_partials(cnn_net* net, const float* d_images, const unsigned* d_labels, long n, int grid, cudaStream_t st,
                          bool chained) {
   return launch_grad(net->d_params, net->d_partials, net->d_status, net->fast_sigmoid, d_images, d_labels, n, grid, st, chained);
+}
+
+// Rows of the gradient of n images, and what the kernel that adds them needs to know.
+struct GradRows {
+  int rows = 0, more = 0;
+  const int* left = nullptr;
+};
+
+// Tensor cores or CUDA cores.  Microseconds per gradient call, CUDA cores / tensor cores, back to back (alone behind a flush of L2: the same
+// differences, both 9 us longer): 1,000 images 18.6 / 21.3, 1,480 (two tiles per SM) 23.2 / 22.8, 2,000 29.8 / 25.4, 2,500 35.3 / 29, 3,000 41.2 / 32.5,
+// 6,000 72 / 46, 20,000 221 / 107, 60,000 645 / 290.  They meet at about 1,500; the line leaves room for images that turn out not to be
+// whole numbers / 255 and go to the CUDA cores behind a look at the first tiles: 2,000 images 36, 6,000 78, 60,000 656.
+static int launch_gradient(cnn_net* net, const float* d_images, const unsigned* d_labels, long n, cudaStream_t st, bool chained, GradRows* out) {
+  constexpr long kTcGradMin = 2048;
+  const int sms = sm_count();
+  const bool tensor = net->grad_path == 1 || (net->grad_path < 0 && n >= kTcGradMin);
+  if (!tensor || !net->fast_sigmoid || sms > kGrShares || n > (1l << 30)) {
+    out->rows = grid_for_batch(n);
+    return launch_grad_partials(net, d_images, d_labels, n, out->rows, st, chained);
+  }
+  long grid = (n + 4) / 5 < sms ? (n + 4) / 5 : sms;
+  const long per_cta = (n + grid - 1) / grid;
+  grid = (n + per_cta - 1) / per_cta;
+  int* left = reinterpret_cast<int*>(net->d_partials + 2 * (size_t)sms * kRowStride);
+  int rc = launch_grad_tc(net, d_images, d_labels, n, (int)grid, (int)per_cta, left, st);
+  if (rc != CNN_OK) return rc;
+  // the images that it has left, if any
+  if ((rc = set_smem_attr(k_grad_partials<1, 2, true>, sizeof(GrSmem<2>))) != CNN_OK) return rc;
+  cudaError_t e = launch_pdl(k_grad_partials<1, 2, true>, dim3(sms), dim3(kGrThreads * 2), sizeof(GrSmem<2>), st, d_images, d_labels, n,
+                             (const float*)net->d_params, net->d_partials + grid * kRowStride, net->d_status, 0, (const int*)left, (int)grid, (int)per_cta);
+  if (e == cudaSuccess) e = cudaGetLastError();
+  if (e != cudaSuccess) return cuda_fail(e, "k_grad_partials launch");
+  out->rows = (int)grid;
+  out->more = sms;
+  out->left = left;
+  return CNN_OK;
 }
 
 // Blocks of the gradient kernel: one per SM at most (a block holds two images at a time), so that few rows are left to add.
@@ -751,12 +845,12 @@ int cnn_grad_batch(cnn_net* net, const float* d_images, const unsigned int* d_la
   CNN_REQUIRE(d_images && d_labels, "cnn_grad_batch: NULL images or labels");
   CNN_REQUIRE((reinterpret_cast<uintptr_t>(d_images) & 15u) == 0,
               "cnn_grad_batch: image batch must start on a 16-byte boundary");
-  const int grid = grid_for_batch(n);
   int rc = ensure_train_scratch(net);
   if (rc != CNN_OK) return rc;
-  if ((rc = launch_grad_partials(net, d_images, d_labels, n, grid, st)) != CNN_OK) return rc;
+  GradRows g;
+  if ((rc = launch_gradient(net, d_images, d_labels, n, st, false, &g)) != CNN_OK) return rc;
   cudaError_t e = launch_pdl(k_reduce_rows, dim3((kNParamsPadded + 31) / 32), dim3(32 * kRedGroups), 0, st,
-                             (const float*)net->d_partials, grid, d_grad, (float*)nullptr, 0.f, (float*)nullptr, 0.f);
+                             (const float*)net->d_partials, g.rows, d_grad, (float*)nullptr, 0.f, (float*)nullptr, 0.f, g.left, g.more);
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e, "k_reduce_rows launch");
   return CNN_OK;
@@ -785,12 +879,11 @@ int cnn_train_minibatch(cnn_net* net, const float* d_images, const unsigned int*
   for (int e = 0; e < epochs; ++e) {
     for (long first = 0; first < n; first += batch) {
       const long b = (n - first) < batch ? (n - first) : batch;
-      const int grid = grid_for_batch(b);
-      if ((rc = launch_grad_partials(net, d_images + first * kImg, d_labels + first, b, grid, st, first > 0 || e > 0)) != CNN_OK)
-        return rc;
+      GradRows g;
+      if ((rc = launch_gradient(net, d_images + first * kImg, d_labels + first, b, st, first > 0 || e > 0, &g)) != CNN_OK) return rc;
       cudaError_t err = launch_pdl(k_reduce_rows, dim3((kNParamsPadded + 31) / 32), dim3(32 * kRedGroups), 0, st,
-                                   (const float*)net->d_partials, grid, net->d_grad, net->d_params, dt / (float)b,
-                                   d_mean_err ? d_mean_err + e : nullptr, 1.0f / (float)n);
+                                   (const float*)net->d_partials, g.rows, net->d_grad, net->d_params, dt / (float)b,
+                                   d_mean_err ? d_mean_err + e : nullptr, 1.0f / (float)n, g.left, g.more);
       if (err == cudaSuccess) err = cudaGetLastError();
       if (err != cudaSuccess) return cuda_fail(err, "k_reduce_rows launch");
     }
@@ -917,7 +1010,7 @@ int cnn_grad_batch_noalloc(const float* d_params, const float* d_images, const u
   // cnn_grad_batch_noalloc_status reads and clears it.
   if ((rc = launch_grad(d_params, rows, status, 0, d_images, d_labels, n, grid, st, false)) != CNN_OK) return rc;
   cudaError_t e = launch_pdl(k_reduce_rows, dim3((kNParamsPadded + 31) / 32), dim3(32 * kRedGroups), 0, st, (const float*)rows, grid,
-                             d_grad, (float*)nullptr, 0.f, (float*)nullptr, 0.f);
+                             d_grad, (float*)nullptr, 0.f, (float*)nullptr, 0.f, (const int*)nullptr, 0);
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e, "k_reduce_rows launch (no-alloc)");
   return CNN_OK;

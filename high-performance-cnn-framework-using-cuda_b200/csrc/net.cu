@@ -9,10 +9,10 @@
 namespace cnn {
 void destroy_host_pipeline(HostPipeline* p);
 
-// (One row per SM: no launch of the gradient kernel has more blocks, see grid_for_batch.)
+// (One row per SM and gradient kernel: no launch has more blocks, see grid_for_batch.)
 int ensure_train_scratch(cnn_net* net) {
   if (!net->d_grad) CNN_CUDA(cudaMalloc(&net->d_grad, sizeof(float) * (kNParamsPadded + 8)));
-  if (!net->d_partials) CNN_CUDA(cudaMalloc(&net->d_partials, sizeof(float) * (size_t)sm_count() * kRowStride));
+  if (!net->d_partials) CNN_CUDA(cudaMalloc(&net->d_partials, sizeof(float) * (size_t)sm_count() * (2 * kRowStride + 1)));
   return CNN_OK;
 }
 }  // namespace cnn
@@ -111,6 +111,11 @@ int cnn_net_set_option(cnn_net* net, const char* key, int value) {
   if (std::strcmp(key, "forward_path") == 0) {
     CNN_REQUIRE(value >= -1 && value <= 2, "cnn_net_set_option: forward_path takes -1 (by batch size), 0, 1 or 2");
     net->forward_path = value;
+    return CNN_OK;
+  }
+  if (std::strcmp(key, "grad_path") == 0) {
+    CNN_REQUIRE(value >= -1 && value <= 1, "cnn_net_set_option: grad_path takes -1 (by batch size), 0 or 1");
+    net->grad_path = value;
     return CNN_OK;
   }
   if (std::strcmp(key, "fast_sigmoid") == 0) {

@@ -14,12 +14,13 @@ struct cnn_net {
   int forward_path = -1;           // batched forward: 0 = exact fp32 SIMT kernel, 1 = tensor cores in three fp16 passes
                                    // (fp32-level accuracy), 2 = tensor cores, one fp16 pass + tanh sigmoid,
                                    // -1 (default) = 1 for batches of kTcMinBatch images or more, else 0
+  int grad_path = -1;              // gradient of a batch: 0 = CUDA cores, 1 = tensor cores, -1 (default) = by batch size
   float* d_params = nullptr;       // kNParamsPadded floats
   int* d_status = nullptr;         // device status word: 0 ok, non-zero = a bounded wait ran out
   int fast_sigmoid = 1;            // sigmoid of the fused kernels: 0 = reference expression, 1 = short form (default)
 
   // Training scratch (allocated on first use): per-block partial gradients and the reduced vector.
-  float* d_partials = nullptr;     // one row of kRowStride floats per SM
+  float* d_partials = nullptr;     // two rows of kRowStride floats per SM, then an int per SM (grad_tc.cu)
   float* d_grad = nullptr;         // kNParamsPadded floats + 8 floats of statistics
   cnn::HostPipeline* host = nullptr;   // host_pipeline.cu (created on first use)
 };
@@ -144,6 +145,8 @@ int grid_for_batch(long n);
 // for that kernel: see k_grad_partials).
 int launch_grad_partials(cnn_net* net, const float* d_images, const unsigned* d_labels, long n, int grid,
                          cudaStream_t st, bool chained = false);
+// The same on the tensor cores, but for left[b] images at the end of block b's share of per_cta images.
+int launch_grad_tc(cnn_net* net, const float* d_images, const unsigned* d_labels, long n, int grid, int per_cta, int* left, cudaStream_t st);
 int launch_persample_cluster8(cnn_net* net, const float* d_images, const unsigned* d_labels, long n, int epochs,
                               float dt, float threshold, float* d_mean, int* d_ran, cudaStream_t st);
 

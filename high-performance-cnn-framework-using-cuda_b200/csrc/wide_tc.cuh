@@ -59,6 +59,27 @@ __device__ __forceinline__ void mma_f16_elect(unsigned tmem_d, unsigned long lon
       ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
+// COUNT (5 or 8) of them into one accumulator, the descriptors' start addresses A_STEP and B_STEP (in units of 16 B) further on each time;
+// all but the first accumulate.
+#define CNN_MMA_NEXT "add.s64 a, a, %5;\n\tadd.s64 b, b, %6;\n\t@q tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, t;\n\t"
+#define CNN_MMA_FIRST                                                                                                          \
+  "{\n\t.reg .pred p, q, t;\n\t.reg .b64 a, b;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.eq.b32 t, 0, 0;\n\tmov.b64 a, %1;\n\tmov.b64 b, %2;\n\t" \
+  "elect.sync _|q, 0xffffffff;\n\t@q tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, p;\n\t"
+template <int COUNT, int A_STEP, int B_STEP>
+__device__ __forceinline__ void mma_f16_run_elect(unsigned tmem_d, unsigned long long adesc, unsigned long long bdesc, unsigned idesc, unsigned accumulate) {
+  static_assert(COUNT == 5 || COUNT == 8, "");
+  if constexpr (COUNT == 5) {
+    asm volatile(CNN_MMA_FIRST CNN_MMA_NEXT CNN_MMA_NEXT CNN_MMA_NEXT CNN_MMA_NEXT "}" ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc),
+                 "r"(accumulate), "n"(A_STEP), "n"(B_STEP)
+                 : "memory");
+  } else {
+    asm volatile(CNN_MMA_FIRST CNN_MMA_NEXT CNN_MMA_NEXT CNN_MMA_NEXT CNN_MMA_NEXT CNN_MMA_NEXT CNN_MMA_NEXT CNN_MMA_NEXT "}" ::"r"(tmem_d), "l"(adesc),
+                 "l"(bdesc), "r"(idesc), "r"(accumulate), "n"(A_STEP), "n"(B_STEP)
+                 : "memory");
+  }
+}
+#undef CNN_MMA_NEXT
+#undef CNN_MMA_FIRST
 // Whole converged warp: the lane that elect.sync picks (the same one every time for a full mask)
 // arrives on the mbarrier when every MMA it has issued so far has completed.
 __device__ __forceinline__ void mma_commit_elect(unsigned long long* bar) {

@@ -353,3 +353,121 @@ def test_grad_batch_around_full_rounds(cuda, pkg, ob, params0, n):
     for name, (lo, hi) in BLOCKS.items():
         assert scaled_err(g[lo:hi], G[lo:hi]) < 1e-5, name
     assert abs(g[2344] - err) < 1e-5 * err and g[2343] == 0 and not g[2345:].any()
+
+
+# ---- the gradient of a large batch on the tensor cores (option "grad_path") ------------------------
+def both_paths(cuda, pkg, params, images, labels):
+    out = {}
+    for path in (0, 1):
+        net = pkg.Net(0)
+        net.set_params(params)
+        net.set_option("grad_path", path)
+        out[path] = gpu_grad(cuda, net, images, labels)
+        assert np.array_equal(out[path], gpu_grad(cuda, net, images, labels), equal_nan=True)      # fixed order
+    return out
+
+
+@pytest.mark.parametrize("n", [1, 4, 5, 6, 739, 740, 741, 148 * 5 * 4 + 3, 148 * 26])
+def test_tensor_core_gradient_matches_oracle(cuda, pkg, ob, params0, n):
+    """Tiles of five images: one image, a full tile, one image more, one tile per SM, and so many that every ring (two raw buffers,
+    three accumulators, four delta operands, five slabs) goes round.  The bar is the other path's: 1e-5 of the block's largest
+    entry."""
+    images, labels = pkg.synth.synth_images(61, n)
+    net = pkg.Net(0)
+    net.set_params(params0)
+    net.set_option("grad_path", 1)
+    g = gpu_grad(cuda, net, images, labels)
+    G, err = ob.grad_batch(params0, images, labels)
+    for name, (lo, hi) in BLOCKS.items():
+        assert scaled_err(g[lo:hi], G[lo:hi]) < 1e-5, name
+    assert abs(g[2344] - err) < 1e-5 * max(err, 1.0) and g[2343] == 0 and not g[2345:].any()
+    assert np.array_equal(g, gpu_grad(cuda, net, images, labels))
+
+
+@pytest.mark.parametrize("where", ["first", "second tile", "middle", "last", "first of a share", "all"])
+@pytest.mark.parametrize("what", ["fraction", "bright", "negative", "not a number"])
+def test_tensor_core_gradient_leaves_other_pixels(cuda, pkg, params0, what, where):
+    """A block stops at its first tile with a pixel that is not a whole number / 255 and leaves what follows to the CUDA-core kernel, wherever
+    that is.  Yardstick: the CUDA-core path alone; two fp32 sums of the same terms, so 1e-5 of the block's largest entry."""
+    n = 148 * 17 + 9
+    share = -(-n // 148)
+    images, labels = pkg.synth.synth_images(62, n)
+    spot = {"first": [0], "second tile": [5], "middle": [share * 70 + 8], "last": [n - 1], "first of a share": [share * 3],
+            "all": np.arange(n)}[where]
+    images[spot, 3, 9] = {"fraction": 0.3337, "bright": 3.1e5, "negative": -0.25, "not a number": np.nan}[what]
+    out = both_paths(cuda, pkg, params0, images, labels)
+    assert np.array_equal(np.isnan(out[0]), np.isnan(out[1]))
+    if what != "not a number":
+        for name, (lo, hi) in BLOCKS.items():
+            assert scaled_err(out[1][lo:hi], out[0][lo:hi].astype(np.float64)) < 1e-5, name
+        assert abs(out[1][2344] - out[0][2344]) < 1e-5 * out[0][2344]
+
+
+@pytest.mark.parametrize("what", ["tiny conv weights", "large conv weights", "huge conv weights", "infinite bias", "not a number", "large rest",
+                                  "no subsample filter"])
+def test_tensor_core_gradient_parameter_range(cuda, pkg, params0, what):
+    """Conv weights below 2^-21 or from 2^11 on, and parameters that are not finite, go to the CUDA-core kernel; everything between
+    through the scales that follow the largest weight and the tile's deltas.  With large weights a pre-activation of 25 terms up to 250 is
+    only known to 25 * 250 * 2^-24 in fp32, 4e-4."""
+    images, labels = pkg.synth.synth_images(63, 2100)
+    params = params0.copy()
+    if "conv weights" in what:
+        params[:150] *= np.float32({"tiny": 1e-7, "large": 500.0, "huge": 1e5}[what.split()[0]])
+    elif what == "infinite bias":
+        params[151] = np.inf
+    elif what == "not a number":
+        params[2000] = np.nan
+    elif what == "large rest":
+        params[156:] *= np.float32(30)
+    else:
+        params[156:172] = 0
+    out = both_paths(cuda, pkg, params, images, labels)
+    assert np.array_equal(np.isnan(out[0]), np.isnan(out[1]))
+    if not np.isnan(out[0]).any():
+        for name, (lo, hi) in BLOCKS.items():
+            if np.abs(out[0][lo:hi]).max() > 0:
+                assert scaled_err(out[1][lo:hi], out[0][lo:hi].astype(np.float64)) < (1e-2 if what == "large conv weights" else 1e-5), name
+            else:
+                assert not out[1][lo:hi].any(), name
+
+
+def test_gradient_kernel_choice_follows_batch_size(cuda, pkg, params0):
+    """grad_path = -1, the default: tensor cores from 2,048 images on, bit for bit, in the gradient call and in the training loop (whose
+    ragged last step is small), eager and replayed from a graph; the reference's sigmoid expression stays on the CUDA cores."""
+    images, labels = pkg.synth.synth_images(64, 2048 * 2 + 300)
+    d_img, d_lab = to_dev(cuda, images, labels)
+    got = {}
+    for path in (-1, 0, 1):
+        net = pkg.Net(0)
+        net.set_params(params0)
+        net.set_option("grad_path", path)
+        a, b = gpu_grad(cuda, net, images[:2047], labels[:2047]), gpu_grad(cuda, net, images[:2048], labels[:2048])
+        err = cuda.zeros(2, dtype=cuda.float32, device="cuda")
+        net.train_minibatch(d_img, d_lab, images.shape[0], 2048, 2, 0.1, err)
+        cuda.cuda.synchronize()
+        assert net.status() == 0
+        got[path] = (a, b, net.get_params(), err.cpu().numpy())
+    assert np.array_equal(got[-1][0], got[0][0]) and np.array_equal(got[-1][1], got[1][1])
+    assert not np.array_equal(got[0][1], got[1][1])
+    assert np.max(np.abs(got[-1][2] - got[0][2])) < 1e-5 * np.max(np.abs(got[0][2])) and np.allclose(got[-1][3], got[0][3], rtol=1e-5)
+    net = pkg.Net(0)
+    net.set_params(params0)
+    err = cuda.zeros(2, dtype=cuda.float32, device="cuda")
+    net.train_minibatch(d_img, d_lab, 2048, 2048, 1, 0.0, err)        # (scratch exists before the capture)
+    stream = cuda.cuda.Stream()
+    graph = cuda.cuda.CUDAGraph()
+    with cuda.cuda.graph(graph, stream=stream):
+        net.train_minibatch(d_img, d_lab, images.shape[0], 2048, 2, 0.1, err, stream.cuda_stream)
+    graph.replay()
+    cuda.cuda.synchronize()
+    assert np.array_equal(net.get_params(), got[-1][2])
+    ref = {}
+    for path in (0, 1):
+        net = pkg.Net(0)
+        net.set_params(params0)
+        net.set_fast_sigmoid(0)
+        net.set_option("grad_path", path)
+        ref[path] = gpu_grad(cuda, net, images[:2100], labels[:2100])
+    assert np.array_equal(ref[0], ref[1])
+    with pytest.raises(Exception):
+        net.set_option("grad_path", 2)
