@@ -568,7 +568,9 @@ k_grad_partials(const float* images, const unsigned* labels, long n,
 // (The data-parallel exchange kernel adds a rank's rows in exactly this order.)
 constexpr int kRedGroups = 32;
 
-// With `left` (grad_tc.cu: images left by each of the n_rows blocks) n_rows more rows follow if any block has left some.
+// LEFT: `left` says how many images each of the n_rows blocks has left (grad_tc.cu); if any has, `more` rows follow.  (A variant of its own: looking
+// at a null pointer costs a training step 0.1 us.)
+template <bool LEFT>
 __global__ void __launch_bounds__(32 * kRedGroups)
 k_reduce_rows(const float* rows, int n_rows, float* __restrict__ G,
               float* __restrict__ params, float scale, float* __restrict__ mean_err, float err_scale, const int* left, int more) {
@@ -577,7 +579,7 @@ k_reduce_rows(const float* rows, int n_rows, float* __restrict__ G,
   const int col = blockIdx.x * 32 + lane;
   pdl_launch_dependents();   // the next step's gradient kernel may set itself up now
   pdl_wait();                // the rows are complete
-  if (left && __syncthreads_or((int)threadIdx.x < n_rows && left[threadIdx.x] != 0)) n_rows += more;
+  if (LEFT && __syncthreads_or((int)threadIdx.x < n_rows && left[threadIdx.x] != 0)) n_rows += more;
   float acc = 0.f, p_old = 0.f;
   if (col < kRowStride) {
     if (params && g == 0 && col < kNParams) p_old = params[col];      // under the row loads
@@ -849,7 +851,7 @@ int cnn_grad_batch(cnn_net* net, const float* d_images, const unsigned int* d_la
   if (rc != CNN_OK) return rc;
   GradRows g;
   if ((rc = launch_gradient(net, d_images, d_labels, n, st, false, &g)) != CNN_OK) return rc;
-  cudaError_t e = launch_pdl(k_reduce_rows, dim3((kNParamsPadded + 31) / 32), dim3(32 * kRedGroups), 0, st,
+  cudaError_t e = launch_pdl(g.left ? k_reduce_rows<true> : k_reduce_rows<false>, dim3((kNParamsPadded + 31) / 32), dim3(32 * kRedGroups), 0, st,
                              (const float*)net->d_partials, g.rows, d_grad, (float*)nullptr, 0.f, (float*)nullptr, 0.f, g.left, g.more);
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e, "k_reduce_rows launch");
@@ -881,7 +883,7 @@ int cnn_train_minibatch(cnn_net* net, const float* d_images, const unsigned int*
       const long b = (n - first) < batch ? (n - first) : batch;
       GradRows g;
       if ((rc = launch_gradient(net, d_images + first * kImg, d_labels + first, b, st, first > 0 || e > 0, &g)) != CNN_OK) return rc;
-      cudaError_t err = launch_pdl(k_reduce_rows, dim3((kNParamsPadded + 31) / 32), dim3(32 * kRedGroups), 0, st,
+      cudaError_t err = launch_pdl(g.left ? k_reduce_rows<true> : k_reduce_rows<false>, dim3((kNParamsPadded + 31) / 32), dim3(32 * kRedGroups), 0, st,
                                    (const float*)net->d_partials, g.rows, net->d_grad, net->d_params, dt / (float)b,
                                    d_mean_err ? d_mean_err + e : nullptr, 1.0f / (float)n, g.left, g.more);
       if (err == cudaSuccess) err = cudaGetLastError();
@@ -1009,7 +1011,7 @@ int cnn_grad_batch_noalloc(const float* d_params, const float* d_images, const u
   // the library is loaded, is only ever set by a wait that ran out, and stays set until
   // cnn_grad_batch_noalloc_status reads and clears it.
   if ((rc = launch_grad(d_params, rows, status, 0, d_images, d_labels, n, grid, st, false)) != CNN_OK) return rc;
-  cudaError_t e = launch_pdl(k_reduce_rows, dim3((kNParamsPadded + 31) / 32), dim3(32 * kRedGroups), 0, st, (const float*)rows, grid,
+  cudaError_t e = launch_pdl(k_reduce_rows<false>, dim3((kNParamsPadded + 31) / 32), dim3(32 * kRedGroups), 0, st, (const float*)rows, grid,
                              d_grad, (float*)nullptr, 0.f, (float*)nullptr, 0.f, (const int*)nullptr, 0);
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e, "k_reduce_rows launch (no-alloc)");
