@@ -84,8 +84,12 @@ k_train_persample_cluster8(const float* __restrict__ images, const unsigned* __r
   const bool service = (warp == kC8Compute);
   const int slot = lane >> 1, half = lane & 1;
   const bool live = !service && slot < kC8WinPerWarp;
-  const int win = live ? kC8WinPerWarp * warp + slot : 35;
-  const int p = win / 6, q = win % 6;
+  // Four windows (eight lanes) at a time are read together, 16 bytes per lane from rows of seven: (4 p + 6 half + q) mod 8 is the bank group.  Columns
+  // 0, 1, 4, 5 of the warp's first row of windows, of its second, and columns 2, 3 of both ask eight different ones.
+  const int quad = slot >> 2, in_quad = slot & 3;
+  const int p = live ? 2 * warp + (quad < 2 ? quad : in_quad >> 1) : 5;
+  const int q = live ? (quad < 2 ? in_quad + (in_quad & 2) : 2 + (in_quad & 1)) : 5;
+  const int win = 6 * p + q;
   const int y0 = 4 * p + 2 * half, x0 = 4 * q;
   const int svc0 = kC8Compute * 32;          // first thread of the service warp
 
@@ -293,16 +297,14 @@ k_train_persample_cluster8(const float* __restrict__ images, const unsigned* __r
       // ---- output layer on lanes 0..9 of every warp ------------------------------------------------
       float delta = 0.f;
       if (lane < kOut) {
-        float z = 0.f;
+        float zc[kClCtas];
 #pragma unroll
         for (int c = 0; c < kClCtas; ++c) {
-          float zc = 0.f;
-#pragma unroll
-          for (int ww = 0; ww < kC8Compute; ++ww) zc += sm.xfc[stage][c][ww][lane < 5 ? lane : lane + 3];
-          z += zc;
+          const float (&x)[kC8Compute][16] = sm.xfc[stage][c];
+          const int k = lane < 5 ? lane : lane + 3;
+          zc[c] = (x[0][k] + x[1][k]) + x[2][k];
         }
-        z += sm.bf[lane];
-        const float o = sigmoidf<FLAVOR>(z);
+        const float o = sigmoidf<FLAVOR>(((zc[0] + zc[1]) + (zc[2] + zc[3])) + ((zc[4] + zc[5]) + sm.bf[lane]));
         delta = ((label == (unsigned)lane) ? 1.0f : 0.0f) - o;   // makeError
       }
 
@@ -318,52 +320,52 @@ k_train_persample_cluster8(const float* __restrict__ images, const unsigned* __r
         float d[5];
 #pragma unroll
         for (int j = 0; j < 5; ++j) d[j] = __shfl_sync(0xffffffffu, delta, 5 * half + j);
-        float das = wfk[0] * d[0];
-#pragma unroll
-        for (int j = 1; j < 5; ++j) das = fmaf(wfk[j], d[j], das);
+        float das = fmaf(wfk[4], d[4], fmaf(wfk[1], d[1], wfk[0] * d[0]) + fmaf(wfk[3], d[3], wfk[2] * d[2]));
         das += __shfl_xor_sync(0xffffffffu, das, 1);
         const float delta_s = live ? das * as * (1.f - as) : 0.f;
-        if (live) {
-#pragma unroll
-          for (int j = 0; j < 5; ++j) sm.wf[5 * half + j][win] = fmaf(dt, d[j] * as, wfk[j]);  // bp_weight_f + apply_grad
-        }
-        // subsample filter gradient: this thread's two filter rows, reduce-scattered over the warp's
-        // 16 window slots (lane bits 4, 3, 2 pick the element, bit 1 is summed last); bias term
-        float gs[8];
+        // Two reductions over the warp, level by level together, so that the waits of one are filled by the other: the thread's 25
+        // conv-filter gradient terms, its bias term (both the window's delta times what was prepared under the exchange) and the
+        // subsample bias' term, reduce-scattered over the lanes; and the subsample filter's gradient, this thread's two filter rows, over the
+        // 16 window slots (lane bits 4, 3, 2 pick the element, bit 1 is summed last).
+        float gs[8], g[32];
 #pragma unroll
         for (int rr = 0; rr < 2; ++rr)
 #pragma unroll
           for (int c = 0; c < 4; ++c) gs[rr * 4 + c] = delta_s * a[rr][c];
-        float gb = (half == 0) ? delta_s * inv_s : 0.f;
 #pragma unroll
-        for (int keep_n = 4; keep_n >= 1; keep_n >>= 1) {
-          const int mask = keep_n << 2;   // 16, 8, 4
+        for (int t = 0; t < 26; ++t) g[t] = delta_s * h[t];
+        g[26] = (half == 0) ? delta_s * inv_s : 0.f;
+#pragma unroll
+        for (int t = 27; t < 32; ++t) g[t] = 0.f;
+        CNN_PHASE(6);   // deltas, the thread's gradient terms
+#pragma unroll
+        for (int mask = 16; mask >= 1; mask >>= 1) {
           const bool upper = (lane & mask) != 0;
+          const int keep_n = mask >> 2;      // 4, 2, 1
 #pragma unroll
           for (int i = 0; i < keep_n; ++i) {
             const float send = upper ? gs[i] : gs[i + keep_n];
             const float keep = upper ? gs[i + keep_n] : gs[i];
             gs[i] = keep + __shfl_xor_sync(0xffffffffu, send, mask);
           }
-        }
-        gs[0] += __shfl_xor_sync(0xffffffffu, gs[0], 2);
+          if (mask == 2) gs[0] += __shfl_xor_sync(0xffffffffu, gs[0], 2);
 #pragma unroll
-        for (int m = 2; m <= 16; m <<= 1) gb += __shfl_xor_sync(0xffffffffu, gb, m);
+          for (int i = 0; i < mask; ++i) {
+            const float send = upper ? g[i] : g[i + mask];
+            const float keep = upper ? g[i + mask] : g[i];
+            g[i] = keep + __shfl_xor_sync(0xffffffffu, send, mask);
+          }
+          if (mask == 4 && live) {
+#pragma unroll
+            for (int j = 0; j < 5; ++j) sm.wf[5 * half + j][win] = fmaf(dt, d[j] * as, wfk[j]);  // bp_weight_f + apply_grad
+          }
+        }
+        if (lane < 26) sm.c_part[warp][lane] = g[0];
+        if (lane == 26) sm.s_part[warp][16] = g[0];
         if ((lane & 2) == 0) {
           const int idx = ((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1);   // rr * 4 + c
           sm.s_part[warp][(2 * half + (idx >> 2)) * 4 + (idx & 3)] = gs[0];
         }
-        if (lane == 0) sm.s_part[warp][16] = gb;
-        // the thread's 25 filter-gradient terms and its bias term: the window's delta times what was
-        // prepared under the exchange
-        float g[32];
-#pragma unroll
-        for (int t = 0; t < 26; ++t) g[t] = delta_s * h[t];
-        CNN_PHASE(6);   // deltas, subsample gradient, the thread's gradient terms
-#pragma unroll
-        for (int t = 26; t < 32; ++t) g[t] = 0.f;
-        const float mine = warp_reduce_scatter32(g, lane);
-        if (lane < 26) sm.c_part[warp][lane] = mine;
       }
       // (the service warp is the last to leave the stretch between B2 and E: what it can read or
       // compute before B2 it does here, while it waits for the compute warps anyway)
