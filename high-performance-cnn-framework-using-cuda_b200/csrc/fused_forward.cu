@@ -91,8 +91,10 @@ k_forward_one(const void* images, long n, const float* params,
   // thread -> (window, pair, half): half fastest, so that a window's halves are neighbouring lanes
   const bool live = tid < kFwLive;
   const int half = tid & 1, unit = (live ? tid : 0) >> 1;
-  const int pr = unit / 36, w = unit % 36;
-  const int p = w / 6, q = w % 6;
+  // (the order of the windows keeps eight neighbouring threads' 16-byte reads out of one another's banks: see k_grad_partials)
+  const int pr = unit / 36, twelve = unit % 36 / 12, quad = unit % 12 / 4, in_quad = unit % 4;
+  const int p = 2 * twelve + (quad < 2 ? quad : in_quad >> 1), q = quad < 2 ? in_quad + (in_quad & 2) : 2 + (in_quad & 1);
+  const int w = 6 * p + q;
   f32x2 wt[25];
 #pragma unroll
   for (int t = 0; t < 25; ++t) wt[t] = *reinterpret_cast<const f32x2*>(&sm.wc[t][2 * pr]);
@@ -280,8 +282,15 @@ k_forward_tiles(const void* images, long n, const float* params,
   }
   __syncthreads();
 
-  const int img = tid / 36, w = tid % 36;
-  const int p = w / 6, q = w % 6;
+  // Eight neighbouring threads read 16 bytes each at a time, of rows of seven: (4 p + q) mod 8 (plus 4 in every other image) is the bank group.  Twelve
+  // threads own two rows of windows; columns 0-3 of both ask eight different ones, columns 4, 5 of both together with columns 2, 3 of the next
+  // two rows, too, and what remains of those takes two turns: 4 turns for 24 windows, the least there is (in the windows' own order 6).
+  const int twelve = tid / 12, t12 = tid % 12, img = twelve / 3;
+  const bool odd12 = (twelve & 1) != 0;
+  const int sub = t12 & 3, third = t12 >> 2;
+  const int second_row = odd12 ? (third == 0 ? sub >> 1 : third - 1) : (third < 2 ? third : sub >> 1);
+  const int q = odd12 ? (third == 0 ? 2 + (sub & 1) : sub + (sub & 2)) : (third < 2 ? sub : 4 + (sub & 1));
+  const int p = 2 * (twelve % 3) + second_row, w = 6 * p + q;
   bool gave_up = false;
   int it = 0;
   for (long tile = blockIdx.x; tile < n_tiles; tile += gridDim.x, ++it) {

@@ -247,6 +247,15 @@ k_grad_partials(const float* images, const unsigned* labels, long n,
     return end - sm.before[share + 1] + im;
   };
   [[maybe_unused]] int share_copied = 0, share_read = 0;
+  const bool live = tid < kS;
+  const int half = tid & 1, unit = (live ? tid : 0) >> 1;      // (the eight idle threads shadow thread 0 and add zeros)
+  // Eight neighbouring threads, four windows, read 16 bytes each of rows of seven at a time: (4 p + 6 half + q) mod 8 is the bank group.  Of
+  // twelve windows (two rows) four with columns 0, 1, 4, 5 of the first row, four of the second, and columns 2, 3 of both ask eight different ones
+  // (in the windows' own order every load took two turns: a third of this kernel's shared-memory cycles).
+  const int pr = unit / 36, twelve = unit % 36 / 12, quad = unit % 12 / 4, in_quad = unit % 4;
+  const int p = 2 * twelve + (quad < 2 ? quad : in_quad >> 1), q = quad < 2 ? in_quad + (in_quad & 2) : 2 + (in_quad & 1);
+  const int w = 6 * p + q;
+  const int patch_at = (4 * p + 2 * half) * kH + 4 * q;
   // Image i of this team is first + i * step.
   const long first = (long)blockIdx.x + (long)team * gridDim.x, step = (long)TEAMS * gridDim.x;
   auto issue = [&](int i, auto mapped) {
@@ -300,7 +309,6 @@ k_grad_partials(const float* images, const unsigned* labels, long n,
     for (int i = 0; i < kGrStages; ++i) issue(i, std::integral_constant<bool, LEFT>());
   // Parameters: every load of a thread is under way before the first of them is stored (one L2 latency, not one per
   // group of loads: 2.4 -> 0.75 us of a step).
-  const bool live = tid < kS;
   {
     float wf[kOut / TEAMS], small;
     const int k0 = team * (kOut / TEAMS);
@@ -321,10 +329,6 @@ k_grad_partials(const float* images, const unsigned* labels, long n,
   }
   __syncthreads();
 
-  const int half = tid & 1, unit = (live ? tid : 0) >> 1;      // (the eight idle threads shadow thread 0 and add zeros)
-  const int pr = unit / 36, w = unit % 36;
-  const int p = w / 6, q = w % 6;
-  const int patch_at = (4 * p + 2 * half) * kH + 4 * q;
   // With one team there are registers enough to keep the taps.
   f32x2 wt[TEAMS == 1 ? 25 : 1];
   if (TEAMS == 1) {
