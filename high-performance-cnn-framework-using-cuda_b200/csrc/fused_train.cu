@@ -228,7 +228,9 @@ __device__ __forceinline__ void team_sync(int team) {
 
 // LEFT: the images that the tensor-core kernel (grad_tc.cu) has left, the last left[b] of each share b of per_cta images; no rows are
 // written if there are none.
-template <int FAST, int TEAMS, bool LEFT = false>
+// ONCE: no team has more than one image.  Then the gradient's registers are free during the forward pass and hold the taps (which two teams
+// otherwise read from shared memory as they go: a quarter of a small batch's shared-memory cycles).
+template <int FAST, int TEAMS, bool ONCE, bool LEFT = false>
 __global__ void __launch_bounds__(kGrThreads * TEAMS, 1)
 k_grad_partials(const float* images, const unsigned* labels, long n,
                 const float* params, float* __restrict__ rows, int* __restrict__ status, int chained,
@@ -329,11 +331,12 @@ k_grad_partials(const float* images, const unsigned* labels, long n,
   }
   __syncthreads();
 
-  // With one team there are registers enough to keep the taps.
-  f32x2 wt[TEAMS == 1 ? 25 : 1];
-  if (TEAMS == 1) {
+  // With one team, or one image, there are registers enough to keep the taps.
+  constexpr bool kTaps = TEAMS == 1 || ONCE;
+  f32x2 wt[kTaps ? 25 : 1];
+  if (kTaps) {
 #pragma unroll
-    for (int t = 0; t < 25; ++t) wt[TEAMS == 1 ? t : 0] = *reinterpret_cast<const f32x2*>(&sm.wc[t][2 * pr]);
+    for (int t = 0; t < 25; ++t) wt[kTaps ? t : 0] = *reinterpret_cast<const f32x2*>(&sm.wc[t][2 * pr]);
   }
 
   f32x2 g[26], gf[5];
@@ -377,7 +380,7 @@ k_grad_partials(const float* images, const unsigned* labels, long n,
         if (i < 0 || i > 4) continue;
 #pragma unroll
         for (int j = 0; j < 5; ++j) {
-          const f32x2 tap = TEAMS == 1 ? wt[TEAMS == 1 ? i * 5 + j : 0] : *reinterpret_cast<const f32x2*>(&sm.wc[i * 5 + j][2 * pr]);
+          const f32x2 tap = kTaps ? wt[kTaps ? i * 5 + j : 0] : *reinterpret_cast<const f32x2*>(&sm.wc[i * 5 + j][2 * pr]);
 #pragma unroll
           for (int x = 0; x < 4; ++x) a[y][x] = fma2(tap, v[x + j], a[y][x]);
         }
@@ -419,7 +422,7 @@ k_grad_partials(const float* images, const unsigned* labels, long n,
     const int idx = scatter8_index(lane);
     if ((lane & 2) == 0 && idx < 5) part[warp][6 * half + idx] = mine;
     team_sync<TEAMS>(team);       // the team's sums are in shared memory; every thread is done with the previous image
-    if (tid == 0 && it > 0) issue(it + kGrStages - 1, mapped);
+    if (!ONCE && tid == 0 && it > 0) issue(it + kGrStages - 1, mapped);
 
     // ---- output layer on lanes 0..9 of every warp -------------------------------------------------
     float delta = 0.f;
@@ -481,8 +484,8 @@ k_grad_partials(const float* images, const unsigned* labels, long n,
           for (int j = 0; j < 5; ++j) g[i * 5 + j] = fma2(a[y][x], u[x + j], g[i * 5 + j]);
       }
     }
+    if (ONCE) break;
   }
-
   };
   // (Where all images are left, as a rule because none has whole numbers / 255 as pixels, there is nothing to look up: 7 % less.)
   if constexpr (LEFT) {
@@ -767,18 +770,21 @@ static int launch_grad(const float* d_params, float* rows, int* status, int fast
                        long n, int grid, cudaStream_t st, bool chained) {
   int rc;
   cudaError_t le = cudaSuccess;
-#define CNN_LAUNCH_GRAD(FL, TEAMS)                                                                            \
+#define CNN_LAUNCH_GRAD(FL, TEAMS, ONCE)                                                                      \
   do {                                                                                                       \
-    if ((rc = set_smem_attr(k_grad_partials<FL, TEAMS>, sizeof(GrSmem<TEAMS>))) != CNN_OK) return rc;         \
-    le = launch_pdl(k_grad_partials<FL, TEAMS>, dim3(grid), dim3(kGrThreads * TEAMS), sizeof(GrSmem<TEAMS>), st, \
+    if ((rc = set_smem_attr(k_grad_partials<FL, TEAMS, ONCE>, sizeof(GrSmem<TEAMS>))) != CNN_OK) return rc;   \
+    le = launch_pdl(k_grad_partials<FL, TEAMS, ONCE>, dim3(grid), dim3(kGrThreads * TEAMS), sizeof(GrSmem<TEAMS>), st, \
                     d_images, d_labels, n, d_params, rows, status, chained ? 1 : 0, (const int*)nullptr, 0, 0); \
   } while (0)
   if (n <= grid) {
-    if (fast) CNN_LAUNCH_GRAD(1, 1);
-    else CNN_LAUNCH_GRAD(0, 1);
+    if (fast) CNN_LAUNCH_GRAD(1, 1, true);
+    else CNN_LAUNCH_GRAD(0, 1, true);
+  } else if (n <= 2l * grid) {
+    if (fast) CNN_LAUNCH_GRAD(1, 2, true);
+    else CNN_LAUNCH_GRAD(0, 2, true);
   } else {
-    if (fast) CNN_LAUNCH_GRAD(1, 2);
-    else CNN_LAUNCH_GRAD(0, 2);
+    if (fast) CNN_LAUNCH_GRAD(1, 2, false);
+    else CNN_LAUNCH_GRAD(0, 2, false);
   }
 #undef CNN_LAUNCH_GRAD
   if (le == cudaSuccess) le = cudaGetLastError();
@@ -816,8 +822,8 @@ static int launch_gradient(cnn_net* net, const float* d_images, const unsigned* 
   int rc = launch_grad_tc(net, d_images, d_labels, n, (int)grid, (int)per_cta, left, st);
   if (rc != CNN_OK) return rc;
   // the images that it has left, if any
-  if ((rc = set_smem_attr(k_grad_partials<1, 2, true>, sizeof(GrSmem<2>))) != CNN_OK) return rc;
-  cudaError_t e = launch_pdl(k_grad_partials<1, 2, true>, dim3(sms), dim3(kGrThreads * 2), sizeof(GrSmem<2>), st, d_images, d_labels, n,
+  if ((rc = set_smem_attr(k_grad_partials<1, 2, false, true>, sizeof(GrSmem<2>))) != CNN_OK) return rc;
+  cudaError_t e = launch_pdl(k_grad_partials<1, 2, false, true>, dim3(sms), dim3(kGrThreads * 2), sizeof(GrSmem<2>), st, d_images, d_labels, n,
                              (const float*)net->d_params, net->d_partials + grid * kRowStride, net->d_status, 0, (const int*)left, (int)grid, (int)per_cta);
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e, "k_grad_partials launch");
