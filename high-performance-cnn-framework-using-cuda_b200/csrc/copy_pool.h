@@ -165,22 +165,17 @@ class CopyPool {
   static constexpr int kSlots = 4;             // ring: pieces of kPiece bytes at most (a copy to the device costs 4 us before
   static constexpr size_t kPiece = 2 * 1024 * 1024;      // its first byte: pieces of 256 KB run at 30 GB/s)
 
-  // The source is cut into chunks, each chunk into pieces; piece p goes to ring slot p % kSlots.
+  // The source is cut into pieces; piece p is the bytes from at[p] to at[p + 1] and goes to ring slot p % kSlots.
   struct Job {
     const unsigned char* src = nullptr;
     unsigned char* ring = nullptr;
-    size_t total = 0, chunk_bytes = 0, piece_bytes = 0;
-    long pieces_per_chunk = 1, pieces = 0;
+    const size_t* at = nullptr;
+    long pieces = 0;
     std::atomic<long> released{0};             // pieces whose ring slot may be written
     std::atomic<int> done[kSlots];          // per ring slot: helpers that have written their share
     std::atomic<bool> cancelled{false};
 
-    size_t offset(long p) const { return (size_t)(p / pieces_per_chunk) * chunk_bytes + (size_t)(p % pieces_per_chunk) * piece_bytes; }
-    size_t bytes(long p) const {
-      const size_t in_chunk = (size_t)(p % pieces_per_chunk) * piece_bytes, at = offset(p);
-      size_t b = chunk_bytes - in_chunk < piece_bytes ? chunk_bytes - in_chunk : piece_bytes;
-      return total - at < b ? total - at : b;
-    }
+    size_t bytes(long p) const { return at[p + 1] - at[p]; }
     unsigned char* slot(long p) const { return ring + (size_t)(p % kSlots) * kPiece; }
   };
 
@@ -223,7 +218,7 @@ class CopyPool {
   // Share `who` of `parts` of piece p (whole cache lines).
   static void copy_share(const Job& j, long p, int who, int parts) {
     const size_t bytes = j.bytes(p), share = ((bytes + parts - 1) / parts + 63) & ~(size_t)63, lo = share * who;
-    if (lo < bytes) copy_past_caches(j.slot(p) + lo, j.src + j.offset(p) + lo, bytes - lo < share ? bytes - lo : share);
+    if (lo < bytes) copy_past_caches(j.slot(p) + lo, j.src + j.at[p] + lo, bytes - lo < share ? bytes - lo : share);
   }
   // dst is 64-byte aligned.  The copy is written around the caches: the device reads it next, and lines that lie modified
   // in some core's cache come over the bus at a fraction of its rate (10,000 uint8 images: 383 against 625 us with the same pieces).

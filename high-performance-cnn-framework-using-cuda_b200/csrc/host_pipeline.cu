@@ -1,8 +1,9 @@
 // The forward pass through host buffers: copy in, kernel and results out, in chunks that overlap.
 //
-// A request is cut into chunks of images; three slots (a device buffer, a stream and a result buffer each) take them in
-// turn, so that the copies of the next chunks run under a chunk's kernel.  Pinned images are copied from where they lie.
-// Pageable images go through a pinned ring that several cores fill (copy_pool.h): 10,000 uint8 images 620-750 -> 270 us on a B200
+// A request is cut into chunks of images; four slots (a device buffer, a stream and a result buffer each) take them in
+// turn, so that the copies of the next chunks run under a chunk's kernel.  The last chunk is a quarter of the request at most: its kernel and results
+// come behind everything else.  Pinned images are copied from where they lie.
+// Pageable images go through a pinned ring that several cores fill (copy_pool.h): 10,000 uint8 images 620-750 -> 250 us on a B200
 // (the driver's own staging fills its buffer with one core, 12 GB/s; the bus carries 55 GB/s).  Results for pageable
 // buffers go through pinned memory too, one copy per chunk.  (Written there by the kernel itself, over the bus, they cost
 // 80 us per 2,500 images.)
@@ -21,8 +22,8 @@ int forward_device(cnn_net* net, int path, const float* d_images, long n, float*
 int forward_device_u8(cnn_net* net, int path, const unsigned char* d_pixels, long n, float* d_out, int* d_argmax,
                       cudaStream_t stream);
 
-constexpr int kHpSlots = 3;
-constexpr long kHpMaxChunk = 8192, kHpMinChunk = 1024;      // images per chunk
+constexpr int kHpSlots = 4;
+constexpr long kHpMaxChunk = 8192, kHpMinChunk = 512;       // images per chunk
 static_assert(kHpSlots * (sizeof(float) * (kOut + 1) * kHpMaxChunk + 256) + sizeof(int) * kHpSlots <= PinnedBlock::kPage, "results fit a lease");
 constexpr size_t kHpMinStaged = 128 * 1024;                 // below, the driver's own staging is as fast
 
@@ -110,8 +111,16 @@ struct HostRequest {
   int* argmax;
   size_t image_bytes;
   bool pinned_results, staged;
-  long chunk;
+  // Chunks: equal ones, and a last one.
+  long chunk, rest;                              // images of an equal chunk, and of all of them
   int slots, path;
+  std::unique_ptr<size_t[]> at = nullptr;        // where the pieces of a staged request begin, and where the last one ends
+  std::unique_ptr<long[]> chunk_end = nullptr;   // per piece: the number of images up to the chunk that it completes, else 0
+
+  long count_at(long first) const {
+    if (first >= rest) return n - rest;
+    return rest - first < chunk ? rest - first : chunk;
+  }
 
   // Pageable results of the chunk that was in this slot.
   int hand_over(HostPipeline::Slot& s) {
@@ -139,14 +148,15 @@ struct HostRequest {
       if (out) CNN_CUDA(cudaMemcpyAsync(out + first * kOut, o, sizeof(float) * kOut * (size_t)count, cudaMemcpyDeviceToHost, s.stream));
       if (argmax) CNN_CUDA(cudaMemcpyAsync(argmax + first, a, sizeof(int) * (size_t)count, cudaMemcpyDeviceToHost, s.stream));
     }
-    if (first + (long)slots * chunk >= n)       // this slot's last chunk
+    const long equal = (rest + chunk - 1) / chunk;
+    if ((first < rest ? first / chunk : equal) + slots >= equal + 1)      // this slot's last chunk
       CNN_CUDA(cudaMemcpyAsync(&hp.h_status[si], net->d_status, sizeof(int), cudaMemcpyDeviceToHost, s.stream));
     return CNN_OK;
   }
   int run_direct() {
     int si = 0;
-    for (long first = 0; first < n; first += chunk, si = (si + 1) % slots) {
-      const long count = n - first < chunk ? n - first : chunk;
+    for (long first = 0; first < n; first += count_at(first), si = (si + 1) % slots) {
+      const long count = count_at(first);
       int rc = hand_over(hp.slot[si]);
       if (rc != CNN_OK) return rc;
       CNN_CUDA(cudaMemcpyAsync(hp.slot[si].d_img, images + (size_t)first * image_bytes, (size_t)count * image_bytes,
@@ -155,21 +165,50 @@ struct HostRequest {
     }
     return CNN_OK;
   }
+  // Pieces of the staged copy.  The cores fill them about as fast as the bus takes them, so nothing but the first piece's filling and the last
+  // one's way over the bus is not under something else: these are short (and so the ones next to them), the others as long as a slot, because
+  // every copy costs some microseconds.
+  bool cut(long& pieces) {
+    const long most = (long)((size_t)n * image_bytes / (CopyPool::kPiece / 4)) + 2 * (n / chunk + 3);
+    at.reset(new (std::nothrow) size_t[most + 1]);
+    chunk_end.reset(new (std::nothrow) long[most]);
+    if (!at || !chunk_end) return false;
+    pieces = 0;
+    at[0] = 0;
+    for (long first = 0; first < n;) {
+      const long end = first + count_at(first);
+      const bool last = end == n;
+      const size_t end_byte = (size_t)end * image_bytes;
+      while (at[pieces] < end_byte) {
+        const size_t left = end_byte - at[pieces];
+        size_t take = pieces == 0 ? CopyPool::kPiece / 4 : (pieces == 1 || last ? CopyPool::kPiece / 2 : CopyPool::kPiece);
+        if (take >= left || left - take < CopyPool::kPiece / 8) take = left < CopyPool::kPiece ? left : CopyPool::kPiece / 2;
+        chunk_end[pieces] = at[pieces] + take == end_byte ? end : 0;
+        at[pieces + 1] = at[pieces] + take;
+        ++pieces;
+      }
+      first = end;
+    }
+    return true;
+  }
   int run_pieces(CopyPool::Job& job, int helpers) {
+    long first = 0;                              // the piece's chunk: its first image and its slot
+    int si = 0;
+    bool begins = true;
     for (long p = 0; p < job.pieces; ++p) {
-      const long c = p / job.pieces_per_chunk, in_chunk = p % job.pieces_per_chunk;
-      const int si = (int)(c % slots);
       HostPipeline::Slot& s = hp.slot[si];
       CopyPool::copy_share(job, p, 0, helpers + 1);
       while (job.done[p % CopyPool::kSlots].load(std::memory_order_acquire) != helpers) CopyPool::pause();
       job.done[p % CopyPool::kSlots].store(0, std::memory_order_relaxed);
       int rc;
-      if (in_chunk == 0 && (rc = hand_over(s)) != CNN_OK) return rc;
-      CNN_CUDA(cudaMemcpyAsync(s.d_img + (size_t)in_chunk * job.piece_bytes, job.slot(p), job.bytes(p), cudaMemcpyHostToDevice, s.stream));
+      if (begins && (rc = hand_over(s)) != CNN_OK) return rc;
+      CNN_CUDA(cudaMemcpyAsync(s.d_img + (job.at[p] - (size_t)first * image_bytes), job.slot(p), job.bytes(p), cudaMemcpyHostToDevice, s.stream));
       CNN_CUDA(cudaEventRecord(hp.piece[p % CopyPool::kSlots], s.stream));
-      if (in_chunk == job.pieces_per_chunk - 1 || p == job.pieces - 1) {
-        const long first = c * chunk;
-        if ((rc = compute(si, first, n - first < chunk ? n - first : chunk)) != CNN_OK) return rc;
+      begins = chunk_end[p] != 0;
+      if (begins) {
+        if ((rc = compute(si, first, chunk_end[p] - first)) != CNN_OK) return rc;
+        first = chunk_end[p];
+        si = (si + 1) % slots;
       }
       // Give back the slot of the piece half a ring behind: its copy is done or nearly so.
       const long next = job.released.load(std::memory_order_relaxed);
@@ -182,12 +221,9 @@ struct HostRequest {
   }
   int run_staged() {
     CopyPool::Job job;
+    if (!cut(job.pieces)) return run_direct();
     job.src = images;
-    job.total = (size_t)n * image_bytes;
-    job.chunk_bytes = (size_t)chunk * image_bytes;
-    job.pieces_per_chunk = (long)((job.chunk_bytes + CopyPool::kPiece - 1) / CopyPool::kPiece);
-    job.piece_bytes = ((job.chunk_bytes + job.pieces_per_chunk - 1) / job.pieces_per_chunk + 63) & ~(size_t)63;
-    for (job.pieces = n / chunk * job.pieces_per_chunk; job.pieces == 0 || job.offset(job.pieces - 1) + job.bytes(job.pieces - 1) < job.total;) ++job.pieces;
+    job.at = at.get();
     for (int i = 0; i < CopyPool::kSlots; ++i) job.done[i].store(0, std::memory_order_relaxed);
     job.released.store(job.pieces < CopyPool::kSlots ? job.pieces : CopyPool::kSlots, std::memory_order_release);
     const int helpers = hp.pool ? CopyPool::get().begin(&job) : 0;
@@ -199,8 +235,8 @@ struct HostRequest {
     CopyPool::get().end();
     return rc;
   }
-  int run() {
-    int rc = hp.reserve(slots, chunk, image_bytes, pinned_results, staged);
+  int run(long largest) {
+    int rc = hp.reserve(slots, largest, image_bytes, pinned_results, staged);
     if (rc != CNN_OK) return rc;
     // The streams are first put behind everything queued so far on the legacy default stream (a parameter update, a
     // training call), so that a forward issued right after such work sees its result; work on a caller's own non-blocking
@@ -230,24 +266,26 @@ static int forward_host_impl(cnn_net* net, const void* h_images, bool u8, long n
   HostPipeline& hp = *net->host;
   const size_t image_bytes = u8 ? (size_t)kImg : sizeof(float) * kImg;
   const bool pageable = is_pageable(h_images);
-  // Half of the request per chunk: half of the kernel time is under copies, and there are few hand-overs (quarters: 20 us
-  // more for 10,000 uint8 images).
-  long chunk = (n + 1) / 2;
-  chunk = chunk < kHpMinChunk ? kHpMinChunk : (chunk > kHpMaxChunk ? kHpMaxChunk : chunk);
-  if (chunk > n) chunk = n;
-  const int slots = n > 2 * chunk ? 3 : (n > chunk ? 2 : 1);
+  // Behind the last copy there is the last chunk's kernel, the way of its results back and, for pageable result buffers, a copy of them: a
+  // quarter of the request (halves, in pieces of equal length: 262 us for 10,000 uint8 images instead of 250; quarters all over: more hand-overs, 280).
+  long last = n / 4;
+  last = last < kHpMinChunk ? kHpMinChunk : (last > kHpMaxChunk / 4 ? kHpMaxChunk / 4 : last);
+  if (n <= 2 * kHpMinChunk) last = n;
+  const long rest = n - last, parts = (rest + kHpMaxChunk - 1) / kHpMaxChunk;
+  const long chunk = parts > 0 ? (rest + parts - 1) / parts : last;
+  const int slots = parts + 1 < kHpSlots ? (int)parts + 1 : kHpSlots;
   HostRequest req{net, hp, static_cast<const unsigned char*>(h_images), u8, n, h_out, h_argmax, image_bytes,
                   (h_out && is_pageable(h_out)) || (h_argmax && is_pageable(h_argmax)),
-                  pageable && (size_t)n * image_bytes >= kHpMinStaged, chunk, slots,
+                  pageable && (size_t)n * image_bytes >= kHpMinStaged, chunk, rest, slots,
                   forward_kernel_for(net, n, u8)};     // one kernel for the whole request, whatever the chunking
-  const int rc = req.run();
+  const int rc = req.run(chunk > last ? chunk : last);
   if (rc != CNN_OK) {
     // nothing of this request may still read the caller's buffers or write into them when the call returns
     for (auto& s : hp.slot)
       if (s.stream) cudaStreamSynchronize(s.stream);
     return rc;
   }
-  if (hp.h_status[0] | hp.h_status[1] | hp.h_status[2]) {
+  if (hp.h_status[0] | hp.h_status[1] | hp.h_status[2] | hp.h_status[3]) {
     set_error("cnn_forward_batched_host: a bounded device-side wait ran out");
     int zero = 0;
     cudaMemcpy(net->d_status, &zero, sizeof(int), cudaMemcpyHostToDevice);

@@ -561,3 +561,21 @@ def test_forward_host_with_nets_that_come_and_go(cuda, pkg, params0):
         net.forward_u8_host(pix, n, out, None)
         assert np.array_equal(np.asarray(out), want)
         net.close()
+
+
+@pytest.mark.parametrize("n", [1026, 2047, 41000])
+def test_forward_host_last_chunk_is_shorter(cuda, pkg, params0, n):
+    """Equal chunks and a last one of a quarter of the request at most: two chunks of about 500, the least, and six chunks in four slots, whose
+    pageable results are handed over before a slot is used again; always the bits of the device call."""
+    pix = pkg.synth.synth_pixels_u8(48, n)
+    net = pkg.Net(0)
+    net.set_params(params0)
+    d_out = cuda.empty((n, 10), dtype=cuda.float32, device="cuda")
+    d_arg = cuda.empty(n, dtype=cuda.int32, device="cuda")
+    net.forward_u8(cuda.from_numpy(pix).cuda(), n, d_out, d_arg)
+    cuda.cuda.synchronize()
+    for pinned in (False, True):
+        img = cuda.from_numpy(pix).pin_memory() if pinned else pix
+        out, arg = np.full((n, 10), -1, np.float32), np.full(n, -1, np.int32)
+        net.forward_u8_host(img, n, out, arg)
+        assert np.array_equal(out, d_out.cpu().numpy()) and np.array_equal(arg, d_arg.cpu().numpy())
