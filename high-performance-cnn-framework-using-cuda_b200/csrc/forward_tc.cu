@@ -238,6 +238,9 @@ k_forward_tc(const void* images, long n, long imgs_per_cta, const float* params,
     for (int w = 0; w < kTfFinishers; ++w) sm.finished[w] = 0;
   }
   if (tid < kTfRange) sm.out_of_range[tid] = 0;
+  if (kLow)      // no remainders yet (written by the first tiles instead: 1.3 us more per call)
+    for (int i = tid; i < kTfSlabsTotal / 2 * kTfSlabBytes / 16; i += kTfThreads)
+      reinterpret_cast<uint4*>(sm.slab[kTfSlabsTotal / 2])[i] = make_uint4(0, 0, 0, 0);
   if (tid < 8 * kTfSlots) sm.as[tid >> 3][216 + (tid & 7)] = 0.f;     // the padding meets zero weights and has to be finite
   if (warp == kTfMmaWarp) tc::tmem_alloc(&sm.tmem_base, 512);
   pdl_wait();
@@ -479,8 +482,8 @@ k_forward_tc(const void* images, long n, long imgs_per_cta, const float* params,
     const __half2 s1 = __float2half2_rn(__int_as_float((127 + e1) << 23)), s2 = __float2half2_rn(__int_as_float((127 + e2) << 23));
     const __half2 base1 = __float2half2_rn(-1024.f * __int_as_float((127 + e1) << 23));
     const f32x2 px_scale2 = pack2(px_scale, px_scale);
-    unsigned stale = (1u << kTfSlabs) - 1;      // slabs whose low part, this warp's share of it, is not all zeros
-    bool expect_low = true;
+    unsigned stale = 0;      // slabs whose low part, this warp's share of it, is not all zeros
+    bool expect_low = false;
     for (int k = 0; k < n_tiles; ++k) {
       const int s = k % kTfSlabs, r = k % kTfRaw;
       CNN_PHASE(0);

@@ -190,10 +190,11 @@ __device__ __forceinline__ int scatter8_index(int lane) { return ((lane >> 4) & 
 // subsample taps) until the block's reduction at the end (shuffles and shared memory, fixed order, no atomics).
 //
 // Batches of up to 2,047 images, and what grad_tc.cu leaves.  Small batches are a chain of latencies, large ones are bound by the FMA pipe (852 cycles
-// of it per warp and image; 318 us for 60,000 images).  Measured: a step of 256 images in a training loop 15.4 -> 9.6 us (of which the
-// parameters 0.7, forward 2.5, backward 1.5, this kernel's reduction 1.2, the row sums 1.2 and the two hand-overs 1.5 us),
-// the gradient of 60,000 images 1,030 -> 640 us.  (Before: a thread per window and map, scalar, two blocks of seven warps per SM at 128 registers
-// with the patch and all gradient terms in registers, two barriers per image, a row per image up to 296.)
+// of it per warp and image; 318 us for 60,000 images).  Measured: a step of 256 images in a training loop 15.4 -> 8.8 us (of which the
+// parameters 0.7, forward 1.9, backward 1.5, this kernel's reduction 1.2, the row sums 1.2 and the two hand-overs 1.5 us),
+// the gradient of 60,000 images 1,030 -> 645 us.  (Before: a thread per window and map, scalar, two blocks of seven warps per SM at 128 registers
+// with the patch and all gradient terms in registers, two barriers per image, a row per image up to 296; then, until 9.5 us, taps from shared
+// memory for every image and patch loads that took two turns each.)
 // ----------------------------------------------------------------------------------------------
 constexpr int kGrThreads = 224;                 // threads of a team: 216 with work
 constexpr int kGrWarps = kGrThreads / 32;
