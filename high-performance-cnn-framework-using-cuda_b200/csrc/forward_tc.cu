@@ -270,6 +270,22 @@ k_forward_tc(const void* images, long n, long imgs_per_cta, const float* params,
     }
 
   // ---- set-up: weight scale, B operand (banded weights), FC table, small parameters -------------------------
+  // Every load of a thread is under way before the first value is used: one wait for L2 instead of three in a row.
+  constexpr int kBRows = 5 * 2 * kTfBN, kBTurns = (kBRows + kTfThreads - 1) / kTfThreads;      // 16-byte rows of the B operand
+  float bw[kBTurns][5], wfc[kOut], small;
+#pragma unroll
+  for (int t = 0; t < kBTurns; ++t) {
+    const int e = min(tid + t * kTfThreads, kBRows - 1), nn = e % kTfBN, r = nn % 24;
+    const int at = nn < 72 ? kOffWc + (2 * (r / 8) + (r & 1)) * 25 + e / (2 * kTfBN) * 5 : 0;
+#pragma unroll
+    for (int d = 0; d < 5; ++d) bw[t][d] = params[at + d];
+  }
+  {
+    const int u = min(tid, kS - 1), p = u / 36, q = (u % 36) / 6, f = u % 6, t = tid - 256;
+#pragma unroll
+    for (int k = 0; k < kOut; ++k) wfc[k] = params[kOffWf + k * kS + f * 36 + p * 6 + q];
+    small = params[t < 0 || t > 40 ? 0 : (t < 16 ? kOffWs + t : (t < 28 ? kOffBf + min(t - 16, kOut - 1) : (t < 28 + kF ? kOffBc + t - 28 : kOffBs)))];
+  }
   float wmax = 0.f;
   bool finite = true;
 #pragma unroll
@@ -290,14 +306,17 @@ k_forward_tc(const void* images, long n, long imgs_per_cta, const float* params,
   const float w_scale = __int_as_float((127 + 16 - wexp) << 23), px_scale = 255.f * __int_as_float((127 - 3 + wexp) << 23);
   constexpr float w_unscale = 1.0f / 8192.0f;
 
-  for (int e = tid; e < 5 * 2 * kTfBN; e += kTfThreads) {     // one 16-byte row of a chunk: 8 columns of one accumulator column
+#pragma unroll
+  for (int turn = 0; turn < kBTurns; ++turn) {     // one 16-byte row of a chunk: 8 columns of one accumulator column
+    const int e = tid + turn * kTfThreads;
+    if (e >= kBRows) break;
     const int i = e / (2 * kTfBN), rem = e % (2 * kTfBN);
     const int ch = rem / kTfBN, nn = rem % kTfBN;
     // accumulator column nn = 24 * (window column in the block) + 8 * (map / 2) + 2 * (column in the window) + map % 2
-    const int qq = nn / 24, r = nn % 24, f = 2 * (r / 8) + (r & 1), x = 4 * qq + ((r & 7) >> 1);
+    const int qq = nn / 24, r = nn % 24, x = 4 * qq + ((r & 7) >> 1);
     float w[5];
 #pragma unroll
-    for (int d = 0; d < 5; ++d) w[d] = (nn < 72) ? w_scale * params[kOffWc + f * 25 + i * 5 + d] : 0.f;
+    for (int d = 0; d < 5; ++d) w[d] = (nn < 72) ? w_scale * bw[turn][d] : 0.f;
     __half2 hi[4], lo[4];
     constexpr double kFactor = (double)kPre / 255.0;            // in two parts, so that the factor costs the weights no bit
     constexpr float kFactorHi = (float)kFactor, kFactorLo = (float)(kFactor - (double)kFactorHi);
@@ -320,20 +339,18 @@ k_forward_tc(const void* images, long n, long imgs_per_cta, const float* params,
     if (kPrecise) *reinterpret_cast<uint4*>(sm.b_lo + off) = *reinterpret_cast<uint4*>(lo);
   }
   if (tid < kTfAsStride) {       // FC table
-    const int p = tid / 36, q = (tid % 36) / 6, f = tid % 6;
-    const float* wf = params + kOffWf + (tid < kS ? f * 36 + p * 6 + q : 0);
     float w[12];
 #pragma unroll
-    for (int k = 0; k < 12; ++k) w[k] = (tid < kS && k < kOut) ? wf[(k < kOut ? k : 0) * kS] : 0.f;
+    for (int k = 0; k < 12; ++k) w[k] = (tid < kS && k < kOut) ? wfc[k < kOut ? k : 0] : 0.f;
 #pragma unroll
     for (int k = 0; k < 3; ++k)
       *reinterpret_cast<float4*>(sm.wf[tid >> 5][k][tid & 31]) = make_float4(w[4 * k], w[4 * k + 1], w[4 * k + 2], w[4 * k + 3]);
   } else if (tid >= 256 && tid < 256 + 64) {
     const int t = tid - 256;
-    if (t < 16) sm.ws[t] = params[kOffWs + t];
-    else if (t < 28) sm.bf[t - 16] = (t - 16 < kOut) ? params[kOffBf + t - 16] : 0.f;
-    else if (t < 28 + kF) sm.bc[t - 28] = kPre * params[kOffBc + t - 28];
-    else if (t == 40) sm.bs[0] = params[kOffBs];
+    if (t < 16) sm.ws[t] = small;
+    else if (t < 28) sm.bf[t - 16] = (t - 16 < kOut) ? small : 0.f;
+    else if (t < 28 + kF) sm.bc[t - 28] = kPre * small;
+    else if (t == 40) sm.bs[0] = small;
   }
   tc::fence_async_smem();      // the B operand was written through the generic proxy
   tc::fence_before_sync();
