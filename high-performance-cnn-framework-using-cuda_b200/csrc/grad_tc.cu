@@ -167,6 +167,28 @@ k_grad_tc(const float* images, const unsigned* labels, long n, int per_cta, cons
     const int i = min(tid + kGtThreads * j, min(kGtImgs, imgs_here) * (kImg / 4) - 1);
     px[j] = reinterpret_cast<const float4*>(images + img0 * kImg)[i];
   }
+  // The parameters as well: every load of the set-up is under way before the first value is used.
+  constexpr int kBRows = 3 * 5 * kGtBN, kBTurns = (kBRows + kGtThreads - 1) / kGtThreads;      // 16-byte rows of the conv operand
+  constexpr int kAll = (kNParams + kGtThreads - 1) / kGtThreads;
+  float bw[kBTurns][5], wfc[kOut], small, share[kAll], taps[5], wsmax;
+#pragma unroll
+  for (int t = 0; t < kBTurns; ++t) {
+    const int e = min(tid + t * kGtThreads, kBRows - 1), i = e / kGtBN % 5, r = e % kGtBN % 24;
+#pragma unroll
+    for (int d = 0; d < 5; ++d) bw[t][d] = params[kOffWc + (2 * (r >> 3) + (r & 1)) * 25 + i * 5 + d];
+  }
+  {
+    const float* wf = params + kOffWf + (min(tid, kS - 1) % 6) * 36 + min(tid, kS - 1) / 6;      // slot entry u = 36 p + 6 q + f: input 36 f + 6 p + q
+    const int t = tid - 256;
+#pragma unroll
+    for (int k = 0; k < kOut; ++k) wfc[k] = wf[k * kS];
+    small = params[t < 0 || t > 40 ? 0 : (t < 16 ? kOffWs + t : (t < 28 ? kOffBf + min(t - 16, kOut - 1) : (t < 28 + kF ? kOffBc + t - 28 : kOffBs)))];
+  }
+#pragma unroll
+  for (int j = 0; j < kAll; ++j) share[j] = params[min(tid + kGtThreads * j, kNParams - 1)];
+#pragma unroll
+  for (int j = 0; j < 5; ++j) taps[j] = params[min(lane + 32 * j, kOffBc - 1)];
+  wsmax = fabsf(params[kOffWs + (lane & 15)]);
   for (int i = tid; i < kGtSlabs * kGtSlabBytes / 16; i += kGtThreads) reinterpret_cast<uint4*>(sm.slab)[i] = make_uint4(0, 0, 0, 0);
   if (tid < 36) sm.zeros[tid] = 0.f;
   {
@@ -189,19 +211,12 @@ k_grad_tc(const float* images, const unsigned* labels, long n, int per_cta, cons
     for (int k = 0; k < kGtRaw && k < n_tiles; ++k) fetch(k);
 
   // ---- set-up: scales, conv weights, FC table, small parameters ----------------------------------------------
-  float wmax = 0.f, wsmax = 0.f;
+  float wmax = 0.f;
   bool sane = true;
 #pragma unroll
-  for (int j = 0; j < 5; ++j) {
-    const int e = lane + 32 * j;
-    if (e < kOffBc) wmax = fmaxf(wmax, fabsf(params[e]));
-  }
-  if (lane < 16) wsmax = fabsf(params[kOffWs + lane]);
+  for (int j = 0; j < 5; ++j) wmax = fmaxf(wmax, fabsf(taps[j]));
 #pragma unroll
-  for (int j = 0; j < (kNParams + kGtThreads - 1) / kGtThreads; ++j) {
-    const int e = tid + kGtThreads * j;
-    if (e < kNParams) sane = sane && fabsf(params[e]) <= 1e9f;
-  }
+  for (int j = 0; j < kAll; ++j) sane = sane && fabsf(share[j]) <= 1e9f;
 #pragma unroll
   for (int m = 16; m > 0; m >>= 1) {
     wmax = fmaxf(wmax, __shfl_xor_sync(0xffffffffu, wmax, m));
@@ -214,13 +229,16 @@ k_grad_tc(const float* images, const unsigned* labels, long n, int per_cta, cons
   const float w_scale = __int_as_float((127 + 16 - wexp) << 23);
   constexpr float w_unscale = 1.0f / 8192.0f;
 
-  for (int e = tid; e < 3 * 5 * kGtBN; e += kGtThreads) {     // one 16-byte row: 8 input columns of one accumulator column
+#pragma unroll
+  for (int turn = 0; turn < kBTurns; ++turn) {     // one 16-byte row: 8 input columns of one accumulator column
+    const int e = tid + turn * kGtThreads;
+    if (e >= kBRows) break;
     const int variant = e / (5 * kGtBN), i = e / kGtBN % 5, nn = e % kGtBN;
     // accumulator column nn = 24 * (window column in the block) + 8 * (map / 2) + 2 * (column in the window) + map % 2
-    const int qq = nn / 24, r = nn % 24, f = 2 * (r >> 3) + (r & 1), x = 4 * qq + ((r & 7) >> 1);
+    const int qq = nn / 24, r = nn % 24, x = 4 * qq + ((r & 7) >> 1);
     float w[5];
 #pragma unroll
-    for (int d = 0; d < 5; ++d) w[d] = w_scale * params[kOffWc + f * 25 + i * 5 + d];
+    for (int d = 0; d < 5; ++d) w[d] = w_scale * bw[turn][d];
     __half2 hi[4], lo[4];
     constexpr double kFactor = (double)kPre / 255.0;            // in two parts, so that the factor costs the weights no bit
     constexpr float kFactorHi = (float)kFactor, kFactorLo = (float)(kFactor - (double)kFactorHi);
@@ -244,15 +262,14 @@ k_grad_tc(const float* images, const unsigned* labels, long n, int per_cta, cons
     *reinterpret_cast<uint4*>(sm.b[1] + off) = *reinterpret_cast<uint4*>(lo);
   }
   if (tid < kS) {
-    const float* wf = params + kOffWf + (tid % 6) * 36 + tid / 6;      // slot entry u = 36 p + 6 q + f: input 36 f + 6 p + q
 #pragma unroll
-    for (int k = 0; k < kOut; ++k) sm.wf[k][tid] = wf[k * kS];
+    for (int k = 0; k < kOut; ++k) sm.wf[k][tid] = wfc[k];
   } else if (tid >= 256 && tid < 256 + 64) {
     const int t = tid - 256;
-    if (t < 16) sm.ws[t] = params[kOffWs + t];
-    else if (t < 28) sm.bf[t - 16] = (t - 16 < kOut) ? params[kOffBf + t - 16] : 0.f;
-    else if (t < 28 + kF) sm.bc[t - 28] = kPre * params[kOffBc + t - 28];
-    else if (t == 40) sm.bs[0] = params[kOffBs];
+    if (t < 16) sm.ws[t] = small;
+    else if (t < 28) sm.bf[t - 16] = (t - 16 < kOut) ? small : 0.f;
+    else if (t < 28 + kF) sm.bc[t - 28] = kPre * small;
+    else if (t == 40) sm.bs[0] = small;
   }
   tc::fence_async_smem();      // the operands were written through the generic proxy
   tc::fence_before_sync();
