@@ -76,16 +76,23 @@ k_forward_one(const void* images, long n, const float* params,
       if (im < n) issue(s, im);
     }
   }
-  // Parameters: 9.4 KB from global (L2-resident after the first block) into shared memory.
-  for (int i = tid; i < kOut * kS; i += kFwThreads) {
-    const int k = i / kS, s = i % kS;
-    sm.wf[k][s % 36][s / 36] = params[kOffWf + i];
+  // Parameters: 9.4 KB, L2-resident after the first block.  Every load of a thread is under way before the first is stored (one wait for L2).
+  {
+    const int at = tid < kS ? tid : kS - 1;
+    float wf[kOut];
+#pragma unroll
+    for (int k = 0; k < kOut; ++k) wf[k] = params[kOffWf + k * kS + at];
+    const float small = params[tid < kOffWf ? tid : kOffBf + (tid - kOffWf < kOut ? tid - kOffWf : 0)];
+    if (tid < kS) {
+#pragma unroll
+      for (int k = 0; k < kOut; ++k) sm.wf[k][tid % 36][tid / 36] = wf[k];
+    }
+    if (tid < kOffBc) sm.wc[tid % 25][tid / 25] = kPre * small;
+    else if (tid < kOffWs) sm.bc[tid - kOffBc] = kPre * small;
+    else if (tid < kOffBs) sm.ws[tid - kOffWs] = small;
+    else if (tid == kOffBs) sm.bs[0] = small;
+    else if (tid < kOffWf + kOut) sm.bf[tid - kOffWf] = small;
   }
-  if (tid < kF * 25) sm.wc[tid % 25][tid / 25] = kPre * params[kOffWc + tid];
-  if (tid < kF) sm.bc[tid] = kPre * params[kOffBc + tid];
-  if (tid < 16) sm.ws[tid] = params[kOffWs + tid];
-  if (tid == 0) sm.bs[0] = params[kOffBs];
-  if (tid < kOut) sm.bf[tid] = params[kOffBf + tid];
   __syncthreads();
 
   // thread -> (window, pair, half): half fastest, so that a window's halves are neighbouring lanes
@@ -262,23 +269,28 @@ k_forward_tiles(const void* images, long n, const float* params,
       if (t < n_tiles) issue(s, t);
     }
   }
-  if (tid < kFwPairs * 2 * 36) {          // 216 threads, ten FC weights each
-    const int f = tid / 36, w = tid % 36;
-    float* dst = sm.wf[f >> 1][w][f & 1];
+  // Parameters: every load of a thread is under way before the first is stored (one wait for L2).
+  {
+    const int f = tid / 36, w = tid % 36, tap_f = tid / kFtTaps, tap = tid % kFtTaps;
+    float wf[kOut];
 #pragma unroll
-    for (int k = 0; k < kOut; ++k) dst[k] = params[kOffWf + k * kS + tid];
-  } else if (tid < 232) {
-    sm.ws[tid - 216][0] = sm.ws[tid - 216][1] = params[kOffWs + tid - 216];
-  } else if (tid < 242) {
-    sm.bf[tid - 232] = params[kOffBf + tid - 232];
-  } else if (tid < 248) {
-    sm.bc[tid - 242] = kPre * params[kOffBc + tid - 242];
-  } else if (tid == 248) {
-    sm.bs[0] = params[kOffBs];
-  }
-  if (tid < kF * kFtTaps) {
-    const int f = tid / kFtTaps, t = tid % kFtTaps;
-    sm.wc[f >> 1][t][f & 1] = (t < 25) ? kPre * params[kOffWc + f * 25 + t] : 0.f;
+    for (int k = 0; k < kOut; ++k) wf[k] = params[kOffWf + k * kS + (tid < kS ? tid : kS - 1)];
+    const float taps = params[kOffWc + (tap_f < kF && tap < 25 ? tap_f * 25 + tap : 0)];
+    const float small = params[tid < 216 ? 0 : (tid < 232 ? kOffWs + tid - 216 : (tid < 242 ? kOffBf + tid - 232 : (tid < 248 ? kOffBc + tid - 242 : kOffBs)))];
+    if (tid < kS) {                       // 216 threads, ten FC weights each
+      float* dst = sm.wf[f >> 1][w][f & 1];
+#pragma unroll
+      for (int k = 0; k < kOut; ++k) dst[k] = wf[k];
+    } else if (tid < 232) {
+      sm.ws[tid - 216][0] = sm.ws[tid - 216][1] = small;
+    } else if (tid < 242) {
+      sm.bf[tid - 232] = small;
+    } else if (tid < 248) {
+      sm.bc[tid - 242] = kPre * small;
+    } else if (tid == 248) {
+      sm.bs[0] = small;
+    }
+    if (tid < kF * kFtTaps) sm.wc[tap_f >> 1][tap][tap_f & 1] = (tap < 25) ? kPre * taps : 0.f;
   }
   __syncthreads();
 
