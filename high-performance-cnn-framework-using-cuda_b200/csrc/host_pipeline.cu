@@ -1,8 +1,8 @@
 // The forward pass through host buffers: copy in, kernel and results out, in chunks that overlap.
 //
 // A request is cut into chunks of images; four slots (a device buffer, a stream and a result buffer each) take them in
-// turn, so that the copies of the next chunks run under a chunk's kernel.  The last chunk is a quarter of the request at most: its kernel and results
-// come behind everything else.  Pinned images are copied from where they lie.
+// turn, so that the copies of the next chunks run under a chunk's kernel.  The last chunk is the short one: its kernel and results come behind
+// everything else.  Pinned images are copied from where they lie.
 // Pageable images go through a pinned ring that several cores fill (copy_pool.h): 10,000 uint8 images 620-750 -> 250 us on a B200
 // (the driver's own staging fills its buffer with one core, 12 GB/s; the bus carries 55 GB/s).  Results for pageable
 // buffers go through pinned memory too, one copy per chunk.  (Written there by the kernel itself, over the bus, they cost
@@ -25,6 +25,7 @@ int forward_device_u8(cnn_net* net, int path, const unsigned char* d_pixels, lon
 constexpr int kHpSlots = 4;
 constexpr long kHpMaxChunk = 8192, kHpMinChunk = 512;       // images per chunk
 static_assert(kHpSlots * (sizeof(float) * (kOut + 1) * kHpMaxChunk + 256) + sizeof(int) * kHpSlots <= PinnedBlock::kPage, "results fit a lease");
+constexpr size_t kHpMinQuarter = 4608 * 1024;               // pinned images: below, two halves
 constexpr size_t kHpMinStaged = 128 * 1024;                 // below, the driver's own staging is as fast
 
 struct HostPipeline {
@@ -165,29 +166,24 @@ struct HostRequest {
     }
     return CNN_OK;
   }
-  // Pieces of the staged copy.  The cores fill them about as fast as the bus takes them, so nothing but the first piece's filling and the last
-  // one's way over the bus is not under something else: these are short (and so the ones next to them), the others as long as a slot, because
-  // every copy costs some microseconds.
+  // Pieces of the staged copy: as many as a chunk needs, of equal length.  (A short first piece and short pieces in the last chunk, so that less of
+  // the filling and of the bus comes before and behind everything else: 1-8 % slower below 10 MB, every copy costs some microseconds, and 0-2 % faster above.)
   bool cut(long& pieces) {
-    const long most = (long)((size_t)n * image_bytes / (CopyPool::kPiece / 4)) + 2 * (n / chunk + 3);
+    const long most = (long)((size_t)n * image_bytes / CopyPool::kPiece) + n / chunk + 3;
     at.reset(new (std::nothrow) size_t[most + 1]);
     chunk_end.reset(new (std::nothrow) long[most]);
     if (!at || !chunk_end) return false;
     pieces = 0;
     at[0] = 0;
-    for (long first = 0; first < n;) {
-      const long end = first + count_at(first);
-      const bool last = end == n;
-      const size_t end_byte = (size_t)end * image_bytes;
+    for (long first = 0, end; first < n; first = end) {
+      end = first + count_at(first);
+      const size_t end_byte = (size_t)end * image_bytes, bytes = end_byte - (size_t)first * image_bytes;
+      const size_t parts = (bytes + CopyPool::kPiece - 1) / CopyPool::kPiece, length = ((bytes + parts - 1) / parts + 63) & ~(size_t)63;
       while (at[pieces] < end_byte) {
-        const size_t left = end_byte - at[pieces];
-        size_t take = pieces == 0 ? CopyPool::kPiece / 4 : (pieces == 1 || last ? CopyPool::kPiece / 2 : CopyPool::kPiece);
-        if (take >= left || left - take < CopyPool::kPiece / 8) take = left < CopyPool::kPiece ? left : CopyPool::kPiece / 2;
-        chunk_end[pieces] = at[pieces] + take == end_byte ? end : 0;
-        at[pieces + 1] = at[pieces] + take;
+        at[pieces + 1] = end_byte - at[pieces] > length ? at[pieces] + length : end_byte;
+        chunk_end[pieces] = at[pieces + 1] == end_byte ? end : 0;
         ++pieces;
       }
-      first = end;
     }
     return true;
   }
@@ -267,9 +263,12 @@ static int forward_host_impl(cnn_net* net, const void* h_images, bool u8, long n
   const size_t image_bytes = u8 ? (size_t)kImg : sizeof(float) * kImg;
   const bool pageable = is_pageable(h_images);
   // Behind the last copy there is the last chunk's kernel, the way of its results back and, for pageable result buffers, a copy of them: a
-  // quarter of the request (halves, in pieces of equal length: 262 us for 10,000 uint8 images instead of 250; quarters all over: more hand-overs, 280).
-  long last = n / 4;
-  last = last < kHpMinChunk ? kHpMinChunk : (last > kHpMaxChunk / 4 ? kHpMaxChunk / 4 : last);
+  // quarter of the request (halves: 10,000 uint8 images 256 instead of 249 us, 6,000 181 instead of 172; quarters all over: more hand-overs, 280).
+  // Pinned images, without the filling of the ring, leave a small request nothing to gain: halves below 4.5 MB (quarter, half: 5,000 uint8 images
+  // 141, 131 us, 1,300 fp32 125, 119; 6,000 uint8 144, 151, 1,500 fp32 131, 136).
+  const bool quarter = pageable || (size_t)n * image_bytes >= kHpMinQuarter;
+  long last = quarter ? n / 4 : (n / 2 < n - 2 * kHpMinChunk ? n / 2 : n - 2 * kHpMinChunk);
+  if (quarter) last = last < kHpMinChunk ? kHpMinChunk : (last > kHpMaxChunk / 4 ? kHpMaxChunk / 4 : last);
   if (n <= 2 * kHpMinChunk) last = n;
   const long rest = n - last, parts = (rest + kHpMaxChunk - 1) / kHpMaxChunk;
   const long chunk = parts > 0 ? (rest + parts - 1) / parts : last;
