@@ -14,12 +14,12 @@
 //    outputs on a 6x8 patch, 200 packed FMAs, the 25 tap pairs in registers for the whole launch.  The two halves of a window
 //    meet in one shuffle, each computes five of the ten FC partial sums, which are added up over the warp by a
 //    shuffle reduce-scatter and over the block's seven warps through shared memory.  Bound by the chain launch -
-//    parameters - patch - 25 x 8 FMAs - two sigmoids - sums - sigmoid: 1 image 10.2 -> 4.5 us, 300 images 10.6 -> 6.1 us
-//    (before: the next kernel's shape at every size, scalar).
-//  * k_forward_tiles: tiles of seven images, thread = window for all six maps (three packed pairs one after another), FC
+//    parameters - patch - 25 x 8 FMAs - two sigmoids - sums - sigmoid: 1 image 10.2 -> 4.0 us, 300 images 10.6 -> 4.4 us
+//    (before: the next kernel's shape at every size, scalar; until 4.5 us the parameters were loaded in several groups, one wait for L2 each).
+//  * k_forward_tiles: tiles of up to seven images, thread = window for all six maps (three packed pairs one after another), FC
 //    partial sums in registers, one barrier pair per tile.  Bound by the FMA pipe (92,016 FMAs = 719 SM-cycles per
-//    image; 63 % of it at 6,143 images): 2,000 images 16.4 -> 10.8 us, 6,143 images 34.9 -> 27.3 us (scalar FMAs on a
-//    patch in registers before).
+//    image; 65 % of it at 6,143 images): 1,000 images 10.5 -> 6.6 us (tiles of equal length), 2,000 images 16.4 -> 10.5 us, 6,143 images
+//    34.9 -> 26.5 us (scalar FMAs on a patch in registers before).
 #include "net.cuh"
 
 namespace cnn {
@@ -236,14 +236,21 @@ struct FtSmem {
   unsigned long long full[kFwStages];
 };
 
-template <int FAST, bool U8>
+// ONE_ROUND: a tile per block, per_tile images each and one more in the first `more`; otherwise tiles of seven, the last one of what is left.
+template <int FAST, bool U8, bool ONE_ROUND>
 __global__ void __launch_bounds__(kFtThreads, kFtBlocksPerSm)
-k_forward_tiles(const void* images, long n, const float* params,
+k_forward_tiles(const void* images, long n, int per_tile, int more, const float* params,
                 float* __restrict__ out, int* __restrict__ argmax, int* __restrict__ status) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   FtSmem& sm = *reinterpret_cast<FtSmem*>(smem_raw);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const long n_tiles = (n + kFtImgs - 1) / kFtImgs;
+  const long n_tiles = ONE_ROUND ? gridDim.x : (n + kFtImgs - 1) / kFtImgs;
+  auto first_of = [&](long tile) -> long { return ONE_ROUND ? tile * per_tile + (tile < more ? tile : more) : tile * kFtImgs; };
+  auto count_of = [&](long tile) -> int {
+    if (ONE_ROUND) return per_tile + (tile < more ? 1 : 0);
+    const long left = n - tile * kFtImgs;
+    return left < kFtImgs ? (int)left : kFtImgs;
+  };
   constexpr float kPre = (FAST == 1) ? -1.4426950408889634f : 1.0f;
   constexpr unsigned kImageBytes = (U8 ? 1u : 4u) * (unsigned)kImg;
 
@@ -252,8 +259,8 @@ k_forward_tiles(const void* images, long n, const float* params,
     return U8 ? reinterpret_cast<unsigned char*>(&sm.img[1][0][0]) + stage * (kFtImgs * kImg) : reinterpret_cast<unsigned char*>(&sm.img[stage][0][0]);
   };
   auto issue = [&](int stage, long tile) {
-    const long first = tile * kFtImgs, left = n - first;
-    const unsigned bytes = (unsigned)(left < kFtImgs ? left : kFtImgs) * kImageBytes;
+    const long first = first_of(tile);
+    const unsigned bytes = (unsigned)count_of(tile) * kImageBytes;
     mbar_expect_tx(&sm.full[stage], bytes);
     bulk_g2s(raw(stage), static_cast<const unsigned char*>(images) + (size_t)first * kImageBytes, bytes, &sm.full[stage]);
   };
@@ -308,9 +315,11 @@ k_forward_tiles(const void* images, long n, const float* params,
   for (long tile = blockIdx.x; tile < n_tiles; tile += gridDim.x, ++it) {
     const int stage = it % kFwStages;
     mbar_wait_bounded(&sm.full[stage], (unsigned)(it / kFwStages) & 1u, status, gave_up);
-    const long first = tile * kFtImgs;
-    const int imgs_here = (int)((n - first) < kFtImgs ? (n - first) : kFtImgs);
+    const long first = first_of(tile);
+    const int imgs_here = count_of(tile);
     const bool live = img < imgs_here;
+    // Warps without an image leave the pipes to the others.  (uint8 pixels in several rounds: the test costs 2 %, and few warps have none.)
+    const bool work = (U8 && !ONE_ROUND) || __any_sync(0xffffffffu, live);
     const int at = (live ? img : 0) * kImg + (4 * p) * kH + 4 * q;         // first pixel of the thread's patch
     if constexpr (U8) {                    // (the previous tile's patches were read before its barriers)
       const unsigned* src = reinterpret_cast<const unsigned*>(raw(stage));
@@ -326,7 +335,7 @@ k_forward_tiles(const void* images, long n, const float* params,
 #pragma unroll
     for (int k = 0; k < kOut / 2; ++k) fc[k] = pack2(0.f, 0.f);
 #pragma unroll 1
-    for (int pr = 0; pr < kFwPairs; ++pr) {
+    for (int pr = work ? 0 : kFwPairs; pr < kFwPairs; ++pr) {
       int again = at;                      // hidden from the compiler: keeping the 8x8 patch over the pairs would spill
       asm volatile("" : "+r"(again));
       const float* base = &sm.img[U8 ? 0 : stage][0][0] + again;
@@ -440,10 +449,18 @@ static int launch_variant(cnn_net* net, int path, const void* d_images, long n, 
     e = launch_pdl(k_forward_one<FAST, U8>, dim3((unsigned)(n < resident ? n : resident)), dim3(kFwThreads), 0, stream, d_images, n,
                    (const float*)net->d_params, d_out, d_argmax, net->d_status);
   } else {
-    const long n_tiles = (n + kFtImgs - 1) / kFtImgs, resident = (long)kFtBlocksPerSm * sm_count();
-    CNN_CUDA(cudaFuncSetAttribute(k_forward_tiles<FAST, U8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(FtSmem)));
-    e = launch_pdl(k_forward_tiles<FAST, U8>, dim3((unsigned)(n_tiles < resident ? n_tiles : resident)), dim3(kFtThreads),
-                   sizeof(FtSmem), stream, d_images, n, (const float*)net->d_params, d_out, d_argmax, net->d_status);
+    // One round of tiles: a tile per block, of equal length to one image, because a round takes as long as its longest tile and warps without an image
+    // leave the pipes to the others (tiles of seven: 889 images 10.5 us, 1,036 6.7, 1,184 10.5, 2,072 10.7; equal ones 6.5, 6.6, 8.7, 10.5).  Up to
+    // seven images per SM that is a block on each SM: fewer would leave SMs idle that take two blocks of the next launch.  With more rounds
+    // tiles of seven, but for the last one, are the better ones (2,500 images 14.4 against 16.2 us, 5,000 22.7 against 26.2; 3,000 18.9 against 17.7).
+    const long sms = sm_count(), resident = kFtBlocksPerSm * sms;
+    const bool one_round = n <= resident * kFtImgs;
+    const long most = n <= sms * kFtImgs ? sms : resident, n_tiles = one_round ? (n < most ? n : most) : (n + kFtImgs - 1) / kFtImgs;
+    const long grid = n_tiles < resident ? n_tiles : resident;
+    auto* const kernel = one_round ? k_forward_tiles<FAST, U8, true> : k_forward_tiles<FAST, U8, false>;
+    CNN_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(FtSmem)));
+    e = launch_pdl(kernel, dim3((unsigned)grid), dim3(kFtThreads), sizeof(FtSmem), stream, d_images, n, (int)(n / n_tiles), (int)(n % n_tiles),
+                   (const float*)net->d_params, d_out, d_argmax, net->d_status);
   }
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e, "fused forward launch");
@@ -453,18 +470,20 @@ static int launch_variant(cnn_net* net, int path, const void* d_images, long n, 
 // The kernel a call over n_total images uses: 0 = k_forward_tiles, kForwardOne = k_forward_one, 1 / 2 = forward_tc.cu.
 // Default (-1): the three-pass tensor-core kernel for batches of kTcMinBatch images and more, this file's below.  The line is the one
 // that the interface promises (the two sides differ in their last bits); it is not where the kernels meet.  That is at one round of
-// tiles, 14 images per SM: 2,072 images 10.9 us here, 11.1 on the tensor cores; 2,073 images 14.2 and 11.1; 4,144: 19.1 and 15.4; 6,143: 27.3 and
-// 18.8 (uint8: 11.5 / 10.9, 14.9 / 10.9, 21.0 / 14.9, 29.9 / 18.0).
+// tiles, 14 images per SM: 2,072 images 10.5 us here, 10.3 on the tensor cores; 2,073 images 11.9 and 10.3; 4,144: 18.6 and 13.8; 6,143: 26.5 and
+// 16.7 (uint8: 10.8 / 9.5, 14.8 / 9.5, 20.8 / 12.7, 29.7 / 15.2).
 // uint8 pixels follow the same rule, so that they give the same bits as the fp32
 // images they stand for (the reduced-precision path 2 is for fp32 images only).  All keep the 1e-5 parity bar.
-// With the reference's sigmoid expression asked for (fast_sigmoid = 0) the default stays in this file.  Up to six images
-// per SM the one-image kernel is the faster one: 600 images 8.0 us, 1,000 images 11.0 us, against 10.6 us for a round of
-// tiles, which is what anything up to 2,072 images costs there.
+// With the reference's sigmoid expression asked for (fast_sigmoid = 0) the default stays in this file.
+// One-image kernel / a tile on each SM, fp32 and uint8: 148 images 3.4 / 4.6 us and 3.3 / 4.6, 350 images 4.5 / 4.6 and 4.7 / 4.9, 444 images
+// 5.7 / 4.7 and 5.8 / 4.9 (up to three images a tile's warps have a scheduler each), 445 images 5.7 / 6.1 and 5.8 / 6.7, 660 images 6.3 / 6.5 and
+// 6.5 / 6.9, 700 images 7.3 / 6.5 and 7.7 / 6.9, 888 images 7.5 / 6.5 and 7.9 / 6.8: the lines lie at 2.5, 3 and 4.5 images per SM.
 int forward_kernel_for(const cnn_net* net, long n_total, bool u8) {
   constexpr long kTcMinBatch = 6144;
   int path = net->forward_path;
   if (path < 0 || (u8 && path == 2)) path = (net->fast_sigmoid && n_total >= kTcMinBatch) ? 1 : 0;
-  return (path == 0 && n_total <= 6L * sm_count()) ? kForwardOne : path;
+  const long sms = sm_count();
+  return (path == 0 && (2 * n_total <= 5 * sms || (n_total > 3 * sms && 2 * n_total <= 9 * sms))) ? kForwardOne : path;
 }
 
 // `path` as returned by forward_kernel_for: callers that cut a request into chunks decide once for the

@@ -489,6 +489,25 @@ def test_cuda_core_forward_around_its_dispatch(cuda, pkg, params0, n, fast):
     assert net.status() == 0 and np.array_equal(d_out.cpu().numpy(), out)
 
 
+@pytest.mark.parametrize("n", [370, 371, 444, 445, 666, 667, 1035, 1036, 1037, 2071, 2072, 2081, 4147])
+def test_cuda_core_forward_tiles_of_equal_length(cuda, pkg, params0, n):
+    """Both sides of the lines at 2.5, 3 and 4.5 images per SM (148 of them) between the one-image and the tile kernel, of a tile on each
+    SM and of a round of tiles, and last tiles of two and three images with warps that have none.  Reference as above."""
+    pix = pkg.synth.synth_pixels_u8(47, n)
+    images = pkg.synth.u8_to_float(pix)
+    net = pkg.Net(0)
+    net.set_params(params0)
+    net.set_option("forward_path", 1)
+    ref, _ = run_forward(cuda, net, images)
+    net.set_option("forward_path", 0)
+    out, arg = run_forward(cuda, net, images)
+    assert rel_err(out, ref) < 1e-5 and np.array_equal(arg, np.argmax(out, axis=1).astype(np.int32))
+    d_pix, d_out = cuda.from_numpy(pix).cuda(), cuda.empty((n, 10), dtype=cuda.float32, device="cuda")
+    net.forward_u8(d_pix, n, d_out, None)
+    cuda.cuda.synchronize()
+    assert net.status() == 0 and np.array_equal(d_out.cpu().numpy(), out)
+
+
 @pytest.mark.parametrize("u8", [False, True])
 @pytest.mark.parametrize("n", [41, 200, 1024, 1025, 9001, 17000])
 def test_forward_host_buffers_pageable_and_pinned(cuda, pkg, params0, n, u8):
