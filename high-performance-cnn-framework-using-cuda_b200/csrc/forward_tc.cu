@@ -53,8 +53,8 @@
 //               output, so the weights are read once for three images), reduce-scatter, output
 //               sigmoid, argmax (lowest index wins ties), 44 bytes per image to HBM.
 //
-// Measured on a B200 (three passes whatever the pixels, a table for uint8 before, now): 65,536 fp32 images 138 -> 115 us, 30,011 uint8 images
-// 65 -> 54 us, path 2 on 65,536 images 98 -> 92 us (loader without bank conflicts).  What bounds it now, per tile of 5.33 images
+// Measured on a B200 (three passes whatever the pixels, a table for uint8 before, now): 65,536 fp32 images 138 -> 114 us, 30,011 uint8 images
+// 65 -> 53 us, path 2 on 65,536 images 98 -> 91 us (loader without bank conflicts).  What bounds it now, per tile of 5.33 images
 // (2,400 cycles): the shared-memory data pipe (20 MMAs fetch 130 KB of operands, 1,040 cycles, the other warps and the copies take 900),
 // and next the special-function unit (1,600 cycles) and instruction issue (1,400); path 2: the special-function unit, 75 % busy.
 #include <type_traits>

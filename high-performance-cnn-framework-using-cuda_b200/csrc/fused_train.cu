@@ -807,9 +807,9 @@ struct GradRows {
 };
 
 // Tensor cores or CUDA cores.  Microseconds per gradient call, CUDA cores / tensor cores, back to back (alone behind a flush of L2: the same
-// differences, both 9 us longer): 1,000 images 18.6 / 21.3, 1,480 (two tiles per SM) 23.2 / 22.8, 2,000 29.8 / 25.4, 2,500 35.3 / 29, 3,000 41.2 / 32.5,
-// 6,000 72 / 46, 20,000 221 / 107, 60,000 645 / 290.  They meet at about 1,500; the line leaves room for images that turn out not to be
-// whole numbers / 255 and go to the CUDA cores behind a look at the first tiles: 2,000 images 36, 6,000 78, 60,000 656.
+// differences, both 9 us longer): 1,480 images (two tiles per SM) 23.4 / 21.1, 2,000 30.0 / 24.2, 3,000 41.5 / 31.1,
+// 6,000 72.9 / 44.2, 20,000 220 / 107, 60,000 643 / 290.  They meet at about 1,300; the line leaves room for images that turn out not to be
+// whole numbers / 255 and go to the CUDA cores behind a look at the first tiles: 2,000 images 37, 6,000 79, 60,000 666.
 static int launch_gradient(cnn_net* net, const float* d_images, const unsigned* d_labels, long n, cudaStream_t st, bool chained, GradRows* out) {
   constexpr long kTcGradMin = 2048;
   const int sms = sm_count();
