@@ -19,10 +19,15 @@
 // other pixel, and images from there on are left to k_grad_partials (fused_train.cu), as are all of them where a parameter is not finite or
 // far out of range.  The tensor core truncates its additions, which over a tile's 48 would cost a gradient 1e-6.  Here they are exact: deltas are
 // scaled by a power of two so that the tile's bound on them (max |ds| * max |Ws| / 4) lies in [1024, 2048), and cut into a whole
-// number, at most 11 bits, and the rest.  Products of whole numbers with bytes have 19 bits and their sums stay below 2^24 (incoherent sums of
-// a tile's 4,600 terms by far; what a coherent one might truncate is below 2^-24 of it).  The rest in fp16 is good to 2^-24 of the bound.
-// D is added to fp32 sums in registers after every tile.  Distance of the gradient from fp64, geometric mean of eight nets and batches: 5.0e-8 of
-// its norm for 8,000 images and 5.2e-8 for 60,000 (k_grad_partials 5.1e-8 and 5.2e-8; conv weights alone 5.2e-8 and 6.0e-8, there 4.8e-8 and 6.0e-8).
+// number, at most 11 bits, and the rest, which in fp16 is good to 2^-24 of the bound.  Products of whole numbers with bytes have 19 bits.  A D adds 720 of
+// them: with deltas of one sign and bright pixels up to 2^28, of which truncation took 0.9e-6 on average and 3e-6 at most, always towards zero.  So
+// pixels are taken from a level, the whole number next to the mean of a sample of the block's images; what it adds to a pre-activation is in the bias, and
+// what it adds to a tap's gradient is the level times the bias gradient, which is summed in fp32.  Sums of centred pixels stay below 2^24: over nets as drawn
+// and trained, and nets with deltas of one sign, with strokes, inverted strokes, both mixed, noise and smooth bright images, a tile's
+// largest lies between 2^14 and 2^23.5 (without the level up to 2^26.9).
+// D is added to fp32 sums in registers after every tile.  Distance of the gradient from fp64, geometric mean over 12 nets and batches of 2,048,
+// 4,500, 8,000, 20,000 and 60,000 images: 4.90e-8 of its norm (k_grad_partials 4.93e-8), conv weights alone 4.98e-8 (4.83e-8), conv biases 4.77e-8
+// (5.78e-8); nets with deltas of one sign 4.52e-8 (4.51e-8), conv weights 4.79e-8 (4.74e-8).
 //
 // Pipeline (one CTA per SM, 20 warps, mbarriers with bounded waits):
 //   warps 4-7   one bulk copy per tile, two tiles ahead; pixels -> fp16 operand; drain D of the tile that had the slab before;
@@ -64,6 +69,7 @@ constexpr unsigned kGtDeltaBlock = 128 * 16;                 // [eight columns: 
 constexpr int kGtDeltaBytes = 6 * kGtDeltaBlock;             // three map pairs, high and low parts
 constexpr int kGtGradN = 40, kGtGradCol = kGtSets * 3 * kGtBN;     // D of even and odd tiles behind the accumulators: 432 + 2 * 40 = 512
 constexpr int kGtFcThreads = 64, kGtFcRounds = 4;            // 216 = 3 * 64 + 24
+constexpr int kGtPlaces = 2 * kGtThreads / 32;                // places of the share that are looked at first, 128 pixels each
 constexpr int kGtWfStride = 234;              // five rows of weights, 10 (mod 32) words apart, by six parts of nine inputs: thirty banks
 constexpr int kGtConvWarp = 2, kGtGradWarp = 3, kGtLoadWarp0 = 4, kGtEpiWarp0 = 8;
 
@@ -82,6 +88,7 @@ struct GtSmem {
   float tile_unscale[kGtSlabs];
   unsigned long long raw_full[kGtRaw], a_full[kGtSlabs], a_free[kGtSlabs], d_full[3 * kGtSets], d_free[3 * kGtSets], df_ready[kGtSets], df_free[kGtSets],
       dl_full[kGtWindows], dl_free[kGtWindows], g_free[2];
+  int px_sum[kGtThreads / 32];                               // whole pixels of the sample, by warp
   int stop;                                                  // tiles that take part
   unsigned tmem_base;
   long long clock_base;                                      // phase clocks only
@@ -160,17 +167,18 @@ k_grad_tc(const float* images, const unsigned* labels, long n, int per_cta, cons
     mbar_expect_tx(&sm.raw_full[k % kGtRaw], bytes);
     bulk_g2s(sm.raw[k % kGtRaw], images + (img0 + k * kGtImgs) * kImg, bytes, &sm.raw_full[k % kGtRaw]);
   };
-  // ---- the first tile's pixels: images that are not whole numbers / 255 are as a rule all of that kind, and this block has nothing to do then ----
+  // ---- a sample of the share's pixels, 128 neighbours at each of kGtPlaces places: its mean is the level that pixels are taken from, and images that
+  // are not whole numbers / 255 are as a rule all of that kind (this block has nothing to do then) ----
   float4 px[2];
 #pragma unroll
   for (int j = 0; j < 2; ++j) {
-    const int i = min(tid + kGtThreads * j, min(kGtImgs, imgs_here) * (kImg / 4) - 1);
-    px[j] = reinterpret_cast<const float4*>(images + img0 * kImg)[i];
+    const long pieces = (long)imgs_here * (kImg / 4), first = (2 * warp + j) * (pieces - 32) / (kGtPlaces - 1);
+    px[j] = reinterpret_cast<const float4*>(images + img0 * kImg)[first + lane];
   }
   // The parameters as well: every load of the set-up is under way before the first value is used.
   constexpr int kBRows = 3 * 5 * kGtBN, kBTurns = (kBRows + kGtThreads - 1) / kGtThreads;      // 16-byte rows of the conv operand
   constexpr int kAll = (kNParams + kGtThreads - 1) / kGtThreads;
-  float bw[kBTurns][5], wfc[kOut], small, share[kAll], taps[5], wsmax;
+  float bw[kBTurns][5], wfc[kOut], small, share[kAll], taps[5], wsmax;      // (taps: the 150 and the six biases)
 #pragma unroll
   for (int t = 0; t < kBTurns; ++t) {
     const int e = min(tid + t * kGtThreads, kBRows - 1), i = e / kGtBN % 5, r = e % kGtBN % 24;
@@ -187,18 +195,24 @@ k_grad_tc(const float* images, const unsigned* labels, long n, int per_cta, cons
 #pragma unroll
   for (int j = 0; j < kAll; ++j) share[j] = params[min(tid + kGtThreads * j, kNParams - 1)];
 #pragma unroll
-  for (int j = 0; j < 5; ++j) taps[j] = params[min(lane + 32 * j, kOffBc - 1)];
+  for (int j = 0; j < 5; ++j) taps[j] = params[min(lane + 32 * j, kOffWs - 1)];
   wsmax = fabsf(params[kOffWs + (lane & 15)]);
   for (int i = tid; i < kGtSlabs * kGtSlabBytes / 16; i += kGtThreads) reinterpret_cast<uint4*>(sm.slab)[i] = make_uint4(0, 0, 0, 0);
   if (tid < 36) sm.zeros[tid] = 0.f;
   {
     bool other = false;
+    int sum = 0;
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
       const float x[4] = {px[j].x * 255.f, px[j].y * 255.f, px[j].z * 255.f, px[j].w * 255.f};
 #pragma unroll
-      for (int c = 0; c < 4; ++c) other = other || !(x[c] == rintf(x[c]) && fabsf(x[c]) <= 255.f);
+      for (int c = 0; c < 4; ++c) {
+        other = other || !(x[c] == rintf(x[c]) && fabsf(x[c]) <= 255.f);
+        sum += (int)fminf(fmaxf(x[c], 0.f), 255.f);
+      }
     }
+    sum = __reduce_add_sync(0xffffffffu, sum);
+    if (lane == 0) sm.px_sum[warp] = sum;
     if (__syncthreads_or(other)) {
       float* row = rows + (size_t)blockIdx.x * kRowStride;
       for (int i = tid; i < kRowStride; i += kGtThreads) row[i] = 0.f;
@@ -214,7 +228,7 @@ k_grad_tc(const float* images, const unsigned* labels, long n, int per_cta, cons
   float wmax = 0.f;
   bool sane = true;
 #pragma unroll
-  for (int j = 0; j < 5; ++j) wmax = fmaxf(wmax, fabsf(taps[j]));
+  for (int j = 0; j < 5; ++j) wmax = fmaxf(wmax, lane + 32 * j < kOffBc ? fabsf(taps[j]) : 0.f);
 #pragma unroll
   for (int j = 0; j < kAll; ++j) sane = sane && fabsf(share[j]) <= 1e9f;
 #pragma unroll
@@ -228,6 +242,10 @@ k_grad_tc(const float* images, const unsigned* labels, long n, int per_cta, cons
   wexp = min(max(wexp, -21), 11);
   const float w_scale = __int_as_float((127 + 16 - wexp) << 23);
   constexpr float w_unscale = 1.0f / 8192.0f;
+  int level = 0;                                 // the sample's mean pixel, a whole number
+#pragma unroll
+  for (int w = 0; w < kGtThreads / 32; ++w) level += sm.px_sum[w];
+  level = wexp > 10 ? 0 : (level + 128 * kGtPlaces / 2) / (128 * kGtPlaces);      // (a negative pixel may be 510 below it)
 
 #pragma unroll
   for (int turn = 0; turn < kBTurns; ++turn) {     // one 16-byte row: 8 input columns of one accumulator column
@@ -240,7 +258,8 @@ k_grad_tc(const float* images, const unsigned* labels, long n, int per_cta, cons
 #pragma unroll
     for (int d = 0; d < 5; ++d) w[d] = w_scale * bw[turn][d];
     __half2 hi[4], lo[4];
-    constexpr double kFactor = (double)kPre / 255.0;            // in two parts, so that the factor costs the weights no bit
+    // In two parts, so that the factor costs the weights no bit.  (A byte / 255 in fp32 is 2.37e-8 of itself too large on average: the pixels are bytes.)
+    constexpr double kFactor = (double)kPre / 255.0 * (1.0 + 2.37e-8);
     constexpr float kFactorHi = (float)kFactor, kFactorLo = (float)(kFactor - (double)kFactorHi);
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
@@ -268,8 +287,16 @@ k_grad_tc(const float* images, const unsigned* labels, long n, int per_cta, cons
     const int t = tid - 256;
     if (t < 16) sm.ws[t] = small;
     else if (t < 28) sm.bf[t - 16] = (t - 16 < kOut) ? small : 0.f;
-    else if (t < 28 + kF) sm.bc[t - 28] = kPre * small;
     else if (t == 40) sm.bs[0] = small;
+  }
+  if (warp < kF) {               // a map's bias, and what the level adds to its pre-activations
+    float sum = 0.f;
+#pragma unroll
+    for (int j = 0; j < 5; ++j) sum += (lane + 32 * j) / 25 == warp ? taps[j] : 0.f;
+#pragma unroll
+    for (int m = 16; m > 0; m >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, m);
+    const float bias = __shfl_sync(0xffffffffu, taps[4], kOffBc - 128 + warp);
+    if (lane == 0) sm.bc[warp] = kPre * fmaf((float)level / 255.f, sum, bias);
   }
   tc::fence_async_smem();      // the operands were written through the generic proxy
   tc::fence_before_sync();
@@ -438,6 +465,7 @@ k_grad_tc(const float* images, const unsigned* labels, long n, int per_cta, cons
       dst[j] |= i < kGtPieces ? (swap ? before | own << 2 : own | before << 2) << 16 : 0u;
     }
     const __half2 px_scale = __float2half2_rn(__int_as_float((127 + wexp - 3) << 23)), magic = __float2half2_rn(1536.f);
+    const __half2 minus_level = __float2half2_rn(-(float)level * __int_as_float((127 + wexp - 3) << 23));
     const f32x2 k255 = pack2(255.f, 255.f);
     f32x2 sum[kGtGradN / 2];
 #pragma unroll
@@ -495,7 +523,7 @@ k_grad_tc(const float* images, const unsigned* labels, long n, int per_cta, cons
             const __half2 p = __floats2half2_rn(x[2 * c], x[2 * c + 1]);
             const __half2 w = __hsub2(__hadd2(p, magic), magic);      // whole numbers below 512 as they are
             odd |= *reinterpret_cast<const unsigned*>(&p) ^ *reinterpret_cast<const unsigned*>(&w);
-            const __half2 q = __hmul2(p, px_scale);
+            const __half2 q = __hfma2(p, px_scale, minus_level);
             h[c] = *reinterpret_cast<const unsigned*>(&q);
           }
           const unsigned to = lt + kGtLoaders * (j0 + j) < pieces ? dst[j0 + j] : 0u, own = slab + (to & 0xffffu);
@@ -836,7 +864,10 @@ k_grad_tc(const float* images, const unsigned* labels, long n, int per_cta, cons
     for (int part = 0; part < 2; ++part)
 #pragma unroll
       for (int x = 0; x < 4; ++x) s[part] += end.d[24 * part + 8 * (f >> 1) + 2 * x + (f & 1)][8 * i + x + j];
-    row[kOffWc + tid] = (s[1] - s[0]) * __int_as_float((127 + 3 - wexp) << 23) / (255.f * kC * kC);
+    float b = 0.f;
+#pragma unroll
+    for (int w = 0; w < 12; ++w) b += end.bc[w][f];
+    row[kOffWc + tid] = (s[1] - s[0]) * __int_as_float((127 + 3 - wexp) << 23) / (255.f * kC * kC) + (float)level / 255.f * (b / (float)(kC * kC));
   } else if (tid < kOffWs) {
     float s = 0.f;
 #pragma unroll

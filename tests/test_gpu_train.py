@@ -403,6 +403,34 @@ def test_tensor_core_gradient_leaves_other_pixels(cuda, pkg, params0, what, wher
         assert abs(out[1][2344] - out[0][2344]) < 1e-5 * out[0][2344]
 
 
+@pytest.mark.parametrize("n", [5, 743])
+@pytest.mark.parametrize("what", ["bright", "white", "inverted", "both"])
+def test_tensor_core_gradient_of_dense_bright_images(cuda, pkg, what, n):
+    """Bytes of 200 to 255, of 254 and 255, inverted strokes, and strokes of which every second image is inverted, with deltas of one sign: sums
+    of 720 products that all add up, which the tensor core must not truncate (2^-23 for each of 48 additions, half of it on average, half of the
+    sum on average: 1.4e-6).  Yardstick: the CUDA-core path, which shares the activations' approximations; what is left are fp32 roundings of
+    a delta, its parts, the bias and the sums, five of 2^-24 on either side."""
+    rng = np.random.default_rng(7)
+    images, labels = pkg.synth.synth_images(65, n)
+    pixels = np.rint(images * 255)
+    if what == "bright":
+        pixels = rng.integers(200, 256, pixels.shape)
+    elif what == "white":
+        pixels = rng.integers(254, 256, pixels.shape)
+    elif what == "inverted":
+        pixels = 255 - pixels
+    else:
+        pixels[::2] = 255 - pixels[::2]
+    images = (pixels / 255).astype(np.float32)
+    for seed in range(3):
+        params = pkg.Net(seed).get_params()
+        params[173:2333] = 0.02 * (1 + 0.3 * rng.random(2160))
+        params[156:172] = 0.3 + 0.2 * rng.random(16)
+        out = both_paths(cuda, pkg, params, images, labels)
+        for name, (lo, hi) in BLOCKS.items():
+            assert scaled_err(out[1][lo:hi], out[0][lo:hi].astype(np.float64)) < 10 * 2.0**-24, name
+
+
 @pytest.mark.parametrize("what", ["tiny conv weights", "large conv weights", "huge conv weights", "infinite bias", "not a number", "large rest",
                                   "no subsample filter"])
 def test_tensor_core_gradient_parameter_range(cuda, pkg, params0, what):
