@@ -189,10 +189,10 @@ __device__ __forceinline__ int scatter8_index(int lane) { return ((lane >> 4) & 
 // The gradient of a team's images stays in registers (26 pairs of conv taps and bias, five pairs of FC weights, eight
 // subsample taps) until the block's reduction at the end (shuffles and shared memory, fixed order, no atomics).
 //
-// Batches of up to 2,047 images, and what grad_tc.cu leaves.  Small batches are a chain of latencies, large ones are bound by the FMA pipe (852 cycles
+// Batches of up to 2,047 images; k_grad_left below does what grad_tc.cu leaves.  Small batches are a chain of latencies, large ones are bound by the FMA pipe (852 cycles
 // of it per warp and image; 318 us for 60,000 images).  Measured: a step of 256 images in a training loop 15.4 -> 8.8 us (of which the
 // parameters 0.7, forward 1.9, backward 1.5, this kernel's reduction 1.2, the row sums 1.2 and the two hand-overs 1.5 us),
-// the gradient of 60,000 images 1,030 -> 645 us.  (Before: a thread per window and map, scalar, two blocks of seven warps per SM at 128 registers
+// the gradient of 60,000 images 1,030 -> 643 us.  (Before: a thread per window and map, scalar, two blocks of seven warps per SM at 128 registers
 // with the patch and all gradient terms in registers, two barriers per image, a row per image up to 296; then, until 9.5 us, taps from shared
 // memory for every image and patch loads that took two turns each.)
 // ----------------------------------------------------------------------------------------------
@@ -200,8 +200,6 @@ constexpr int kGrThreads = 224;                 // threads of a team: 216 with w
 constexpr int kGrWarps = kGrThreads / 32;
 constexpr int kGrStages = 3;                    // image buffers of a team
 constexpr int kGrRed = 27;                      // pairs per thread in the reduction: 25 taps + bias, padded to an odd number
-
-constexpr int kGrShares = 256;                  // most blocks that may have left images (LEFT)
 
 template <int TEAMS>
 struct GrSmem {
@@ -217,7 +215,6 @@ struct GrSmem {
   float red_f[kS][kOut];                        // two teams: FC gradient of the second
   float red_b[TEAMS][12];                       // FC bias gradient and error sum of a team
   unsigned long long full[TEAMS][kGrStages];
-  int before[kGrShares + 1];                    // LEFT only: images left in the shares before this one
 };
 
 // Barrier of one team's threads.
@@ -227,98 +224,58 @@ __device__ __forceinline__ void team_sync(int team) {
   else asm volatile("bar.sync %0, %1;" ::"r"(team + 1), "n"(kGrThreads) : "memory");
 }
 
-// LEFT: the images that the tensor-core kernel (grad_tc.cu) has left, the last left[b] of each share b of per_cta images; no rows are
-// written if there are none.
-// ONCE: no team has more than one image (one team never has).  Then the gradient's registers are free during the forward pass and hold the taps (which two teams
-// otherwise read from shared memory as they go: a quarter of a small batch's shared-memory cycles).
-template <int FAST, int TEAMS, bool ONCE, bool LEFT = false>
-__global__ void __launch_bounds__(kGrThreads * TEAMS, 1)
-k_grad_partials(const float* images, const unsigned* labels, long n,
-                const float* params, float* __restrict__ rows, int* __restrict__ status, int chained,
-                const int* left, int shares, int per_cta) {
-  extern __shared__ __align__(128) unsigned char smem_raw[];
-  GrSmem<TEAMS>& sm = *reinterpret_cast<GrSmem<TEAMS>*>(smem_raw);
-  const int team = TEAMS == 1 ? 0 : threadIdx.x / kGrThreads;
-  const int tid = threadIdx.x - team * kGrThreads, warp = tid >> 5, lane = threadIdx.x & 31;
-  constexpr float kPre = (FAST == 1) ? -1.4426950408889634f : 1.0f;   // the short sigmoid form's factor, folded into the conv weights
+// The images of one team, by turn.  Those of a batch go round the teams of all blocks.
+struct BatchImages {
+  const float* images;
+  const unsigned* labels;
+  long n, first, step;
+  __device__ bool has(int i) const { return first + i * step < n; }
+  __device__ long number(int i) const { return first + i * step; }
+};
+// What the tensor-core kernel has left of a share (`images` and `labels` are the share's): listed images of the tiles that it left out, then those from `from` on.
+template <int TEAMS>
+struct LeftImages {
+  const float* images;
+  const unsigned* labels;
+  int n, team, listed, from;
+  const int* tile;
+  __device__ bool has(int i) const { return team + i * TEAMS < n; }
+  __device__ long number(int i) const {
+    const int im = team + i * TEAMS;
+    if (listed == 0) return from + im;
+    return im < listed ? kGradTile * tile[im / kGradTile] + im % kGradTile : from + (im - listed);
+  }
+};
 
-  // Number of the im-th image, one of share `share` or a later one.
-  const long n_all = n;
-  auto at = [&](long im, [[maybe_unused]] int& share) -> long {
-    while (im >= sm.before[share + 1]) ++share;
-    const long end = (long)(share + 1) * per_cta < n_all ? (long)(share + 1) * per_cta : n_all;
-    return end - sm.before[share + 1] + im;
-  };
-  [[maybe_unused]] int share_copied = 0, share_read = 0;
-  const bool live = tid < kS;
-  const int half = tid & 1, unit = (live ? tid : 0) >> 1;      // (the eight idle threads shadow thread 0 and add zeros)
-  // Eight neighbouring threads, four windows, read 16 bytes each of rows of seven at a time: (4 p + 6 half + q) mod 8 is the bank group.  Of
-  // twelve windows (two rows) four with columns 0, 1, 4, 5 of the first row, four of the second, and columns 2, 3 of both ask eight different ones
-  // (in the windows' own order every load took two turns: a third of this kernel's shared-memory cycles).
-  const int pr = unit / 36, twelve = unit % 36 / 12, quad = unit % 12 / 4, in_quad = unit % 4;
-  const int p = 2 * twelve + (quad < 2 ? quad : in_quad >> 1), q = quad < 2 ? in_quad + (in_quad & 2) : 2 + (in_quad & 1);
-  const int w = 6 * p + q;
-  const int patch_at = (4 * p + 2 * half) * kH + 4 * q;
-  // Image i of this team is first + i * step.
-  const long first = (long)blockIdx.x + (long)team * gridDim.x, step = (long)TEAMS * gridDim.x;
-  auto issue = [&](int i, auto mapped) {
-    long im = first + (long)i * step;
-    if (im >= n) return;
-    if constexpr (decltype(mapped)::value) im = at(im, share_copied);
-    unsigned long long* bar = &sm.full[team][i % kGrStages];
-    mbar_expect_tx(bar, kImg * sizeof(float));
-    bulk_g2s(&sm.img[team][i % kGrStages][0], images + im * kImg, kImg * sizeof(float), bar);
-  };
-  if (chained) pdl_launch_dependents();
-  if (tid == 0) {
-    for (int s = 0; s < kGrStages; ++s) mbar_init(&sm.full[team][s], 1);
-    mbar_fence_init();
-    // In a training loop the kernel before this one is the previous step's reduce + update kernel, which does not touch
-    // the images: their copies may leave while it still runs.  Whatever wrote the images is complete by then, because the loop's
-    // first gradient kernel (the one that is not chained) lets its successors start only behind its own wait; kernels that
-    // triggered before their waits could otherwise all start while the writer still runs.
-    if (chained)
-      for (int i = 0; i < kGrStages; ++i) issue(i, std::false_type());
-  }
-  pdl_wait();      // the parameters (and the row buffer this kernel writes at its end) belong to the predecessor until here
-  if (!chained) pdl_launch_dependents();
-  if constexpr (LEFT) {
-    const int mine = (int)threadIdx.x < shares ? left[threadIdx.x] : 0;
-    if ((int)threadIdx.x < shares) sm.before[threadIdx.x + 1] = mine;
-    if (!__syncthreads_or(mine)) return;
-    if (threadIdx.x < 32) {        // running sums, kGrShares / 32 shares per lane
-      int upto[kGrShares / 32], sum = 0;
-#pragma unroll
-      for (int i = 0; i < kGrShares / 32; ++i) {
-        const int b = lane * (kGrShares / 32) + i;
-        sum += b < shares ? sm.before[b + 1] : 0;
-        upto[i] = sum;
-      }
-      int ahead = sum;
-#pragma unroll
-      for (int m = 1; m < 32; m <<= 1) {
-        const int v = __shfl_up_sync(0xffffffffu, ahead, m);
-        if (lane >= m) ahead += v;
-      }
-      ahead -= sum;
-#pragma unroll
-      for (int i = 0; i < kGrShares / 32; ++i) sm.before[lane * (kGrShares / 32) + i + 1] = ahead + upto[i];
-      if (lane == 0) sm.before[0] = 0;
-    }
-    __syncthreads();
-    n = sm.before[shares];
-  }
-  if (tid == 0 && !chained)
-    for (int i = 0; i < kGrStages; ++i) issue(i, std::integral_constant<bool, LEFT>());
-  // Parameters: every load of a thread is under way before the first of them is stored (one L2 latency, not one per
-  // group of loads: 2.4 -> 0.75 us of a step).
-  {
-    float wf[kOut / TEAMS], small;
+template <int TEAMS, class Images>
+__device__ __forceinline__ void copy_image(GrSmem<TEAMS>& sm, int team, const Images& src, int i) {
+  if (!src.has(i)) return;
+  unsigned long long* bar = &sm.full[team][i % kGrStages];
+  mbar_expect_tx(bar, kImg * sizeof(float));
+  bulk_g2s(&sm.img[team][i % kGrStages][0], src.images + src.number(i) * kImg, kImg * sizeof(float), bar);
+}
+
+template <int TEAMS>
+__device__ __forceinline__ void init_image_barriers(GrSmem<TEAMS>& sm, int team) {
+  for (int s = 0; s < kGrStages; ++s) mbar_init(&sm.full[team][s], 1);
+  mbar_fence_init();
+}
+
+// A thread's share of the parameters: every load is under way before the first of them is stored (one L2 latency, not one per
+// group of loads: 2.4 -> 0.75 us of a step).
+template <int FAST, int TEAMS>
+struct ParamShare {
+  float wf[kOut / TEAMS], small;
+  __device__ __forceinline__ void load(const float* params, int team, int tid) {
     const int k0 = team * (kOut / TEAMS);
 #pragma unroll
-    for (int k = 0; k < kOut / TEAMS; ++k) wf[k] = params[kOffWf + (k0 + k) * kS + (live ? tid : 0)];
+    for (int k = 0; k < kOut / TEAMS; ++k) wf[k] = params[kOffWf + (k0 + k) * kS + (tid < kS ? tid : 0)];
     if (team == 0) small = params[tid < kOffWf ? tid : kOffBf + (tid - kOffWf < kOut ? tid - kOffWf : 0)];
-    if (live) {
+  }
+  __device__ __forceinline__ void store(GrSmem<TEAMS>& sm, int team, int tid) const {
+    constexpr float kPre = (FAST == 1) ? -1.4426950408889634f : 1.0f;   // the short sigmoid form's factor, folded into the conv weights
+    const int k0 = team * (kOut / TEAMS);
+    if (tid < kS) {
 #pragma unroll
       for (int k = 0; k < kOut / TEAMS; ++k) sm.wf[k0 + k][tid % 36][tid / 36] = wf[k];
     }
@@ -330,7 +287,23 @@ k_grad_partials(const float* images, const unsigned* labels, long n,
       else if (tid < kOffWf + kOut) sm.bf[tid - kOffWf] = small;
     }
   }
-  __syncthreads();
+};
+
+// Gradient of both teams' images (the first kGrStages of each are on their way) into the block's row, or added to what is there.
+// ONCE: no team has more than one image (one team never has).  Then the gradient's registers are free during the forward pass and hold the taps (which two teams
+// otherwise read from shared memory as they go: a quarter of a small batch's shared-memory cycles).
+template <int FAST, int TEAMS, bool ONCE, class Images>
+__device__ __forceinline__ void grad_images(GrSmem<TEAMS>& sm, const Images& src, int team, int tid, float* row, bool add, int* status) {
+  const int warp = tid >> 5, lane = threadIdx.x & 31;
+  const bool live = tid < kS;
+  const int half = tid & 1, unit = (live ? tid : 0) >> 1;      // (the eight idle threads shadow thread 0 and add zeros)
+  // Eight neighbouring threads, four windows, read 16 bytes each of rows of seven at a time: (4 p + 6 half + q) mod 8 is the bank group.  Of
+  // twelve windows (two rows) four with columns 0, 1, 4, 5 of the first row, four of the second, and columns 2, 3 of both ask eight different ones
+  // (in the windows' own order every load took two turns: a third of this kernel's shared-memory cycles).
+  const int pr = unit / 36, twelve = unit % 36 / 12, quad = unit % 12 / 4, in_quad = unit % 4;
+  const int p = 2 * twelve + (quad < 2 ? quad : in_quad >> 1), q = quad < 2 ? in_quad + (in_quad & 2) : 2 + (in_quad & 1);
+  const int w = 6 * p + q;
+  const int patch_at = (4 * p + 2 * half) * kH + 4 * q;
 
   f32x2 wt[ONCE ? 25 : 1];
   if (ONCE) {
@@ -350,14 +323,9 @@ k_grad_partials(const float* images, const unsigned* labels, long n,
   const float inv_c = 1.0f / (float)(kC * kC);
 
   bool gave_up = false;
-  auto run = [&](auto mapped) {
-  int it = 0;
-  for (long im = first; im < n; im += step, ++it) {
+  for (int it = 0; src.has(it); ++it) {
     unsigned label = 0;
-    if (lane < kOut) {
-      if constexpr (decltype(mapped)::value) label = labels[at(im, share_read)];
-      else label = labels[im];
-    }
+    if (lane < kOut) label = src.labels[src.number(it)];
     mbar_wait_bounded(&sm.full[team][it % kGrStages], (unsigned)(it / kGrStages) & 1u, status, gave_up);
     const float* patch = &sm.img[team][it % kGrStages][0] + patch_at;
 
@@ -421,7 +389,7 @@ k_grad_partials(const float* images, const unsigned* labels, long n,
     const int idx = scatter8_index(lane);
     if ((lane & 2) == 0 && idx < 5) part[warp][6 * half + idx] = mine;
     team_sync<TEAMS>(team);       // the team's sums are in shared memory; every thread is done with the previous image
-    if (!ONCE && tid == 0 && it > 0) issue(it + kGrStages - 1, mapped);
+    if (!ONCE && tid == 0 && it > 0) copy_image(sm, team, src, it + kGrStages - 1);
 
     // ---- output layer on lanes 0..9 of every warp -------------------------------------------------
     float delta = 0.f;
@@ -485,17 +453,9 @@ k_grad_partials(const float* images, const unsigned* labels, long n,
     }
     if (ONCE) break;
   }
-  };
-  // (Where all images are left, as a rule because none has whole numbers / 255 as pixels, there is nothing to look up: 7 % less.)
-  if constexpr (LEFT) {
-    if (n < n_all) run(std::true_type());
-    else run(std::false_type());
-  } else {
-    run(std::false_type());
-  }
 
   // ---- block-level reduction, fixed order ----------------------------------------------------
-  float* row = rows + (size_t)blockIdx.x * kRowStride;
+  auto put = [&](float* dst, float v) { *dst = add ? *dst + v : v; };
   if (live) {
 #pragma unroll
     for (int t = 0; t < 26; ++t) sm.red[team * kS + tid][t] = g[t];
@@ -521,8 +481,8 @@ k_grad_partials(const float* images, const unsigned* labels, long n,
       unpack2(gf[j], f0, f1);
       if (TEAMS == 2) { f0 += sm.red_f[tid][2 * j]; f1 += sm.red_f[tid][2 * j + 1]; }
       float* dst = row + kOffWf + (5 * half + j) * kS + 2 * pr * 36 + w;
-      dst[0] = f0;
-      dst[36] = f1;
+      put(dst, f0);
+      put(dst + 36, f1);
     }
   }
   // conv taps and biases: 78 pair columns, 2 TEAMS neighbouring threads each, 36 rows per thread
@@ -549,23 +509,108 @@ k_grad_partials(const float* images, const unsigned* labels, long n,
     }
     if (part == 0) {
       float* dst = t < 25 ? row + kOffWc + 2 * cp * 25 + t : row + kOffBc + 2 * cp;
-      dst[0] = lo;
-      dst[t < 25 ? 25 : 1] = hi;
+      put(dst, lo);
+      put(dst + (t < 25 ? 25 : 1), hi);
     }
   } else if (threadIdx.x >= kGrThreads * TEAMS - 32) {      // the last warp: subsample filter and bias, FC biases, error sum, padding
     if (lane < 17) {
       float sum = 0.f;
 #pragma unroll
       for (int ww = 0; ww < TEAMS * kGrWarps; ++ww) sum += sm.red_s[ww][lane];
-      row[lane < 16 ? kOffWs + lane : kOffBs] = sum;
+      put(row + (lane < 16 ? kOffWs + lane : kOffBs), sum);
     } else if (lane < 28) {
       const float sum = TEAMS == 2 ? sm.red_b[0][lane - 17] + sm.red_b[1][lane - 17] : sm.red_b[0][lane - 17];
-      row[lane < 27 ? kOffBf + lane - 17 : kRowErr] = sum;
+      put(row + (lane < 27 ? kOffBf + lane - 17 : kRowErr), sum);
     }
     // zero the padding so that reductions and collectives over the padded row stay finite
     for (int i = kNParams + lane; i < kRowStride; i += 32)
       if (i != kRowErr) row[i] = 0.f;
   }
+}
+
+// The looping kernel gets 128 registers, what 512 threads would have: with the 144 that it could get it is slower (2,048 images 30.1 us instead of 29.0;
+// with 120 and fewer what is spilled costs more, 60,000 images 652 us and up instead of 643).
+template <int FAST, int TEAMS, bool ONCE>
+__global__ void __launch_bounds__(ONCE ? kGrThreads * TEAMS : 512, 1)
+k_grad_partials(const float* images, const unsigned* labels, long n,
+                const float* params, float* __restrict__ rows, int* __restrict__ status, int chained) {
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  GrSmem<TEAMS>& sm = *reinterpret_cast<GrSmem<TEAMS>*>(smem_raw);
+  const int team = TEAMS == 1 ? 0 : threadIdx.x / kGrThreads, tid = threadIdx.x - team * kGrThreads;
+  const BatchImages src = {images, labels, n, (long)blockIdx.x + (long)team * gridDim.x, (long)TEAMS * gridDim.x};
+  if (chained) pdl_launch_dependents();
+  if (tid == 0) {
+    init_image_barriers(sm, team);
+    // In a training loop the kernel before this one is the previous step's reduce + update kernel, which does not touch
+    // the images: their copies may leave while it still runs.  Whatever wrote the images is complete by then, because the loop's
+    // first gradient kernel (the one that is not chained) lets its successors start only behind its own wait; kernels that
+    // triggered before their waits could otherwise all start while the writer still runs.
+    if (chained)
+      for (int i = 0; i < kGrStages; ++i) copy_image(sm, team, src, i);
+  }
+  pdl_wait();      // the parameters (and the row buffer this kernel writes at its end) belong to the predecessor until here
+  if (!chained) pdl_launch_dependents();
+  if (tid == 0 && !chained)
+    for (int i = 0; i < kGrStages; ++i) copy_image(sm, team, src, i);
+  ParamShare<FAST, TEAMS> share;
+  share.load(params, team, tid);
+  share.store(sm, team, tid);
+  __syncthreads();
+  grad_images<FAST, TEAMS, ONCE>(sm, src, team, tid, rows + (size_t)blockIdx.x * kRowStride, false, status);
+}
+
+// What the tensor-core kernel (grad_tc.cu) has left, added to the rows that it wrote.  A block takes the share that is next in the queue of those with
+// something left, as a rule before that kernel is complete (an SM is free for this block because one of its blocks has finished), else, and for good if there
+// is none, when it is.  So shares that are left as a whole are under way beside the others' tiles, and a batch without a byte image takes 4 us longer than
+// on k_grad_partials (7 to 23 us when this kernel waited for the other's end and wrote rows of its own).  Parameters and images may be read before the wait: the kernel before this
+// one writes neither, and lets this one start only when whatever did is complete.
+template <int FAST>
+__global__ void __launch_bounds__(512, 1)
+k_grad_left(const float* images, const unsigned* labels, GradShares shares,
+            const float* params, float* __restrict__ rows, int* __restrict__ status, GradLeft* left, int* pushed) {
+  constexpr int TEAMS = 2;
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  GrSmem<TEAMS>& sm = *reinterpret_cast<GrSmem<TEAMS>*>(smem_raw);
+  __shared__ int next;
+  const int team = threadIdx.x / kGrThreads, tid = threadIdx.x - team * kGrThreads;
+  ParamShare<FAST, TEAMS> share;
+  share.load(params, team, tid);
+  if (tid == 0) init_image_barriers(sm, team);
+  auto take = [&] {
+    if (threadIdx.x == 0) {
+      int b;
+      asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(b) : "l"(&left[blockIdx.x].next) : "memory");
+      next = b;
+    }
+    __syncthreads();
+    return next - 1;
+  };
+  int b = take();
+  if (b < 0) {
+    pdl_wait();
+    __syncthreads();      // (everybody has looked)
+    b = take();
+  }
+  pdl_launch_dependents();
+  if (b >= 0) {
+    const long img0 = shares.first(b);
+    const GradLeft& mine = left[b];
+    const int imgs = shares.size(b), skips = mine.skips, from = mine.from;
+    int listed = 0;
+    if (skips > 0) {
+      const int last = kGradTile * (mine.tile[skips - 1] + 1);      // (the share's last tile may be short)
+      listed = kGradTile * skips - (last > imgs ? last - imgs : 0);
+    }
+    const LeftImages<TEAMS> src = {images + img0 * kImg, labels + img0, listed + imgs - from, team, listed, from, mine.tile};
+    if (tid == 0)
+      for (int i = 0; i < kGrStages; ++i) copy_image(sm, team, src, i);
+    share.store(sm, team, tid);
+    __syncthreads();
+    grad_images<FAST, TEAMS, false>(sm, src, team, tid, rows + (size_t)b * kRowStride, mine.written != 0, status);
+    if (threadIdx.x == 0) left[blockIdx.x].next = 0;
+    pdl_wait();
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) *pushed = 0;      // behind the wait: all blocks have pushed what they push
 }
 
 // G[i] = sum over rows (fixed order: thirty-two interleaved row groups, then a fixed tree over the
@@ -574,18 +619,14 @@ k_grad_partials(const float* images, const unsigned* labels, long n,
 // (The data-parallel exchange kernel adds a rank's rows in exactly this order.)
 constexpr int kRedGroups = 32;
 
-// LEFT: `left` says how many images each of the n_rows blocks has left (grad_tc.cu); if any has, `more` rows follow.  (A variant of its own: looking
-// at a null pointer costs a training step 0.1 us.)
-template <bool LEFT>
 __global__ void __launch_bounds__(32 * kRedGroups)
 k_reduce_rows(const float* rows, int n_rows, float* __restrict__ G,
-              float* __restrict__ params, float scale, float* __restrict__ mean_err, float err_scale, const int* left, int more) {
+              float* __restrict__ params, float scale, float* __restrict__ mean_err, float err_scale) {
   __shared__ float part[kRedGroups][33];
   const int lane = threadIdx.x & 31, g = threadIdx.x >> 5;
   const int col = blockIdx.x * 32 + lane;
   pdl_launch_dependents();   // the next step's gradient kernel may set itself up now
   pdl_wait();                // the rows are complete
-  if (LEFT && __syncthreads_or((int)threadIdx.x < n_rows && left[threadIdx.x] != 0)) n_rows += more;
   float acc = 0.f, p_old = 0.f;
   if (col < kRowStride) {
     if (params && g == 0 && col < kNParams) p_old = params[col];      // under the row loads
@@ -776,7 +817,7 @@ static int launch_grad(const float* d_params, float* rows, int* status, int fast
   do {                                                                                                       \
     if ((rc = set_smem_attr(k_grad_partials<FL, TEAMS, ONCE>, CNN_GRAD_SMEM(TEAMS))) != CNN_OK) return rc;     \
     le = launch_pdl(k_grad_partials<FL, TEAMS, ONCE>, dim3(grid), dim3(kGrThreads * TEAMS), CNN_GRAD_SMEM(TEAMS), st, \
-                    d_images, d_labels, n, d_params, rows, status, chained ? 1 : 0, (const int*)nullptr, 0, 0); \
+                    d_images, d_labels, n, d_params, rows, status, chained ? 1 : 0); \
   } while (0)
   if (n <= grid) {
     if (fast) CNN_LAUNCH_GRAD(1, 1, true);
@@ -800,39 +841,34 @@ int launch_grad_partials(cnn_net* net, const float* d_images, const unsigned* d_
   return launch_grad(net->d_params, net->d_partials, net->d_status, net->fast_sigmoid, d_images, d_labels, n, grid, st, chained);
 }
 
-// Rows of the gradient of n images, and what the kernel that adds them needs to know.
-struct GradRows {
-  int rows = 0, more = 0;
-  const int* left = nullptr;
-};
-
-// Tensor cores or CUDA cores.  Microseconds per gradient call, CUDA cores / tensor cores, back to back (alone behind a flush of L2: the same
-// differences, both 9 us longer): 1,480 images (two tiles per SM) 23.4 / 21.1, 2,000 30.0 / 24.2, 3,000 41.5 / 31.1,
-// 6,000 72.9 / 44.2, 20,000 220 / 107, 60,000 643 / 290.  They meet at about 1,300; the line leaves room for images that turn out not to be
-// whole numbers / 255 and go to the CUDA cores behind a look at the first tiles: 2,000 images 37, 6,000 79, 60,000 666.
-static int launch_gradient(cnn_net* net, const float* d_images, const unsigned* d_labels, long n, cudaStream_t st, bool chained, GradRows* out) {
+// Tensor cores or CUDA cores.  Microseconds per gradient call, CUDA cores / tensor cores, back to back: 740 images 14.6 / 17.6, 1,000 18.0 / 20.7,
+// 1,250 21.6 / 20.8, 1,480 (two tiles per SM) 22.6 / 20.8, 2,000 28.9 / 24.1, 3,000 40.2 / 30.4, 6,000 71.8 / 43.5, 20,000 220 / 106, 60,000 643 / 281.
+// They meet at about 1,250; the line leaves room for images that turn out not to be whole numbers / 255 and go to the CUDA cores behind a
+// look at a sample: 2,048 images 33.2 (29.0 without the look), 6,000 76 (72), 60,000 652 (643).  With other pixels in one image of a hundred 60,000
+// images are 367 us, with other pixels in the second half of them 678.
+static int launch_gradient(cnn_net* net, const float* d_images, const unsigned* d_labels, long n, cudaStream_t st, bool chained, int* rows) {
   constexpr long kTcGradMin = 2048;
   const int sms = sm_count();
   const bool tensor = net->grad_path == 1 || (net->grad_path < 0 && n >= kTcGradMin);
-  if (!tensor || !net->fast_sigmoid || sms > kGrShares || n > (1l << 30)) {
-    out->rows = grid_for_batch(n);
-    return launch_grad_partials(net, d_images, d_labels, n, out->rows, st, chained);
+  if (!tensor || !net->fast_sigmoid || n > (1l << 30)) {
+    *rows = grid_for_batch(n);
+    return launch_grad_partials(net, d_images, d_labels, n, *rows, st, chained);
   }
-  long grid = (n + 4) / 5 < sms ? (n + 4) / 5 : sms;
-  const long per_cta = (n + grid - 1) / grid;
-  grid = (n + per_cta - 1) / per_cta;
-  int* left = reinterpret_cast<int*>(net->d_partials + 2 * (size_t)sms * kRowStride);
-  int rc = launch_grad_tc(net, d_images, d_labels, n, (int)grid, (int)per_cta, left, st);
+  const long grid = (n + kGradTile - 1) / kGradTile < sms ? (n + kGradTile - 1) / kGradTile : sms;
+  const GradShares shares = {(int)grid, (int)(n / grid), (int)(n % grid)};
+  GradLeft* left = reinterpret_cast<GradLeft*>(net->d_partials + (size_t)sms * kRowStride);
+  int* pushed = reinterpret_cast<int*>(left + sms);
+  int rc = set_smem_attr(k_grad_left<1>, sizeof(GrSmem<2>));
+  if (rc == CNN_OK) rc = launch_grad_tc(net, d_images, d_labels, shares, left, pushed, st);
   if (rc != CNN_OK) return rc;
-  // the images that it has left, if any
-  if ((rc = set_smem_attr(k_grad_partials<1, 2, false, true>, sizeof(GrSmem<2>))) != CNN_OK) return rc;
-  cudaError_t e = launch_pdl(k_grad_partials<1, 2, false, true>, dim3(sms), dim3(kGrThreads * 2), sizeof(GrSmem<2>), st, d_images, d_labels, n,
-                             (const float*)net->d_params, net->d_partials + grid * kRowStride, net->d_status, 0, (const int*)left, (int)grid, (int)per_cta);
+  cudaError_t e = launch_pdl(k_grad_left<1>, dim3((unsigned)grid), dim3(kGrThreads * 2), sizeof(GrSmem<2>), st, d_images, d_labels, shares,
+                             (const float*)net->d_params, net->d_partials, net->d_status, left, pushed);
   if (e == cudaSuccess) e = cudaGetLastError();
-  if (e != cudaSuccess) return cuda_fail(e, "k_grad_partials launch");
-  out->rows = (int)grid;
-  out->more = sms;
-  out->left = left;
+  if (e != cudaSuccess) {
+    cudaMemsetAsync(left, 0, sizeof(GradLeft) * sms + sizeof(int), st);      // nobody takes what the kernel before has queued
+    return cuda_fail(e, "k_grad_left launch");
+  }
+  *rows = (int)grid;
   return CNN_OK;
 }
 
@@ -862,10 +898,10 @@ int cnn_grad_batch(cnn_net* net, const float* d_images, const unsigned int* d_la
               "cnn_grad_batch: image batch must start on a 16-byte boundary");
   int rc = ensure_train_scratch(net);
   if (rc != CNN_OK) return rc;
-  GradRows g;
-  if ((rc = launch_gradient(net, d_images, d_labels, n, st, false, &g)) != CNN_OK) return rc;
-  cudaError_t e = launch_pdl(g.left ? k_reduce_rows<true> : k_reduce_rows<false>, dim3((kNParamsPadded + 31) / 32), dim3(32 * kRedGroups), 0, st,
-                             (const float*)net->d_partials, g.rows, d_grad, (float*)nullptr, 0.f, (float*)nullptr, 0.f, g.left, g.more);
+  int rows = 0;
+  if ((rc = launch_gradient(net, d_images, d_labels, n, st, false, &rows)) != CNN_OK) return rc;
+  cudaError_t e = launch_pdl(k_reduce_rows, dim3((kNParamsPadded + 31) / 32), dim3(32 * kRedGroups), 0, st,
+                             (const float*)net->d_partials, rows, d_grad, (float*)nullptr, 0.f, (float*)nullptr, 0.f);
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e, "k_reduce_rows launch");
   return CNN_OK;
@@ -894,11 +930,11 @@ int cnn_train_minibatch(cnn_net* net, const float* d_images, const unsigned int*
   for (int e = 0; e < epochs; ++e) {
     for (long first = 0; first < n; first += batch) {
       const long b = (n - first) < batch ? (n - first) : batch;
-      GradRows g;
-      if ((rc = launch_gradient(net, d_images + first * kImg, d_labels + first, b, st, first > 0 || e > 0, &g)) != CNN_OK) return rc;
-      cudaError_t err = launch_pdl(g.left ? k_reduce_rows<true> : k_reduce_rows<false>, dim3((kNParamsPadded + 31) / 32), dim3(32 * kRedGroups), 0, st,
-                                   (const float*)net->d_partials, g.rows, net->d_grad, net->d_params, dt / (float)b,
-                                   d_mean_err ? d_mean_err + e : nullptr, 1.0f / (float)n, g.left, g.more);
+      int rows = 0;
+      if ((rc = launch_gradient(net, d_images + first * kImg, d_labels + first, b, st, first > 0 || e > 0, &rows)) != CNN_OK) return rc;
+      cudaError_t err = launch_pdl(k_reduce_rows, dim3((kNParamsPadded + 31) / 32), dim3(32 * kRedGroups), 0, st,
+                                   (const float*)net->d_partials, rows, net->d_grad, net->d_params, dt / (float)b,
+                                   d_mean_err ? d_mean_err + e : nullptr, 1.0f / (float)n);
       if (err == cudaSuccess) err = cudaGetLastError();
       if (err != cudaSuccess) return cuda_fail(err, "k_reduce_rows launch");
     }
@@ -1024,8 +1060,8 @@ int cnn_grad_batch_noalloc(const float* d_params, const float* d_images, const u
   // the library is loaded, is only ever set by a wait that ran out, and stays set until
   // cnn_grad_batch_noalloc_status reads and clears it.
   if ((rc = launch_grad(d_params, rows, status, 0, d_images, d_labels, n, grid, st, false)) != CNN_OK) return rc;
-  cudaError_t e = launch_pdl(k_reduce_rows<false>, dim3((kNParamsPadded + 31) / 32), dim3(32 * kRedGroups), 0, st, (const float*)rows, grid,
-                             d_grad, (float*)nullptr, 0.f, (float*)nullptr, 0.f, (const int*)nullptr, 0);
+  cudaError_t e = launch_pdl(k_reduce_rows, dim3((kNParamsPadded + 31) / 32), dim3(32 * kRedGroups), 0, st, (const float*)rows, grid,
+                             d_grad, (float*)nullptr, 0.f, (float*)nullptr, 0.f);
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e, "k_reduce_rows launch (no-alloc)");
   return CNN_OK;

@@ -15,9 +15,9 @@
 //                 (five kernel rows of eight columns).  All six window columns add to one D.  The deltas are the A operand, M-contiguous as the
 //                 epilogue's lanes (rows) have them, the slab is the N-contiguous B operand: a row is 16 bytes, so it may start at any.
 //
-// Accuracy.  Pixels that are whole numbers / 255 (image files' bytes) are exact in fp16 (forward_tc.cu); a CTA stops at the first tile with any
-// other pixel, and images from there on are left to k_grad_partials (fused_train.cu), as are all of them where a parameter is not finite or
-// far out of range.  The tensor core truncates its additions, which over a tile's 48 would cost a gradient 1e-6.  Here they are exact: deltas are
+// Accuracy.  Pixels that are whole numbers / 255 (image files' bytes) are exact in fp16 (forward_tc.cu).  A tile with any other pixel goes through as
+// an empty one, and its images are left to k_grad_partials (fused_train.cu); so is the whole share of a CTA whose sample of pixels has others in several
+// places, what comes behind too many such tiles, and everything where a parameter is not finite or far out of range.  The tensor core truncates its additions, which over a tile's 48 would cost a gradient 1e-6.  Here they are exact: deltas are
 // scaled by a power of two so that the tile's bound on them (max |ds| * max |Ws| / 4) lies in [1024, 2048), and cut into a whole
 // number, at most 11 bits, and the rest, which in fp16 is good to 2^-24 of the bound.  Products of whole numbers with bytes have 19 bits.  A D adds 720 of
 // them: with deltas of one sign and bright pixels up to 2^28, of which truncation took 0.9e-6 on average and 3e-6 at most, always towards zero.  So
@@ -26,8 +26,8 @@
 // and trained, and nets with deltas of one sign, with strokes, inverted strokes, both mixed, noise and smooth bright images, a tile's
 // largest lies between 2^14 and 2^23.5 (without the level up to 2^26.9).
 // D is added to fp32 sums in registers after every tile.  Distance of the gradient from fp64, geometric mean over 12 nets and batches of 2,048,
-// 4,500, 8,000, 20,000 and 60,000 images: 4.90e-8 of its norm (k_grad_partials 4.93e-8), conv weights alone 4.98e-8 (4.83e-8), conv biases 4.77e-8
-// (5.78e-8); nets with deltas of one sign 4.52e-8 (4.51e-8), conv weights 4.79e-8 (4.74e-8).
+// 4,500, 8,000, 20,000 and 60,000 images: 4.94e-8 of its norm (k_grad_partials 4.93e-8), conv weights alone 4.79e-8 (4.83e-8), conv biases 4.8e-8
+// (5.8e-8); nets with deltas of one sign 4.52e-8 (4.51e-8), conv weights 4.93e-8 (4.74e-8).
 //
 // Pipeline (one CTA per SM, 20 warps, mbarriers with bounded waits):
 //   warps 4-7   one bulk copy per tile, two tiles ahead; pixels -> fp16 operand; drain D of the tile that had the slab before;
@@ -38,12 +38,10 @@
 //               deltas.  Stage 2: conv deltas, subsample-filter and bias gradients, delta operand (its whole parts negated: one instruction less);
 //   warps 0-1   FC gradient in registers (a thread owns three or four of the 216 inputs), from what the groups leave in shared memory.
 //
-// Measured on a B200, 60,000 images with the kernels around it: 645 us (k_grad_partials) -> 290 us.  What bounds it, per tile of five images (6,300 cycles):
-// the shared-memory data pipe, 89 % busy (operands of the 78 MMAs 2,590 cycles, other warps 3,020: delta operands 580, FC layer
-// 700, loader 350, conflicts with the tensor core 570); instruction issue 59 %, the special-function unit 37 %.  On the way there: one warp for
-// both kinds of MMA 332 us (it issues in order, and waits for one kind held up the other); four activations per reciprocal in both stages, the exponentials kept
-// instead of the activations, 349 us; the FC layer on three warps of its own 348 us with two thirds of its latency in the groups' way; four
-// operand slabs instead of five 468 us.
+// Measured on a B200, 60,000 images with the kernels around it: 643 us (k_grad_partials) -> 281 us.  What bounds it, per tile of five images (6,200 cycles):
+// the shared-memory data pipe (operands of the 78 MMAs 2,590 cycles, other warps 3,020: delta operands 580, FC layer
+// 700, loader 350, conflicts with the tensor core 570); instruction issue about 60 %, the special-function unit 37 %.  2,048 images are 24.0 us, of which a launch's
+// set-up is 3.2 us.
 #include "cluster_exchange.cuh"
 #include "net.cuh"
 #include "phase_clocks.cuh"
@@ -52,7 +50,7 @@
 namespace cnn {
 
 constexpr int kGtThreads = 640;
-constexpr int kGtImgs = 5;                    // images per tile
+constexpr int kGtImgs = kGradTile;            // images per tile
 constexpr int kGtRaw = 2, kGtSlabs = 5;       // tiles of raw images, and of operands, in shared memory
 constexpr int kGtSets = 3;                    // groups of epilogue warps, and accumulators
 constexpr unsigned kGtGroupStride = 12 * 16;  // a group's twelve rows
@@ -69,8 +67,12 @@ constexpr unsigned kGtDeltaBlock = 128 * 16;                 // [eight columns: 
 constexpr int kGtDeltaBytes = 6 * kGtDeltaBlock;             // three map pairs, high and low parts
 constexpr int kGtGradN = 40, kGtGradCol = kGtSets * 3 * kGtBN;     // D of even and odd tiles behind the accumulators: 432 + 2 * 40 = 512
 constexpr int kGtFcThreads = 64, kGtFcRounds = 4;            // 216 = 3 * 64 + 24
-constexpr int kGtPlaces = 2 * kGtThreads / 32;                // places of the share that are looked at first, 128 pixels each
+// Places of the share that are looked at first, 128 pixels each, and how many with other than whole numbers / 255 leave it to the CUDA cores.  Images of
+// strokes that are all of other numbers show them in half of the places or more (a fifth of a canvas is not zero); where one image in ten has them, a tile's worth
+// of images in ten tiles is still cheaper left out (an empty tile 3.5 us, five images on the CUDA cores 8).
+constexpr int kGtPlaces = 2 * kGtThreads / 32, kGtPlacesOther = 8;
 constexpr int kGtWfStride = 234;              // five rows of weights, 10 (mod 32) words apart, by six parts of nine inputs: thirty banks
+constexpr float kGtUnscale = 1.0f / 8192.0f;                 // of the convolution's accumulators
 constexpr int kGtConvWarp = 2, kGtGradWarp = 3, kGtLoadWarp0 = 4, kGtEpiWarp0 = 8;
 
 struct GtSmem {
@@ -84,11 +86,14 @@ struct GtSmem {
   alignas(16) float df[kGtSets][kGtImgs][12];                // output deltas
   alignas(16) float zeros[36];                               // subsample deltas of the unused group
   float bc[8], ws[16], bs[4], bf[12];
+  float most;                                                // largest pixel that is finite in fp16 with and without level and scale
   unsigned ds_max[kGtSets][4];
   float tile_unscale[kGtSlabs];
   unsigned long long raw_full[kGtRaw], a_full[kGtSlabs], a_free[kGtSlabs], d_full[3 * kGtSets], d_free[3 * kGtSets], df_ready[kGtSets], df_free[kGtSets],
       dl_full[kGtWindows], dl_free[kGtWindows], g_free[2];
   int px_sum[kGtThreads / 32];                               // whole pixels of the sample, by warp
+  int skips, skipped[kGradSkips];                            // tiles left out: how many, and which
+  int empty[kGtSlabs];                                       // the last of them that was in a slab
   int stop;                                                  // tiles that take part
   unsigned tmem_base;
   long long clock_base;                                      // phase clocks only
@@ -136,17 +141,463 @@ __device__ __forceinline__ void store_if(unsigned smem_addr, const unsigned (&v)
 
 __device__ __forceinline__ f32x2 ld2(const float* p) { return *reinterpret_cast<const f32x2*>(p); }
 
-// left[b]: images at the end of block b's share (per_cta images each) that are not in its row.
+// The loaders: tile k has other pixels.  It goes through all the same, with output deltas of zero, if what is in its slab is finite in fp16.
+// Returns how many tiles take part: as many as before, or k where the block stops with this one.
+__device__ __noinline__ int other_tile(GtSmem& sm, int k, int tiles, float big, int lt) {
+  const int skips = sm.skips;
+  if (barrier_any(1, !(big <= sm.most)) || skips == kGradSkips || 2 * skips > k + 4) {
+    if (lt == 0) *const_cast<volatile int*>(&sm.stop) = k;
+    return k;
+  }
+  if (lt == 0) {
+    sm.skipped[skips] = k;
+    *const_cast<volatile int*>(&sm.empty[k % kGtSlabs]) = k;
+    sm.skips = skips + 1;
+  }
+  return tiles;
+}
+
+// One thread: the images of tile k of a share.
+__device__ __forceinline__ void fetch_tile(GtSmem& sm, const float* images, int imgs_here, int k) {
+  const unsigned bytes = (unsigned)(min(kGtImgs, imgs_here - k * kGtImgs) * kImg) * (unsigned)sizeof(float);
+  mbar_expect_tx(&sm.raw_full[k % kGtRaw], bytes);
+  bulk_g2s(sm.raw[k % kGtRaw], images + (long)k * kGtImgs * kImg, bytes, &sm.raw_full[k % kGtRaw]);
+}
+
+// The loaders' part (warps 4-7): tiles to operands, and what the gradient's MMAs have added up.  A function of its own, as run_group is: as parts of the
+// kernel their registers and schedules changed with every line of the set-up (60,000 images 288 to 321 us, as functions 277 to 281).
+__device__ __noinline__ void load_tiles(GtSmem& sm, const float* images, int imgs_here, int n_tiles, int wexp, int level, unsigned tmem_base, int* status) {
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+  bool gave_up = false;
+  CNN_PHASE_ROLE(blockIdx.x == 0, sm.clock_base)
+  const int lt = tid - 32 * kGtLoadWarp0, quarter = warp & 3;
+  // Piece i = lt + 128 j: four pixels (column 4 c) of one row, the second half of chunk c - 1 and the first of chunk c, in one group or two.
+  // Lanes eight apart write the two halves of 16 bytes in opposite order, so that no bank is asked twice: first to `own + at[0]`, then to
+  // `own + at[1]`.  Bits 16 to 19: whether the first place exists, whether a second group has it (64 bytes before), and the same of the second.
+  unsigned dst[kGtUnits];
+  const int swap = (lane >> 3) & 1;
+  const unsigned at[2] = {swap ? 8u - kGtChunk : 0u, swap ? 0u : 8u - kGtChunk};
+#pragma unroll
+  for (int j = 0; j < kGtUnits; ++j) {
+    const int i = lt + kGtLoaders * j, img = i / (kImg / 4), rest = i % (kImg / 4), r = rest / 7, c = rest % 7;
+    const int g = min(r >> 3, 2);
+    dst[j] = (unsigned)(((3 * img + g) * 12 + (r - 8 * g)) * 16) + (unsigned)c * kGtChunk;
+    const unsigned two = g > 0 && r - 8 * g < 4 ? 3u : 1u, own = c < 6 ? two : 0u, before = c > 0 ? two : 0u;
+    dst[j] |= i < kGtPieces ? (swap ? before | own << 2 : own | before << 2) << 16 : 0u;
+  }
+  const __half2 px_scale = __float2half2_rn(__int_as_float((127 + wexp - 3) << 23)), magic = __float2half2_rn(1536.f);
+  const __half2 minus_level = __float2half2_rn(-(float)level * __int_as_float((127 + wexp - 3) << 23));
+  const f32x2 k255 = pack2(255.f, 255.f);
+  f32x2 sum[kGtGradN / 2];
+#pragma unroll
+  for (int i = 0; i < kGtGradN / 2; ++i) sum[i] = pack2(0.f, 0.f);
+  auto drain = [&](int k) {
+    mbar_wait_bounded(&sm.a_free[k % kGtSlabs], (unsigned)(k / kGtSlabs) & 1u, status, gave_up);
+    __syncwarp();
+    if (quarter == 3) return;
+    tc::fence_after_sync();
+    const float f = *const_cast<const volatile float*>(&sm.tile_unscale[k % kGtSlabs]);
+    const f32x2 f2 = pack2(f, f);
+    const unsigned t0 = tmem_base + (unsigned)(kGtGradCol + (k & 1) * kGtGradN) + ((unsigned)(quarter * 32) << 16);
+#pragma unroll
+    for (int c = 0; c < kGtGradN; c += 8) {
+      unsigned v[8];
+      tc::tmem_ld8_nowait(t0 + (unsigned)c, v);
+      tc::tmem_wait8(v);
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        sum[c / 2 + i] = fma2(pack2(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1])), f2, sum[c / 2 + i]);
+    }
+    tc::fence_before_sync();
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&sm.g_free[k & 1]);
+  };
+  int tiles = *const_cast<const volatile int*>(&sm.stop);
+  int k = 0, drained = 0;
+  for (; k < tiles; ++k) {
+    const int s = k % kGtSlabs, r = k % kGtRaw;
+    CNN_PHASE(0);
+    if (k >= kGtSlabs) drain(drained++);
+    CNN_PHASE(1);
+    mbar_wait_bounded(&sm.raw_full[r], (unsigned)(k / kGtRaw) & 1u, status, gave_up);
+    CNN_PHASE(2);
+    const int pieces = min(kGtImgs, imgs_here - k * kGtImgs) * (kImg / 4);
+    const unsigned slab = smem_u32(sm.slab[s]);
+    unsigned bits = 0, odd = 0;
+    float big = 0.f;
+#pragma unroll
+    for (int j0 = 0; j0 < kGtUnits; j0 += 4) {
+      float4 v[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) v[j] = *reinterpret_cast<const float4*>(&sm.raw[r][4 * min(lt + kGtLoaders * (j0 + j), pieces - 1)]);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        float x[4];
+        unpack2(mul2(pack2(v[j].x, v[j].y), k255), x[0], x[1]);
+        unpack2(mul2(pack2(v[j].z, v[j].w), k255), x[2], x[3]);
+        big = max_abs_nan(max_abs_nan(big, x[0], x[1]), x[2], x[3]);
+        bits |= __float_as_uint(x[0]) | __float_as_uint(x[1]) | __float_as_uint(x[2]) | __float_as_uint(x[3]);
+        unsigned h[2];
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          const __half2 p = __floats2half2_rn(x[2 * c], x[2 * c + 1]);
+          const __half2 w = __hsub2(__hadd2(p, magic), magic);      // whole numbers below 512 as they are
+          odd |= *reinterpret_cast<const unsigned*>(&p) ^ *reinterpret_cast<const unsigned*>(&w);
+          const __half2 q = __hfma2(p, px_scale, minus_level);
+          h[c] = *reinterpret_cast<const unsigned*>(&q);
+        }
+        const unsigned to = lt + kGtLoaders * (j0 + j) < pieces ? dst[j0 + j] : 0u, own = slab + (to & 0xffffu);
+#pragma unroll
+        for (int turn = 0; turn < 2; ++turn) {
+          store_if(own + at[turn], h, to & (1u << (16 + 2 * turn)));
+          store_if(own + at[turn] - 64u, h, to & (1u << (17 + 2 * turn)));
+        }
+      }
+    }
+    tc::fence_async_smem();    // generic-proxy writes -> visible to the tensor core's operand reads
+    if (barrier_any(1, (bits & 0x1fffu) != 0 || odd != 0 || !(big <= 255.f))) tiles = other_tile(sm, k, tiles, big, lt);
+    if (lt == 0) {
+      if (k + kGtRaw < n_tiles) fetch_tile(sm, images, imgs_here, k + kGtRaw);
+      mbar_arrive(&sm.a_full[s]);
+    }
+    __syncwarp();
+    CNN_PHASE(3);
+  }
+  // copies that are still on their way land before their memory is used for anything else
+  for (int j = k; j < min(k + kGtRaw, n_tiles); ++j)
+    mbar_wait_bounded(&sm.raw_full[j % kGtRaw], (unsigned)(j / kGtRaw) & 1u, status, gave_up);
+  for (; drained < tiles; ++drained) drain(drained);      // (`tiles` take part, k may be one more)
+  __syncthreads();
+  if (quarter < 3 && lane < 16) {
+    GtEnd& end = *reinterpret_cast<GtEnd*>(sm.raw);
+    float* to = end.d[16 * quarter + lane];
+#pragma unroll
+    for (int i = 0; i < kGtGradN / 2; ++i) unpack2(sum[i], to[2 * i], to[2 * i + 1]);
+  }
+  CNN_PHASE_END(g_phase_clocks_gt);
+}
+
+// The part of a group of epilogue warps (8-19).
+__device__ __noinline__ void run_group(GtSmem& sm, const unsigned* labels, int imgs_here, int n_tiles, float wsmax, unsigned tmem_base, int* status) {
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+  const volatile int& stop = sm.stop;
+  bool gave_up = false;
+  CNN_PHASE_ROLE(blockIdx.x == 0, sm.clock_base)
+  const int set = (warp - kGtEpiWarp0) >> 2;     // accumulator / tile residue this group owns
+  const int quarter = warp & 3;                  // tensor-memory lanes 32 * quarter ..
+  const int rsub = lane & 3;                     // row of the 4x4 window
+  const int g = quarter * 4 + (lane >> 3);       // group of 8 output rows this lane's row belongs to
+  const int img = g / 3, p = 2 * (g % 3) + ((lane >> 2) & 1);      // image of the tile (5: the unused group), window row
+  const bool used = img < kGtImgs;
+  const bool b0 = (lane & 1) != 0, b1 = (lane & 2) != 0;
+  f32x2 bc2[kF / 2], gws[4], gbc[kF / 2];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) gws[j] = pack2(0.f, 0.f);
+#pragma unroll
+  for (int f = 0; f < kF; f += 2) {
+    bc2[f / 2] = pack2(sm.bc[f], sm.bc[f + 1]);
+    gbc[f / 2] = pack2(0.f, 0.f);
+  }
+  const f32x2 unscale2 = pack2(kGtUnscale, kGtUnscale), one2 = pack2(1.f, 1.f);
+  const float bs = sm.bs[0];
+  float* const as_slot = used ? &sm.as[set][img][p * 36] : nullptr;
+  const float* const ds_slot = used ? &sm.ds[set][img][p * 36] : sm.zeros;
+  // FC forward: 54 inputs per warp, lane = nine of them (of six parts) and outputs fk and fk + 5, for all five images
+  const int fk = lane < 30 ? lane % 5 : 4, fpart = lane < 30 ? lane / 5 : 5, first_in = 54 * quarter + 9 * fpart;
+  const int gt = 32 * quarter + lane;            // thread of the group: inputs gt and gt + 128
+  float g_bs = 0.f;
+  const unsigned t0 = tmem_base + (unsigned)(set * 3 * kGtBN) + ((unsigned)(quarter * 32) << 16);
+
+  for (int k = set; k < n_tiles; k += kGtSets) {
+    const unsigned turn = (unsigned)(k / kGtSets) & 1u;
+    bool halt = false;
+    // output layer: quarter 0 images 0-2, quarter 1 images 3-4, lane 10 j + o
+    const int oj = 3 * quarter + lane / 10, oo = lane % 10;
+    const bool outputs = quarter < 2 && lane < (quarter ? 20 : 30);
+    unsigned label = ~0u;
+    if (outputs && k * kGtImgs + oj < imgs_here) label = labels[k * kGtImgs + oj];
+    CNN_PHASE(0);
+    if (k >= kGtSets) mbar_wait_bounded(&sm.df_free[set], turn ^ 1u, status, gave_up);      // this group's tile before this one
+    {
+      f32x2 ws2[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float w = sm.ws[rsub * 4 + j];
+        ws2[j] = pack2(w, w);
+      }
+#pragma unroll 1
+      for (int xb = 0; xb < 3; ++xb) {              // one block of two window columns
+        mbar_wait_bounded(&sm.d_full[3 * set + xb], turn, status, gave_up);
+        if (xb == 0) {
+          halt = barrier_any(2 + set, k >= stop);      // (all of the group, or none)
+          CNN_PHASE(1);
+        }
+        if (halt) break;
+        __syncwarp();
+        tc::fence_after_sync();
+        unsigned nxt[8];
+        tc::tmem_ld8_nowait(t0 + (unsigned)(xb * kGtBN), nxt);
+        tc::tmem_wait8(nxt);
+        float z[12];
+        f32x2 d2[4];               // 1 + 2^t of the row's four columns (of two maps), one step behind
+        // Step ch turns 8 accumulator columns (window column ch / 3, maps 2 * (ch % 3) + {0, 1}) into exponentials and
+        // finishes the columns of step ch - 1, so that two chains of dependent instructions are always under way.
+#pragma unroll
+        for (int ch = 0; ch < 7; ++ch) {
+          f32x2 e2[4];
+          if (ch < 6) {
+            if (ch > 0) tc::tmem_wait8(nxt);
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+              e2[j] = fma2(pack2(__uint_as_float(nxt[2 * j]), __uint_as_float(nxt[2 * j + 1])), unscale2, bc2[ch % 3]);
+            if (ch < 5) tc::tmem_ld8_nowait(t0 + (unsigned)(xb * kGtBN + (ch + 1) * 8), nxt);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              float x, y;
+              unpack2(e2[j], x, y);
+              e2[j] = pack2(exp2f_approx(x), exp2f_approx(y));
+            }
+          }
+          if (ch > 0) {
+            f32x2 z2;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              float x, y;
+              unpack2(d2[j], x, y);
+              d2[j] = pack2(rcp_approx(x), rcp_approx(y));
+              z2 = j == 0 ? mul2(ws2[0], d2[0]) : fma2(ws2[j], d2[j], z2);
+            }
+            tmem_st8(t0 + (unsigned)(xb * kGtBN + (ch - 1) * 8), d2);      // the activations, for stage 2
+            unpack2(z2, z[2 * (ch - 1)], z[2 * (ch - 1) + 1]);
+          }
+          if (ch < 6) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) d2[j] = add2(e2[j], one2);
+          }
+        }
+        // the window's four rows are lanes 4g..4g+3: reduce-scatter the block's 12 sums
+        float w6[6];
+#pragma unroll
+        for (int i = 0; i < 6; ++i) {
+          const float send = b0 ? z[i] : z[i + 6], keep = b0 ? z[i + 6] : z[i];
+          w6[i] = keep + __shfl_xor_sync(0xffffffffu, send, 1);
+        }
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+          const float send = b1 ? w6[i] : w6[i + 3], keep = b1 ? w6[i + 3] : w6[i];
+          const float as = sigmoidf<1>(keep + __shfl_xor_sync(0xffffffffu, send, 2) + bs);
+          if (used) as_slot[12 * xb + (b0 ? 6 : 0) + (b1 ? 3 : 0) + i] = as;
+        }
+      }
+    }
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+    if (halt) {
+      if (lane == 0 && quarter < 2) mbar_arrive(&sm.df_ready[set]);
+      if (k == stop) {        // the gradient warp waits for this tile's first window: its turn, empty
+        const int win = (6 * k) % kGtWindows;
+        if (k >= 2) mbar_wait_bounded(&sm.a_free[(k - 2) % kGtSlabs], (unsigned)((k - 2) / kGtSlabs) & 1u, status, gave_up);
+        mbar_wait_bounded(&sm.dl_free[win], ((unsigned)(6 * k / kGtWindows) & 1u) ^ 1u, status, gave_up);
+        if (lane == 0) mbar_arrive(&sm.dl_full[win]);
+      }
+      break;
+    }
+    CNN_PHASE(2);
+    // ---- the output layer, its error, and the subsample deltas, by the group's 128 threads ----
+    group_sync(set);
+    {
+      const float *as = &sm.as[set][0][first_in], *w0 = &sm.wf[fk][first_in], *w1 = &sm.wf[fk + 5][first_in];
+      f32x2 z[kGtImgs];
+#pragma unroll
+      for (int jj = 0; jj < kGtImgs; ++jj) z[jj] = pack2(0.f, 0.f);
+#pragma unroll
+      for (int i = 0; i < 9; ++i) {
+        const f32x2 w2 = pack2(w0[i], w1[i]);
+#pragma unroll
+        for (int jj = 0; jj < kGtImgs; ++jj) {
+          const float a = as[jj * kS + i];
+          z[jj] = fma2(w2, pack2(a, a), z[jj]);
+        }
+      }
+      // parts 3-5 to parts 0-2, the twelve sums of the group to shared memory (where the subsample deltas come later)
+      float* part = &sm.ds[set][0][0] + (3 * quarter + fpart) * 50 + fk;
+#pragma unroll
+      for (int jj = 0; jj < kGtImgs; ++jj) {
+        float lo, hi;
+        unpack2(z[jj], lo, hi);
+        lo += __shfl_down_sync(0xffffffffu, lo, 15);
+        hi += __shfl_down_sync(0xffffffffu, hi, 15);
+        if (lane < 15) {
+          part[10 * jj] = lo;
+          part[10 * jj + 5] = hi;
+        }
+      }
+    }
+    CNN_PHASE(9);
+    group_sync(set);
+    CNN_PHASE(10);
+    if (quarter < 2) {
+      if (outputs) {
+        const float* part = &sm.ds[set][0][0] + 10 * oj + oo;
+        float z = 0.f;
+#pragma unroll
+        for (int i = 0; i < 12; i += 4) z += (part[50 * i] + part[50 * i + 50]) + (part[50 * i + 100] + part[50 * i + 150]);
+        const float d = (label == (unsigned)oo ? 1.0f : 0.0f) - sigmoidf<1>(z + sm.bf[oo]);       // makeError
+        const bool counts = k * kGtImgs + oj < imgs_here && *const_cast<const volatile int*>(&sm.empty[k % kGtSlabs]) != k;
+        sm.df[set][oj][oo] = counts ? d : 0.f;
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&sm.df_ready[set]);
+    }
+    CNN_PHASE(11);
+    group_sync(set);
+    CNN_PHASE(12);
+    float most = 0.f;
+    {
+      f32x2 wk[2][kOut / 2];
+      const bool second = gt + 128 < kS;
+      const int u[2] = {gt, second ? gt + 128 : gt};
+#pragma unroll
+      for (int r = 0; r < 2; ++r)
+#pragma unroll
+        for (int kk = 0; kk < kOut / 2; ++kk) wk[r][kk] = pack2(sm.wf[2 * kk][u[r]], sm.wf[2 * kk + 1][u[r]]);
+#pragma unroll
+      for (int jj = 0; jj < kGtImgs; ++jj) {
+        const ulonglong2 e0 = *reinterpret_cast<const ulonglong2*>(&sm.df[set][jj][0]), e1 = *reinterpret_cast<const ulonglong2*>(&sm.df[set][jj][4]);
+        const f32x2 e4 = ld2(&sm.df[set][jj][8]);
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+          const float a = sm.as[set][jj][u[r]];
+          float lo, hi;
+          unpack2(fma2(wk[r][4], e4, fma2(wk[r][3], e1.y, fma2(wk[r][2], e1.x, fma2(wk[r][1], e0.y, mul2(wk[r][0], e0.x))))), lo, hi);
+          const float ds = (lo + hi) * a * (1.f - a);
+          if (r == 0 || second) {
+            sm.ds[set][jj][u[r]] = ds;
+            g_bs += ds;
+          }
+          most = fmaxf(most, fabsf(ds));
+        }
+      }
+    }
+    const unsigned m32 = __reduce_max_sync(0xffffffffu, __float_as_uint(most));
+    if (lane == 0) sm.ds_max[set][quarter] = m32;
+    group_sync(set);
+    CNN_PHASE(3);
+    CNN_PHASE(7);
+    // The delta operands go round: a window's turn is told by a parity, which is unambiguous while no more than two tiles are at it.
+    if (k >= 2) mbar_wait_bounded(&sm.a_free[(k - 2) % kGtSlabs], (unsigned)((k - 2) / kGtSlabs) & 1u, status, gave_up);
+    CNN_PHASE(8);
+    // |conv delta * 576| <= max |ds| * max |Ws| / 4: scaled by 2^e into [1024, 2048) at most
+    const unsigned ds_bits = max(max(sm.ds_max[set][0], sm.ds_max[set][1]), max(sm.ds_max[set][2], sm.ds_max[set][3]));
+    const float bound = __uint_as_float(ds_bits) * wsmax * 0.25f;
+    const int e = min(max(10 - ((int)(__float_as_uint(bound) >> 23) - 127), -100), 100);
+    const float scale = __int_as_float((127 + e) << 23), unscale = __int_as_float((127 - e) << 23);
+    if (quarter == 0 && lane == 0) *const_cast<volatile float*>(&sm.tile_unscale[k % kGtSlabs]) = unscale;
+    f32x2 ws2[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float w = sm.ws[rsub * 4 + j] * scale;
+      ws2[j] = pack2(w, w);
+    }
+    const f32x2 back2 = pack2(unscale, unscale), minus2 = pack2(-1.f, -1.f);
+    const f32x2 magic2 = pack2(12582912.f, 12582912.f);      // 1.5 * 2^23: adding it rounds to a whole number
+    unsigned nxt[8];
+    tc::tmem_ld8_nowait(t0, nxt);
+#pragma unroll 1
+    for (int w = 0; w < 6; ++w) {                 // window columns
+      const int at = 6 * k + w, win = at % kGtWindows;
+      unsigned char* const to = sm.delta[win] + (32 * quarter + lane) * 16;
+      CNN_PHASE(5);
+      mbar_wait_bounded(&sm.dl_free[win], ((unsigned)(at / kGtWindows) & 1u) ^ 1u, status, gave_up);
+      __syncwarp();
+      CNN_PHASE(6);
+#pragma unroll
+      for (int m = 0; m < 3; ++m) {               // map pairs
+        tc::tmem_wait8(nxt);
+        f32x2 a2[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) a2[j] = pack2(__uint_as_float(nxt[2 * j]), __uint_as_float(nxt[2 * j + 1]));
+        if (m < 2 || w < 5) tc::tmem_ld8_nowait(t0 + (unsigned)(24 * w + 8 * m + 8), nxt);
+        if (m == 2 && (w & 1)) {                   // the last columns of a block are in registers: hand it back to the MMA warp
+          tc::fence_before_sync();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&sm.d_free[3 * set + (w >> 1)]);
+        }
+        const f32x2 ds2 = ld2(ds_slot + 6 * w + 2 * m);
+        unsigned hi[4], lo[4];
+        f32x2 total;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          gws[j] = fma2(ds2, a2[j], gws[j]);
+          const f32x2 slope = mul2(a2[j], fma2(a2[j], minus2, one2)), c = mul2(ds2, ws2[j]);      // the delta is their product
+          total = j == 0 ? mul2(slope, c) : fma2(slope, c, total);
+          const f32x2 whole = fma2(fma2(slope, c, magic2), minus2, magic2);                        // minus the delta, rounded
+          float q0, q1, l0, l1;
+          unpack2(whole, q0, q1);
+          unpack2(fma2(slope, c, whole), l0, l1);
+          const __half2 hh = __floats2half2_rn(q0, q1), hl = __floats2half2_rn(l0, l1);
+          hi[j] = *reinterpret_cast<const unsigned*>(&hh);
+          lo[j] = *reinterpret_cast<const unsigned*>(&hl);
+        }
+        gbc[m] = fma2(total, back2, gbc[m]);
+        *reinterpret_cast<uint4*>(to + m * kGtDeltaBlock) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+        *reinterpret_cast<uint4*>(to + (3 + m) * kGtDeltaBlock) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+      }
+      tc::fence_async_smem();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&sm.dl_full[win]);
+    }
+    CNN_PHASE(4);
+  }
+  // ---- what this warp has gathered: lanes 0-3 the taps 4 * lane + j, lane 0 the biases ----
+  float t[4], b[kF];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    float lo, hi;
+    unpack2(gws[j], lo, hi);
+    t[j] = lo + hi;
+#pragma unroll
+    for (int m = 4; m <= 16; m <<= 1) t[j] += __shfl_xor_sync(0xffffffffu, t[j], m);
+  }
+#pragma unroll
+  for (int f = 0; f < kF; f += 2) unpack2(gbc[f / 2], b[f], b[f + 1]);
+#pragma unroll
+  for (int f = 0; f < kF; ++f)
+#pragma unroll
+    for (int m = 1; m <= 16; m <<= 1) b[f] += __shfl_xor_sync(0xffffffffu, b[f], m);
+#pragma unroll
+  for (int m = 1; m <= 16; m <<= 1) g_bs += __shfl_xor_sync(0xffffffffu, g_bs, m);
+  __syncthreads();
+  GtEnd& end = *reinterpret_cast<GtEnd*>(sm.raw);
+  if (lane < 4) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) end.ws[warp - kGtEpiWarp0][4 * lane + j] = t[j];
+  }
+  if (lane == 0) {
+#pragma unroll
+    for (int f = 0; f < kF; ++f) end.bc[warp - kGtEpiWarp0][f] = b[f];
+    end.bs[warp - kGtEpiWarp0] = g_bs;
+  }
+  CNN_PHASE_END(g_phase_clocks_gt);
+}
+
+// One thread: this block has left something, and has written what, and its row.
+__device__ __forceinline__ void push_left(GradLeft* left, int* pushed) {
+  __threadfence();
+  const int at = atomicAdd(pushed, 1);
+  asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(&left[at].next), "r"((int)blockIdx.x + 1) : "memory");
+}
+
+// left[b]: what of block b's share is not in its row.
 __global__ void __launch_bounds__(kGtThreads, 1)
-k_grad_tc(const float* images, const unsigned* labels, long n, int per_cta, const float* params, float* __restrict__ rows,
-          int* __restrict__ left, int* __restrict__ status) {
+k_grad_tc(const float* images, const unsigned* labels, GradShares shares, const float* params, float* __restrict__ rows,
+          GradLeft* left, int* pushed, int* __restrict__ status) {
   extern __shared__ unsigned char smem_raw[];
   GtSmem& sm = *reinterpret_cast<GtSmem*>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~(uintptr_t)127);
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   constexpr float kPre = -1.4426950408889634f;      // the short sigmoid form's factor, in the conv weights and biases
 
-  const long img0 = (long)blockIdx.x * per_cta;
-  const int imgs_here = (int)min((long)per_cta, n - img0);
+  const long img0 = shares.first(blockIdx.x);
+  const int imgs_here = shares.size(blockIdx.x);
   const int n_tiles = (imgs_here + kGtImgs - 1) / kGtImgs;
 
   if (tid == 0) {
@@ -162,21 +613,18 @@ k_grad_tc(const float* images, const unsigned* labels, long n, int per_cta, cons
   pdl_wait();
   pdl_launch_dependents();
 
-  auto fetch = [&](int k) {       // one thread: the images of tile k
-    const unsigned bytes = (unsigned)(min(kGtImgs, imgs_here - k * kGtImgs) * kImg) * (unsigned)sizeof(float);
-    mbar_expect_tx(&sm.raw_full[k % kGtRaw], bytes);
-    bulk_g2s(sm.raw[k % kGtRaw], images + (img0 + k * kGtImgs) * kImg, bytes, &sm.raw_full[k % kGtRaw]);
-  };
-  // ---- a sample of the share's pixels, 128 neighbours at each of kGtPlaces places: its mean is the level that pixels are taken from, and images that
-  // are not whole numbers / 255 are as a rule all of that kind (this block has nothing to do then) ----
+  // ---- a sample of the share's pixels, 128 neighbours at each of kGtPlaces places: its mean is the level that pixels are taken from, and images with
+  // other pixels than whole numbers / 255 are as a rule many (this block has nothing to do then) ----
   float4 px[2];
 #pragma unroll
   for (int j = 0; j < 2; ++j) {
-    const long pieces = (long)imgs_here * (kImg / 4), first = (2 * warp + j) * (pieces - 32) / (kGtPlaces - 1);
+    const int first = (2 * warp + j) * ((imgs_here * (kImg / 4) - 32) / (kGtPlaces - 1));
     px[j] = reinterpret_cast<const float4*>(images + img0 * kImg)[first + lane];
   }
   // The parameters as well: every load of the set-up is under way before the first value is used.
   constexpr int kBRows = 3 * 5 * kGtBN, kBTurns = (kBRows + kGtThreads - 1) / kGtThreads;      // 16-byte rows of the conv operand
+  // The first 80 threads build two of them; the FC table, the small parameters and the biases are others' (all by the first: 0.4 us more per launch).
+  constexpr int kFcFrom = 96, kSmallFrom = 320, kBiasWarp = 12;
   constexpr int kAll = (kNParams + kGtThreads - 1) / kGtThreads;
   float bw[kBTurns][5], wfc[kOut], small, share[kAll], taps[5], wsmax;      // (taps: the 150 and the six biases)
 #pragma unroll
@@ -186,43 +634,53 @@ k_grad_tc(const float* images, const unsigned* labels, long n, int per_cta, cons
     for (int d = 0; d < 5; ++d) bw[t][d] = params[kOffWc + (2 * (r >> 3) + (r & 1)) * 25 + i * 5 + d];
   }
   {
-    const float* wf = params + kOffWf + (min(tid, kS - 1) % 6) * 36 + min(tid, kS - 1) / 6;      // slot entry u = 36 p + 6 q + f: input 36 f + 6 p + q
-    const int t = tid - 256;
+    const int u = min(max(tid - kFcFrom, 0), kS - 1), t = tid - kSmallFrom;
+    const float* wf = params + kOffWf + (u % 6) * 36 + u / 6;      // slot entry u = 36 p + 6 q + f: input 36 f + 6 p + q
 #pragma unroll
     for (int k = 0; k < kOut; ++k) wfc[k] = wf[k * kS];
-    small = params[t < 0 || t > 40 ? 0 : (t < 16 ? kOffWs + t : (t < 28 ? kOffBf + min(t - 16, kOut - 1) : (t < 28 + kF ? kOffBc + t - 28 : kOffBs)))];
+    small = params[t < 0 || t > 28 ? 0 : (t < 16 ? kOffWs + t : (t < 28 ? kOffBf + min(t - 16, kOut - 1) : kOffBs))];
   }
 #pragma unroll
   for (int j = 0; j < kAll; ++j) share[j] = params[min(tid + kGtThreads * j, kNParams - 1)];
 #pragma unroll
   for (int j = 0; j < 5; ++j) taps[j] = params[min(lane + 32 * j, kOffWs - 1)];
   wsmax = fabsf(params[kOffWs + (lane & 15)]);
-  for (int i = tid; i < kGtSlabs * kGtSlabBytes / 16; i += kGtThreads) reinterpret_cast<uint4*>(sm.slab)[i] = make_uint4(0, 0, 0, 0);
+  // What no tile of five images writes of a slab: behind each chunk, and behind the last.  The slab of a shorter tile, the share's last, as a whole.
+  for (int i = tid; i < kGtSlabs * 28; i += kGtThreads) {
+    const int j = i % 28;
+    const unsigned off = j < 3 * kGtChunks ? j / 3 * kGtChunk + 15 * kGtGroupStride + j % 3 * 16 : kGtChunks * kGtChunk + (j - 3 * kGtChunks) * 16;
+    *reinterpret_cast<uint4*>(sm.slab[i / 28] + off) = make_uint4(0, 0, 0, 0);
+  }
+  if (imgs_here % kGtImgs != 0)
+    for (int i = tid; i < kGtSlabBytes / 16; i += kGtThreads) reinterpret_cast<uint4*>(sm.slab[(n_tiles - 1) % kGtSlabs])[i] = make_uint4(0, 0, 0, 0);
   if (tid < 36) sm.zeros[tid] = 0.f;
+  if (tid < kGtSlabs) sm.empty[tid] = -1;
   {
-    bool other = false;
+    bool other[2] = {false, false};
     int sum = 0;
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
       const float x[4] = {px[j].x * 255.f, px[j].y * 255.f, px[j].z * 255.f, px[j].w * 255.f};
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
-        other = other || !(x[c] == rintf(x[c]) && fabsf(x[c]) <= 255.f);
+        other[j] = other[j] || !(x[c] == rintf(x[c]) && fabsf(x[c]) <= 255.f);
         sum += (int)fminf(fmaxf(x[c], 0.f), 255.f);
       }
     }
     sum = __reduce_add_sync(0xffffffffu, sum);
     if (lane == 0) sm.px_sum[warp] = sum;
-    if (__syncthreads_or(other)) {
-      float* row = rows + (size_t)blockIdx.x * kRowStride;
-      for (int i = tid; i < kRowStride; i += kGtThreads) row[i] = 0.f;
-      if (tid == 0) left[blockIdx.x] = imgs_here;
+    const bool first = __any_sync(0xffffffffu, other[0]), second = __any_sync(0xffffffffu, other[1]);
+    if (__syncthreads_count((lane == 0 && first) || (lane == 1 && second)) >= kGtPlacesOther) {
+      if (tid == 0) {
+        left[blockIdx.x].from = left[blockIdx.x].written = left[blockIdx.x].skips = 0;
+        push_left(left, pushed);
+      }
       if (warp == kGtGradWarp) tc::tmem_dealloc(sm.tmem_base, 512);
       return;
     }
   }
   if (tid == 0)        // the thread that initialised the barriers
-    for (int k = 0; k < kGtRaw && k < n_tiles; ++k) fetch(k);
+    for (int k = 0; k < kGtRaw && k < n_tiles; ++k) fetch_tile(sm, images + img0 * kImg, imgs_here, k);
 
   // ---- set-up: scales, conv weights, FC table, small parameters ----------------------------------------------
   float wmax = 0.f;
@@ -231,20 +689,14 @@ k_grad_tc(const float* images, const unsigned* labels, long n, int per_cta, cons
   for (int j = 0; j < 5; ++j) wmax = fmaxf(wmax, lane + 32 * j < kOffBc ? fabsf(taps[j]) : 0.f);
 #pragma unroll
   for (int j = 0; j < kAll; ++j) sane = sane && fabsf(share[j]) <= 1e9f;
-#pragma unroll
-  for (int m = 16; m > 0; m >>= 1) {
-    wmax = fmaxf(wmax, __shfl_xor_sync(0xffffffffu, wmax, m));
-    wsmax = fmaxf(wsmax, __shfl_xor_sync(0xffffffffu, wsmax, m));
-  }
+  wmax = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(wmax)));      // (magnitudes compare as their bits)
+  wsmax = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(wsmax)));
   // With 2^E <= max |kPre * w| < 2^(E+1) weights are scaled by 2^(16-E) / 255 and pixels by 255 * 2^(E-3): the accumulator carries 2^13.
   int wexp = (int)((__float_as_uint(fabsf(kPre) * wmax) >> 23) & 255u) - 127;
   sane = sane && wexp >= -21 && wexp <= 11;      // fp16 holds 255 * 2^(E-3)
   wexp = min(max(wexp, -21), 11);
   const float w_scale = __int_as_float((127 + 16 - wexp) << 23);
-  constexpr float w_unscale = 1.0f / 8192.0f;
-  int level = 0;                                 // the sample's mean pixel, a whole number
-#pragma unroll
-  for (int w = 0; w < kGtThreads / 32; ++w) level += sm.px_sum[w];
+  int level = __reduce_add_sync(0xffffffffu, lane < kGtThreads / 32 ? sm.px_sum[lane] : 0);       // the sample's mean pixel, a whole number
   level = wexp > 10 ? 0 : (level + 128 * kGtPlaces / 2) / (128 * kGtPlaces);      // (a negative pixel may be 510 below it)
 
 #pragma unroll
@@ -280,28 +732,32 @@ k_grad_tc(const float* images, const unsigned* labels, long n, int per_cta, cons
     *reinterpret_cast<uint4*>(sm.b[0] + off) = *reinterpret_cast<uint4*>(hi);
     *reinterpret_cast<uint4*>(sm.b[1] + off) = *reinterpret_cast<uint4*>(lo);
   }
-  if (tid < kS) {
+  if (tid >= kFcFrom && tid < kFcFrom + kS) {
 #pragma unroll
-    for (int k = 0; k < kOut; ++k) sm.wf[k][tid] = wfc[k];
-  } else if (tid >= 256 && tid < 256 + 64) {
-    const int t = tid - 256;
+    for (int k = 0; k < kOut; ++k) sm.wf[k][tid - kFcFrom] = wfc[k];
+  } else if (tid >= kSmallFrom && tid <= kSmallFrom + 28) {
+    const int t = tid - kSmallFrom;
     if (t < 16) sm.ws[t] = small;
     else if (t < 28) sm.bf[t - 16] = (t - 16 < kOut) ? small : 0.f;
-    else if (t == 40) sm.bs[0] = small;
+    else sm.bs[0] = small;
   }
-  if (warp < kF) {               // a map's bias, and what the level adds to its pre-activations
+  if (warp >= kBiasWarp && warp < kBiasWarp + kF) {               // a map's bias, and what the level adds to its pre-activations
     float sum = 0.f;
 #pragma unroll
-    for (int j = 0; j < 5; ++j) sum += (lane + 32 * j) / 25 == warp ? taps[j] : 0.f;
+    for (int j = 0; j < 5; ++j) sum += (lane + 32 * j) / 25 == warp - kBiasWarp ? taps[j] : 0.f;
 #pragma unroll
     for (int m = 16; m > 0; m >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, m);
-    const float bias = __shfl_sync(0xffffffffu, taps[4], kOffBc - 128 + warp);
-    if (lane == 0) sm.bc[warp] = kPre * fmaf((float)level / 255.f, sum, bias);
+    const float bias = __shfl_sync(0xffffffffu, taps[4], kOffBc - 128 + warp - kBiasWarp);
+    if (lane == 0) sm.bc[warp - kBiasWarp] = kPre * fmaf((float)level / 255.f, sum, bias);
   }
   tc::fence_async_smem();      // the operands were written through the generic proxy
   tc::fence_before_sync();
   const bool all_sane = __syncthreads_and(sane);
-  if (tid == 0) sm.stop = all_sane ? n_tiles : 0;
+  if (tid == 0) {
+    sm.stop = all_sane ? n_tiles : 0;
+    sm.skips = 0;
+    sm.most = 60000.f / fmaxf(1.f, __int_as_float((127 + wexp - 3) << 23)) - 255.f;
+  }
   __syncthreads();
   tc::fence_after_sync();
   const unsigned tmem_base = sm.tmem_base;
@@ -448,410 +904,11 @@ k_grad_tc(const float* images, const unsigned* labels, long n, int per_cta, cons
     __syncwarp();
     __syncthreads();
   } else if (warp < kGtEpiWarp0) {
-    // ================= loaders and drain ================================================================
-    const int lt = tid - 32 * kGtLoadWarp0, quarter = warp & 3;
-    // Piece i = lt + 128 j: four pixels (column 4 c) of one row, the second half of chunk c - 1 and the first of chunk c, in one group or two.
-    // Lanes eight apart write the two halves of 16 bytes in opposite order, so that no bank is asked twice: first to `own + at[0]`, then to
-    // `own + at[1]`.  Bits 16 to 19: whether the first place exists, whether a second group has it (64 bytes before), and the same of the second.
-    unsigned dst[kGtUnits];
-    const int swap = (lane >> 3) & 1;
-    const unsigned at[2] = {swap ? 8u - kGtChunk : 0u, swap ? 0u : 8u - kGtChunk};
-#pragma unroll
-    for (int j = 0; j < kGtUnits; ++j) {
-      const int i = lt + kGtLoaders * j, img = i / (kImg / 4), rest = i % (kImg / 4), r = rest / 7, c = rest % 7;
-      const int g = min(r >> 3, 2);
-      dst[j] = (unsigned)(((3 * img + g) * 12 + (r - 8 * g)) * 16) + (unsigned)c * kGtChunk;
-      const unsigned two = g > 0 && r - 8 * g < 4 ? 3u : 1u, own = c < 6 ? two : 0u, before = c > 0 ? two : 0u;
-      dst[j] |= i < kGtPieces ? (swap ? before | own << 2 : own | before << 2) << 16 : 0u;
-    }
-    const __half2 px_scale = __float2half2_rn(__int_as_float((127 + wexp - 3) << 23)), magic = __float2half2_rn(1536.f);
-    const __half2 minus_level = __float2half2_rn(-(float)level * __int_as_float((127 + wexp - 3) << 23));
-    const f32x2 k255 = pack2(255.f, 255.f);
-    f32x2 sum[kGtGradN / 2];
-#pragma unroll
-    for (int i = 0; i < kGtGradN / 2; ++i) sum[i] = pack2(0.f, 0.f);
-    auto drain = [&](int k) {
-      mbar_wait_bounded(&sm.a_free[k % kGtSlabs], (unsigned)(k / kGtSlabs) & 1u, status, gave_up);
-      __syncwarp();
-      if (quarter == 3) return;
-      tc::fence_after_sync();
-      const float f = *const_cast<const volatile float*>(&sm.tile_unscale[k % kGtSlabs]);
-      const f32x2 f2 = pack2(f, f);
-      const unsigned t0 = tmem_base + (unsigned)(kGtGradCol + (k & 1) * kGtGradN) + ((unsigned)(quarter * 32) << 16);
-#pragma unroll
-      for (int c = 0; c < kGtGradN; c += 8) {
-        unsigned v[8];
-        tc::tmem_ld8_nowait(t0 + (unsigned)c, v);
-        tc::tmem_wait8(v);
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-          sum[c / 2 + i] = fma2(pack2(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1])), f2, sum[c / 2 + i]);
-      }
-      tc::fence_before_sync();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&sm.g_free[k & 1]);
-    };
-    const int tiles = stop;
-    int k = 0, fetched = min(kGtRaw, n_tiles), seen = 0, drained = 0;
-    for (; k < tiles; ++k) {
-      const int s = k % kGtSlabs, r = k % kGtRaw;
-      CNN_PHASE(0);
-      if (k >= kGtSlabs) drain(drained++);
-      CNN_PHASE(1);
-      mbar_wait_bounded(&sm.raw_full[r], (unsigned)(k / kGtRaw) & 1u, status, gave_up);
-      ++seen;
-      CNN_PHASE(2);
-      const int pieces = min(kGtImgs, imgs_here - k * kGtImgs) * (kImg / 4);
-      const unsigned slab = smem_u32(sm.slab[s]);
-      unsigned bits = 0, odd = 0;
-      float big = 0.f;
-#pragma unroll
-      for (int j0 = 0; j0 < kGtUnits; j0 += 4) {
-        float4 v[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) v[j] = *reinterpret_cast<const float4*>(&sm.raw[r][4 * min(lt + kGtLoaders * (j0 + j), pieces - 1)]);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          float x[4];
-          unpack2(mul2(pack2(v[j].x, v[j].y), k255), x[0], x[1]);
-          unpack2(mul2(pack2(v[j].z, v[j].w), k255), x[2], x[3]);
-          big = max_abs_nan(max_abs_nan(big, x[0], x[1]), x[2], x[3]);
-          bits |= __float_as_uint(x[0]) | __float_as_uint(x[1]) | __float_as_uint(x[2]) | __float_as_uint(x[3]);
-          unsigned h[2];
-#pragma unroll
-          for (int c = 0; c < 2; ++c) {
-            const __half2 p = __floats2half2_rn(x[2 * c], x[2 * c + 1]);
-            const __half2 w = __hsub2(__hadd2(p, magic), magic);      // whole numbers below 512 as they are
-            odd |= *reinterpret_cast<const unsigned*>(&p) ^ *reinterpret_cast<const unsigned*>(&w);
-            const __half2 q = __hfma2(p, px_scale, minus_level);
-            h[c] = *reinterpret_cast<const unsigned*>(&q);
-          }
-          const unsigned to = lt + kGtLoaders * (j0 + j) < pieces ? dst[j0 + j] : 0u, own = slab + (to & 0xffffu);
-#pragma unroll
-          for (int turn = 0; turn < 2; ++turn) {
-            store_if(own + at[turn], h, to & (1u << (16 + 2 * turn)));
-            store_if(own + at[turn] - 64u, h, to & (1u << (17 + 2 * turn)));
-          }
-        }
-      }
-      const bool other = (bits & 0x1fffu) != 0 || odd != 0 || !(big <= 255.f);
-      tc::fence_async_smem();    // generic-proxy writes -> visible to the tensor core's operand reads
-      const bool halt = barrier_any(1, other);
-      if (lt == 0) {
-        if (halt) *const_cast<volatile int*>(&sm.stop) = k;
-        else if (k + kGtRaw < n_tiles) fetch(k + kGtRaw);
-        mbar_arrive(&sm.a_full[s]);
-      }
-      __syncwarp();
-      if (halt) break;
-      fetched = min(k + kGtRaw + 1, n_tiles);
-      CNN_PHASE(3);
-    }
-    // k tiles take part; copies that are still on their way land before their memory is used for anything else
-    for (int j = seen; j < fetched; ++j) mbar_wait_bounded(&sm.raw_full[j % kGtRaw], (unsigned)(j / kGtRaw) & 1u, status, gave_up);
-    for (; drained < k; ++drained) drain(drained);
-    __syncthreads();
-    if (quarter < 3 && lane < 16) {
-      float* to = end.d[16 * quarter + lane];
-#pragma unroll
-      for (int i = 0; i < kGtGradN / 2; ++i) unpack2(sum[i], to[2 * i], to[2 * i + 1]);
-    }
+    load_tiles(sm, images + img0 * kImg, imgs_here, n_tiles, wexp, level, tmem_base, status);
   } else {
-    // ================= epilogue ====================================================================
-    const int set = (warp - kGtEpiWarp0) >> 2;     // accumulator / tile residue this group owns
-    const int quarter = warp & 3;                  // tensor-memory lanes 32 * quarter ..
-    const int rsub = lane & 3;                     // row of the 4x4 window
-    const int g = quarter * 4 + (lane >> 3);       // group of 8 output rows this lane's row belongs to
-    const int img = g / 3, p = 2 * (g % 3) + ((lane >> 2) & 1);      // image of the tile (5: the unused group), window row
-    const bool used = img < kGtImgs;
-    const bool b0 = (lane & 1) != 0, b1 = (lane & 2) != 0;
-    f32x2 bc2[kF / 2], gws[4], gbc[kF / 2];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) gws[j] = pack2(0.f, 0.f);
-#pragma unroll
-    for (int f = 0; f < kF; f += 2) {
-      bc2[f / 2] = pack2(sm.bc[f], sm.bc[f + 1]);
-      gbc[f / 2] = pack2(0.f, 0.f);
-    }
-    const f32x2 unscale2 = pack2(w_unscale, w_unscale), one2 = pack2(1.f, 1.f);
-    const float bs = sm.bs[0];
-    float* const as_slot = used ? &sm.as[set][img][p * 36] : nullptr;
-    const float* const ds_slot = used ? &sm.ds[set][img][p * 36] : sm.zeros;
-    // FC forward: 54 inputs per warp, lane = nine of them (of six parts) and outputs fk and fk + 5, for all five images
-    const int fk = lane < 30 ? lane % 5 : 4, fpart = lane < 30 ? lane / 5 : 5, first_in = 54 * quarter + 9 * fpart;
-    const int gt = 32 * quarter + lane;            // thread of the group: inputs gt and gt + 128
-    float g_bs = 0.f;
-    const unsigned t0 = tmem_base + (unsigned)(set * 3 * kGtBN) + ((unsigned)(quarter * 32) << 16);
-
-    for (int k = set; k < n_tiles; k += kGtSets) {
-      const unsigned turn = (unsigned)(k / kGtSets) & 1u;
-      bool halt = false;
-      // output layer: quarter 0 images 0-2, quarter 1 images 3-4, lane 10 j + o
-      const int oj = 3 * quarter + lane / 10, oo = lane % 10;
-      const bool outputs = quarter < 2 && lane < (quarter ? 20 : 30);
-      unsigned label = ~0u;
-      if (outputs && k * kGtImgs + oj < imgs_here) label = labels[img0 + k * kGtImgs + oj];
-      CNN_PHASE(0);
-      if (k >= kGtSets) mbar_wait_bounded(&sm.df_free[set], turn ^ 1u, status, gave_up);      // this group's tile before this one
-      {
-        f32x2 ws2[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const float w = sm.ws[rsub * 4 + j];
-          ws2[j] = pack2(w, w);
-        }
-#pragma unroll 1
-        for (int xb = 0; xb < 3; ++xb) {              // one block of two window columns
-          mbar_wait_bounded(&sm.d_full[3 * set + xb], turn, status, gave_up);
-          if (xb == 0) {
-            halt = barrier_any(2 + set, k >= stop);      // (all of the group, or none)
-            CNN_PHASE(1);
-          }
-          if (halt) break;
-          __syncwarp();
-          tc::fence_after_sync();
-          unsigned nxt[8];
-          tc::tmem_ld8_nowait(t0 + (unsigned)(xb * kGtBN), nxt);
-          tc::tmem_wait8(nxt);
-          float z[12];
-          f32x2 d2[4];               // 1 + 2^t of the row's four columns (of two maps), one step behind
-          // Step ch turns 8 accumulator columns (window column ch / 3, maps 2 * (ch % 3) + {0, 1}) into exponentials and
-          // finishes the columns of step ch - 1, so that two chains of dependent instructions are always under way.
-#pragma unroll
-          for (int ch = 0; ch < 7; ++ch) {
-            f32x2 e2[4];
-            if (ch < 6) {
-              if (ch > 0) tc::tmem_wait8(nxt);
-#pragma unroll
-              for (int j = 0; j < 4; ++j)
-                e2[j] = fma2(pack2(__uint_as_float(nxt[2 * j]), __uint_as_float(nxt[2 * j + 1])), unscale2, bc2[ch % 3]);
-              if (ch < 5) tc::tmem_ld8_nowait(t0 + (unsigned)(xb * kGtBN + (ch + 1) * 8), nxt);
-#pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                float x, y;
-                unpack2(e2[j], x, y);
-                e2[j] = pack2(exp2f_approx(x), exp2f_approx(y));
-              }
-            }
-            if (ch > 0) {
-              f32x2 z2;
-#pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                float x, y;
-                unpack2(d2[j], x, y);
-                d2[j] = pack2(rcp_approx(x), rcp_approx(y));
-                z2 = j == 0 ? mul2(ws2[0], d2[0]) : fma2(ws2[j], d2[j], z2);
-              }
-              tmem_st8(t0 + (unsigned)(xb * kGtBN + (ch - 1) * 8), d2);      // the activations, for stage 2
-              unpack2(z2, z[2 * (ch - 1)], z[2 * (ch - 1) + 1]);
-            }
-            if (ch < 6) {
-#pragma unroll
-              for (int j = 0; j < 4; ++j) d2[j] = add2(e2[j], one2);
-            }
-          }
-          // the window's four rows are lanes 4g..4g+3: reduce-scatter the block's 12 sums
-          float w6[6];
-#pragma unroll
-          for (int i = 0; i < 6; ++i) {
-            const float send = b0 ? z[i] : z[i + 6], keep = b0 ? z[i + 6] : z[i];
-            w6[i] = keep + __shfl_xor_sync(0xffffffffu, send, 1);
-          }
-#pragma unroll
-          for (int i = 0; i < 3; ++i) {
-            const float send = b1 ? w6[i] : w6[i + 3], keep = b1 ? w6[i + 3] : w6[i];
-            const float as = sigmoidf<1>(keep + __shfl_xor_sync(0xffffffffu, send, 2) + bs);
-            if (used) as_slot[12 * xb + (b0 ? 6 : 0) + (b1 ? 3 : 0) + i] = as;
-          }
-        }
-      }
-      asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-      if (halt) {
-        if (lane == 0 && quarter < 2) mbar_arrive(&sm.df_ready[set]);
-        if (k == stop) {        // the gradient warp waits for this tile's first window: its turn, empty
-          const int win = (6 * k) % kGtWindows;
-          if (k >= 2) mbar_wait_bounded(&sm.a_free[(k - 2) % kGtSlabs], (unsigned)((k - 2) / kGtSlabs) & 1u, status, gave_up);
-          mbar_wait_bounded(&sm.dl_free[win], ((unsigned)(6 * k / kGtWindows) & 1u) ^ 1u, status, gave_up);
-          if (lane == 0) mbar_arrive(&sm.dl_full[win]);
-        }
-        break;
-      }
-      CNN_PHASE(2);
-      // ---- the output layer, its error, and the subsample deltas, by the group's 128 threads ----
-      group_sync(set);
-      {
-        const float *as = &sm.as[set][0][first_in], *w0 = &sm.wf[fk][first_in], *w1 = &sm.wf[fk + 5][first_in];
-        f32x2 z[kGtImgs];
-#pragma unroll
-        for (int jj = 0; jj < kGtImgs; ++jj) z[jj] = pack2(0.f, 0.f);
-#pragma unroll
-        for (int i = 0; i < 9; ++i) {
-          const f32x2 w2 = pack2(w0[i], w1[i]);
-#pragma unroll
-          for (int jj = 0; jj < kGtImgs; ++jj) {
-            const float a = as[jj * kS + i];
-            z[jj] = fma2(w2, pack2(a, a), z[jj]);
-          }
-        }
-        // parts 3-5 to parts 0-2, the twelve sums of the group to shared memory (where the subsample deltas come later)
-        float* part = &sm.ds[set][0][0] + (3 * quarter + fpart) * 50 + fk;
-#pragma unroll
-        for (int jj = 0; jj < kGtImgs; ++jj) {
-          float lo, hi;
-          unpack2(z[jj], lo, hi);
-          lo += __shfl_down_sync(0xffffffffu, lo, 15);
-          hi += __shfl_down_sync(0xffffffffu, hi, 15);
-          if (lane < 15) {
-            part[10 * jj] = lo;
-            part[10 * jj + 5] = hi;
-          }
-        }
-      }
-      CNN_PHASE(9);
-      group_sync(set);
-      CNN_PHASE(10);
-      if (quarter < 2) {
-        if (outputs) {
-          const float* part = &sm.ds[set][0][0] + 10 * oj + oo;
-          float z = 0.f;
-#pragma unroll
-          for (int i = 0; i < 12; i += 4) z += (part[50 * i] + part[50 * i + 50]) + (part[50 * i + 100] + part[50 * i + 150]);
-          const float d = (label == (unsigned)oo ? 1.0f : 0.0f) - sigmoidf<1>(z + sm.bf[oo]);       // makeError
-          sm.df[set][oj][oo] = k * kGtImgs + oj < imgs_here ? d : 0.f;
-        }
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&sm.df_ready[set]);
-      }
-      CNN_PHASE(11);
-      group_sync(set);
-      CNN_PHASE(12);
-      float most = 0.f;
-      {
-        f32x2 wk[2][kOut / 2];
-        const bool second = gt + 128 < kS;
-        const int u[2] = {gt, second ? gt + 128 : gt};
-#pragma unroll
-        for (int r = 0; r < 2; ++r)
-#pragma unroll
-          for (int kk = 0; kk < kOut / 2; ++kk) wk[r][kk] = pack2(sm.wf[2 * kk][u[r]], sm.wf[2 * kk + 1][u[r]]);
-#pragma unroll
-        for (int jj = 0; jj < kGtImgs; ++jj) {
-          const ulonglong2 e0 = *reinterpret_cast<const ulonglong2*>(&sm.df[set][jj][0]), e1 = *reinterpret_cast<const ulonglong2*>(&sm.df[set][jj][4]);
-          const f32x2 e4 = ld2(&sm.df[set][jj][8]);
-#pragma unroll
-          for (int r = 0; r < 2; ++r) {
-            const float a = sm.as[set][jj][u[r]];
-            float lo, hi;
-            unpack2(fma2(wk[r][4], e4, fma2(wk[r][3], e1.y, fma2(wk[r][2], e1.x, fma2(wk[r][1], e0.y, mul2(wk[r][0], e0.x))))), lo, hi);
-            const float ds = (lo + hi) * a * (1.f - a);
-            if (r == 0 || second) {
-              sm.ds[set][jj][u[r]] = ds;
-              g_bs += ds;
-            }
-            most = fmaxf(most, fabsf(ds));
-          }
-        }
-      }
-      const unsigned m32 = __reduce_max_sync(0xffffffffu, __float_as_uint(most));
-      if (lane == 0) sm.ds_max[set][quarter] = m32;
-      group_sync(set);
-      CNN_PHASE(3);
-      CNN_PHASE(7);
-      // The delta operands go round: a window's turn is told by a parity, which is unambiguous while no more than two tiles are at it.
-      if (k >= 2) mbar_wait_bounded(&sm.a_free[(k - 2) % kGtSlabs], (unsigned)((k - 2) / kGtSlabs) & 1u, status, gave_up);
-      CNN_PHASE(8);
-      // |conv delta * 576| <= max |ds| * max |Ws| / 4: scaled by 2^e into [1024, 2048) at most
-      const unsigned ds_bits = max(max(sm.ds_max[set][0], sm.ds_max[set][1]), max(sm.ds_max[set][2], sm.ds_max[set][3]));
-      const float bound = __uint_as_float(ds_bits) * wsmax * 0.25f;
-      const int e = min(max(10 - ((int)(__float_as_uint(bound) >> 23) - 127), -100), 100);
-      const float scale = __int_as_float((127 + e) << 23), unscale = __int_as_float((127 - e) << 23);
-      if (quarter == 0 && lane == 0) *const_cast<volatile float*>(&sm.tile_unscale[k % kGtSlabs]) = unscale;
-      f32x2 ws2[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float w = sm.ws[rsub * 4 + j] * scale;
-        ws2[j] = pack2(w, w);
-      }
-      const f32x2 back2 = pack2(unscale, unscale), minus2 = pack2(-1.f, -1.f);
-      const f32x2 magic2 = pack2(12582912.f, 12582912.f);      // 1.5 * 2^23: adding it rounds to a whole number
-      unsigned nxt[8];
-      tc::tmem_ld8_nowait(t0, nxt);
-#pragma unroll 1
-      for (int w = 0; w < 6; ++w) {                 // window columns
-        const int at = 6 * k + w, win = at % kGtWindows;
-        unsigned char* const to = sm.delta[win] + (32 * quarter + lane) * 16;
-        CNN_PHASE(5);
-        mbar_wait_bounded(&sm.dl_free[win], ((unsigned)(at / kGtWindows) & 1u) ^ 1u, status, gave_up);
-        __syncwarp();
-        CNN_PHASE(6);
-#pragma unroll
-        for (int m = 0; m < 3; ++m) {               // map pairs
-          tc::tmem_wait8(nxt);
-          f32x2 a2[4];
-#pragma unroll
-          for (int j = 0; j < 4; ++j) a2[j] = pack2(__uint_as_float(nxt[2 * j]), __uint_as_float(nxt[2 * j + 1]));
-          if (m < 2 || w < 5) tc::tmem_ld8_nowait(t0 + (unsigned)(24 * w + 8 * m + 8), nxt);
-          if (m == 2 && (w & 1)) {                   // the last columns of a block are in registers: hand it back to the MMA warp
-            tc::fence_before_sync();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&sm.d_free[3 * set + (w >> 1)]);
-          }
-          const f32x2 ds2 = ld2(ds_slot + 6 * w + 2 * m);
-          unsigned hi[4], lo[4];
-          f32x2 total;
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            gws[j] = fma2(ds2, a2[j], gws[j]);
-            const f32x2 slope = mul2(a2[j], fma2(a2[j], minus2, one2)), c = mul2(ds2, ws2[j]);      // the delta is their product
-            total = j == 0 ? mul2(slope, c) : fma2(slope, c, total);
-            const f32x2 whole = fma2(fma2(slope, c, magic2), minus2, magic2);                        // minus the delta, rounded
-            float q0, q1, l0, l1;
-            unpack2(whole, q0, q1);
-            unpack2(fma2(slope, c, whole), l0, l1);
-            const __half2 hh = __floats2half2_rn(q0, q1), hl = __floats2half2_rn(l0, l1);
-            hi[j] = *reinterpret_cast<const unsigned*>(&hh);
-            lo[j] = *reinterpret_cast<const unsigned*>(&hl);
-          }
-          gbc[m] = fma2(total, back2, gbc[m]);
-          *reinterpret_cast<uint4*>(to + m * kGtDeltaBlock) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-          *reinterpret_cast<uint4*>(to + (3 + m) * kGtDeltaBlock) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
-        }
-        tc::fence_async_smem();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&sm.dl_full[win]);
-      }
-      CNN_PHASE(4);
-    }
-    // ---- what this warp has gathered: lanes 0-3 the taps 4 * lane + j, lane 0 the biases ----
-    float t[4], b[kF];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      float lo, hi;
-      unpack2(gws[j], lo, hi);
-      t[j] = lo + hi;
-#pragma unroll
-      for (int m = 4; m <= 16; m <<= 1) t[j] += __shfl_xor_sync(0xffffffffu, t[j], m);
-    }
-#pragma unroll
-    for (int f = 0; f < kF; f += 2) unpack2(gbc[f / 2], b[f], b[f + 1]);
-#pragma unroll
-    for (int f = 0; f < kF; ++f)
-#pragma unroll
-      for (int m = 1; m <= 16; m <<= 1) b[f] += __shfl_xor_sync(0xffffffffu, b[f], m);
-#pragma unroll
-    for (int m = 1; m <= 16; m <<= 1) g_bs += __shfl_xor_sync(0xffffffffu, g_bs, m);
-    __syncthreads();
-    if (lane < 4) {
-#pragma unroll
-      for (int j = 0; j < 4; ++j) end.ws[warp - kGtEpiWarp0][4 * lane + j] = t[j];
-    }
-    if (lane == 0) {
-#pragma unroll
-      for (int f = 0; f < kF; ++f) end.bc[warp - kGtEpiWarp0][f] = b[f];
-      end.bs[warp - kGtEpiWarp0] = g_bs;
-    }
+    run_group(sm, labels + img0, imgs_here, n_tiles, wsmax, tmem_base, status);
   }
-  CNN_PHASE_END(g_phase_clocks_gt);
+  if (warp < kGtLoadWarp0) { CNN_PHASE_END(g_phase_clocks_gt); }
 
   tc::fence_before_sync();
   __syncthreads();
@@ -867,7 +924,8 @@ k_grad_tc(const float* images, const unsigned* labels, long n, int per_cta, cons
     float b = 0.f;
 #pragma unroll
     for (int w = 0; w < 12; ++w) b += end.bc[w][f];
-    row[kOffWc + tid] = (s[1] - s[0]) * __int_as_float((127 + 3 - wexp) << 23) / (255.f * kC * kC) + (float)level / 255.f * (b / (float)(kC * kC));
+    // (not a division: 1 / (255 * 576) in fp32 is 2.9e-8 of itself too large, as the pixels are by 2.4e-8)
+    row[kOffWc + tid] = fmaf((float)level, b, (s[1] - s[0]) * __int_as_float((127 + 3 - wexp) << 23)) * (1.f / (255.f * kC * kC));
   } else if (tid < kOffWs) {
     float s = 0.f;
 #pragma unroll
@@ -889,17 +947,21 @@ k_grad_tc(const float* images, const unsigned* labels, long n, int per_cta, cons
   } else if (tid >= 192 && tid < 192 + kRowStride - kNParams) {
     const int i = kNParams + tid - 192;
     row[i] = i == kRowErr ? end.err : 0.f;
-  } else if (tid == 256) {
-    left[blockIdx.x] = imgs_here - min(imgs_here, (int)stop * kGtImgs);
+  } else if (tid >= 256 && tid < 256 + 3 + kGradSkips) {
+    const int i = tid - 256;
+    reinterpret_cast<int*>(left + blockIdx.x)[i] = i == 0 ? min(imgs_here, (int)stop * kGtImgs) : (i == 1 ? 1 : (i == 2 ? sm.skips : sm.skipped[i - 3]));
+  }
+  if (sm.skips > 0 || stop < n_tiles) {
+    __syncthreads();
+    if (tid == 0) push_left(left, pushed);
   }
 }
 
-// Shares of per_cta images, `grid` blocks.
-int launch_grad_tc(cnn_net* net, const float* d_images, const unsigned* d_labels, long n, int grid, int per_cta, int* left, cudaStream_t st) {
+int launch_grad_tc(cnn_net* net, const float* d_images, const unsigned* d_labels, GradShares shares, GradLeft* left, int* pushed, cudaStream_t st) {
   const size_t smem = sizeof(GtSmem) + 128;
   CNN_CUDA(cudaFuncSetAttribute(k_grad_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  cudaError_t e = launch_pdl(k_grad_tc, dim3(grid), dim3(kGtThreads), smem, st, d_images, d_labels, n, per_cta, (const float*)net->d_params,
-                             net->d_partials, left, net->d_status);
+  cudaError_t e = launch_pdl(k_grad_tc, dim3(shares.blocks), dim3(kGtThreads), smem, st, d_images, d_labels, shares, (const float*)net->d_params,
+                             net->d_partials, left, pushed, net->d_status);
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e, "k_grad_tc launch");
   return CNN_OK;

@@ -12,7 +12,12 @@ void destroy_host_pipeline(HostPipeline* p);
 // (One row per SM and gradient kernel: no launch has more blocks, see grid_for_batch.)
 int ensure_train_scratch(cnn_net* net) {
   if (!net->d_grad) CNN_CUDA(cudaMalloc(&net->d_grad, sizeof(float) * (kNParamsPadded + 8)));
-  if (!net->d_partials) CNN_CUDA(cudaMalloc(&net->d_partials, sizeof(float) * (size_t)sm_count() * (2 * kRowStride + 1)));
+  if (!net->d_partials) {
+    const size_t rows = sizeof(float) * kRowStride * sm_count(), left = sizeof(GradLeft) * sm_count() + sizeof(int);
+    CNN_CUDA(cudaMalloc(&net->d_partials, rows + left));
+    CNN_CUDA(cudaMemset(reinterpret_cast<unsigned char*>(net->d_partials) + rows, 0, left));      // an empty queue
+    CNN_CUDA(cudaDeviceSynchronize());      // (the caller's stream need not wait for the null stream)
+  }
   return CNN_OK;
 }
 }  // namespace cnn

@@ -20,7 +20,7 @@ struct cnn_net {
   int fast_sigmoid = 1;            // sigmoid of the fused kernels: 0 = reference expression, 1 = short form (default)
 
   // Training scratch (allocated on first use): per-block partial gradients and the reduced vector.
-  float* d_partials = nullptr;     // two rows of kRowStride floats per SM, then an int per SM (grad_tc.cu)
+  float* d_partials = nullptr;     // a row of kRowStride floats per SM, then a GradLeft per SM and the number of blocks in their queue
   float* d_grad = nullptr;         // kNParamsPadded floats + 8 floats of statistics
   cnn::HostPipeline* host = nullptr;   // host_pipeline.cu (created on first use)
 };
@@ -112,6 +112,21 @@ __device__ __forceinline__ bool mbar_wait_bounded(unsigned long long* bar, unsig
 constexpr int kRowStride = kNParamsPadded + 8;
 constexpr int kRowErr = kNParams + 1;  // 2344
 
+// Shares of a batch: the first `more` blocks have one image more than the others.  (Fewer blocks with equal shares would leave SMs idle, where k_grad_left's
+// first blocks would start before anything is left.)
+struct GradShares {
+  int blocks, each, more;
+  __host__ __device__ long first(int b) const { return (long)b * each + (b < more ? b : more); }
+  __host__ __device__ int size(int b) const { return each + (b < more ? 1 : 0); }
+};
+
+// What of a block's share of a batch the tensor-core gradient kernel (grad_tc.cu) leaves to the CUDA cores: the images from `from` on, and before
+// them some tiles of kGradTile images.  `next` is a queue beside it: block numbers + 1, in the order in which blocks that leave something finish; 0 = no more yet.
+constexpr int kGradTile = 5, kGradSkips = 28;
+struct GradLeft {
+  int from, written, skips, tile[kGradSkips], next;      // written: the block's row holds the gradient of what is not left
+};
+
 // Column `col` of rows g, g + GROUPS, g + 2 GROUPS, ... added in that order; five loads at a time are under way (with one
 // row per SM and 32 groups that is all of them).
 template <int GROUPS>
@@ -145,8 +160,8 @@ int grid_for_batch(long n);
 // for that kernel: see k_grad_partials).
 int launch_grad_partials(cnn_net* net, const float* d_images, const unsigned* d_labels, long n, int grid,
                          cudaStream_t st, bool chained = false);
-// The same on the tensor cores, but for left[b] images at the end of block b's share of per_cta images.
-int launch_grad_tc(cnn_net* net, const float* d_images, const unsigned* d_labels, long n, int grid, int per_cta, int* left, cudaStream_t st);
+// The same on the tensor cores, but for what left[b] says of block b's share.
+int launch_grad_tc(cnn_net* net, const float* d_images, const unsigned* d_labels, GradShares shares, GradLeft* left, int* pushed, cudaStream_t st);
 int launch_persample_cluster8(cnn_net* net, const float* d_images, const unsigned* d_labels, long n, int epochs,
                               float dt, float threshold, float* d_mean, int* d_ran, cudaStream_t st);
 

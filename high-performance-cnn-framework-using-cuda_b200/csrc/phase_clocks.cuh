@@ -19,6 +19,11 @@
   if (threadIdx.x == 0) (slot) = clock64();                                           \
   __syncthreads();                                                                    \
   const long long ph_base_ = (slot);
+// The same in a function that some warps call behind CNN_PHASE_BEGIN.
+#define CNN_PHASE_ROLE(owner, slot)                                                   \
+  long long ph_[16] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};               \
+  const bool ph_on_ = (owner) && (threadIdx.x & 31) == 0;                             \
+  const long long ph_base_ = (slot);
 #define CNN_PHASE(i)                                                                  \
   do {                                                                                \
     if (ph_on_) {                                                                     \
@@ -35,6 +40,7 @@
 #else
 #define CNN_PHASE_TABLE(name, warps)
 #define CNN_PHASE_BEGIN(owner, slot)
+#define CNN_PHASE_ROLE(owner, slot)
 #define CNN_PHASE(i) do { } while (0)
 #define CNN_PHASE_END(name) do { } while (0)
 #endif
