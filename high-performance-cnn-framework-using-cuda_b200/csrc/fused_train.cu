@@ -856,8 +856,8 @@ static int launch_gradient(cnn_net* net, const float* d_images, const unsigned* 
   }
   const long grid = (n + kGradTile - 1) / kGradTile < sms ? (n + kGradTile - 1) / kGradTile : sms;
   const GradShares shares = {(int)grid, (int)(n / grid), (int)(n % grid)};
-  GradLeft* left = reinterpret_cast<GradLeft*>(net->d_partials + (size_t)sms * kRowStride);
-  int* pushed = reinterpret_cast<int*>(left + sms);
+  GradLeft* left = grad_left(net);
+  int* pushed = grad_queued(net);
   int rc = set_smem_attr(k_grad_left<1>, sizeof(GrSmem<2>));
   if (rc == CNN_OK) rc = launch_grad_tc(net, d_images, d_labels, shares, left, pushed, st);
   if (rc != CNN_OK) return rc;
@@ -865,7 +865,7 @@ static int launch_gradient(cnn_net* net, const float* d_images, const unsigned* 
                              (const float*)net->d_params, net->d_partials, net->d_status, left, pushed);
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e != cudaSuccess) {
-    cudaMemsetAsync(left, 0, sizeof(GradLeft) * sms + sizeof(int), st);      // nobody takes what the kernel before has queued
+    cudaMemsetAsync(pushed, 0, sizeof(GradLeft) * (1 + (size_t)sms) - sizeof(int), st);      // nobody takes what the kernel before has queued
     return cuda_fail(e, "k_grad_left launch");
   }
   *rows = (int)grid;

@@ -9,15 +9,12 @@
 namespace cnn {
 void destroy_host_pipeline(HostPipeline* p);
 
-// (One row per SM and gradient kernel: no launch has more blocks, see grid_for_batch.)
+// One allocation, in the first training call of a net.  (One row per SM: no gradient kernel has more blocks, see grid_for_batch.)
 int ensure_train_scratch(cnn_net* net) {
-  if (!net->d_grad) CNN_CUDA(cudaMalloc(&net->d_grad, sizeof(float) * (kNParamsPadded + 8)));
-  if (!net->d_partials) {
-    const size_t rows = sizeof(float) * kRowStride * sm_count(), left = sizeof(GradLeft) * sm_count() + sizeof(int);
-    CNN_CUDA(cudaMalloc(&net->d_partials, rows + left));
-    CNN_CUDA(cudaMemset(reinterpret_cast<unsigned char*>(net->d_partials) + rows, 0, left));      // an empty queue
-    CNN_CUDA(cudaDeviceSynchronize());      // (the caller's stream need not wait for the null stream)
-  }
+  if (net->d_grad) return CNN_OK;
+  constexpr size_t kGrad = kNParamsPadded + 32;
+  CNN_CUDA(cudaMalloc(&net->d_grad, sizeof(float) * (kGrad + (size_t)kRowStride * sm_count())));
+  net->d_partials = net->d_grad + kGrad;
   return CNN_OK;
 }
 }  // namespace cnn
@@ -34,8 +31,9 @@ int cnn_net_create(unsigned int seed, cnn_net** out) {
   net->seed = seed;
   cudaError_t e = cudaGetDevice(&net->device);
   if (e == cudaSuccess) e = cudaMalloc(&net->d_params, sizeof(float) * kNParamsPadded);
-  if (e == cudaSuccess) e = cudaMalloc(&net->d_status, sizeof(int));
-  if (e == cudaSuccess) e = cudaMemset(net->d_status, 0, sizeof(int));
+  const size_t status_bytes = sizeof(GradLeft) * (1 + (size_t)sm_count());      // status word, length of the queue, and the queue of GradLeft
+  if (e == cudaSuccess) e = cudaMalloc(&net->d_status, status_bytes);
+  if (e == cudaSuccess) e = cudaMemset(net->d_status, 0, status_bytes);
   if (e != cudaSuccess) {
     cnn_net_destroy(net);
     return cuda_fail(e, "cnn_net_create");
@@ -70,8 +68,7 @@ int cnn_net_destroy(cnn_net* net) {
   if (!net) return CNN_OK;
   cudaFree(net->d_params);
   cudaFree(net->d_status);
-  cudaFree(net->d_partials);
-  cudaFree(net->d_grad);
+  cudaFree(net->d_grad);      // and d_partials behind it
   destroy_host_pipeline(net->host);
   delete net;
   return CNN_OK;

@@ -16,11 +16,11 @@ struct cnn_net {
                                    // -1 (default) = 1 for batches of kTcMinBatch images or more, else 0
   int grad_path = -1;              // gradient of a batch: 0 = CUDA cores, 1 = tensor cores, -1 (default) = by batch size
   float* d_params = nullptr;       // kNParamsPadded floats
-  int* d_status = nullptr;         // device status word: 0 ok, non-zero = a bounded wait ran out
+  int* d_status = nullptr;         // device status word: 0 ok, non-zero = a bounded wait ran out; behind it what GradLeft describes
   int fast_sigmoid = 1;            // sigmoid of the fused kernels: 0 = reference expression, 1 = short form (default)
 
-  // Training scratch (allocated on first use): per-block partial gradients and the reduced vector.
-  float* d_partials = nullptr;     // a row of kRowStride floats per SM, then a GradLeft per SM and the number of blocks in their queue
+  // Training scratch, one allocation on first use: the reduced vector, and behind it per-block partial gradients.
+  float* d_partials = nullptr;     // a row of kRowStride floats per SM
   float* d_grad = nullptr;         // kNParamsPadded floats + 8 floats of statistics
   cnn::HostPipeline* host = nullptr;   // host_pipeline.cu (created on first use)
 };
@@ -126,6 +126,9 @@ constexpr int kGradTile = 5, kGradSkips = 28;
 struct GradLeft {
   int from, written, skips, tile[kGradSkips], next;      // written: the block's row holds the gradient of what is not left
 };
+// They lie behind the net's status word, one per SM, and before them the number of entries in the queue; all zero between two calls.
+inline int* grad_queued(cnn_net* net) { return net->d_status + 1; }
+inline GradLeft* grad_left(cnn_net* net) { return reinterpret_cast<GradLeft*>(net->d_status) + 1; }
 
 // Column `col` of rows g, g + GROUPS, g + 2 GROUPS, ... added in that order; five loads at a time are under way (with one
 // row per SM and 32 groups that is all of them).

@@ -463,6 +463,22 @@ def test_tensor_core_gradient_of_a_mixture_takes_no_longer(cuda, pkg, which, n, 
     assert np.median(times[-1]) < bar * np.median(times[0])
 
 
+def test_first_gradient_of_a_net_allocates_one_granule(cuda, pkg):
+    """The training scratch comes with a net's first gradient call, so that call pays for it: a row per SM, 1.4 MB, which fits one 2 MiB granule of
+    device memory.  Median over nets, because small allocations share granules."""
+    images, labels = pkg.synth.synth_images(67, 2048)
+    d_img, d_lab = to_dev(cuda, images, labels)
+    d_g = cuda.empty(2368, dtype=cuda.float32, device="cuda")
+    nets, taken = [], []
+    for seed in range(9):
+        nets.append(pkg.Net(seed))
+        before = cuda.cuda.mem_get_info()[0]
+        nets[-1].grad_batch(d_img, d_lab, 2048, d_g)
+        cuda.cuda.synchronize()
+        taken.append(before - cuda.cuda.mem_get_info()[0])
+    assert sorted(taken)[len(taken) // 2] <= 2 << 20
+
+
 @pytest.mark.parametrize("n", [5, 743])
 @pytest.mark.parametrize("what", ["bright", "white", "inverted", "both"])
 def test_tensor_core_gradient_of_dense_bright_images(cuda, pkg, what, n):
