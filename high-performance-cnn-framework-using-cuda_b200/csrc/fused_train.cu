@@ -836,9 +836,10 @@ static int launch_grad(const float* d_params, float* rows, int* status, int fast
   return CNN_OK;
 }
 
-int launch_grad_partials(cnn_net* net, const float* d_images, const unsigned* d_labels, long n, int grid, cudaStream_t st,
-                         bool chained) {
-  return launch_grad(net->d_params, net->d_partials, net->d_status, net->fast_sigmoid, d_images, d_labels, n, grid, st, chained);
+// Blocks of k_grad_partials: one per SM at most (a block holds two images at a time), so that few rows are left to add.
+static int grid_for_batch(long n) {
+  const long sms = sm_count();
+  return (int)(n < sms ? n : sms);
 }
 
 // Tensor cores or CUDA cores.  Microseconds per gradient call, CUDA cores / tensor cores, back to back: 740 images 14.6 / 17.6, 1,000 18.0 / 20.7,
@@ -846,13 +847,13 @@ int launch_grad_partials(cnn_net* net, const float* d_images, const unsigned* d_
 // They meet at about 1,250; the line leaves room for images that turn out not to be whole numbers / 255 and go to the CUDA cores behind a
 // look at a sample: 2,048 images 33.2 (29.0 without the look), 6,000 76 (72), 60,000 652 (643).  With other pixels in one image of a hundred 60,000
 // images are 367 us, with other pixels in the second half of them 678.
-static int launch_gradient(cnn_net* net, const float* d_images, const unsigned* d_labels, long n, cudaStream_t st, bool chained, int* rows) {
+int launch_gradient(cnn_net* net, const float* d_images, const unsigned* d_labels, long n, cudaStream_t st, bool chained, int* rows) {
   constexpr long kTcGradMin = 2048;
   const int sms = sm_count();
   const bool tensor = net->grad_path == 1 || (net->grad_path < 0 && n >= kTcGradMin);
   if (!tensor || !net->fast_sigmoid || n > (1l << 30)) {
     *rows = grid_for_batch(n);
-    return launch_grad_partials(net, d_images, d_labels, n, *rows, st, chained);
+    return launch_grad(net->d_params, net->d_partials, net->d_status, net->fast_sigmoid, d_images, d_labels, n, *rows, st, chained);
   }
   const long grid = (n + kGradTile - 1) / kGradTile < sms ? (n + kGradTile - 1) / kGradTile : sms;
   const GradShares shares = {(int)grid, (int)(n / grid), (int)(n % grid)};
@@ -870,12 +871,6 @@ static int launch_gradient(cnn_net* net, const float* d_images, const unsigned* 
   }
   *rows = (int)grid;
   return CNN_OK;
-}
-
-// Blocks of the gradient kernel: one per SM at most (a block holds two images at a time), so that few rows are left to add.
-int grid_for_batch(long n) {
-  const long sms = sm_count();
-  return (int)(n < sms ? n : sms);
 }
 
 }  // namespace cnn

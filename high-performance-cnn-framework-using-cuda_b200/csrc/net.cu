@@ -9,7 +9,7 @@
 namespace cnn {
 void destroy_host_pipeline(HostPipeline* p);
 
-// One allocation, in the first training call of a net.  (One row per SM: no gradient kernel has more blocks, see grid_for_batch.)
+// One allocation, in the first training call of a net.  (One row per SM: no gradient kernel has more blocks.)
 int ensure_train_scratch(cnn_net* net) {
   if (net->d_grad) return CNN_OK;
   constexpr size_t kGrad = kNParamsPadded + 32;

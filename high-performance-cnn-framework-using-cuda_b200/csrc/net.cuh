@@ -155,15 +155,12 @@ int forward_device_tc(cnn_net* net, int path, const float* d_images, long n, flo
 int forward_device_tc_u8(cnn_net* net, const unsigned char* d_pixels, long n, float* d_out, int* d_argmax,
                          cudaStream_t stream);
 int ensure_train_scratch(cnn_net* net);
-// Blocks of the minibatch gradient kernel for a batch of n images (one partial row per block).
-int grid_for_batch(long n);
-// Fused forward + backward of n images at fixed parameters: `grid` partial rows into net->d_partials.
+// Fused forward + backward of n images at fixed parameters, on the CUDA cores or the tensor cores: *rows partial rows in net->d_partials.
 // `chained`: the kernel before this one on the stream is this library's reduce + update kernel of the previous
 // step of the same call (then, and only then, the gradient kernel may fetch its first images before waiting
 // for that kernel: see k_grad_partials).
-int launch_grad_partials(cnn_net* net, const float* d_images, const unsigned* d_labels, long n, int grid,
-                         cudaStream_t st, bool chained = false);
-// The same on the tensor cores, but for what left[b] says of block b's share.
+int launch_gradient(cnn_net* net, const float* d_images, const unsigned* d_labels, long n, cudaStream_t st, bool chained, int* rows);
+// Its tensor-core part: a row per share, but for what left[b] says of block b's.
 int launch_grad_tc(cnn_net* net, const float* d_images, const unsigned* d_labels, GradShares shares, GradLeft* left, int* pushed, cudaStream_t st);
 int launch_persample_cluster8(cnn_net* net, const float* d_images, const unsigned* d_labels, long n, int epochs,
                               float dt, float threshold, float* d_mean, int* d_ran, cudaStream_t st);

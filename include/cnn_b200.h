@@ -178,9 +178,11 @@ int cnn_synth_images(unsigned long long seed, long first_index, long n, float* d
                      unsigned int* d_labels, void* stream);
 
 /* Options, by name:
- *   "grad_path"        kernel behind cnn_grad_batch and the steps of cnn_train_minibatch: 0 = fp32 on the CUDA cores, 1 = the
+ *   "grad_path"        kernel behind cnn_grad_batch and the steps of cnn_train_minibatch and of the data-parallel calls (by the
+ *                      images of one rank): 0 = fp32 on the CUDA cores, 1 = the
  *                      convolution and its weight gradient on the tensor cores at fp32-level accuracy (images whose pixels are
- *                      whole numbers / 255; others are computed on the CUDA cores), -1 (default) = 1 from 2,048 images on, else 0;
+ *                      float(byte / 255.0), as a division gives them; others, a byte times 1 / 255 among them, are noticed and computed
+ *                      on the CUDA cores, 4 to 9 us later than under 0), -1 (default) = 1 from 2,048 images on, else 0;
  *                      fast_sigmoid = 0 stays on the CUDA cores.
  *   "forward_path"     kernel behind cnn_forward_batched and cnn_forward_batched_u8: 0 = exact fp32 on the CUDA
  *                      cores; 1 = the convolution on the tensor cores (tcgen05), both operands in two fp16 parts and

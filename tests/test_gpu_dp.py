@@ -40,6 +40,35 @@ def test_single_rank_exchange_equals_minibatch_kernel(cuda, pkg, params0):
     dp.close()
 
 
+@pytest.mark.parametrize("path", [-1, 0, 1])
+def test_single_rank_takes_the_gradient_kernel_of_the_net(cuda, pkg, params0, path):
+    """Steps of 2,500 images and a ragged last one, some images with other pixels than whole numbers / 255: the data-parallel calls follow
+    grad_path as cnn_train_minibatch does, bit for bit, so a one-rank run changes nothing."""
+    n, batch = 2500 + 2500 + 140, 2500
+    images, labels = pkg.synth.synth_images(83, n)
+    images[[7, 2400, 4000], 9, 9] = 0.3337
+    d_img = cuda.from_numpy(images).cuda()
+    d_lab = cuda.from_numpy(labels.astype(np.int32)).cuda()
+    nets, errs = [], []
+    for of_dp in (False, True):
+        net = pkg.Net(0)
+        net.set_params(params0)
+        net.set_option("grad_path", path)
+        err = cuda.zeros(2, dtype=cuda.float32, device="cuda")
+        if of_dp:
+            dp = pkg.DataParallel(net)
+            dp.train_minibatch(d_img, d_lab, n, batch, 2, 0.1, err)
+            cuda.cuda.synchronize()
+            dp.close()
+        else:
+            net.train_minibatch(d_img, d_lab, n, batch, 2, 0.1, err)
+            cuda.cuda.synchronize()
+        assert net.status() == 0
+        nets.append(net)
+        errs.append(err)
+    assert np.array_equal(nets[0].get_params(), nets[1].get_params()) and cuda.equal(errs[0], errs[1])
+
+
 def test_exchange_uses_the_scratch_of_a_net_that_trained_alone(cuda, pkg, params0):
     """A net keeps its training scratch: a data-parallel step behind ordinary ones allocates nothing (and frees nothing, which
     would wait for the device)."""
