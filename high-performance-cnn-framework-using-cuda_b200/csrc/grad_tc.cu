@@ -25,9 +25,11 @@
 // what it adds to a tap's gradient is the level times the bias gradient, which is summed in fp32.  Sums of centred pixels stay below 2^24: over nets as drawn
 // and trained, and nets with deltas of one sign, with strokes, inverted strokes, both mixed, noise and smooth bright images, a tile's
 // largest lies between 2^14 and 2^23.5 (without the level up to 2^26.9).
-// D is added to fp32 sums in registers after every tile.  Distance of the gradient from fp64, geometric mean over 12 nets and batches of 2,048,
-// 4,500, 8,000, 20,000 and 60,000 images: 4.94e-8 of its norm (k_grad_partials 4.93e-8), conv weights alone 4.79e-8 (4.83e-8), conv biases 4.8e-8
-// (5.8e-8); nets with deltas of one sign 4.52e-8 (4.51e-8), conv weights 4.93e-8 (4.74e-8).
+// D is added to fp32 sums in registers after every tile.  Distance of the gradient from fp64 in 1e-8 of its norm, k_grad_partials / here, geometric means: strokes, nets
+// as drawn, 12 nets and batches of 2,048 to 60,000 images 4.93 / 4.93, conv weights alone 4.83 / 4.8, conv biases 5.8 / 4.8.  4,000 images and six to ten nets, conv
+// weights alone: strokes 4.7 / 4.8, inverted 9.0 / 5.9, bright (200-255) 7.4 / 5.1, strokes and inverted ones 8.3 / 7.4, dim (0-126) 5.9 / 5.1; with deltas of one sign
+// 4.9 / 5.1, 7.8 / 7.1, 8.6 / 8.6, 7.4 / 6.8, 6.6 / 6.9 (27 to 51 without the level).  With conv weights 30 times as large, where pre-activations are the limit: strokes
+// 11.5 / 12.9, inverted 31 / 19, bright 80 / 64, both 22 / 21, dim 7.3 / 7.4, the whole gradient of strokes 4.8 / 5.4.
 //
 // Pipeline (one CTA per SM, 20 warps, mbarriers with bounded waits):
 //   warps 4-7   one bulk copy per tile, two tiles ahead; pixels -> fp16 operand; drain D of the tile that had the slab before;
@@ -710,8 +712,10 @@ k_grad_tc(const float* images, const unsigned* labels, GradShares shares, const 
 #pragma unroll
     for (int d = 0; d < 5; ++d) w[d] = w_scale * bw[turn][d];
     __half2 hi[4], lo[4];
-    // In two parts, so that the factor costs the weights no bit.  (A byte / 255 in fp32 is 2.37e-8 of itself too large on average: the pixels are bytes.)
-    constexpr double kFactor = (double)kPre / 255.0 * (1.0 + 2.37e-8);
+    // In two parts, so that the factor costs the weights no bit.  A byte / 255 in fp32 is 2.37e-8 of itself too large on average, and the pixels are bytes.  And
+    // truncated additions take 4e-8 of a pre-activation: with that the conv weights' gradient is nearest to fp64 (strokes, weights eight times as
+    // large: 8.8e-8 without, 7.6e-8, 8.6e-8 with twice as much).
+    constexpr double kFactor = (double)kPre / 255.0 * (1.0 + 2.37e-8 + 4e-8);
     constexpr float kFactorHi = (float)kFactor, kFactorLo = (float)(kFactor - (double)kFactorHi);
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
@@ -741,14 +745,16 @@ k_grad_tc(const float* images, const unsigned* labels, GradShares shares, const 
     else if (t < 28) sm.bf[t - 16] = (t - 16 < kOut) ? small : 0.f;
     else sm.bs[0] = small;
   }
-  if (warp >= kBiasWarp && warp < kBiasWarp + kF) {               // a map's bias, and what the level adds to its pre-activations
-    float sum = 0.f;
+  // A map's bias, and what the level adds to its pre-activations: an error here is the same in every window, so it is rounded once (in fp32: the gradient of
+  // dense bright images at weights up to 15 three times as far from fp64).
+  if (warp >= kBiasWarp && warp < kBiasWarp + kF) {
+    double sum = 0.0;
 #pragma unroll
-    for (int j = 0; j < 5; ++j) sum += (lane + 32 * j) / 25 == warp - kBiasWarp ? taps[j] : 0.f;
-#pragma unroll
+    for (int j = 0; j < 5; ++j) sum += (lane + 32 * j) / 25 == warp - kBiasWarp ? (double)taps[j] : 0.0;
+#pragma unroll 1
     for (int m = 16; m > 0; m >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, m);
     const float bias = __shfl_sync(0xffffffffu, taps[4], kOffBc - 128 + warp - kBiasWarp);
-    if (lane == 0) sm.bc[warp - kBiasWarp] = kPre * fmaf((float)level / 255.f, sum, bias);
+    if (lane == 0) sm.bc[warp - kBiasWarp] = (float)(-1.4426950408889634 * ((double)bias + (double)level * (1.0 / 255.0) * sum));
   }
   tc::fence_async_smem();      // the operands were written through the generic proxy
   tc::fence_before_sync();

@@ -507,6 +507,47 @@ def test_tensor_core_gradient_of_dense_bright_images(cuda, pkg, what, n):
             assert scaled_err(out[1][lo:hi], out[0][lo:hi].astype(np.float64)) < 10 * 2.0**-24, name
 
 
+def fp64_gradient(torch, params, images, labels):
+    """The gradient of a batch in fp64, from the formulas."""
+    p = torch.from_numpy(params.astype(np.float64)).cuda()
+    x, n = torch.from_numpy(images.astype(np.float64)).cuda(), images.shape[0]
+    w_conv, w_sub, w_fc = p[:150].view(6, 25), p[156:172].view(4, 4), p[173:2333].view(10, 216)
+    patches = torch.nn.functional.unfold(x.view(n, 1, 28, 28), 5)
+    a = torch.sigmoid(torch.einsum("ft,ntp->nfp", w_conv, patches) + p[150:156, None]).view(n, 6, 6, 4, 6, 4)
+    s = torch.sigmoid(torch.einsum("nfpiqj,ij->nfpq", a, w_sub) + p[172]).reshape(n, 216)
+    d = torch.nn.functional.one_hot(torch.from_numpy(labels.astype(np.int64)).cuda(), 10) - torch.sigmoid(s @ w_fc.t() + p[2333:])
+    ds = ((d @ w_fc) * s * (1 - s)).view(n, 6, 6, 6)
+    dc = (ds.view(n, 6, 6, 1, 6, 1) * w_sub.view(1, 1, 1, 4, 1, 4) * a * (1 - a)).reshape(n, 6, 576) / 576
+    parts = [torch.einsum("nfp,ntp->ft", dc, patches), dc.sum((0, 2)), torch.einsum("nfpq,nfpiqj->ij", ds, a), ds.sum()[None] / 216, d.t() @ s, d.sum(0)]
+    return torch.cat([q.reshape(-1) for q in parts]).cpu().numpy()
+
+
+@pytest.mark.parametrize("scale", [1, 30])
+@pytest.mark.parametrize("what", ["strokes", "bright", "inverted"])
+def test_tensor_core_gradient_is_as_close_to_fp64(cuda, pkg, what, scale):
+    """Distance from fp64 of the whole gradient and of the conv weights' part, by the two paths, geometric mean over nets (where that part is not lost
+    in saturation).  With conv weights 30 times as large pre-activations are the limit, and of dense bright images their common part.  Two fp32
+    results of the same precision: half as far again, for chance."""
+    images, labels = pkg.synth.synth_images(68, 743)
+    pixels = np.rint(images * 255)
+    if what == "bright":
+        pixels = np.random.default_rng(5).integers(200, 256, pixels.shape)
+    elif what == "inverted":
+        pixels = 255 - pixels
+    images = (pixels / 255).astype(np.float32)
+    ratios = []
+    for seed in range(1, 9):
+        params = pkg.Net(seed).get_params()
+        params[:150] *= np.float32(scale)
+        want = fp64_gradient(cuda, params, images, labels)
+        out = both_paths(cuda, pkg, params, images, labels)
+        ratios.append([])
+        for hi in (2343, 150):
+            away = [np.linalg.norm(out[path][:hi] - want[:hi]) for path in (0, 1)]
+            ratios[-1].append(away[1] / away[0] if np.linalg.norm(want[:hi]) > 1e-6 * np.linalg.norm(want) else np.nan)
+    assert (np.exp(np.nanmean(np.log(ratios), axis=0)) < 1.5).all(), ratios
+
+
 @pytest.mark.parametrize("what", ["tiny conv weights", "large conv weights", "huge conv weights", "infinite bias", "not a number", "large rest",
                                   "no subsample filter"])
 def test_tensor_core_gradient_parameter_range(cuda, pkg, params0, what):
@@ -530,7 +571,7 @@ def test_tensor_core_gradient_parameter_range(cuda, pkg, params0, what):
     if not np.isnan(out[0]).any():
         for name, (lo, hi) in BLOCKS.items():
             if np.abs(out[0][lo:hi]).max() > 0:
-                assert scaled_err(out[1][lo:hi], out[0][lo:hi].astype(np.float64)) < (1e-2 if what == "large conv weights" else 1e-5), name
+                assert scaled_err(out[1][lo:hi], out[0][lo:hi].astype(np.float64)) < (4e-4 if what == "large conv weights" else 1e-5), name
             else:
                 assert not out[1][lo:hi].any(), name
 
