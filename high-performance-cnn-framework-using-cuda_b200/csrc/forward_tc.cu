@@ -59,6 +59,7 @@
 // and next the special-function unit (1,600 cycles) and instruction issue (1,400); path 2: the special-function unit, 75 % busy.
 #include <type_traits>
 
+#include "banded_conv.cuh"
 #include "cluster_exchange.cuh"
 #include "net.cuh"
 #include "wide_tc.cuh"
@@ -275,8 +276,8 @@ k_forward_tc(const void* images, long n, long imgs_per_cta, const float* params,
   float bw[kBTurns][5], wfc[kOut], small;
 #pragma unroll
   for (int t = 0; t < kBTurns; ++t) {
-    const int e = min(tid + t * kTfThreads, kBRows - 1), nn = e % kTfBN, r = nn % 24;
-    const int at = nn < 72 ? kOffWc + (2 * (r / 8) + (r & 1)) * 25 + e / (2 * kTfBN) * 5 : 0;
+    const int e = min(tid + t * kTfThreads, kBRows - 1), nn = e % kTfBN;
+    const int at = nn < 72 ? kOffWc + band_map(nn) * 25 + e / (2 * kTfBN) * 5 : 0;
 #pragma unroll
     for (int d = 0; d < 5; ++d) bw[t][d] = params[at + d];
   }
@@ -311,29 +312,13 @@ k_forward_tc(const void* images, long n, long imgs_per_cta, const float* params,
     const int e = tid + turn * kTfThreads;
     if (e >= kBRows) break;
     const int i = e / (2 * kTfBN), rem = e % (2 * kTfBN);
-    const int ch = rem / kTfBN, nn = rem % kTfBN;
-    // accumulator column nn = 24 * (window column in the block) + 8 * (map / 2) + 2 * (column in the window) + map % 2
-    const int qq = nn / 24, r = nn % 24, x = 4 * qq + ((r & 7) >> 1);
+    const int ch = rem / kTfBN, nn = rem % kTfBN, x = band_column(nn);
     float w[5];
 #pragma unroll
     for (int d = 0; d < 5; ++d) w[d] = (nn < 72) ? w_scale * bw[turn][d] : 0.f;
     __half2 hi[4], lo[4];
-    constexpr double kFactor = (double)kPre / 255.0;            // in two parts, so that the factor costs the weights no bit
-    constexpr float kFactorHi = (float)kFactor, kFactorLo = (float)(kFactor - (double)kFactorHi);
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      float t[2];
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int d = 8 * ch + 2 * c + h - x;
-        t[h] = 0.f;
-#pragma unroll
-        for (int dd = 0; dd < 5; ++dd) t[h] = (d == dd) ? w[dd] : t[h];
-      }
-      hi[c] = __floats2half2_rn(t[0] * kFactorHi, t[1] * kFactorHi);
-      const float2 b = __half22float2(hi[c]);
-      lo[c] = __floats2half2_rn(fmaf(t[0], kFactorLo, fmaf(t[0], kFactorHi, -b.x)), fmaf(t[1], kFactorLo, fmaf(t[1], kFactorHi, -b.y)));
-    }
+    constexpr TwoPart kFactor = two_part((double)kPre / 255.0);
+    band_row(w, 8 * ch - x, kFactor, hi, lo);
     const unsigned off = (unsigned)i * kTfBRow + (unsigned)ch * kTfBChunk + (unsigned)nn * 16u;
     *reinterpret_cast<uint4*>(sm.b_hi + off) = *reinterpret_cast<uint4*>(hi);
     if (kPrecise) *reinterpret_cast<uint4*>(sm.b_lo + off) = *reinterpret_cast<uint4*>(lo);

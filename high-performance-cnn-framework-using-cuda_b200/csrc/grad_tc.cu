@@ -44,6 +44,7 @@
 // the shared-memory data pipe (operands of the 78 MMAs 2,590 cycles, other warps 3,020: delta operands 580, FC layer
 // 700, loader 350, conflicts with the tensor core 570); instruction issue about 60 %, the special-function unit 37 %.  2,048 images are 24.0 us, of which a launch's
 // set-up is 3.2 us.
+#include "banded_conv.cuh"
 #include "cluster_exchange.cuh"
 #include "net.cuh"
 #include "phase_clocks.cuh"
@@ -597,6 +598,7 @@ k_grad_tc(const float* images, const unsigned* labels, GradShares shares, const 
   GtSmem& sm = *reinterpret_cast<GtSmem*>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~(uintptr_t)127);
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   constexpr float kPre = -1.4426950408889634f;      // the short sigmoid form's factor, in the conv weights and biases
+  constexpr double kByteExcess = 2.37e-8;
 
   const long img0 = shares.first(blockIdx.x);
   const int imgs_here = shares.size(blockIdx.x);
@@ -631,9 +633,9 @@ k_grad_tc(const float* images, const unsigned* labels, GradShares shares, const 
   float bw[kBTurns][5], wfc[kOut], small, share[kAll], taps[5], wsmax;      // (taps: the 150 and the six biases)
 #pragma unroll
   for (int t = 0; t < kBTurns; ++t) {
-    const int e = min(tid + t * kGtThreads, kBRows - 1), i = e / kGtBN % 5, r = e % kGtBN % 24;
+    const int e = min(tid + t * kGtThreads, kBRows - 1), i = e / kGtBN % 5;
 #pragma unroll
-    for (int d = 0; d < 5; ++d) bw[t][d] = params[kOffWc + (2 * (r >> 3) + (r & 1)) * 25 + i * 5 + d];
+    for (int d = 0; d < 5; ++d) bw[t][d] = params[kOffWc + band_map(e % kGtBN) * 25 + i * 5 + d];
   }
   {
     const int u = min(max(tid - kFcFrom, 0), kS - 1), t = tid - kSmallFrom;
@@ -705,33 +707,18 @@ k_grad_tc(const float* images, const unsigned* labels, GradShares shares, const 
   for (int turn = 0; turn < kBTurns; ++turn) {     // one 16-byte row: 8 input columns of one accumulator column
     const int e = tid + turn * kGtThreads;
     if (e >= kBRows) break;
-    const int variant = e / (5 * kGtBN), i = e / kGtBN % 5, nn = e % kGtBN;
-    // accumulator column nn = 24 * (window column in the block) + 8 * (map / 2) + 2 * (column in the window) + map % 2
-    const int qq = nn / 24, r = nn % 24, x = 4 * qq + ((r & 7) >> 1);
+    const int variant = e / (5 * kGtBN), i = e / kGtBN % 5, nn = e % kGtBN, x = band_column(nn);
     float w[5];
 #pragma unroll
     for (int d = 0; d < 5; ++d) w[d] = w_scale * bw[turn][d];
     __half2 hi[4], lo[4];
-    // In two parts, so that the factor costs the weights no bit.  A byte / 255 in fp32 is 2.37e-8 of itself too large on average, and the pixels are bytes.  And
-    // truncated additions take 4e-8 of a pre-activation: with that the conv weights' gradient is nearest to fp64 (strokes, weights eight times as
-    // large: 8.8e-8 without, 7.6e-8, 8.6e-8 with twice as much).
-    constexpr double kFactor = (double)kPre / 255.0 * (1.0 + 2.37e-8 + 4e-8);
-    constexpr float kFactorHi = (float)kFactor, kFactorLo = (float)(kFactor - (double)kFactorHi);
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      float t[2];
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        // input column of the block: 0-7, 8-15, or 4-11 of which the first four are in the first chunk
-        const int col = variant == 0 ? 2 * c + h : (variant == 1 ? 8 + 2 * c + h : (c >= 2 ? 4 + 2 * c + h : -64));
-        t[h] = 0.f;
-#pragma unroll
-        for (int dd = 0; dd < 5; ++dd) t[h] = (col - x == dd) ? w[dd] : t[h];
-      }
-      hi[c] = __floats2half2_rn(t[0] * kFactorHi, t[1] * kFactorHi);
-      const float2 b = __half22float2(hi[c]);
-      lo[c] = __floats2half2_rn(fmaf(t[0], kFactorLo, fmaf(t[0], kFactorHi, -b.x)), fmaf(t[1], kFactorLo, fmaf(t[1], kFactorHi, -b.y)));
-    }
+    // A byte / 255 in fp32 is kByteExcess of itself too large on average, and the pixels are bytes.  And truncated additions take 4e-8 of a
+    // pre-activation: with that the conv weights' gradient is nearest to fp64 (strokes, weights eight times as large: 8.8e-8 without, 7.6e-8, 8.6e-8 with
+    // twice as much).
+    constexpr TwoPart kFactor = two_part((double)kPre / 255.0 * (1.0 + kByteExcess + 4e-8));
+    // Input columns of the block: 0-7, 8-15, or 4-11 of which the first four are in the first chunk.
+    band_row(w, (variant == 0 ? 0 : (variant == 1 ? 8 : 4)) - x, kFactor, hi, lo);
+    if (variant == 2) hi[0] = hi[1] = lo[0] = lo[1] = __half2half2(__ushort_as_half(0));
     const unsigned off = (unsigned)variant * kGtBChunk + (unsigned)(i * kGtBN + nn) * 16u;
     *reinterpret_cast<uint4*>(sm.b[0] + off) = *reinterpret_cast<uint4*>(hi);
     *reinterpret_cast<uint4*>(sm.b[1] + off) = *reinterpret_cast<uint4*>(lo);
@@ -754,7 +741,7 @@ k_grad_tc(const float* images, const unsigned* labels, GradShares shares, const 
 #pragma unroll 1
     for (int m = 16; m > 0; m >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, m);
     const float bias = __shfl_sync(0xffffffffu, taps[4], kOffBc - 128 + warp - kBiasWarp);
-    if (lane == 0) sm.bc[warp - kBiasWarp] = (float)(-1.4426950408889634 * ((double)bias + (double)level * (1.0 / 255.0) * sum));
+    if (lane == 0) sm.bc[warp - kBiasWarp] = (float)(-1.4426950408889634 * ((double)bias + (double)level * ((1.0 + kByteExcess) / 255.0) * sum));
   }
   tc::fence_async_smem();      // the operands were written through the generic proxy
   tc::fence_before_sync();
