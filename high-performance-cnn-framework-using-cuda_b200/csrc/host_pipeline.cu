@@ -37,8 +37,7 @@ struct HostPipeline {
     long first = 0, count = 0;                 // the chunk whose results wait in h_res (count 0: none)
   } slot[kHpSlots];
   unsigned char* d_block = nullptr;            // all slots' images and results
-  size_t d_slot_bytes = 0;                     // what a slot has of it
-  int d_slots = 0;
+  size_t d_bytes = 0;
   PinnedHeap::Lease h_block;                   // all slots' results (for pageable ones), and behind them:
   int* h_status = nullptr;                     // the net's status word after each slot's last kernel
   cudaEvent_t piece[CopyPool::kSlots] = {};    // a ring slot's copy to the device is done
@@ -54,7 +53,8 @@ struct HostPipeline {
     if (order_event) cudaEventDestroy(order_event);
   }
 
-  // One allocation each for all slots: a cudaMalloc costs 0.4 ms whatever its size.
+  // One allocation each for all slots, which only grows: a cudaMalloc costs 0.4 ms whatever its size, and of two requests the larger one may have
+  // the shorter or the fewer slots (10,000 images two of 7,952, 11,000 three of 4,476).
   int reserve(int slots, long chunk, size_t image_bytes, bool pinned_results, bool staged) {
     if (!order_event) {
       for (Slot& s : slot)
@@ -62,13 +62,12 @@ struct HostPipeline {
       CNN_CUDA(cudaEventCreateWithFlags(&order_event, cudaEventDisableTiming));
     }
     const size_t img = ((size_t)chunk * image_bytes + 255) & ~(size_t)255, res = (sizeof(float) * (kOut + 1) * (size_t)chunk + 255) & ~(size_t)255;
-    if (d_slot_bytes < img + res || d_slots < slots) {
+    if (d_bytes < (img + res) * slots) {
       cudaFree(d_block);
       d_block = nullptr;
-      d_slots = 0;
+      d_bytes = 0;
       CNN_CUDA(cudaMalloc(&d_block, (img + res) * slots));
-      d_slot_bytes = img + res;
-      d_slots = slots;
+      d_bytes = (img + res) * slots;
     }
     const size_t pinned = (pinned_results ? res * slots : 0) + sizeof(int) * kHpSlots;
     if (h_block.bytes() < pinned && !h_block.take(pinned)) {
@@ -76,7 +75,7 @@ struct HostPipeline {
       return CNN_ERR_CUDA;
     }
     for (int i = 0; i < slots; ++i) {
-      slot[i].d_img = d_block + d_slot_bytes * i;
+      slot[i].d_img = d_block + (img + res) * i;
       slot[i].d_res = reinterpret_cast<float*>(slot[i].d_img + img);
       slot[i].h_res = pinned_results ? reinterpret_cast<float*>(h_block.get() + res * i) : nullptr;
     }

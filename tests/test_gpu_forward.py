@@ -598,3 +598,24 @@ def test_forward_host_last_chunk_is_shorter(cuda, pkg, params0, n):
         out, arg = np.full((n, 10), -1, np.float32), np.full(n, -1, np.int32)
         net.forward_u8_host(img, n, out, arg)
         assert np.array_equal(out, d_out.cpu().numpy()) and np.array_equal(arg, d_arg.cpu().numpy())
+
+
+def test_forward_host_memory_stays_whatever_the_order_of_sizes(cuda, pkg, params0):
+    """The chunks of a larger request can be the shorter ones (10,000 images 7,952 and the rest, 11,000 two of 4,476): a net that has seen all sizes
+    allocates nothing any more, whichever comes next, and the results are the bits of the device call at every one."""
+    sizes = [10000, 11000, 20000, 1500]
+    pix = pkg.synth.synth_pixels_u8(46, max(sizes))
+    d_pix = cuda.from_numpy(pix).cuda()
+    d_out = cuda.empty((max(sizes), 10), dtype=cuda.float32, device="cuda")
+    net = pkg.Net(0)
+    net.set_params(params0)
+    free = []
+    for turn in range(3):
+        for n in sizes if turn < 2 else sizes[::-1]:
+            out = np.empty((n, 10), np.float32)
+            net.forward_u8_host(pix[:n], n, out, None)
+            free.append((turn, cuda.cuda.mem_get_info()[0]))
+            net.forward_u8(d_pix, n, d_out, None)
+            cuda.cuda.synchronize()
+            assert np.array_equal(out, d_out[:n].cpu().numpy())
+    assert len({left for turn, left in free if turn > 0}) == 1
