@@ -262,11 +262,11 @@ static int forward_host_impl(cnn_net* net, const void* h_images, bool u8, long n
   const size_t image_bytes = u8 ? (size_t)kImg : sizeof(float) * kImg;
   const bool pageable = is_pageable(h_images);
   // Behind the last copy there is the last chunk's kernel, the way of its results back and, for pageable result buffers, a copy of them: a
-  // quarter of the request (halves: 10,000 uint8 images 256 instead of 249 us, 6,000 181 instead of 172; quarters all over: more hand-overs, 280).
+  // quarter of the request, at least 512 images and at most 2,048 (halves: 10,000 uint8 images 256 instead of 249 us, 6,000 181 instead of 172; quarters all over: more hand-overs, 280).
   // Pinned images, without the filling of the ring, leave a small request nothing to gain: halves below 4.5 MB (quarter, half: 5,000 uint8 images
   // 141, 131 us, 1,300 fp32 125, 119; 6,000 uint8 144, 151, 1,500 fp32 131, 136).
   const bool quarter = pageable || (size_t)n * image_bytes >= kHpMinQuarter;
-  long last = quarter ? n / 4 : (n / 2 < n - 2 * kHpMinChunk ? n / 2 : n - 2 * kHpMinChunk);
+  long last = quarter ? n / 4 : n / 2;
   if (quarter) last = last < kHpMinChunk ? kHpMinChunk : (last > kHpMaxChunk / 4 ? kHpMaxChunk / 4 : last);
   if (n <= 2 * kHpMinChunk) last = n;
   const long rest = n - last, parts = (rest + kHpMaxChunk - 1) / kHpMaxChunk;

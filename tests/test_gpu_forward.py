@@ -584,8 +584,9 @@ def test_forward_host_with_nets_that_come_and_go(cuda, pkg, params0):
 
 @pytest.mark.parametrize("n", [1026, 2047, 41000])
 def test_forward_host_last_chunk_is_shorter(cuda, pkg, params0, n):
-    """Equal chunks and a last one of a quarter of the request at most: two chunks of about 500, the least, and six chunks in four slots, whose
-    pageable results are handed over before a slot is used again; always the bits of the device call."""
+    """Equal chunks and a last one, for pageable images of a quarter of the request, 512 at least and 2,048 at most (514 and 512, 1,535 and 512), for
+    pinned ones of so few bytes of half of it (513 twice, 1,024 and 1,023); and six chunks in four slots, whose pageable results are handed over
+    before a slot is used again; always the bits of the device call."""
     pix = pkg.synth.synth_pixels_u8(48, n)
     net = pkg.Net(0)
     net.set_params(params0)
@@ -619,3 +620,25 @@ def test_forward_host_memory_stays_whatever_the_order_of_sizes(cuda, pkg, params
             cuda.cuda.synchronize()
             assert np.array_equal(out, d_out[:n].cpu().numpy())
     assert len({left for turn, left in free if turn > 0}) == 1
+
+
+def test_forward_host_small_pinned_requests_run_in_halves(cuda, pkg, params0):
+    """1,100 pinned images are two chunks of 550, for which a new net takes 3.5 MB of device memory (1,024 and 76: 6.5 MB).
+    Behind a request of 20, which creates the streams; median over nets, because small allocations share granules."""
+    n = 1100
+    images = cuda.from_numpy(pkg.synth.u8_to_float(pkg.synth.synth_pixels_u8(49, n))).pin_memory()
+    want = cuda.empty((n, 10), dtype=cuda.float32, device="cuda")
+    nets, taken = [], []
+    for _ in range(9):
+        nets.append(pkg.Net(0))
+        nets[-1].set_params(params0)
+        out = cuda.empty((n, 10)).pin_memory()
+        nets[-1].forward_host(images[:20], 20, out[:20], None)
+        cuda.cuda.synchronize()
+        before = cuda.cuda.mem_get_info()[0]
+        nets[-1].forward_host(images, n, out, None)
+        taken.append(before - cuda.cuda.mem_get_info()[0])
+        nets[-1].forward(images.cuda(), n, want, None)
+        cuda.cuda.synchronize()
+        assert cuda.equal(out, want.cpu())
+    assert sorted(taken)[len(taken) // 2] <= 4 << 20
