@@ -828,6 +828,7 @@ static int launch_grad(const float* d_params, float* rows, int* status, int fast
   cudaError_t le = cudaSuccess;
   // A block that needs little (one team, no registers for a loop) is given half an SM's shared memory and more, so that no two share an SM: batches of
   // 148 images 6.7 us a step, 8.6 without (7.0 with a loop's registers, which kept others away too).
+  static_assert(sizeof(GrSmem<1>) <= 120 * 1024, "");
 #define CNN_GRAD_SMEM(TEAMS) (TEAMS == 1 ? 120 * 1024 : sizeof(GrSmem<TEAMS>))
 #define CNN_LAUNCH_GRAD(FL, TEAMS, ONCE)                                                                      \
   do {                                                                                                       \

@@ -298,6 +298,7 @@ k_train_persample_cluster8(const float* __restrict__ images, const unsigned* __r
       // ---- output layer on lanes 0..9 of every warp ------------------------------------------------
       float delta = 0.f;
       if (lane < kOut) {
+        static_assert(kC8Compute == 3 && kClCtas == 6, "the sums below are written out");
         float zc[kClCtas];
 #pragma unroll
         for (int c = 0; c < kClCtas; ++c) {
