@@ -360,7 +360,7 @@ def run_ours(args):
     net.set_params(params)
     net.set_fast_sigmoid(args.fast_sigmoid)
     net.set_option("forward_path", args.forward_path)
-    # -1 = the library's default: the three-pass tensor-core kernel from 6,144 images per call on
+    # -1 = the library's default: the tensor-core kernel in two or three passes from 6,144 images per call on
     eff_path = args.forward_path if args.forward_path >= 0 else (1 if (args.fast_sigmoid and BATCH >= 6144) else 0)
     stream = torch.cuda.current_stream()
     peak, peak_kind = measured_peak_gbs()
@@ -429,7 +429,7 @@ def run_ours(args):
     # ---- the same launch through the other forward kernels --------------------------------------------
     def forward_paths_leg():
         names = {0: "exact fp32 on the CUDA cores (k_forward_tiles)",
-                 1: "conv on tcgen05, three passes of fp16 parts (k_forward_tc path 1), 1e-5 parity",
+                 1: "conv on tcgen05, two passes of fp16 parts, three where pixels are no bytes / 255 (k_forward_tc path 1), 1e-5 parity",
                  2: "conv on tcgen05, one fp16 pass + tanh.approx sigmoid (k_forward_tc path 2), reduced precision"}
         res = {}
         for path in (0, 1, 2):
@@ -844,7 +844,7 @@ def main():
     ap.add_argument("--fast-sigmoid", type=int, default=1)
     ap.add_argument("--forward-path", type=int, default=-1,
                     help="kernel of the headline: -1 the library's default (1 at this batch size), 0 exact fp32 SIMT, "
-                         "1 tcgen05 three passes of fp16 parts (1e-5 parity), 2 tcgen05 one pass + tanh (reduced precision)")
+                         "1 tcgen05 two or three passes of fp16 parts (1e-5 parity), 2 tcgen05 one pass + tanh (reduced precision)")
     ap.add_argument("--only-train", type=int, default=0,
                     help="run only the training legs of the reference net (for ncu launch lists)")
     ap.add_argument("--only-wide", type=int, default=0,

@@ -2,7 +2,7 @@
 // 94 % of the forward MACs) on the 5th-generation tensor cores (tcgen05, accumulators in tensor
 // memory), and everything after it -- bias, sigmoid, shared 4x4 subsample, sigmoid, FC 216->10,
 // sigmoid, argmax -- done by the epilogue warps straight out of tensor memory.  Selected with the
-// option "forward_path" = 1 (three passes, fp32-level accuracy; the default for large batches, fp32 images
+// option "forward_path" = 1 (two passes, three where pixels leave a remainder, fp32-level accuracy; the default for large batches, fp32 images
 // or uint8 pixels) or 2 (one pass and a tanh.approx sigmoid: an explicitly reduced-precision inference mode).
 //
 // The convolution as a GEMM WITHOUT an im2col copy.  For kernel row i the conv is a product of image rows
@@ -31,6 +31,8 @@
 // arithmetic exactly, its high part all of it and its remainder zero.  A tile of such images takes two passes instead
 // of three; the third would add zeros, so what an image gives does not depend on its neighbours.  (65,536 images: 138 -> 115 us; images
 // of other numbers 134 -> 127 us, by the loader alone.)  Such a pixel kept as a byte needs no table: fp16(byte) is two instructions per pair.
+// Another pixel's product with 255 is rounded, which does not show: outputs of noise and of normalised noise, eight nets as drawn, are 7.0e-8 and 7.1e-8
+// of their norm from fp64 with the power of two alone, with 255, and with the remainder of the exact product (146 us).
 // An image with a scaled pixel of 65,520 or more (a pixel of 1,000 to 2,000 where w = 1: its pre-activations are no longer
 // of order one) is noticed by the loader, and a finisher warp computes it in plain fp32 instead (slow, 0.1 ms per image; no
 // image data is expected there).  uint8 pixels reach that limit only where w is above 1,000: the finishers look for themselves
@@ -56,7 +58,7 @@
 // Measured on a B200 (three passes whatever the pixels, a table for uint8 before, now): 65,536 fp32 images 138 -> 114 us, 30,011 uint8 images
 // 65 -> 53 us, path 2 on 65,536 images 98 -> 91 us (loader without bank conflicts).  What bounds it now, per tile of 5.33 images
 // (2,400 cycles): the shared-memory data pipe (20 MMAs fetch 130 KB of operands, 1,040 cycles, the other warps and the copies take 900),
-// and next the special-function unit (1,600 cycles) and instruction issue (1,400); path 2: the special-function unit, 75 % busy.
+// and next the special-function unit (1,600 cycles) and instruction issue (1,400); path 2: the same pipe, 88 % busy, then the special-function unit, 64 %.
 #include <type_traits>
 
 #include "banded_conv.cuh"
@@ -196,7 +198,7 @@ __device__ __noinline__ float finish_plain_u8(const unsigned char* pixels, const
   return z;
 }
 
-// PATH 1: three passes, sigmoid flavour SIG (0 or 1).  PATH 2: one pass, tanh sigmoid.  U8: `images` points at
+// PATH 1: two or three passes, sigmoid flavour SIG (0 or 1).  PATH 2: one pass, tanh sigmoid.  U8: `images` points at
 // uint8 pixels and the kernel applies the reference's ingest, float(pixel / 255.0) (mnist.h:145, main.cu:57-65).
 template <int PATH, int SIG, bool U8>
 __global__ void __launch_bounds__(kTfThreads, 1)

@@ -468,7 +468,7 @@ static int launch_variant(cnn_net* net, int path, const void* d_images, long n, 
 }
 
 // The kernel a call over n_total images uses: 0 = k_forward_tiles, kForwardOne = k_forward_one, 1 / 2 = forward_tc.cu.
-// Default (-1): the three-pass tensor-core kernel for batches of kTcMinBatch images and more, this file's below.  The line is the one
+// Default (-1): the tensor-core kernel in two or three passes for batches of kTcMinBatch images and more, this file's below.  The line is the one
 // that the interface promises (the two sides differ in their last bits); it is not where the kernels meet.  That is at one round of
 // tiles, 14 images per SM: 2,072 images 10.5 us here, 10.3 on the tensor cores; 2,073 images 11.9 and 10.3; 4,144: 18.6 and 13.8; 6,143: 26.5 and
 // 16.7 (uint8: 10.8 / 9.5, 14.8 / 9.5, 20.8 / 12.7, 29.7 / 15.2).

@@ -16,7 +16,7 @@
 //                 epilogue's lanes (rows) have them, the slab is the N-contiguous B operand: a row is 16 bytes, so it may start at any.
 //
 // Accuracy.  Pixels that are whole numbers / 255 (image files' bytes) are exact in fp16 (forward_tc.cu).  A tile with any other pixel goes through as
-// an empty one, and its images are left to k_grad_partials (fused_train.cu); so is the whole share of a CTA whose sample of pixels has others in several
+// an empty one, and its images are left to k_grad_left (fused_train.cu); so is the whole share of a CTA whose sample of pixels has others in several
 // places, what comes behind too many such tiles, and everything where a parameter is not finite or far out of range.  The tensor core truncates its additions, which over a tile's 48 would cost a gradient 1e-6.  Here they are exact: deltas are
 // scaled by a power of two so that the tile's bound on them (max |ds| * max |Ws| / 4) lies in [1024, 2048), and cut into a whole
 // number, at most 11 bits, and the rest, which in fp16 is good to 2^-24 of the bound.  Products of whole numbers with bytes have 19 bits.  A D adds 720 of
@@ -40,7 +40,7 @@
 //               deltas.  Stage 2: conv deltas, subsample-filter and bias gradients, delta operand (its whole parts negated: one instruction less);
 //   warps 0-1   FC gradient in registers (a thread owns three or four of the 216 inputs), from what the groups leave in shared memory.
 //
-// Measured on a B200, 60,000 images with the kernels around it: 643 us (k_grad_partials) -> 281 us.  What bounds it, per tile of five images (6,200 cycles):
+// Measured on a B200, 60,000 images with the kernels around it: 643 us (k_grad_partials) -> 282 us.  What bounds it, per tile of five images (6,200 cycles):
 // the shared-memory data pipe (operands of the 78 MMAs 2,590 cycles, other warps 3,020: delta operands 580, FC layer
 // 700, loader 350, conflicts with the tensor core 570); instruction issue about 60 %, the special-function unit 37 %.  2,048 images are 24.0 us, of which a launch's
 // set-up is 3.2 us.

@@ -11,7 +11,7 @@ struct cnn_net {
   int device = 0;
   unsigned seed = 0;               // what cnn_net_create drew the initial parameters from (kept for checkpoints)
   int ps_kernel = 1;               // per-sample SGD: 1 = six-CTA cluster kernel (default), 0 = single persistent block
-  int forward_path = -1;           // batched forward: 0 = exact fp32 SIMT kernel, 1 = tensor cores in three fp16 passes
+  int forward_path = -1;           // batched forward: 0 = exact fp32 SIMT kernel, 1 = tensor cores in two or three fp16 passes
                                    // (fp32-level accuracy), 2 = tensor cores, one fp16 pass + tanh sigmoid,
                                    // -1 (default) = 1 for batches of kTcMinBatch images or more, else 0
   int grad_path = -1;              // gradient of a batch: 0 = CUDA cores, 1 = tensor cores, -1 (default) = by batch size

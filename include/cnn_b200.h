@@ -182,11 +182,12 @@ int cnn_synth_images(unsigned long long seed, long first_index, long n, float* d
  *                      images of one rank): 0 = fp32 on the CUDA cores, 1 = the
  *                      convolution and its weight gradient on the tensor cores at fp32-level accuracy (images whose pixels are
  *                      float(byte / 255.0), as a division gives them; others, a byte times 1 / 255 among them, are noticed and computed
- *                      on the CUDA cores, 4 to 9 us later than under 0), -1 (default) = 1 from 2,048 images on, else 0;
+ *                      on the CUDA cores, 4 to 10 us later than under 0), -1 (default) = 1 from 2,048 images on, else 0;
  *                      fast_sigmoid = 0 stays on the CUDA cores.
  *   "forward_path"     kernel behind cnn_forward_batched and cnn_forward_batched_u8: 0 = exact fp32 on the CUDA
  *                      cores; 1 = the convolution on the tensor cores (tcgen05), both operands in two fp16 parts and
- *                      three passes, fp32-level accuracy, same 1e-5 parity bar; -1 (default) = 1 for batches of 6,144
+ *                      two passes, a third for images whose pixels are not float(byte / 255.0); fp32-level accuracy, same
+ *                      1e-5 parity bar; -1 (default) = 1 for batches of 6,144
  *                      images or more and 0 below, or always 0 when the
  *                      reference's sigmoid expression is selected; 2 = (fp32 images) one fp16 pass and a tanh.approx
  *                      sigmoid: about 1e-4 on the outputs, argmax equal wherever the top-two margin is
