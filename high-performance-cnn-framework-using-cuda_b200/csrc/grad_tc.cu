@@ -76,6 +76,8 @@ constexpr int kGtFcThreads = 64, kGtFcRounds = 4;            // 216 = 3 * 64 + 2
 constexpr int kGtPlaces = 2 * kGtThreads / 32, kGtPlacesOther = 8;
 constexpr int kGtWfStride = 234;              // five rows of weights, 10 (mod 32) words apart, by six parts of nine inputs: thirty banks
 constexpr float kGtUnscale = 1.0f / 8192.0f;                 // of the convolution's accumulators
+constexpr int kGtMaxExp = 100;                               // deltas are scaled by 2^100 at most, where they are zero or nearly so
+constexpr float kGtMost = 67108864.f;                        // largest parameter, 2^26: a tap of the subsample filter times that scale is finite
 constexpr int kGtConvWarp = 2, kGtGradWarp = 3, kGtLoadWarp0 = 4, kGtEpiWarp0 = 8;
 
 struct GtSmem {
@@ -492,7 +494,7 @@ __device__ __noinline__ void run_group(GtSmem& sm, const unsigned* labels, int i
     // |conv delta * 576| <= max |ds| * max |Ws| / 4: scaled by 2^e into [1024, 2048) at most
     const unsigned ds_bits = max(max(sm.ds_max[set][0], sm.ds_max[set][1]), max(sm.ds_max[set][2], sm.ds_max[set][3]));
     const float bound = __uint_as_float(ds_bits) * wsmax * 0.25f;
-    const int e = min(max(10 - ((int)(__float_as_uint(bound) >> 23) - 127), -100), 100);
+    const int e = min(max(10 - ((int)(__float_as_uint(bound) >> 23) - 127), -kGtMaxExp), kGtMaxExp);
     const float scale = __int_as_float((127 + e) << 23), unscale = __int_as_float((127 - e) << 23);
     if (quarter == 0 && lane == 0) *const_cast<volatile float*>(&sm.tile_unscale[k % kGtSlabs]) = unscale;
     f32x2 ws2[4];
@@ -692,7 +694,7 @@ k_grad_tc(const float* images, const unsigned* labels, GradShares shares, const 
 #pragma unroll
   for (int j = 0; j < 5; ++j) wmax = fmaxf(wmax, lane + 32 * j < kOffBc ? fabsf(taps[j]) : 0.f);
 #pragma unroll
-  for (int j = 0; j < kAll; ++j) sane = sane && fabsf(share[j]) <= 1e9f;
+  for (int j = 0; j < kAll; ++j) sane = sane && fabsf(share[j]) <= kGtMost;
   wmax = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(wmax)));      // (magnitudes compare as their bits)
   wsmax = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(wsmax)));
   // With 2^E <= max |kPre * w| < 2^(E+1) weights are scaled by 2^(16-E) / 255 and pixels by 255 * 2^(E-3): the accumulator carries 2^13.

@@ -549,11 +549,13 @@ def test_tensor_core_gradient_is_as_close_to_fp64(cuda, pkg, what, scale):
 
 
 @pytest.mark.parametrize("what", ["conv weights x 1e-7", "conv weights x 5e-6", "conv weights x 1e-3", "conv weights x 30", "conv weights x 100",
-                                  "conv weights x 500", "conv weights x 1e5", "infinite bias", "not a number", "large rest", "no subsample filter"])
+                                  "conv weights x 500", "conv weights x 1e5", "infinite bias", "not a number", "large rest", "no subsample filter",
+                                  "subsample filter of 6e7", "subsample filter of 5e8", "subsample filter of 5e9"])
 def test_tensor_core_gradient_parameter_range(cuda, pkg, params0, what):
     """Conv weights below 2^-21 (x 1e-7) or from 2^11 on (x 1e5), and parameters that are not finite, go to the CUDA-core kernel; everything between
     through the scales that follow the largest weight and the tile's deltas.  Yardstick: the CUDA-core path.  With large weights a pre-activation
-    of 25 terms up to 0.5 * factor is only known to 25 * 0.5 * factor * 2^-24 in fp32."""
+    of 25 terms up to 0.5 * factor is only known to 25 * 0.5 * factor * 2^-24 in fp32.  A subsample filter that saturates its sigmoids leaves deltas of
+    zero, whose scale is the largest there is and must not take the filter's taps out of range (they go to the CUDA cores above 2^26)."""
     images, labels = pkg.synth.synth_images(63, 2100)
     params, factor = params0.copy(), 1.0
     if "conv weights" in what:
@@ -566,8 +568,9 @@ def test_tensor_core_gradient_parameter_range(cuda, pkg, params0, what):
     elif what == "large rest":
         params[156:] *= np.float32(30)
     else:
-        params[156:172] = 0
+        params[156:172] = float(what.split()[-1]) if " of " in what else 0
     out = both_paths(cuda, pkg, params, images, labels)
+    assert np.isfinite(out[0]).all() or what in ("infinite bias", "not a number")
     assert np.array_equal(np.isnan(out[0]), np.isnan(out[1]))
     if not np.isnan(out[0]).any():
         bar = max(1e-5, 25 * 0.5 * factor * 2.0**-24) if factor < 1e5 else 1e-5
