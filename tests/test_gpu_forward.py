@@ -364,12 +364,12 @@ def test_tensor_core_forward_operand_range(cuda, pkg, params0, what, n):
     images = pkg.synth.u8_to_float(pix)
     params = params0.copy()
     spots = [0, n // 2, n - 1]
-    limit = 65520.0 / 2.0 ** (5 + np.floor(np.log2(np.abs(params[:150]).max() * 1.442695)))
+    limit = 65520.0 / (255 * 2.0 ** (np.floor(np.log2(np.abs(params[:150]).max() * 1.442695)) - 3))
     if what == "largest":
         images[spots, 5, 7] = limit * (1 - 1e-4)
     elif what == "out of range":
-        images[spots, 27, 27] = limit
-        images[spots, 0, 0] = -3e6
+        images[spots, 27, 27] = limit * (1 + 1e-6)
+        images[spots[0], 0, 0] = -3e6
     elif what == "not a number":
         images[spots, 11, 12] = np.nan
     elif what.endswith("weights"):
